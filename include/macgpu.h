@@ -162,11 +162,15 @@ typedef struct {
      no_normalize != 0 leaves the positions unwrapped. */
   double box_rmin;
   int no_normalize;
-  /* Ewald k-space engine of the FP32 path: 0 = each pass on the tensor
-     cores when its shared-memory tiles fit (else on the FP32 cores); 1 =
-     both passes on the FP32 cores; 2 = pass 2 on the tensor cores, pass 1 on
-     the FP32 cores; 3 = both passes on the tensor cores.  The tensor-core
-     passes run TF32 split into three products with FP32 accuracy. */
+  /* Ewald k-space engine of the FP32 path.  0 = automatic: the force
+     evaluations sum over the same k set by non-uniform Fourier transforms
+     (mg_nufft.cu) where cells are re-binned at every evaluation (skin <= 0)
+     and the k set fits (|n| up to about 40 per edge); otherwise, and in
+     mg_ewald, each pass directly, on the tensor cores when its shared-memory
+     tiles fit, else on the FP32 cores.  1 = both passes directly on the FP32
+     cores; 2 = pass 2 on the tensor cores, pass 1 on the FP32 cores; 3 = both
+     passes on the tensor cores.  The tensor-core passes run TF32 split into
+     three products with FP32 accuracy. */
   int kspace_engine;
   /* Nose-Hoover predictor length k (cook's No.pred = option -p % 10,
      sim/main.c:404-405), 1..8; <=0 selects 2 */
@@ -452,10 +456,10 @@ mg_ctx *mg_batch_box(mg_batch *b, int i);
 /* kernels launched by the last batch call (graph nodes counted per step) */
 int mg_batch_last_launches(const mg_batch *b);
 /* en: NULL or [nbox] energies of the last step.  When every box runs the
-   FP32 path with both Ewald passes on the FP32 cores or both on the tensor
-   cores (kspace_engine 1 or 0; under 0 a box whose tiles do not fit runs on
-   the FP32 cores), the cell pair kernel with 4 warps (pair_variant 0),
-   cells re-binned every step and no Drude charges, dependants, thermostat,
+   FP32 path with its Ewald sums as non-uniform transforms or both passes on
+   the FP32 cores or both on the tensor cores (kspace_engine 0, 1 or 3; under
+   0 a box whose k set does not fit runs its passes directly), the cell pair
+   kernel with 4 warps (pair_variant 0), cells re-binned every step and no Drude charges, dependants, thermostat,
    drmax, drift removal or dipole term, a step is one launch per kernel over
    all boxes (blockIdx.y = box, each box with its single-launch arguments,
    so its results are those of the box run alone); otherwise one graph node

@@ -2,6 +2,7 @@
 // per-call orchestration of the kernels in mg_kernels.cu.
 #include "../../include/macgpu.h"
 #include "mg_internal.h"
+#include "mg_nufft.h"
 
 #include <algorithm>
 #include <cmath>
@@ -103,6 +104,15 @@ struct mg_ctx {
   bool sk_tc = false;
   float* d_zb = nullptr;
   int sk_nch = 1, sk_gpc = 1;
+  // k-space of the force evaluations as non-uniform transforms
+  // (kspace_engine 0 with cells re-binned): the arguments, the launch grids,
+  // one block for the grids and tables
+  bool nf = false;
+  NfBox h_nf{};
+  NfGrid nf_grid{};
+  NfBox* d_nf = nullptr;
+  float* d_nfmem = nullptr;
+  int* d_far = nullptr;
   // SHAKE
   int* d_mol_first = nullptr;
   int* d_mol_cfirst = nullptr;
@@ -288,6 +298,85 @@ cudaError_t upload(T** p, const T* h, size_t n) {
   cudaError_t e = dalloc(p, n);
   if (e != cudaSuccess || n == 0) return e;
   return cudaMemcpy(*p, h, sizeof(T) * n, cudaMemcpyHostToDevice);
+}
+
+// the arguments, tables and grids of the non-uniform transforms
+int setup_nf(mg_ctx* ctx, const int K[3], const std::vector<int4>& kvec,
+             const std::vector<double>& ekk, const std::vector<double>& kind_q,
+             const std::vector<double>& kind_qp) {
+  NfBox& b = ctx->h_nf;
+  b.ns = ctx->ns;
+  b.nsub = ctx->polar ? 2 : 1;
+  const int nc[3] = {ctx->ncx, ctx->ncy, ctx->ncz};
+  for (int d = 0; d < 3; d++) {
+    b.K[d] = K[d];
+    b.M[d] = nf_grid(K[d]);
+    b.nc[d] = nc[d];
+    b.marg[d] = ctx->polar ? (int)std::ceil(NF_MARGIN * b.M[d] / ctx->L[d]) : 0;
+    const double beta = nf_beta(b.M[d], K[d]);
+    b.nb[d] = (float)(-beta * 1.4426950408889634);
+    b.db[d] = (float)(-beta * 4 / (NF_W * NF_W));
+    b.fac[d] = (float)(b.M[d] / ctx->L[d]);
+    b.fix[d] = (float)(4294967296.0 / ctx->L[d]);
+    b.iL[d] = 1 / ctx->L[d];
+    b.cpg[d] = (float)nc[d] / b.M[d];
+    b.step[d] = ~0ull / b.M[d];
+    b.ext[d] = (unsigned)(((unsigned long long)(NF_TILE + NF_W - 1) << 32) / b.M[d]) + 2;
+  }
+  b.dense = nf_dense(ctx->nq, b.M);
+  b.pi2_over_a2 = 9.869604401089358 / (ctx->alpha * ctx->alpha);
+  for (int k = 0; k < ctx->nkind; k++) {
+    b.q[k] = (float)kind_q[k];
+    b.qp[k] = (float)kind_qp[k];
+  }
+  std::vector<float2> fwd[3], inv[3];
+  std::vector<float> wk;
+  nf_tables(K, b.M, kvec, ekk, fwd, inv, &wk);
+  // one allocation: grids, then tables, each on a 256-byte boundary
+  const size_t G = (size_t)b.M[0] * b.M[1] * b.M[2], A = (size_t)(K[0] + 1) * b.M[1] * b.M[2];
+  size_t n = 0;
+  auto take = [&](size_t floats) {
+    const size_t o = n;
+    n += (floats + 63) / 64 * 64;
+    return o;
+  };
+  const size_t oG = take(G), oA = take(2 * A), oW = take(wk.size());
+  size_t of[3], oi[3];
+  for (int d = 0; d < 3; d++) {
+    of[d] = take(2 * fwd[d].size());
+    oi[d] = take(2 * inv[d].size());
+  }
+  CK(dalloc(&ctx->d_nfmem, n));
+  std::vector<float> h(n - oW, 0.f);
+  auto put = [&](size_t o, const void* src, size_t floats) {
+    std::memcpy(h.data() + (o - oW), src, floats * sizeof(float));
+  };
+  put(oW, wk.data(), wk.size());
+  for (int d = 0; d < 3; d++) {
+    put(of[d], fwd[d].data(), 2 * fwd[d].size());
+    put(oi[d], inv[d].data(), 2 * inv[d].size());
+  }
+  CK(cudaMemcpy(ctx->d_nfmem + oW, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  float* m = ctx->d_nfmem;
+  b.G = m + oG;
+  b.A = (float2*)(m + oA);
+  b.wk = m + oW;
+  for (int d = 0; d < 3; d++) {
+    b.fwd[d] = (const float2*)(m + of[d]);
+    b.inv[d] = (const float2*)(m + oi[d]);
+  }
+  CK(dalloc(&ctx->d_far, 1));
+  CK(cudaMemset(ctx->d_far, 0, sizeof(int)));
+  b.pj = ctx->d_pj;
+  b.pdj = ctx->d_pdj;
+  b.order = ctx->d_order;
+  b.cell_start = ctx->d_cell_start;
+  b.far = ctx->d_far;
+  b.ek_part = ctx->d_ekpart;
+  b.f = ctx->d_f;
+  nf_launch(b, &ctx->nf_grid);
+  CK(upload(&ctx->d_nf, &b, 1));
+  return MG_OK;
 }
 
 int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
@@ -630,6 +719,11 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   ctx->nchunk = std::max(1, std::min(std::max(1, ctx->nq / 512),
                                      (p1ctas + ctx->np1job - 1) / ctx->np1job));
   ctx->nkblocks = (nk + 255) / 256;
+  const int nfK[3] = {ctx->Kx, ctx->Ky, ctx->Kz};
+  // non-uniform transforms (mg_nufft.cu) need the cells of the present
+  // positions (no kept lists) and serve the automatic engine
+  ctx->nf = ctx->precision == MG_MIXED && p->kspace_engine == 0 && !ctx->use_list && ctx->nq > 0 &&
+            nf_fits(nfK);
 
   // ---- constraints
   ctx->nc = t->nc;
@@ -766,7 +860,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   CK(upload(&ctx->d_p1job, p1job.data(), p1job.size()));
   CK(upload(&ctx->d_ekk, ekk.data(), ekk.size()));
   CK(dalloc(&ctx->d_S, 2 * (size_t)nk));
-  CK(dalloc(&ctx->d_ekpart, (size_t)ctx->nkblocks * 7));
+  CK(dalloc(&ctx->d_ekpart, (size_t)std::max(ctx->nkblocks, ctx->nf ? NF_CS * (ctx->Kx + 1) : 0) * 7));
   if (ctx->precision == MG_MIXED) {
     CK(dalloc(&ctx->d_pj, ns));
     CK(upload(&ctx->d_ptabf, pf.data(), pf.size()));
@@ -787,6 +881,10 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     CK(dalloc(&ctx->d_fk, 3 * (size_t)ns * (ctx->polar ? 2 : 1)));
     CK(dalloc((float2**)&ctx->d_part, (size_t)std::max(ctx->nchunk, ctx->sk_nch) * nk));
     CK(dalloc(&ctx->d_Wf, nk));
+    if (ctx->nf) {
+      int rc = setup_nf(ctx, nfK, kvec, ekk, kind_q, kind_qp);
+      if (rc) return rc;
+    }
   } else {
     CK(dalloc(&ctx->d_pd, ns));
     CK(upload(&ctx->d_ptabd, pd.data(), pd.size()));
@@ -1169,7 +1267,8 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
   ctx->last_r = r_dev;
   // fork point of the concurrent k-space chain (FP32 path): everything
   // queued before, nothing of this evaluation's r-space work
-  if (ctx->precision == MG_MIXED && ctx->overlap && ctx->nq > 0)
+  // (the non-uniform transforms fork after the cell list, which they read)
+  if (ctx->precision == MG_MIXED && ctx->overlap && ctx->nq > 0 && !ctx->nf)
     CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
   const bool rebuild = !ctx->use_list || ctx->need_build || ctx->since_build >= ctx->nl_every;
   const double iL[3] = {1.0 / ctx->L[0], 1.0 / ctx->L[1], 1.0 / ctx->L[2]};
@@ -1190,7 +1289,25 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
     // its forces go to d_fk and are added at the join
     const bool fork = ctx->overlap && ctx->nq > 0;
     const size_t nf = 3 * (size_t)ns * (ctx->polar ? 2 : 1);
-    if (fork) {
+    if (ctx->nf) {
+      // the transforms up to the potential grid, beside the r-space chain or
+      // before it; the forces are interpolated from it after the r-space
+      // forces, so that both orders add the same terms in the same order
+      if (ctx->polar) {
+        PROF("gather", k_gather_drude(L, ns, r_dev, ctx->d_order, ctx->d_pdj, nullptr));
+        PROF("gather", k_nf_far(L, ns, ctx->d_pdj, NF_MARGIN, ctx->d_far));
+      }
+      cudaStream_t ks = fork ? ctx->kstream : ctx->stream;
+      Launch LK{ks, &ctx->launches};
+      if (fork) {
+        CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
+        CK(cudaStreamWaitEvent(ks, ctx->ev_fork, 0));
+      }
+      PROFS("ewald_sk", ks, k_nf_forward(LK, ctx->d_nf, 1, ctx->nf_grid));
+      PROFS("ewald_sk", ks, k_nf_modes(LK, ctx->d_nf, 1, ctx->nf_grid, measure));
+      PROFS("ewald_kforce", ks, k_nf_back(LK, ctx->d_nf, 1, ctx->nf_grid));
+      if (fork) CK(cudaEventRecord(ctx->ev_join, ks));
+    } else if (fork) {
       cudaStream_t ks = ctx->kstream;
       Launch LK{ks, &ctx->launches};
       KArgs kk = ka;
@@ -1206,7 +1323,8 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
     if (!rebuild)
       PROF("gather", k_gather_mixed(L, ns, r_dev, ctx->d_order, ctx->d_kind, ctx->d_mol, iL,
                                     ctx->d_pj));
-    if (ctx->polar) PROF("gather", k_gather_drude(L, ns, r_dev, ctx->d_order, ctx->d_pdj, nullptr));
+    if (ctx->polar && !ctx->nf)
+      PROF("gather", k_gather_drude(L, ns, r_dev, ctx->d_order, ctx->d_pdj, nullptr));
     if (ctx->use_list) {
       if (rebuild) {
         int rc = build_lists(ctx, r_dev);
@@ -1225,7 +1343,10 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
       PROF("exclusions", k_excl_mixed(L, xa, measure, ctx->polar));
       nerows = ctx->nprows + ctx->nxblocks;
     }
-    if (fork) {
+    if (ctx->nf) {
+      if (fork) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+      PROF("ewald_kforce", k_nf_interp(L, ctx->d_nf, 1, ctx->nf_grid, f_dev));
+    } else if (fork) {
       CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
       PROF("ewald_kforce", k_add_forces(L, nf, ctx->d_fk, f_dev));
     } else if (ctx->nq > 0) {
@@ -1265,7 +1386,9 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
   ctx->have_cells = true;
   if (measure) {
     PROF("reduce", k_reduce_sum(L, ctx->d_epart, nerows, 10, ctx->d_sums));
-    if (ctx->nq > 0) PROF("reduce", k_reduce_sum(L, ctx->d_ekpart, ctx->nkblocks, 7, ctx->d_sums + 10));
+    if (ctx->nq > 0)
+      PROF("reduce", k_reduce_sum(L, ctx->d_ekpart, ctx->nf ? NF_CS * (ctx->Kx + 1) : ctx->nkblocks, 7,
+                                  ctx->d_sums + 10));
   }
   return MG_OK;
 }
@@ -1649,7 +1772,7 @@ int mg_destroy(mg_ctx* ctx) {
   void* bufs[] = {ctx->d_rs, ctx->d_fs, ctx->d_r,      ctx->d_f,       ctx->d_r1,    ctx->d_p,      ctx->d_kind,
                   ctx->d_mol,    ctx->d_key,     ctx->d_pfix,   ctx->d_idx,   ctx->d_key_s,  ctx->d_order,
                   ctx->d_cell_start, ctx->d_ccount, ctx->d_ccursor, ctx->d_spans, ctx->d_gstart,
-                  ctx->d_hspans, ctx->d_facc, ctx->d_tcb,
+                  ctx->d_hspans, ctx->d_facc, ctx->d_tcb, ctx->d_nf, ctx->d_nfmem, ctx->d_far,
                   ctx->d_gcell, ctx->d_pj, ctx->d_pd,  ctx->d_stencil,
                   ctx->d_ptabf,  ctx->d_ptabd,   ctx->d_erd,   ctx->d_eru,    ctx->d_ert,
                   ctx->d_epart,  ctx->d_qsite,   ctx->d_qval,  ctx->d_task,   ctx->d_col,
@@ -2518,6 +2641,9 @@ struct mg_batch {
   int fused_ok = -1;
   BoxStep* d_steps = nullptr;
   TcBox* d_tc = nullptr;
+  NfBox* d_nf = nullptr;   // the boxes whose k-space runs as non-uniform transforms
+  int n_nf = 0;
+  NfGrid nf_grid{};
   BatchGrid grid{};
   // the boxes' status words, gathered into one array after unmeasured steps
   int** d_statp = nullptr;
@@ -2633,6 +2759,7 @@ int mg_batch_destroy(mg_batch* b) {
   if (b->gf_meas) cudaGraphExecDestroy(b->gf_meas);
   if (b->d_steps) cudaFree(b->d_steps);
   if (b->d_tc) cudaFree(b->d_tc);
+  if (b->d_nf) cudaFree(b->d_nf);
   if (b->d_statp) cudaFree(b->d_statp);
   if (b->d_stat) cudaFree(b->d_stat);
   if (b->h_stat) cudaFreeHost(b->h_stat);
@@ -2663,7 +2790,7 @@ namespace {
 // cores, no dipole term
 bool fusable(const mg_ctx* c) {
   return c->precision == MG_MIXED && !c->polar && !c->use_list && !c->allpairs &&
-         c->pair_variant == 0 && c->kspace_tc == c->sk_tc && c->thermostat == 0 &&
+         c->pair_variant == 0 && (c->nf || c->kspace_tc == c->sk_tc) && c->thermostat == 0 &&
          c->ndep == 0 && !c->dipole && c->drmax == 0 && !c->drift_step && c->nq > 0 &&
          !c->prof_on;
 }
@@ -2674,6 +2801,8 @@ int build_fused(mg_batch* b) {
   const int nbox = (int)b->box.size();
   std::vector<BoxStep> h(nbox);
   std::vector<TcBox> tc(nbox);
+  std::vector<NfBox> nf;
+  b->nf_grid = NfGrid{};
   BatchGrid& g = b->grid;
   g = BatchGrid{};
   for (int i = 0; i < nbox; i++) {
@@ -2745,7 +2874,15 @@ int build_fused(mg_batch* b) {
     e.g_kf = kf_mixed_blocks(c->nq);
     e.g_shake = (c->nmol + 127) / 128;
     TcBox& t = tc[i];
-    if (c->kspace_tc) {
+    if (c->nf) {
+      // non-uniform transforms, with the arguments of the box's single
+      // launches
+      nf.push_back(c->h_nf);
+      nf_launch(c->h_nf, &b->nf_grid);
+      e.rrows[1] = NF_CS * (c->Kx + 1);
+      e.g_charge = e.g_phase = e.g_p1x = e.g_p1y = e.g_kf = e.g_skr = 0;
+      t = TcBox{};
+    } else if (c->kspace_tc) {
       // the tensor-core passes, with the arguments of the box's single
       // launches (tc_args); its pass 1 reduces sk_nch chunks
       t = tc_args(c, e.ka, c->d_r);
@@ -2775,8 +2912,14 @@ int build_fused(mg_batch* b) {
     g.kf = std::max(g.kf, e.g_kf);
     g.shake = std::max(g.shake, e.g_shake);
     g.pair_smem = std::max(g.pair_smem, sizeof(PairFS) * (size_t)c->nkind * c->nkind);
-    if (!c->kspace_tc) g.kf_smem = std::max(g.kf_smem, kf_mixed_smem(e.ka));
+    if (!c->nf && !c->kspace_tc) g.kf_smem = std::max(g.kf_smem, kf_mixed_smem(e.ka));
   }
+  b->n_nf = (int)nf.size();
+  if (b->n_nf > 0 &&
+      (cudaMalloc(&b->d_nf, sizeof(NfBox) * nf.size()) != cudaSuccess ||
+       cudaMemcpy(b->d_nf, nf.data(), sizeof(NfBox) * nf.size(), cudaMemcpyHostToDevice) !=
+           cudaSuccess))
+    return bfail(b, MG_ERR_CUDA, "batch: uploading the boxes' transform arguments");
   if (cudaMalloc(&b->d_steps, sizeof(BoxStep) * (size_t)nbox) != cudaSuccess ||
       cudaMemcpy(b->d_steps, h.data(), sizeof(BoxStep) * (size_t)nbox, cudaMemcpyHostToDevice) !=
           cudaSuccess ||
@@ -2806,11 +2949,17 @@ int fused_step_enqueue(mg_batch* b, bool measure, cudaEvent_t* ev = nullptr) {
   BCK(mark(2));
   if (g.any_tc) BCK(k_batch_tc_phase(L, b->d_tc, nbox, g.tc_phase, g.tc_phase_smem));
   BCK(mark(3));
+  if (b->n_nf) BCK(k_nf_forward(L, b->d_nf, b->n_nf, b->nf_grid));
   if (g.any_fp32) BCK(k_batch_pass1(L, b->d_steps, nbox, g));
   if (g.any_tc) BCK(k_batch_sk_tc(L, b->d_tc, nbox, g.tc_sk, g.tc_sk_smem));
   BCK(mark(4));
-  BCK(k_batch_sk_reduce(L, b->d_steps, nbox, g, measure));
+  if (b->n_nf) BCK(k_nf_modes(L, b->d_nf, b->n_nf, b->nf_grid, measure));
+  if (g.skr > 0) BCK(k_batch_sk_reduce(L, b->d_steps, nbox, g, measure));
   BCK(mark(5));
+  if (b->n_nf) {
+    BCK(k_nf_back(L, b->d_nf, b->n_nf, b->nf_grid));
+    BCK(k_nf_interp(L, b->d_nf, b->n_nf, b->nf_grid, nullptr));
+  }
   if (g.any_fp32) BCK(k_batch_pass2(L, b->d_steps, nbox, g));
   if (g.any_tc) BCK(k_batch_kf_tc(L, b->d_tc, nbox, g.tc_vb, g.tc_kf, g.tc_kf_smem));
   BCK(mark(6));

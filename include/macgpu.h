@@ -130,18 +130,17 @@ typedef struct {
   /* Ewald pass 1 work split: charge chunks sized for this many CTAs per SM;
      <=0 selects 10 (FP32) / 8 (FP64).  mg_autotune picks it. */
   int kspace_ctas_per_sm;
-  /* FP32 pair kernel: 8 = the group kernel (a warp per group of 8 home
-     sites; neighbours pruned against the group's bounding box; needs a grid
-     of at least 2 cdiv + 1 cells per edge, else the cell kernel runs);
-     9 = the group kernel with Newton's third law (every pair once, over a
-     half-shell stencil; forces, of the shells too, summed in 64-bit fixed
-     point, 2^-32 K/A, by integer atomics, so still reproducible bit for
-     bit), lanes on the home sites; 10 = the same with lanes on the
-     neighbours (each lane runs one neighbour against the group's home
-     sites; with Drude shells 9 runs);
-     otherwise the cell kernel with bit 0 = 8 warps per home cell (else 4),
-     bit 2 = 16 warps per home cell (over bit 0), bit 1 = the erfc force
-     spline in shared memory (else read through L1).  mg_autotune picks it. */
+  /* FP32 pair kernel: 0 = automatic, the half-shell kernel (every pair once,
+     warps with a group of 8 home sites each against neighbours pruned by the
+     group's bounding box; forces, of the shells too, summed in 64-bit fixed
+     point, 2^-32 K/A, by integer atomics, so reproducible bit for bit), or all
+     pairs in a small box whose cutoff leaves cells of few sites; 9, 10 = the
+     half-shell kernel; 8 = the group kernel (the same pruning, every pair
+     from both ends, no atomics); 1..7 = the cell kernel with bit 0 = 8 warps
+     per home cell (else 4), bit 2 = 16 warps per home cell (over bit 0), bit 1
+     = the erfc force spline in shared memory (else read through L1).  A box
+     held in one cell (cutoff within 6 % of half the box) runs all pairs under
+     every value.  mg_autotune picks it. */
   int pair_variant;
   /* thermostat (sim/thermo.c): 0 none, 1 Berendsen, 2 Bussi (stochastic
      velocity rescaling), both applied after every SHAKE step; 3 Nose-Hoover
@@ -458,8 +457,8 @@ int mg_batch_last_launches(const mg_batch *b);
 /* en: NULL or [nbox] energies of the last step.  When every box runs the
    FP32 path with its Ewald sums as non-uniform transforms or both passes on
    the FP32 cores or both on the tensor cores (kspace_engine 0, 1 or 3; under
-   0 a box whose k set does not fit runs its passes directly), the cell pair
-   kernel with 4 warps (pair_variant 0), cells re-binned every step and no Drude charges, dependants, thermostat,
+   0 a box whose k set does not fit runs its passes directly), the default
+   pair kernel (pair_variant 0), cells re-binned every step and no Drude charges, dependants, thermostat,
    drmax, drift removal or dipole term, a step is one launch per kernel over
    all boxes (blockIdx.y = box, each box with its single-launch arguments,
    so its results are those of the box run alone); otherwise one graph node

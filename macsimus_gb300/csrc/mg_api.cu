@@ -64,8 +64,7 @@ struct mg_ctx {
   // group, its grid; nprows = energy rows of the pair kernel (cell or group)
   int4* d_spans = nullptr;
   int nspans = 0, ngroup_grid = 0, nprows = 0;
-  // its half-shell forms (pair_variant 9, 10): the half stencil as z-runs and the
-  // 64-bit fixed-point force sums (sorted order, zero between evaluations)
+  // the half-shell kernel: the half stencil as z-runs and the 64-bit fixed-point force sums (sorted order, zero between evaluations)
   int4* d_hspans = nullptr;
   int nhspans = 0;
   long long* d_facc = nullptr;
@@ -155,6 +154,11 @@ struct mg_ctx {
   bool dmax_pending = false;
   int nepart = 0;
   int pair_variant = 0;
+  // FP32 path: all pairs (pair_all_kernel), the half-shell kernel; its warps
+  // per group, its kind masks
+  bool small = false, half = false;
+  int split = 1;
+  unsigned heavy = 0, shells = 0;
   // thermostat
   int normalize = 1;
   double box_r0 = 0.15;
@@ -534,6 +538,13 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
                                      qq,           qpc,          qcp,         qpp};
     }
 
+  for (int k = 0; k < ctx->nkind; k++) {
+    if (kind_qp[k] != 0) ctx->shells |= 1u << k;
+    for (int l = 0; l < ctx->nkind; l++)
+      if (pd[k * ctx->nkind + l].E4 != 0) ctx->heavy |= 1u << k;
+  }
+  ctx->heavy |= ctx->shells;
+
   // ---- erfc spline table over [0, cutoff + rplus)
   std::vector<double> ert;
   double rplus = p->rplus > 0 ? p->rplus : 2.5;
@@ -572,6 +583,15 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     if (ok) break;
   }
   ctx->allpairs = allpairs;
+  // the FP32 pair kernel.  One cell: all pairs; so with cells of fewer than
+  // four sites (a cutoff just short of half the box, cut in many to fit) in a
+  // box of up to 8192.  Otherwise variants 9, 10 and the default 0 run the
+  // half-shell kernel
+  ctx->small = allpairs || (ctx->precision == MG_MIXED && !ctx->use_list &&
+                            ctx->pair_variant == 0 && ns <= 8192 &&
+                            ns < 4L * nc3[0] * nc3[1] * nc3[2]);
+  ctx->half = ctx->precision == MG_MIXED && !ctx->use_list && !ctx->small &&
+              (ctx->pair_variant == 0 || ctx->pair_variant >= 9);
   ctx->ntab = (int)(ert.size() / 6);
   ctx->ncx = nc3[0];
   ctx->ncy = nc3[1];
@@ -617,7 +637,18 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   ctx->nhspans = (int)hspans.size();
   // work items of the group kernel: at most ns / GROUP_SITES + ncell
   ctx->ngroup_grid = (int)(((long)ns / GROUP_SITES + ctx->ncell + GROUP_WARPS) / GROUP_WARPS);
-  ctx->nprows = std::max(ctx->ncell, ctx->ngroup_grid);
+  // warps per group of the half-shell kernel: enough groups to give every SM
+  // sub-partition eight warps are not split; others until they do, while every
+  // warp keeps about four batches of candidates (half the stencil's sites)
+  {
+    const double groups = ns / 8.0 + 0.5 * ctx->ncell,
+                 cand = 0.5 * ctx->nstencil * ((double)ns / ctx->ncell);
+    while (ctx->split < 8 && groups * ctx->split < 8 * 4 * PARTITION_SMS &&
+           cand >= 2 * ctx->split * 128)
+      ctx->split *= 2;
+  }
+  ctx->nprows = std::max(std::max(ctx->ncell, ctx->ngroup_grid * (ctx->half ? ctx->split : 1)),
+                         pair_all_blocks(ns));
 
   // ---- k-vectors (cook's set), sorted into (kx,ky) columns of consecutive kz
   double kappa = p->kappa;
@@ -781,7 +812,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   CK(upload(&ctx->d_stencil, st.data(), st.size()));
   CK(upload(&ctx->d_spans, spans.data(), spans.size()));
   CK(upload(&ctx->d_hspans, hspans.data(), hspans.size()));
-  if (ctx->pair_variant >= 9) {
+  if (ctx->half) {
     // centres, then (Drude builds) shells
     const size_t nfix = 3 * (size_t)ns * (t->chargepol ? 2 : 1);
     CK(dalloc(&ctx->d_facc, nfix));
@@ -1178,6 +1209,7 @@ PairArgs make_pair_args(mg_ctx* ctx, double* f_dev) {
   pa.ncz = ctx->ncz;
   pa.nstencil = ctx->nstencil;
   pa.allpairs = ctx->allpairs ? 1 : 0;
+  pa.small = ctx->small ? 1 : 0;
   pa.nkind = ctx->nkind;
   pa.cell_start = ctx->d_cell_start;
   pa.order = ctx->d_order;
@@ -1195,9 +1227,11 @@ PairArgs make_pair_args(mg_ctx* ctx, double* f_dev) {
   pa.pdd = ctx->d_pdd;
   pa.pair_warps = (ctx->pair_variant & 4) ? 16 : ((ctx->pair_variant & 1) ? 8 : 4);
   pa.spline_smem = (ctx->pair_variant & 2) && ctx->ntab * 16 <= 200 * 1024 ? 1 : 0;
-  pa.group = (ctx->pair_variant & 8) ? 1 : 0;
-  // half shell: 1 lanes on the home sites, 2 lanes on the neighbours
-  pa.newton = ctx->pair_variant == 9 ? 1 : (ctx->pair_variant == 10 ? 2 : 0);
+  pa.group = ctx->half || ctx->pair_variant == 8 ? 1 : 0;
+  pa.newton = ctx->half ? 1 : 0;
+  pa.split = ctx->split;
+  pa.heavy = ctx->heavy;
+  pa.shells = ctx->shells;
   pa.hspans = ctx->d_hspans;
   pa.nhspans = ctx->nhspans;
   pa.facc = ctx->d_facc;
@@ -2355,6 +2389,7 @@ PairArgs pair_args(mg_ctx* ctx) {
   pa.ncz = ctx->ncz;
   pa.nstencil = ctx->nstencil;
   pa.allpairs = ctx->allpairs ? 1 : 0;
+  pa.small = ctx->small ? 1 : 0;
   pa.nkind = ctx->nkind;
   pa.cell_start = ctx->d_cell_start;
   pa.order = ctx->d_order;
@@ -2785,12 +2820,12 @@ namespace {
 
 // a box the batched kernels take: the FP32 path without Drude charges,
 // dependants, thermostat, step limiter or drift removal, cells re-binned
-// at every step on a grid of at least 3 cells per edge, the cell pair kernel
-// with 4 warps, both Ewald passes on the FP32 cores or both on the tensor
+// at every step on a grid of at least 3 cells per edge, the default pair
+// kernel, both Ewald passes on the FP32 cores or both on the tensor
 // cores, no dipole term
 bool fusable(const mg_ctx* c) {
   return c->precision == MG_MIXED && !c->polar && !c->use_list && !c->allpairs &&
-         c->pair_variant == 0 && (c->nf || c->kspace_tc == c->sk_tc) && c->thermostat == 0 &&
+         c->pair_variant == 0 && (c->half || c->small) && (c->nf || c->kspace_tc == c->sk_tc) && c->thermostat == 0 &&
          c->ndep == 0 && !c->dipole && c->drmax == 0 && !c->drift_step && c->nq > 0 &&
          !c->prof_on;
 }
@@ -2864,7 +2899,8 @@ int build_fused(mg_batch* b) {
     e.rout[3] = c->d_sums + 32;
     e.g_site = cell_site_blocks(c->ns);
     e.g_order = cell_order_blocks(c->ncell);
-    e.g_pair = c->ncell;
+    e.g_half = c->half ? c->ngroup_grid * c->split : 0;
+    e.g_all = c->small ? pair_all_blocks(c->ns) : 0;
     e.g_excl = c->nmol > 0 ? (c->nmol + EXCL_THREADS - 1) / EXCL_THREADS : 0;
     e.g_charge = (c->nq + 255) / 256;
     e.g_phase = (int)(((long)c->nq * c->row + 255) / 256);
@@ -2902,7 +2938,8 @@ int build_fused(mg_batch* b) {
     g.tc_kf_smem = std::max(g.tc_kf_smem, t.smem_kf);
     g.site = std::max(g.site, e.g_site);
     g.order = std::max(g.order, e.g_order);
-    g.pair = std::max(g.pair, e.g_pair);
+    g.half = std::max(g.half, e.g_half);
+    g.all = std::max(g.all, e.g_all);
     g.excl = std::max(g.excl, e.g_excl);
     g.charge = std::max(g.charge, e.g_charge);
     g.phase = std::max(g.phase, e.g_phase);

@@ -130,6 +130,7 @@ cudaError_t k_gather_drude(const Launch& L, int ns, const double* r, const int* 
 struct PairArgs {
   int ns, ncx, ncy, ncz, nstencil, nkind;
   int allpairs;             // one cell: nearest image taken per pair (FP64 path)
+  int small;                // FP32 path: the all-pairs kernel (pair_all_kernel)
   const int* cell_start;
   const int* order;         // sorted -> site
   const int4* stencil;      // dx,dy,dz
@@ -153,11 +154,13 @@ struct PairArgs {
   const int4* spans;
   int nspans;
   int ngrid;                // CTAs of the group kernel (its energy rows)
-  // the group kernel with Newton's third law (pair_variant 9: 1, lanes on
-  // the home sites; pair_variant 10: 2, lanes on the neighbours, shells as
-  // 1): the half-shell z-runs, and the 64-bit fixed-point force sums (2^-32
-  // K/A units, sorted order, kept zero between evaluations)
+  // the half-shell kernel (every pair once): the half-shell z-runs, and the
+  // 64-bit fixed-point force sums (2^-32 K/A units, sorted order, kept zero
+  // between evaluations); split: warps per group; bit masks of the kinds with
+  // a Lennard-Jones term or a shell, and of those with a shell
   int newton;
+  int split;
+  unsigned heavy, shells;
   const int4* hspans;
   int nhspans;
   long long* facc;
@@ -386,7 +389,7 @@ struct BoxStep {
   int* gstart;
   int4* pj;
   int* gcell;
-  // r-space (the cell pair kernel, 4 warps per home cell)
+  // r-space (the half-shell or the all-pairs kernel)
   PairArgs pa;
   const PairF* ptab;
   const float4* erd;
@@ -406,13 +409,13 @@ struct BoxStep {
   int rrows[4], rwidth[4];
   double* rout[4];
   // CTAs of each kernel
-  int g_site, g_order, g_pair, g_excl, g_charge, g_phase, g_p1x, g_p1y, g_skr, g_kf, g_shake;
+  int g_site, g_order, g_half, g_all, g_excl, g_charge, g_phase, g_p1x, g_p1y, g_skr, g_kf, g_shake;
 };
 // the largest grid and shared memory of each kernel over the boxes (the
 // FP32-core k-space kernels have zero grids for boxes on the tensor cores
 // and the other way round; tc: the TcBox grids and shared memory)
 struct BatchGrid {
-  int site, order, pair, excl, charge, phase, p1x, p1y, skr, kf, shake;
+  int site, order, half, all, excl, charge, phase, p1x, p1y, skr, kf, shake;
   size_t pair_smem, kf_smem;
   int tc_phase, tc_sk, tc_vb, tc_kf;
   size_t tc_phase_smem, tc_sk_smem, tc_kf_smem;
@@ -437,6 +440,7 @@ size_t kf_mixed_smem(const KArgs& a);
 int kf_mixed_blocks(int nq);
 int cell_site_blocks(int ns);
 int cell_order_blocks(int ncell);
+int pair_all_blocks(int ns);
 
 
 // neighbour lists (mg_nlist.cu)

@@ -237,12 +237,43 @@ cell_order_kernel(int ncell, const int* __restrict__ start, const int* __restric
   cell_order_kernel_body(ncell, start, slot_site, pfix, order, key_s, pj, gstart, gcell, blockIdx.x, 0);
 }
 
+// the list of a box held in one cell: the sites in their own order (the pair
+// kernel takes all pairs, so no order helps it), one launch
+__global__ void cell_one_kernel(int ns, const double* __restrict__ r, const __grid_constant__ Inv3 iL,
+                                const int* __restrict__ kind, const int* __restrict__ mol,
+                                int* __restrict__ status, int* __restrict__ order,
+                                int* __restrict__ key_s, int* __restrict__ start,
+                                int* __restrict__ gstart, int4* __restrict__ pj,
+                                int* __restrict__ gcell) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    start[0] = gstart[0] = 0;
+    start[1] = ns;
+    gstart[1] = ngroups(ns);
+  }
+  if (i >= ns) return;
+  const double x = r[3 * i], y = r[3 * i + 1], z = r[3 * i + 2];
+  if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(status, 2);
+  order[i] = i;
+  key_s[i] = 0;
+  if (gcell && i % GROUP_SITES == 0) gcell[i / GROUP_SITES] = 0;
+  if (pj)
+    pj[i] = make_int4(fixed32(x, iL.v[0]), fixed32(y, iL.v[1]), fixed32(z, iL.v[2]),
+                      (mol[i] << 8) | kind[i]);
+}
+
 cudaError_t k_cell_list(const Launch& L, int ns, const double* r, int* status, const double iL[3],
                         int ncx, int ncy, int ncz, const int* kind, const int* mol, int4* pfix,
                         int* key, int* count, int* cursor, int* slot_site, int* order,
                         int* key_s, int* start, int* gstart, int4* pj, int* gcell) {
   const int ncell = ncx * ncy * ncz;
   const Inv3 il{{iL[0], iL[1], iL[2]}};
+  if (ncell == 1) {
+    cell_one_kernel<<<cdiv(ns, 128), 128, 0, L.s>>>(ns, r, il, kind, mol, status, order, key_s,
+                                                    start, gstart, pj, gcell);
+    LAUNCHED(L);
+    return cudaGetLastError();
+  }
   cell_count_kernel<<<cdiv(ns, 256), 256, 0, L.s>>>(ns, r, il, ncx, ncy, ncz, kind, mol, pfix, key,
                                                     count, status);
   LAUNCHED(L);
@@ -308,14 +339,13 @@ constexpr int FOLD = 8;   // stencil cells per FP32 force batch before the FP64 
 // cook/ljqqpol.c (centre-Drude, Drude-centre, Drude-Drude, each at its own
 // separation); Drude forces go to the second half of f.
 //
-// REL (every grid of at least 2 cdiv + 1 cells per edge): a staged site is
-// converted once, as the float offset of its nearest image from the centre
-// of the home cell (exact 32-bit fixed-point difference, then one rounding);
-// a pair then costs three subtractions and no int-to-float conversion
-// (conversions are slow on this GPU).  Every stencil cell lies within half a
-// box of the home-cell centre, so the image taken is the nearest one for
-// every pair inside the cutoff.  Without REL (one cell: all pairs) each pair
-// takes its nearest image from its own fixed-point difference.
+// Every grid has at least 2 cdiv + 1 cells per edge (boxes of one cell run
+// pair_all_kernel): a staged site is converted once, as the float offset of
+// its nearest image from the centre of the home cell (exact 32-bit
+// fixed-point difference, then one rounding); a pair then costs three
+// subtractions and no int-to-float conversion (conversions are slow on this
+// GPU).  Every stencil cell lies within half a box of the home-cell centre,
+// so the image taken is the nearest one for every pair inside the cutoff.
 // NW warps per CTA (the autotuner picks 4, 8 or 16: more warps per home
 // cell finish a cell sooner, which shortens the tail of the grid); STAB: the
 // force spline in
@@ -325,7 +355,7 @@ constexpr int FOLD = 8;   // stencil cells per FP32 force batch before the FP64 
 // FOLD stencil cells and folded into an FP32 sum with a compensation term
 // (Knuth's TwoSum): no FP64 instruction in the loop (the FP64 pipe of this
 // GPU is narrow and also serves the float/double conversions).
-template <bool MEASURE, bool POLAR, bool REL, int NW, bool STAB>
+template <bool MEASURE, bool POLAR, int NW, bool STAB>
 MG_BODY void pair_mixed_kernel_body(const PairArgs& a,
     const int4* __restrict__ pj,
     const PairF* __restrict__ ptab_g,
@@ -395,14 +425,12 @@ MG_BODY void pair_mixed_kernel_body(const PairArgs& a,
       for (int jb = 0; jb < nj; jb += 32) {
         if (jb + lane < nj) {
           int4 q = pj[j0 + jb + lane];
-          if (REL) {
-            // offset of the neighbour's nearest image from the home-cell centre
-            const float4 f = make_float4((float)(int)((unsigned)q.x - refx) * sx,
-                                         (float)(int)((unsigned)q.y - refy) * sy,
-                                         (float)(int)((unsigned)q.z - refz) * sz,
-                                         __int_as_float(q.w));
-            q = make_int4(__float_as_int(f.x), __float_as_int(f.y), __float_as_int(f.z), q.w);
-          }
+          // offset of the neighbour's nearest image from the home-cell centre
+          const float4 f = make_float4((float)(int)((unsigned)q.x - refx) * sx,
+                                       (float)(int)((unsigned)q.y - refy) * sy,
+                                       (float)(int)((unsigned)q.z - refz) * sz,
+                                       __int_as_float(q.w));
+          q = make_int4(__float_as_int(f.x), __float_as_int(f.y), __float_as_int(f.z), q.w);
           sj[warp][lane] = q;
           if (POLAR) sjd[warp][lane] = a.pdj[j0 + jb + lane];
         }
@@ -410,17 +438,8 @@ MG_BODY void pair_mixed_kernel_body(const PairArgs& a,
         const int cnt = min(32, nj - jb);
         for (int jj = 0; jj < cnt; jj++) {
           const int4 q = sj[warp][jj];
-          float dx, dy, dz;
-          if (REL) {
-            dx = xi - __int_as_float(q.x);
-            dy = yi - __int_as_float(q.y);
-            dz = zi - __int_as_float(q.z);
-          } else {
-            // nearest image: 32-bit wrap-around of the fixed-point difference
-            dx = (float)(int)((unsigned)me.x - (unsigned)q.x) * sx;
-            dy = (float)(int)((unsigned)me.y - (unsigned)q.y) * sy;
-            dz = (float)(int)((unsigned)me.z - (unsigned)q.z) * sz;
-          }
+          const float dx = xi - __int_as_float(q.x), dy = yi - __int_as_float(q.y),
+                      dz = zi - __int_as_float(q.z);
           const float rr = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
           // the site itself and its own molecule (exclusions) are skipped
           if (!vi || rr >= cq || (q.w >> 8) == mol_i) continue;
@@ -544,10 +563,10 @@ MG_BODY void pair_mixed_kernel_body(const PairArgs& a,
   }
 }
 
-template <bool MEASURE, bool POLAR, bool REL, int NW, bool STAB>
+template <bool MEASURE, bool POLAR, int NW, bool STAB>
 __global__ void __launch_bounds__(NW * 32)
     pair_mixed_kernel(const __grid_constant__ PairArgs a, const int4* __restrict__ pj, const PairF* __restrict__ ptab_g, const float4* __restrict__ erd_g, const float4* __restrict__ eru, float sx, float sy, float sz, float cq, float sgrid, float alpha) {
-  pair_mixed_kernel_body<MEASURE, POLAR, REL, NW, STAB>(a, pj, ptab_g, erd_g, eru, sx, sy, sz, cq, sgrid, alpha, blockIdx.x, 0);
+  pair_mixed_kernel_body<MEASURE, POLAR, NW, STAB>(a, pj, ptab_g, erd_g, eru, sx, sy, sz, cq, sgrid, alpha, blockIdx.x, 0);
 }
 
 // ------------------------------------------------- group pair kernel --
@@ -772,31 +791,13 @@ __global__ void __launch_bounds__(NW * 32)
   }
 }
 
-// ------------------------------------------- group kernel, half shell --
+// ---------------------------------------- fixed-point force sums --
 //
-// Newton's third law in the group kernel (pair_variant 9, no Drude shells):
-// every unordered pair once.  The stencil is the half shell: the z-runs of
-// the columns with dx > 0, or dx = 0 and dy > 0, whole, and the column
-// (0, 0) from the home cell up; inside the home cell a pair is taken from
-// its site with the lower sorted index (the grid has at least 2 cdiv + 1
-// cells per edge, so no cell reaches another by two stencil offsets and no
-// pair is found twice).  The pair terms are the group kernel's.  Forces go
-// into 64-bit fixed-point sums (FIX_SCALE units per K/A) in sorted order by
-// integer atomics; integer addition does not depend on the order, so the
-// forces come out the same bit for bit on every run.  The neighbour's force
-// of an iteration is summed over the 8 home lanes by a reduce-scatter (three
-// shuffle levels: lanes i = 0, 2, 4 end with x, y, z) and added with one
-// atomic per component; the home sites' own compensated sums once per
-// group.  Every rounding of the force arithmetic is explicit (the `_rn`
-// intrinsics and explicit FMAs), so that the measuring and the plain
-// instantiation run the same arithmetic: nvcc and ptxas may otherwise fuse
-// a product into a following add in one kernel and not in the other, and a
-// measured step would move the sites differently.  finish_forces_kernel
-// turns the sums into the FP64 forces (site order) and clears them for the
-// next evaluation.  Measured on 32768 waters (cells of cutoff/2): 0.37 ms
-// against 0.45 ms for the group kernel.  Pairing two iterations on one
-// conversion and one atomic, and a float-to-integer conversion in FP32
-// arithmetic instead of the one on the FP64 pipe, both measured slower.
+// The half-shell kernel below adds forces as 64-bit fixed-point numbers
+// (FIX_SCALE units per K/A, sorted order) by integer atomics: integer addition
+// does not depend on the order, so the forces come out the same bit for bit
+// on every run.  finish_forces_kernel turns the sums into the FP64 forces
+// (site order) and clears them for the next evaluation.
 constexpr double FIX_SCALE = 4294967296.0;  // 2^32: steps of 2.3e-10 K/A, |F| < 2^31 K/A
 
 
@@ -806,14 +807,22 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
+// a compile-time truth value (which terms a quad of home sites takes)
+template <bool B>
+struct BoolC {
+  static constexpr bool value = B;
+};
+
 // the half-shell kernel's pair force factor f (force on i = f (r_i - r_j))
-// with every rounding explicit; flj: the LJ part.  The same terms as
+// with every rounding explicit; flj: the LJ part, y: (Sq / r^2)^3 for its
+// energy.  The same terms as
 // spline_any and the group kernel: smoothed LJ (core below C1q, quadratic
 // tail up to C2q) and the hyperbolic erfc spline d.x + d.y / (d.z + r^2)
 __device__ __forceinline__ float pair_force_rn(const PairFS& P, float rr,
                                                const float4* __restrict__ erd, float sgrid,
-                                               int ntab, float& flj) {
-  const float x = __fmul_rn(P.Sq, rcp_approx(rr)), y = __fmul_rn(__fmul_rn(x, x), x);
+                                               int ntab, float& flj, float& y) {
+  const float x = __fmul_rn(P.Sq, rcp_approx(rr));
+  y = __fmul_rn(__fmul_rn(x, x), x);
   flj = rr < P.C1q ? __fmul_rn(__fmul_rn(P.E24, __fmaf_rn(__fmul_rn(2.f, y), y, -y)), x)
                    : (rr < P.C2q ? __fmul_rn(P.A4, __fadd_rn(rr, -P.C2q)) : 0.f);
   const int ix = min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
@@ -840,286 +849,222 @@ __device__ __forceinline__ float drude_force_rn(const float4* __restrict__ erd,
   return __fmul_rn(__fmaf_rn(d.y, rcp_approx(__fadd_rn(d.z, r2)), d.x), q);
 }
 
-// 7 CTAs per SM (72 registers, no spills): measured faster than 8 (64) and
-// than no bound (95).  POLAR (Drude shells): four charge terms per pair,
-// forces on both centres and both shells; the neighbour's six components
-// (centre x y z, shell x y z) are reduce-scattered over the 8 home lanes
-// in three levels (keeping 4, 2, 1 of 8 padded components), so lane i ends
-// with component i and lanes 0..5 write them
-template <bool MEASURE, bool POLAR, int NW>
-__global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : (POLAR ? 5 : 7))
-    pair_half_mixed_kernel(PairArgs a, const int4* __restrict__ pj,
-                           const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
-                           const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
-                           float sgrid) {
-  constexpr int NT = NW * 32;
+// ------------------------------------------------- all-pairs kernel --
+//
+// Small boxes (one cell holds every site, or the cutoff sphere covers a good
+// part of the box): a CTA per 8 consecutive sorted sites, its 16 warps taking
+// batches of 32 of all sites in turn, staged in shared memory; lane = (site,
+// one of four neighbours at a time).  Every pair is evaluated from both ends, its nearest image from the
+// exact fixed-point difference.  With the cells of such a box a few dozen
+// warps wait for short runs of sites one after the other; here every SM has
+// work and the only waste is the pairs beyond the cutoff, whose terms are
+// skipped when no lane needs them.  Measured at 1500 sites: 11 us, the cell
+// kernel 85 and the half-shell kernel 17; at 648 sites held in one cell, where
+// one warp of the cell kernel did all the work, a measured evaluation went
+// from 3.2 ms to about 20 us.  From some 2000 sites on the half-shell kernel is
+// the faster one wherever there is a grid for it.  Forces: FP32 per batch, folded into
+// compensated sums, the warps' sums added in order in FP64; every rounding of
+// the force arithmetic is explicit (measured and plain forces are the same).
+constexpr int ALL_WARPS = 16, ALL_SITES = 8;
+
+template <bool MEASURE, bool POLAR>
+MG_BODY void pair_all_kernel_body(const PairArgs& a, const int4* __restrict__ pj,
+                                  const PairF* __restrict__ ptab_g,
+                                  const float4* __restrict__ erd, const float4* __restrict__ eru,
+                                  float sx, float sy, float sz, float cq, float sgrid,
+                                  const int bx_) {
+  constexpr int NW = ALL_WARPS, NT = NW * 32, NC = POLAR ? 6 : 3;
   extern __shared__ float4 dyn_smem[];   // the nk x nk FP32 pair table
-  __shared__ float4 sj[NW][32];
+  __shared__ int4 sj[NW][32];
   __shared__ float4 sjd[POLAR ? NW : 1][32];
-  __shared__ int sjt[NW][32];
-  __shared__ double ered[NT];
+  __shared__ double red[NW][NC][ALL_SITES];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int il = lane & 7, sl = lane >> 3;
   const int nk = a.nkind, ntab = a.ntab;
   PairFS* ptab = reinterpret_cast<PairFS*>(dyn_smem);
   for (int t = threadIdx.x; t < 3 * nk * nk; t += NT)
     dyn_smem[t] = reinterpret_cast<const float4*>(ptab_g + t / 3)[t % 3];
-  __syncthreads();
-  const int ncell = a.ncx * a.ncy * a.ncz;
-  const int nitems = a.gstart[ncell];
-  unsigned long long* facc = reinterpret_cast<unsigned long long*>(a.facc);
-  const long dhalf = 3 * (long)a.ns;   // the shells' sums after the centres'
-  // reduce-scatter roles: without shells lane i ends with component i >> 1
-  // (0 x, 1 y, 2 z, 3 nothing) and lanes i = 0, 2, 4 write it; with shells
-  // lane i ends with component i (0-2 centre, 3-5 shell, 6-7 nothing)
-  const bool b2 = (il & 4) != 0, b1 = (il & 2) != 0, b0 = (il & 1) != 0;
-  const int comp = POLAR ? il : il >> 1;
-  const bool jw = POLAR ? il < 6 : (!b0 && comp < 3);
-  const long joff = POLAR && il >= 3 ? dhalf - 3 : 0;   // shell components
+  const int ti = bx_ * ALL_SITES + (lane & 7), sl = lane >> 3;
+  const bool vi = ti < a.ns;
+  const int4 me = vi ? pj[ti] : make_int4(0, 0, 0, 0);
+  const float4 md = (POLAR && vi) ? a.pdj[ti] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const PairFS* prow = ptab + (me.w & 255) * nk;
+  const float lim = vi ? cq : 0.f;
+  CSum fx, fy, fz, gx, gy, gz;
   CSum es[9];
-
-  for (int item = blockIdx.x * NW + warp; item < nitems; item += gridDim.x * NW) {
-    const int c = a.gcell[item];
-    const int cz = c % a.ncz, cy = (c / a.ncz) % a.ncy, cx = c / (a.ncy * a.ncz);
-    const int hs = a.cell_start[c], he = a.cell_start[c + 1];
-    const int i0 = hs + GROUP_SITES * (item - a.gstart[c]);
-    const int ni = min(GROUP_SITES, he - i0);
-    const unsigned refx = (unsigned)((((unsigned long long)(2 * cx + 1)) << 31) / a.ncx),
-                   refy = (unsigned)((((unsigned long long)(2 * cy + 1)) << 31) / a.ncy),
-                   refz = (unsigned)((((unsigned long long)(2 * cz + 1)) << 31) / a.ncz);
-    const bool vi = il < ni;
-    const int ti = i0 + il;
-    const int4 me = vi ? pj[ti] : make_int4(0, 0, 0, 0);
-    const float4 md = (POLAR && vi) ? a.pdj[ti] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int kind_i = me.w & 255, mol_i = me.w >> 8;
-    const float xi = __fmul_rn((float)(int)((unsigned)me.x - refx), sx),
-                yi = __fmul_rn((float)(int)((unsigned)me.y - refy), sy),
-                zi = __fmul_rn((float)(int)((unsigned)me.z - refz), sz);
-    float blx = vi ? xi : 3e38f, bly = vi ? yi : 3e38f, blz = vi ? zi : 3e38f;
-    float bhx = vi ? xi : -3e38f, bhy = vi ? yi : -3e38f, bhz = vi ? zi : -3e38f;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-      blx = fminf(blx, __shfl_xor_sync(0xffffffffu, blx, o));
-      bly = fminf(bly, __shfl_xor_sync(0xffffffffu, bly, o));
-      blz = fminf(blz, __shfl_xor_sync(0xffffffffu, blz, o));
-      bhx = fmaxf(bhx, __shfl_xor_sync(0xffffffffu, bhx, o));
-      bhy = fmaxf(bhy, __shfl_xor_sync(0xffffffffu, bhy, o));
-      bhz = fmaxf(bhz, __shfl_xor_sync(0xffffffffu, bhz, o));
-    }
-    CSum fx, fy, fz, gx, gy, gz;
-    for (int sp = 0; sp < a.nhspans; sp++) {
-      const int4 o = a.hspans[sp];
-      int x2 = cx + o.x, y2 = cy + o.y;
-      x2 += (x2 < 0) ? a.ncx : (x2 >= a.ncx ? -a.ncx : 0);
-      y2 += (y2 < 0) ? a.ncy : (y2 >= a.ncy ? -a.ncy : 0);
-      const int col = (x2 * a.ncy + y2) * a.ncz;
-      int za = cz + o.z, zb = cz + o.w;
-      if (zb < 0) { za += a.ncz; zb += a.ncz; }
-      if (za >= a.ncz) { za -= a.ncz; zb -= a.ncz; }
-      int ra0, ra1, rb0 = 0, rb1 = -1;
-      if (za < 0) { ra0 = za + a.ncz; ra1 = a.ncz - 1; rb0 = 0; rb1 = zb; }
-      else if (zb >= a.ncz) { ra0 = za; ra1 = a.ncz - 1; rb0 = 0; rb1 = zb - a.ncz; }
-      else { ra0 = za; ra1 = zb; }
-      float ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-      float e_el = 0, e_lj = 0, e_vir = 0;
-      PvF pv;
-      pv.zero();
-      for (int part = 0; part < 2; part++) {
-        const int z0 = part ? rb0 : ra0, z1 = part ? rb1 : ra1;
-        if (z1 < z0) continue;
-        // home-cell sites before the group pair with it from their own group
-        const int j0 = max(a.cell_start[col + z0], col + z0 == c ? i0 : 0),
-                  j1 = a.cell_start[col + z1 + 1];
-        for (int jb = j0; jb < j1; jb += 32) {
-          const int j = jb + lane;
-          bool keep = false;
-          float4 f4 = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (j < j1) {
-            const int4 q = pj[j];
-            f4 = make_float4(__fmul_rn((float)(int)((unsigned)q.x - refx), sx),
-                             __fmul_rn((float)(int)((unsigned)q.y - refy), sy),
-                             __fmul_rn((float)(int)((unsigned)q.z - refz), sz),
-                             __int_as_float(q.w));
-            const float ddx = fmaxf(fmaxf(blx - f4.x, f4.x - bhx), 0.f),
-                        ddy = fmaxf(fmaxf(bly - f4.y, f4.y - bhy), 0.f),
-                        ddz = fmaxf(fmaxf(blz - f4.z, f4.z - bhz), 0.f);
-            keep = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz)) < cq;
-          }
-          const unsigned M = __ballot_sync(0xffffffffu, keep);
-          if (keep) {
-            const int slot = __popc(M & ((1u << lane) - 1u));
-            sj[warp][slot] = f4;
-            sjt[warp][slot] = j;
-            if (POLAR) sjd[warp][slot] = a.pdj[j];
-          }
-          __syncwarp();
-          const int n = __popc(M);
-          // the whole warp iterates: the reduce-scatter needs every lane
-          for (int t0 = 0; t0 < n; t0 += 4) {
-            const int t = t0 + sl;
-            const bool vt = t < n;
-            const float4 q = sj[warp][vt ? t : 0];
-            const int tj = sjt[warp][vt ? t : 0];
-            const float dx = __fadd_rn(xi, -q.x), dy = __fadd_rn(yi, -q.y),
-                        dz = __fadd_rn(zi, -q.z);
-            const float rr = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-            const int qw = __float_as_int(q.w);
-            const bool ok = vt && vi && rr < cq && (qw >> 8) != mol_i &&
-                            (tj > ti || tj >= he || tj < hs);
-            const PairFS P = ptab[kind_i * nk + (qw & 255)];
-            float flj;
-            float f = pair_force_rn(P, rr, erd, sgrid, ntab, flj);
-            f = ok ? f : 0.f;
-            ax = __fmaf_rn(f, dx, ax);
-            ay = __fmaf_rn(f, dy, ay);
-            az = __fmaf_rn(f, dz, az);
-            float px = __fmul_rn(f, dx), py = __fmul_rn(f, dy), pz = __fmul_rn(f, dz);
-            // the neighbour's shell (POLAR)
-            float hx = 0.f, hy = 0.f, hz = 0.f;
-            float e_p = 0.f;
-            if (POLAR) {
-              // shell(i) - centre(j), centre(i) - shell(j), shell(i) - shell(j)
-              const float4 qd = sjd[warp][vt ? t : 0];
-              const float ex = __fadd_rn(dx, md.x), ey = __fadd_rn(dy, md.y),
-                          ez = __fadd_rn(dz, md.z);
-              float fp = drude_force_rn<MEASURE>(erd, eru, ex, ey, ez, sgrid, ntab, P.qpc, e_p);
-              const float cx2 = __fadd_rn(dx, -qd.x), cy2 = __fadd_rn(dy, -qd.y),
-                          cz2 = __fadd_rn(dz, -qd.z);
-              float fc = drude_force_rn<MEASURE>(erd, eru, cx2, cy2, cz2, sgrid, ntab, P.qcp,
-                                                 e_p);
-              const float ux = __fadd_rn(ex, -qd.x), uy = __fadd_rn(ey, -qd.y),
-                          uz = __fadd_rn(ez, -qd.z);
-              float fd = drude_force_rn<MEASURE>(erd, eru, ux, uy, uz, sgrid, ntab, P.qpp, e_p);
-              fp = ok ? fp : 0.f;
-              fc = ok ? fc : 0.f;
-              fd = ok ? fd : 0.f;
-              // home centre: + fc (cx2); home shell: + fp (e) + fd (u)
-              ax = __fmaf_rn(fc, cx2, ax);
-              ay = __fmaf_rn(fc, cy2, ay);
-              az = __fmaf_rn(fc, cz2, az);
-              bx = __fmaf_rn(fp, ex, __fmaf_rn(fd, ux, bx));
-              by = __fmaf_rn(fp, ey, __fmaf_rn(fd, uy, by));
-              bz = __fmaf_rn(fp, ez, __fmaf_rn(fd, uz, bz));
-              // neighbour centre: -(f d + fp e); neighbour shell: -(fc cx2 + fd u)
-              px = __fmaf_rn(fp, ex, px);
-              py = __fmaf_rn(fp, ey, py);
-              pz = __fmaf_rn(fp, ez, pz);
-              hx = __fmaf_rn(fc, cx2, __fmul_rn(fd, ux));
-              hy = __fmaf_rn(fc, cy2, __fmul_rn(fd, uy));
-              hz = __fmaf_rn(fc, cz2, __fmul_rn(fd, uz));
-              if (MEASURE && ok) {
-                pv.add(ex, ey, ez, fp);
-                pv.add(cx2, cy2, cz2, fc);
-                pv.add(ux, uy, uz, fd);
-              }
-            }
-            if (MEASURE && ok) {
-              // energies and virial: no effect on the forces
-              const float x = __fdividef(P.Sq, rr), y = x * x * x, xt = rr - P.C2q;
-              e_lj += rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
-              e_vir += rr * flj;
-              float e_el_p = 0.f;
-              spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
-              e_el += e_el_p + e_p;
-              pv.add(dx, dy, dz, f);
-            }
-            float k;
-            if (POLAR) {
-              // components 0-5 = (px, py, pz, hx, hy, hz), 6-7 zero; level 1
-              // keeps 4 (xor 4), level 2 keeps 2 (xor 2), level 3 keeps 1
-              const float v0 = b2 ? hy : px, v1 = b2 ? hz : py, v2 = b2 ? 0.f : pz,
-                          v3 = b2 ? 0.f : hx;
-              const float w0 = b2 ? px : hy, w1 = b2 ? py : hz, w2 = b2 ? pz : 0.f,
-                          w3 = b2 ? hx : 0.f;
-              const float k0 = __fadd_rn(v0, __shfl_xor_sync(0xffffffffu, w0, 4)),
-                          k1 = __fadd_rn(v1, __shfl_xor_sync(0xffffffffu, w1, 4)),
-                          k2 = __fadd_rn(v2, __shfl_xor_sync(0xffffffffu, w2, 4)),
-                          k3 = __fadd_rn(v3, __shfl_xor_sync(0xffffffffu, w3, 4));
-              const float m0 = __fadd_rn(b1 ? k2 : k0,
-                                         __shfl_xor_sync(0xffffffffu, b1 ? k0 : k2, 2)),
-                          m1 = __fadd_rn(b1 ? k3 : k1,
-                                         __shfl_xor_sync(0xffffffffu, b1 ? k1 : k3, 2));
-              k = __fadd_rn(b0 ? m1 : m0, __shfl_xor_sync(0xffffffffu, b0 ? m0 : m1, 1));
-            } else {
-              float k0 = b2 ? pz : px, k1 = b2 ? 0.f : py;
-              const float s0 = b2 ? px : pz, s1 = b2 ? py : 0.f;
-              k0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 4));
-              k1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 4));
-              k = b1 ? k1 : k0;
-              k = __fadd_rn(k, __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2));
-              k = __fadd_rn(k, __shfl_xor_sync(0xffffffffu, k, 1));
-            }
-            if (jw && vt)
-              atomicAdd(facc + 3 * (long)tj + comp + joff,
-                        (unsigned long long)__float2ll_rn(__fmul_rn(k, -(float)FIX_SCALE)));
-          }
-          __syncwarp();
+  __syncthreads();
+  for (int jb = warp * 32; jb < a.ns; jb += NT) {
+    const int j = jb + lane;
+    __syncwarp();
+    // slots past the last site hold a site of kind 0 (their pairs are masked,
+    // but their kind still indexes the pair table)
+    sj[warp][lane] = j < a.ns ? pj[j] : make_int4(0, 0, 0, 0);
+    if (POLAR) sjd[warp][lane] = j < a.ns ? a.pdj[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    const int cnt = min(32, a.ns - jb);
+    float ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
+    float e_el = 0, e_lj = 0, e_vir = 0;
+    PvF pv;
+    pv.zero();
+#pragma unroll 4
+    for (int j0 = 0; j0 < cnt; j0 += 4) {
+      const int jj = j0 + sl;
+      const int4 q = sj[warp][jj];
+      const float dx = __fmul_rn((float)(int)((unsigned)me.x - (unsigned)q.x), sx),
+                  dy = __fmul_rn((float)(int)((unsigned)me.y - (unsigned)q.y), sy),
+                  dz = __fmul_rn((float)(int)((unsigned)me.z - (unsigned)q.z), sz);
+      const float rr = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+      // the site itself and its own molecule (exclusions) are skipped
+      const bool ok = jj < cnt && rr < lim && ((q.w ^ me.w) >> 8) != 0;
+      if (!__any_sync(0xffffffffu, ok)) continue;
+      const PairFS P = prow[q.w & 255];
+      float flj, y;
+      float f = pair_force_rn(P, ok ? rr : 1.f, erd, sgrid, ntab, flj, y);
+      f = ok ? f : 0.f;
+      ax = __fmaf_rn(f, dx, ax);
+      ay = __fmaf_rn(f, dy, ay);
+      az = __fmaf_rn(f, dz, az);
+      float e_p = 0.f;
+      if (POLAR) {
+        // shell(i) - centre(j), centre(i) - shell(j), shell(i) - shell(j)
+        const float4 qd = sjd[warp][jj];
+        const float ex = __fadd_rn(dx, md.x), ey = __fadd_rn(dy, md.y), ez = __fadd_rn(dz, md.z);
+        const float cx = __fadd_rn(dx, -qd.x), cy = __fadd_rn(dy, -qd.y),
+                    cz = __fadd_rn(dz, -qd.z);
+        const float ux = __fadd_rn(ex, -qd.x), uy = __fadd_rn(ey, -qd.y),
+                    uz = __fadd_rn(ez, -qd.z);
+        float fp = drude_force_rn<MEASURE>(erd, eru, ex, ey, ez, sgrid, ntab, P.qpc, e_p);
+        float fc = drude_force_rn<MEASURE>(erd, eru, cx, cy, cz, sgrid, ntab, P.qcp, e_p);
+        float fd = drude_force_rn<MEASURE>(erd, eru, ux, uy, uz, sgrid, ntab, P.qpp, e_p);
+        fp = ok ? fp : 0.f;
+        fc = ok ? fc : 0.f;
+        fd = ok ? fd : 0.f;
+        ax = __fmaf_rn(fc, cx, ax);
+        ay = __fmaf_rn(fc, cy, ay);
+        az = __fmaf_rn(fc, cz, az);
+        bx = __fmaf_rn(fp, ex, __fmaf_rn(fd, ux, bx));
+        by = __fmaf_rn(fp, ey, __fmaf_rn(fd, uy, by));
+        bz = __fmaf_rn(fp, ez, __fmaf_rn(fd, uz, bz));
+        if (MEASURE && ok) {
+          pv.add(ex, ey, ez, fp);
+          pv.add(cx, cy, cz, fc);
+          pv.add(ux, uy, uz, fd);
         }
       }
-      fx.add(ax); fy.add(ay); fz.add(az);
-      if (POLAR) { gx.add(bx); gy.add(by); gz.add(bz); }
-      if (MEASURE) {
-        es[0].add(e_el); es[1].add(e_lj); es[2].add(e_vir);
-        es[3].add(pv.p0); es[4].add(pv.p1); es[5].add(pv.p2);
-        es[6].add(pv.p3); es[7].add(pv.p4); es[8].add(pv.p5);
+      if (MEASURE && ok) {
+        // energies and virial: no effect on the forces
+        const float xt = rr - P.C2q;
+        e_lj += rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
+        e_vir += rr * flj;
+        float e_el_p = 0.f;
+        spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
+        e_el += e_el_p + e_p;
+        pv.add(dx, dy, dz, f);
       }
     }
-    // the home sites' sums: the four s-lanes in a fixed order, then lane
-    // s = 0, 1, 2 adds component x, y, z (of the centre and the shell)
-    double g[6] = {fx.value(), fy.value(), fz.value(), 0, 0, 0};
-    if (POLAR) {
-      g[3] = gx.value();
-      g[4] = gy.value();
-      g[5] = gz.value();
-    }
-#pragma unroll
-    for (int k = 0; k < (POLAR ? 6 : 3); k++) {
-      g[k] += __shfl_xor_sync(0xffffffffu, g[k], 8);
-      g[k] += __shfl_xor_sync(0xffffffffu, g[k], 16);
-    }
-    if (vi && sl < 3) {
-      atomicAdd(facc + 3 * (long)ti + sl,
-                (unsigned long long)__double2ll_rn((sl == 0 ? g[0] : (sl == 1 ? g[1] : g[2])) *
-                                                   FIX_SCALE));
-      if (POLAR)
-        atomicAdd(facc + dhalf + 3 * (long)ti + sl,
-                  (unsigned long long)__double2ll_rn(
-                      (sl == 0 ? g[3] : (sl == 1 ? g[4] : g[5])) * FIX_SCALE));
+    fx.add(ax); fy.add(ay); fz.add(az);
+    if (POLAR) { gx.add(bx); gy.add(by); gz.add(bz); }
+    if (MEASURE) {
+      es[0].add(e_el); es[1].add(e_lj); es[2].add(e_vir);
+      es[3].add(pv.p0); es[4].add(pv.p1); es[5].add(pv.p2);
+      es[6].add(pv.p3); es[7].add(pv.p4); es[8].add(pv.p5);
     }
   }
+  double g[6] = {fx.value(), fy.value(), fz.value(), gx.value(), gy.value(), gz.value()};
+#pragma unroll
+  for (int k = 0; k < NC; k++) {
+    g[k] += __shfl_xor_sync(0xffffffffu, g[k], 8);
+    g[k] += __shfl_xor_sync(0xffffffffu, g[k], 16);
+    if (sl == 0) red[warp][k][lane] = g[k];
+  }
+  __syncthreads();
+  if (warp == 0 && vi)
+    for (int k = sl; k < NC; k += 4) {
+      double t = 0;
+#pragma unroll
+      for (int w = 0; w < NW; w++) t += red[w][k][lane & 7];
+      a.f[(k >= 3 ? 3 * (long)a.ns : 0) + 3 * (long)a.order[ti] + k % 3] = t;
+    }
   if (MEASURE) {
-    // every unordered pair once; one row per CTA
+    // each unordered pair was visited from both ends; the lanes' sums by
+    // butterfly, compensated in FP32 (the FP64 pipe is narrow), then the
+    // warps in order in FP64
+    double e[9];
+#pragma unroll
     for (int k = 0; k < 9; k++) {
-      ered[threadIdx.x] = es[k].value();
-      __syncthreads();
-      for (int w = NT / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) ered[threadIdx.x] += ered[threadIdx.x + w];
-        __syncthreads();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float s = __shfl_xor_sync(0xffffffffu, es[k].s, o),
+                    c = __shfl_xor_sync(0xffffffffu, es[k].c, o);
+        es[k].add(s);
+        es[k].c += c;
       }
-      if (threadIdx.x == 0) a.epart[blockIdx.x * NEN + k] = ered[0];
-      __syncthreads();
+      e[k] = 0.5 * es[k].value();
+    }
+    __syncthreads();
+    double* er = &red[0][0][0];   // at least 9 NW values
+    static_assert(NC * ALL_SITES >= 9, "energy sums fit the force sums");
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < 9; k++) er[k * NW + warp] = e[k];
+    __syncthreads();
+    if (threadIdx.x < 9) {
+      double t = 0;
+      for (int w = 0; w < NW; w++) t += er[threadIdx.x * NW + w];
+      a.epart[bx_ * NEN + threadIdx.x] = t;
     }
   }
 }
 
+template <bool MEASURE, bool POLAR>
+__global__ void __launch_bounds__(ALL_WARPS * 32, POLAR ? 1 : 2)
+    pair_all_kernel(const __grid_constant__ PairArgs a, const int4* __restrict__ pj,
+                    const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
+                    const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
+                    float sgrid) {
+  pair_all_kernel_body<MEASURE, POLAR>(a, pj, ptab_g, erd, eru, sx, sy, sz, cq, sgrid, blockIdx.x);
+}
+
 // ------------------------------ group kernel, half shell, lanes on the
-// neighbours (pair_variant 10, no Drude shells) --
+// neighbours --
 //
-// The work items, the half-shell z-runs, the candidate pruning against the
-// cutoff sphere around the group's bounding box and the pair terms are
-// those of pair_half_mixed_kernel; the roles of the lanes are transposed.
-// The kept candidates are compacted into a ring of 64 per warp; whenever
-// 32 are queued, each lane takes one and runs it against the group's (up
-// to 8) home sites in turn, which every lane reads from shared memory
+// Every pair once, over a half-shell stencil (the columns with dx > 0, or
+// dx = 0 and dy > 0, whole; the column (0, 0) from the home cell up, pairs
+// inside the home cell taken from their site with the lower sorted index).
+// Work item: a group of up to GROUP_SITES = 8 consecutive sorted sites of a
+// home cell; `split` warps share one, each taking every split-th batch of its
+// candidates (one warp a group fills the GPU from about 40000 sites on;
+// smaller boxes have too few groups).
+//
+// The candidates are the sites of the half-shell's z-runs: one run per lane
+// (its bounds found side by side; one after the other they cost a chain of
+// dependent loads each), read in batches of 32, each loaded before the one
+// before it is used.  Those outside the cutoff sphere around
+// the group's bounding box are dropped, the others compacted into a ring of 64
+// per warp; whenever 32 are queued, each lane takes one and runs it against
+// the group's home sites, which every lane reads from shared memory
 // (broadcast).  The neighbour's force stays in the lane's registers and goes
-// into the fixed-point sums with three atomics after the 8 home sites: no
-// per-pair shuffles, one float-to-integer conversion per component and
-// neighbour.  The home sites' forces stay in 24 registers per lane and are
-// reduce-scattered over the 32 lanes once per group (lane 3 i + d ends with
-// component d of site i).  Home sites beyond the group's end are masked
-// out of the pair test.  Every rounding is explicit, as in the lane-per-home
-// kernel, so the measuring and the plain instantiation move the sites
-// identically; the integer sums make the forces bit-reproducible.
+// into the 64-bit fixed-point sums with three atomics after the home sites;
+// the home sites' forces stay in registers and are reduce-scattered over the
+// warp once per group.
+//
+// The home sites come with those that have a Lennard-Jones term or a shell
+// first, in quads: a quad without any of them takes the Coulomb term alone
+// (half of the quads in water; about 31 instead of 46 instructions a pair).
+// The two quads stand in one block, so that the compiler interleaves their
+// eight independent chains: a branch per quad measured 0.305 ms on 32768
+// waters, a branch per site as slow.
+// With Drude shells (POLAR) a heavy quad takes the four charge terms of a
+// pair, a light one the two of the home centre.
+//
+// Every rounding of the force arithmetic is explicit, so the measuring and
+// the plain instantiation move the sites identically; the integer sums make
+// the forces bit-reproducible.
+//
+// Bound by issue (63 %) and the gathers of the erfc table through L1.  Measured:
+// 0.250 ms on 32768 waters (lane per home site 0.363, without the quads and
+// the side-by-side runs 0.267), 42 us on 12544 sites (61), 23 us on 864 waters
+// (61; cell kernel 110), 0.59 ms with 32768 shells (lane per home site 0.67),
+// 0.61 ms on a batch of 256 ionic boxes (cell kernel 0.94).
 
 // the z-ranges of half-shell span sp around cell (cx, cy, cz): column index
 // col; run [ra0, ra1] and, where the run wraps through the box, [rb0, rb1]
@@ -1142,27 +1087,37 @@ __device__ __forceinline__ void half_span_runs(const PairArgs& a, int sp, int cx
 }
 
 constexpr int HT_RING = 64;   // compacted candidates per warp (a power of two >= 63)
-// 5 CTAs per SM (96 registers): on 32768 waters with cells of half the
-// cutoff 0.283 ms, against 0.294 ms with 6 (80 registers and a spill); the
-// lane-per-home kernel takes 0.363 ms there.  One limit per lane for the
-// pair test (instead of three tests per pair): 0.276 ms, the same forces
-// bit for bit
-#ifndef MG_HALF_T_MINB
-#define MG_HALF_T_MINB 5      // CTAs per SM the register budget is set for
-#endif
 
-template <bool MEASURE, int NW>
-__global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : MG_HALF_T_MINB)
-    pair_half_t_mixed_kernel(PairArgs a, const int4* __restrict__ pj,
-                             const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
-                             const float4* __restrict__ eru, float sx, float sy, float sz,
-                             float cq, float sgrid) {
-  constexpr int NT = NW * 32;
+// the sums v[0..23] of a warp's lanes (v[24..31] zero), in a fixed order: lane
+// k ends with the sum of v[k] in v[0]
+__device__ __forceinline__ void reduce_scatter(float (&v)[32], int lane) {
+#pragma unroll
+  for (int w = 16; w >= 1; w >>= 1) {
+    const bool up = (lane & w) != 0;
+#pragma unroll
+    for (int k = 0; k < w; k++) {
+      const float keepv = up ? v[w + k] : v[k], sendv = up ? v[k] : v[w + k];
+      v[k] = __fadd_rn(keepv, __shfl_xor_sync(0xffffffffu, sendv, w));
+    }
+  }
+}
+
+template <bool MEASURE, bool POLAR, int NW>
+__device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const int4* __restrict__ pj,
+                                   const PairF* __restrict__ ptab_g,
+                                   const float4* __restrict__ erd,
+                                   const float4* __restrict__ eru, float sx, float sy, float sz,
+                                   float cq, float sgrid, const int bx_) {
+  constexpr int NT = NW * 32, GS = GROUP_SITES;
   extern __shared__ float4 dyn_smem[];   // the nk x nk FP32 pair table
   __shared__ float4 sq[NW][HT_RING];     // candidate positions (w: kind | mol << 8)
   __shared__ int sqt[NW][HT_RING];       // candidate sorted index
-  __shared__ float4 sh[NW][GROUP_SITES]; // the group's home sites
-  __shared__ double ered[MEASURE ? NT : 1];
+  __shared__ float4 sqd[POLAR ? NW : 1][HT_RING];   // candidate shells
+  __shared__ float4 sh[NW][GS];          // the group's home sites, heavy ones first
+  __shared__ float4 shd[POLAR ? NW : 1][GS];
+  __shared__ int so[NW][GS];             // their places in the group
+  __shared__ int spm[NW][GS + 1];        // [k]: the home sites of places below k
+  __shared__ int2 runs[NW][64];          // first site and end of the candidate runs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int il = lane & 7;
   const int nk = a.nkind, ntab = a.ntab;
@@ -1171,16 +1126,15 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : MG_HALF_T_MINB)
     dyn_smem[t] = reinterpret_cast<const float4*>(ptab_g + t / 3)[t % 3];
   __syncthreads();
   const int ncell = a.ncx * a.ncy * a.ncz;
-  const int nitems = a.gstart[ncell];
-  unsigned long long* facc = reinterpret_cast<unsigned long long*>(a.facc);
+  const int split = a.split, w = bx_ * NW + warp, item = w / split, part = w - item * split;
   CSum es[9];
 
-  for (int item = blockIdx.x * NW + warp; item < nitems; item += gridDim.x * NW) {
+  if (item < a.gstart[ncell]) {
     const int c = a.gcell[item];
     const int cz = c % a.ncz, cy = (c / a.ncz) % a.ncy, cx = c / (a.ncy * a.ncz);
     const int hs = a.cell_start[c], he = a.cell_start[c + 1];
-    const int i0 = hs + GROUP_SITES * (item - a.gstart[c]);
-    const int ni = min(GROUP_SITES, he - i0);
+    const int i0 = hs + GS * (item - a.gstart[c]);
+    const int ni = min(GS, he - i0);
     const unsigned refx = (unsigned)((((unsigned long long)(2 * cx + 1)) << 31) / a.ncx),
                    refy = (unsigned)((((unsigned long long)(2 * cy + 1)) << 31) / a.ncy),
                    refz = (unsigned)((((unsigned long long)(2 * cz + 1)) << 31) / a.ncz);
@@ -1201,12 +1155,36 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : MG_HALF_T_MINB)
       bhy = fmaxf(bhy, __shfl_xor_sync(0xffffffffu, bhy, o));
       bhz = fmaxf(bhz, __shfl_xor_sync(0xffffffffu, bhz, o));
     }
-    __syncwarp();   // the previous group's readers of sh are done
-    if (lane < GROUP_SITES) sh[warp][lane] = make_float4(xi, yi, zi, __int_as_float(me.w));
-    __syncwarp();
-    float hx[GROUP_SITES], hy[GROUP_SITES], hz[GROUP_SITES];
+    // slots: the heavy sites, the light ones, then the unused (their pairs
+    // are masked; a site of kind 0 at the cell centre keeps them finite)
+    const bool heavy = vi && ((a.heavy >> (me.w & 255)) & 1);
+    const unsigned below = (1u << il) - 1u;
+    const unsigned hm = __ballot_sync(0xffffffffu, heavy) & 255u,
+                   lm = __ballot_sync(0xffffffffu, vi && !heavy) & 255u;
+    const int nh = __popc(hm);
+    const int slot = heavy ? __popc(hm & below)
+                           : (vi ? nh + __popc(lm & below) : il);
+    if (lane < GS) {
+      sh[warp][slot] = make_float4(xi, yi, zi, __int_as_float(me.w));
+      if (POLAR) shd[warp][slot] = vi ? a.pdj[i0 + il] : make_float4(0.f, 0.f, 0.f, 0.f);
+      so[warp][slot] = il;
+    }
+    int pm = 0;
 #pragma unroll
-    for (int i = 0; i < GROUP_SITES; i++) hx[i] = hy[i] = hz[i] = 0.f;
+    for (int k = 0; k < GS; k++) {
+      const int o = __shfl_sync(0xffffffffu, slot, k);
+      if (k < lane && k < ni) pm |= 1 << o;
+    }
+    if (lane <= GS) spm[warp][lane] = pm;
+    __syncwarp();
+    const int all = (1 << ni) - 1;
+    float hx[GS], hy[GS], hz[GS];
+    float gx[POLAR ? GS : 1], gy[POLAR ? GS : 1], gz[POLAR ? GS : 1];
+#pragma unroll
+    for (int i = 0; i < GS; i++) {
+      hx[i] = hy[i] = hz[i] = 0.f;
+      if (POLAR) gx[POLAR ? i : 0] = gy[POLAR ? i : 0] = gz[POLAR ? i : 0] = 0.f;
+    }
 
     // cnt queued candidates from ring slot h0: lane -> one candidate
     // against the home sites
@@ -1215,57 +1193,123 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : MG_HALF_T_MINB)
       const int e = vt ? (h0 + lane) & (HT_RING - 1) : h0;   // a valid slot for idle lanes
       const float4 q = sq[warp][e];
       const int tj = sqt[warp][e];
+      const float4 qd = POLAR ? sqd[POLAR ? warp : 0][e] : make_float4(0.f, 0.f, 0.f, 0.f);
       const int qw = __float_as_int(q.w);
-      const int kj = qw & 255;
-      // the home sites i < lim pair with this candidate: none for an idle
-      // lane, those of the group, and of a candidate in the home cell only
-      // the ones before it
+      const PairFS* pcol = ptab + (qw & 255);
+      // the home sites this candidate pairs with: none for an idle lane, the
+      // group's, and of a candidate in the home cell only those before it
       const bool inh = (unsigned)(tj - hs) < (unsigned)(he - hs);
-      const int lim = !vt ? 0 : (inh ? min(ni, tj - i0) : ni);
-      float px = 0.f, py = 0.f, pz = 0.f;
+      const int mask = !vt ? 0 : (inh ? spm[warp][min(ni, max(tj - i0, 0))] : all);
+      float px = 0.f, py = 0.f, pz = 0.f;            // on the candidate
+      float ux = 0.f, uy = 0.f, uz = 0.f;            // on its shell
       float e_el = 0.f, e_lj = 0.f, e_vir = 0.f;
       PvF pv;
       pv.zero();
-      // the home sites in turn, those beyond the group's end masked (sh
-      // holds finite positions for them): without a branch per site the
-      // compiler interleaves the sites' independent chains (0.283 ms on
-      // 32768 waters against 0.304 ms with a warp-uniform branch per site)
-#pragma unroll
-      for (int i = 0; i < GROUP_SITES; i++) {
-        {
-          const float4 h = sh[warp][i];
-          const float dx = __fadd_rn(h.x, -q.x), dy = __fadd_rn(h.y, -q.y),
-                      dz = __fadd_rn(h.z, -q.z);
-          const float rr = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-          const int hw = __float_as_int(h.w);
-          const bool ok = i < lim && rr < cq && ((hw ^ qw) >> 8) != 0;
-          const PairFS P = ptab[(hw & 255) * nk + kj];
-          float flj;
-          float f = pair_force_rn(P, rr, erd, sgrid, ntab, flj);
-          f = ok ? f : 0.f;
-          hx[i] = __fmaf_rn(f, dx, hx[i]);
-          hy[i] = __fmaf_rn(f, dy, hy[i]);
-          hz[i] = __fmaf_rn(f, dz, hz[i]);
-          px = __fmaf_rn(f, dx, px);
-          py = __fmaf_rn(f, dy, py);
-          pz = __fmaf_rn(f, dz, pz);
-          if (MEASURE && ok) {
-            // energies and virial: no effect on the forces
-            const float x = __fdividef(P.Sq, rr), y = x * x * x, xt = rr - P.C2q;
-            e_lj += rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
-            e_vir += rr * flj;
-            float e_el_p = 0.f;
-            spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
-            e_el += e_el_p;
-            pv.add(dx, dy, dz, f);
+      auto pair = [&](const int i, auto full) {
+        constexpr bool HEAVY = decltype(full)::value;
+        const float4 h = sh[warp][i];
+        const float dx = __fadd_rn(h.x, -q.x), dy = __fadd_rn(h.y, -q.y),
+                    dz = __fadd_rn(h.z, -q.z);
+        const float rr = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+        const int hw = __float_as_int(h.w);
+        const bool ok = (mask >> i & 1) && rr < cq && ((hw ^ qw) >> 8) != 0;
+        const PairFS* pp = pcol + (hw & 255) * nk;
+        float f, flj = 0.f, y = 0.f, e_p = 0.f;
+        PairFS P;
+        if (HEAVY) {
+          P = *pp;
+          f = pair_force_rn(P, rr, erd, sgrid, ntab, flj, y);
+        } else {
+          P.qq = pp->qq;
+          // no LJ at this home site
+          const int ix =
+              min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+          const float4 d = __ldg(erd + ix);
+          f = __fmul_rn(__fmaf_rn(d.y, rcp_approx(__fadd_rn(d.z, rr)), d.x), P.qq);
+        }
+        f = ok ? f : 0.f;
+        hx[i] = __fmaf_rn(f, dx, hx[i]);
+        hy[i] = __fmaf_rn(f, dy, hy[i]);
+        hz[i] = __fmaf_rn(f, dz, hz[i]);
+        px = __fmaf_rn(f, dx, px);
+        py = __fmaf_rn(f, dy, py);
+        pz = __fmaf_rn(f, dz, pz);
+        if (POLAR) {
+          const int ip = POLAR ? i : 0;
+          // centre(i) - shell(j)
+          const float cx2 = __fadd_rn(dx, -qd.x), cy2 = __fadd_rn(dy, -qd.y),
+                      cz2 = __fadd_rn(dz, -qd.z);
+          float fc = drude_force_rn<MEASURE>(erd, eru, cx2, cy2, cz2, sgrid, ntab, pp->qcp, e_p);
+          fc = ok ? fc : 0.f;
+          hx[i] = __fmaf_rn(fc, cx2, hx[i]);
+          hy[i] = __fmaf_rn(fc, cy2, hy[i]);
+          hz[i] = __fmaf_rn(fc, cz2, hz[i]);
+          ux = __fmaf_rn(fc, cx2, ux);
+          uy = __fmaf_rn(fc, cy2, uy);
+          uz = __fmaf_rn(fc, cz2, uz);
+          if (MEASURE) pv.add(cx2, cy2, cz2, fc);
+          if (HEAVY) {
+            // shell(i) - centre(j), shell(i) - shell(j)
+            const float4 md = shd[POLAR ? warp : 0][i];
+            const float ex = __fadd_rn(dx, md.x), ey = __fadd_rn(dy, md.y),
+                        ez = __fadd_rn(dz, md.z);
+            float fp = drude_force_rn<MEASURE>(erd, eru, ex, ey, ez, sgrid, ntab, pp->qpc, e_p);
+            const float sx2 = __fadd_rn(ex, -qd.x), sy2 = __fadd_rn(ey, -qd.y),
+                        sz2 = __fadd_rn(ez, -qd.z);
+            float fd = drude_force_rn<MEASURE>(erd, eru, sx2, sy2, sz2, sgrid, ntab, pp->qpp, e_p);
+            fp = ok ? fp : 0.f;
+            fd = ok ? fd : 0.f;
+            gx[ip] = __fmaf_rn(fp, ex, __fmaf_rn(fd, sx2, gx[ip]));
+            gy[ip] = __fmaf_rn(fp, ey, __fmaf_rn(fd, sy2, gy[ip]));
+            gz[ip] = __fmaf_rn(fp, ez, __fmaf_rn(fd, sz2, gz[ip]));
+            px = __fmaf_rn(fp, ex, px);
+            py = __fmaf_rn(fp, ey, py);
+            pz = __fmaf_rn(fp, ez, pz);
+            ux = __fmaf_rn(fd, sx2, ux);
+            uy = __fmaf_rn(fd, sy2, uy);
+            uz = __fmaf_rn(fd, sz2, uz);
+            if (MEASURE) {
+              pv.add(ex, ey, ez, fp);
+              pv.add(sx2, sy2, sz2, fd);
+            }
           }
         }
-      }
+        if (MEASURE) {
+          // energies and virial: no effect on the forces; masked, not
+          // branched around, as the forces are
+          if (HEAVY) {
+            const float xt = rr - P.C2q;
+            const float u = rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
+            e_lj += ok ? u : 0.f;
+            e_vir += ok ? rr * flj : 0.f;
+          }
+          float e_el_p = 0.f;
+          spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
+          e_el += ok ? e_el_p + e_p : 0.f;
+          pv.add(dx, dy, dz, f);
+        }
+      };
+      // the two quads in one block, their eight chains interleaved
+      auto quad = [&](const int k, auto full) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) pair(k + i, full);
+      };
+      if (nh > 4) { quad(0, BoolC<true>()); quad(4, BoolC<true>()); }
+      else if (nh > 0 && ni > 4) { quad(0, BoolC<true>()); quad(4, BoolC<false>()); }
+      else if (nh > 0) quad(0, BoolC<true>());
+      else if (ni > 4) { quad(0, BoolC<false>()); quad(4, BoolC<false>()); }
+      else quad(0, BoolC<false>());
       if (vt) {
-        unsigned long long* fj = facc + 3 * (long)tj;
+        unsigned long long* fj = reinterpret_cast<unsigned long long*>(a.facc) + 3 * (long)tj;
         atomicAdd(fj, (unsigned long long)__float2ll_rn(__fmul_rn(px, -(float)FIX_SCALE)));
         atomicAdd(fj + 1, (unsigned long long)__float2ll_rn(__fmul_rn(py, -(float)FIX_SCALE)));
         atomicAdd(fj + 2, (unsigned long long)__float2ll_rn(__fmul_rn(pz, -(float)FIX_SCALE)));
+        if (POLAR && ((a.shells >> (qw & 255)) & 1)) {
+          fj += 3 * (long)a.ns;
+          atomicAdd(fj, (unsigned long long)__float2ll_rn(__fmul_rn(ux, -(float)FIX_SCALE)));
+          atomicAdd(fj + 1, (unsigned long long)__float2ll_rn(__fmul_rn(uy, -(float)FIX_SCALE)));
+          atomicAdd(fj + 2, (unsigned long long)__float2ll_rn(__fmul_rn(uz, -(float)FIX_SCALE)));
+        }
       }
       if (MEASURE) {
         es[0].add(e_el); es[1].add(e_lj); es[2].add(e_vir);
@@ -1276,93 +1320,172 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? 1 : MG_HALF_T_MINB)
     };
 
     int qh = 0, qn = 0;   // ring head and count (warp-uniform)
-    for (int sp = 0; sp < a.nhspans; sp++) {
-      int col, ra0, ra1, rb0, rb1;
-      half_span_runs(a, sp, cx, cy, cz, col, ra0, ra1, rb0, rb1);
-      for (int part = 0; part < 2; part++) {
-        const int z0 = part ? rb0 : ra0, z1 = part ? rb1 : ra1;
-        if (z1 < z0) continue;
+    for (int sb = 0; sb < a.nhspans; sb += 32) {
+      // the runs of spans sb .. sb + 31, the wrapped parts after the others
+      int ja = 0, la = 0, jw = 0, lw = 0;
+      if (sb + lane < a.nhspans) {
+        int col, ra0, ra1, rb0, rb1;
+        half_span_runs(a, sb + lane, cx, cy, cz, col, ra0, ra1, rb0, rb1);
         // home-cell sites before the group pair with it from their own group
-        const int j0 = max(a.cell_start[col + z0], col + z0 == c ? i0 : 0),
-                  j1 = a.cell_start[col + z1 + 1];
-        for (int jb = j0; jb < j1; jb += 32) {
-          const int j = jb + lane;
-          bool keep = false;
-          float4 f4 = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (j < j1) {
-            const int4 q = pj[j];
-            f4 = make_float4(__fmul_rn((float)(int)((unsigned)q.x - refx), sx),
-                             __fmul_rn((float)(int)((unsigned)q.y - refy), sy),
-                             __fmul_rn((float)(int)((unsigned)q.z - refz), sz),
-                             __int_as_float(q.w));
-            const float ddx = fmaxf(fmaxf(blx - f4.x, f4.x - bhx), 0.f),
-                        ddy = fmaxf(fmaxf(bly - f4.y, f4.y - bhy), 0.f),
-                        ddz = fmaxf(fmaxf(blz - f4.z, f4.z - bhz), 0.f);
-            keep = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz)) < cq;
-          }
-          const unsigned M = __ballot_sync(0xffffffffu, keep);
-          if (keep) {
-            // qn < 32 here, so the new slots never reach the queued ones
-            const int slot = (qh + qn + __popc(M & ((1u << lane) - 1u))) & (HT_RING - 1);
-            sq[warp][slot] = f4;
-            sqt[warp][slot] = j;
-          }
-          qn += __popc(M);
-          __syncwarp();
-          if (qn >= 32) {
-            run(qh, 32);
-            qh = (qh + 32) & (HT_RING - 1);
-            qn -= 32;
-          }
+        ja = max(a.cell_start[col + ra0], col + ra0 == c ? i0 : 0);
+        la = a.cell_start[col + ra1 + 1] - ja;
+        if (rb1 >= rb0) {
+          jw = max(a.cell_start[col + rb0], col + rb0 == c ? i0 : 0);
+          lw = a.cell_start[col + rb1 + 1] - jw;
+        }
+      }
+      auto sum = [&](int v) {   // inclusive prefix over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        return v;
+      };
+      const int pa = sum(la), ta = __shfl_sync(0xffffffffu, pa, 31);
+      const int pw = sum(lw), total = ta + __shfl_sync(0xffffffffu, pw, 31);
+      // this warp's share [k0, k1) of the candidates: each run cut to it
+      const int share = (total + split - 1) / split, k0 = share * part, k1 = k0 + share;
+      auto cut = [&](int& first, int len, int before) {
+        const int lo = min(max(k0 - before, 0), len), hi = min(max(k1 - before, 0), len);
+        first += lo;
+        return hi - lo;
+      };
+      la = cut(ja, la, pa - la);
+      lw = cut(jw, lw, ta + pw - lw);
+      const unsigned ma = __ballot_sync(0xffffffffu, la > 0),
+                     mw = __ballot_sync(0xffffffffu, lw > 0), lt = (1u << lane) - 1u;
+      const int na = __popc(ma), nr = na + __popc(mw);
+      __syncwarp();
+      if (la > 0) runs[warp][__popc(ma & lt)] = make_int2(ja, ja + la);
+      if (lw > 0) runs[warp][na + __popc(mw & lt)] = make_int2(jw, jw + lw);
+      __syncwarp();
+      if (nr == 0) continue;
+      // batches of 32 of each run, loaded one batch ahead
+      int r = 0;
+      int2 u = runs[warp][0];
+      int jn = u.x + lane;
+      bool in = jn < u.y;
+      int4 pn = in ? pj[jn] : make_int4(0, 0, 0, 0);
+      for (bool more = true; more;) {
+        const int j = in ? jn : -1;
+        const int4 p = pn;
+        u.x += 32;
+        if (u.x >= u.y) {
+          r++;
+          more = r < nr;
+          if (more) u = runs[warp][r];
+        }
+        jn = u.x + lane;
+        in = more && jn < u.y;
+        if (in) pn = pj[jn];
+        const float4 f4 = make_float4(__fmul_rn((float)(int)((unsigned)p.x - refx), sx),
+                                      __fmul_rn((float)(int)((unsigned)p.y - refy), sy),
+                                      __fmul_rn((float)(int)((unsigned)p.z - refz), sz),
+                                      __int_as_float(p.w));
+        const float ddx = fmaxf(fmaxf(blx - f4.x, f4.x - bhx), 0.f),
+                    ddy = fmaxf(fmaxf(bly - f4.y, f4.y - bhy), 0.f),
+                    ddz = fmaxf(fmaxf(blz - f4.z, f4.z - bhz), 0.f);
+        const bool keep = j >= 0 && fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz)) < cq;
+        const unsigned M = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          // qn < 32 here, so the new slots never reach the queued ones
+          const int e = (qh + qn + __popc(M & ((1u << lane) - 1u))) & (HT_RING - 1);
+          sq[warp][e] = f4;
+          sqt[warp][e] = j;
+          if (POLAR) sqd[POLAR ? warp : 0][e] = a.pdj[j];
+        }
+        qn += __popc(M);
+        __syncwarp();
+        if (qn >= 32) {
+          run(qh, 32);
+          qh = (qh + 32) & (HT_RING - 1);
+          qn -= 32;
         }
       }
     }
     if (qn > 0) run(qh, qn);
 
-    // the home sites' sums: reduce-scatter of v[3 i + d] (24 values, 8
-    // zero) over the lanes in a fixed order; lane k ends with v[k]
+    // the home sites' sums: lane 3 i + d ends with component d of slot i
+    unsigned long long* facc = reinterpret_cast<unsigned long long*>(a.facc);
+    const int slot_i = min(lane / 3, GS - 1), d = lane % 3;
+    const long at = 3 * (long)(i0 + so[warp][slot_i]) + d;
     float v[32];
 #pragma unroll
-    for (int i = 0; i < GROUP_SITES; i++) {
+    for (int k = 3 * GS; k < 32; k++) v[k] = 0.f;
+#pragma unroll
+    for (int i = 0; i < GS; i++) {
       v[3 * i] = hx[i];
       v[3 * i + 1] = hy[i];
       v[3 * i + 2] = hz[i];
     }
-#pragma unroll
-    for (int k = 3 * GROUP_SITES; k < 32; k++) v[k] = 0.f;
-#pragma unroll
-    for (int w = 16; w >= 1; w >>= 1) {
-      const bool up = (lane & w) != 0;
-#pragma unroll
-      for (int k = 0; k < w; k++) {
-        const float keepv = up ? v[w + k] : v[k], sendv = up ? v[k] : v[w + k];
-        v[k] = __fadd_rn(keepv, __shfl_xor_sync(0xffffffffu, sendv, w));
-      }
-    }
+    reduce_scatter(v, lane);
     if (lane < 3 * ni)
-      atomicAdd(facc + 3 * (long)i0 + lane,
-                (unsigned long long)__float2ll_rn(__fmul_rn(v[0], (float)FIX_SCALE)));
+      atomicAdd(facc + at, (unsigned long long)__float2ll_rn(__fmul_rn(v[0], (float)FIX_SCALE)));
+    if (POLAR && nh > 0) {
+#pragma unroll
+      for (int k = 3 * GS; k < 32; k++) v[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < GS; i++) {
+        const int ip = POLAR ? i : 0;
+        v[3 * i] = gx[ip];
+        v[3 * i + 1] = gy[ip];
+        v[3 * i + 2] = gz[ip];
+      }
+      reduce_scatter(v, lane);
+      if (lane < 3 * nh)
+        atomicAdd(facc + 3 * (long)a.ns + at,
+                  (unsigned long long)__float2ll_rn(__fmul_rn(v[0], (float)FIX_SCALE)));
+    }
   }
   if (MEASURE) {
-    // every unordered pair once; one row per CTA
-    for (int k = 0; k < 9; k++) {
-      ered[threadIdx.x] = es[k].value();
-      __syncthreads();
-      for (int w = NT / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) ered[threadIdx.x] += ered[threadIdx.x + w];
-        __syncthreads();
+    // every unordered pair once; one row per CTA.  The lanes' sums stay
+    // compensated FP32 (lane 9 t + k adds sum k of the lanes of third t): an
+    // FP64 butterfly of nine sums kept the narrow FP64 pipe busy for 21 us on
+    // 864 waters; the warps' sums are added in FP64, in order
+    __shared__ float2 em[NW][32][9];
+    __shared__ double er[NW][27];
+#pragma unroll
+    for (int k = 0; k < 9; k++) em[warp][lane][k] = make_float2(es[k].s, es[k].c);
+    __syncwarp();
+    if (lane < 27) {
+      const int t = lane / 9, k = lane - 9 * t;
+      CSum e;
+      for (int l = 11 * t; l < min(32, 11 * t + 11); l++) {
+        const float2 v = em[warp][l][k];
+        e.add(v.x);
+        e.c += v.y;
       }
-      if (threadIdx.x == 0) a.epart[blockIdx.x * NEN + k] = ered[0];
-      __syncthreads();
+      er[warp][lane] = e.value();
+    }
+    __syncthreads();
+    if (threadIdx.x < 9) {
+      double e = 0;
+#pragma unroll
+      for (int q = 0; q < NW; q++)
+#pragma unroll
+        for (int t = 0; t < 3; t++) e += er[q][9 * t + threadIdx.x];
+      a.epart[bx_ * NEN + threadIdx.x] = e;
     }
   }
+}
+
+template <bool MEASURE, bool POLAR, int NW>
+__global__ void __launch_bounds__(NW * 32, MEASURE ? (POLAR ? 2 : 3) : (POLAR ? 4 : 5))
+    pair_half_mixed_kernel(const __grid_constant__ PairArgs a, const int4* __restrict__ pj,
+                           const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
+                           const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
+                           float sgrid) {
+  pair_half_kernel_body<MEASURE, POLAR, NW>(a, pj, ptab_g, erd, eru, sx, sy, sz, cq, sgrid,
+                                            blockIdx.x);
 }
 
 // the fixed-point sums (sorted order) into the FP64 forces (site order),
 // with shells the second half of each; the sums are cleared for the next
 // evaluation
-__global__ void finish_forces_kernel(int ns, int halves, const int* __restrict__ order,
-                                     long long* __restrict__ facc, double* __restrict__ f) {
+__device__ __forceinline__ void finish_forces(int ns, int halves, const int* __restrict__ order,
+                                              long long* __restrict__ facc,
+                                              double* __restrict__ f) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ns) return;
   const int site = order[t];
@@ -1376,40 +1499,53 @@ __global__ void finish_forces_kernel(int ns, int halves, const int* __restrict__
   }
 }
 
+__global__ void finish_forces_kernel(int ns, int halves, const int* __restrict__ order,
+                                     long long* __restrict__ facc, double* __restrict__ f) {
+  finish_forces(ns, halves, order, facc, f);
+}
+
 cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, const PairF* ptab,
                          const float4* erd, const float4* eru, bool measure, bool polar) {
   int ncell = a.ncx * a.ncy * a.ncz;
   float sx = (float)(a.Lx / 4294967296.0), sy = (float)(a.Ly / 4294967296.0),
         sz = (float)(a.Lz / 4294967296.0);
   const float cq = (float)a.cutoff_sq, sg = (float)a.sgrid, al = (float)a.alpha;
-  const bool rel = !a.allpairs;
-  if (a.group && a.newton && rel) {
+  if (a.small) {
+    const size_t sm = sizeof(PairFS) * (size_t)a.nkind * a.nkind;
+    cudaError_t se = cudaSuccess;
+    // with the static part (22 KB with shells) this may pass 48 KB
+#define PAIR_ALL(M, P)                                                                          \
+  do {                                                                                          \
+    if (sm > 24 * 1024)                                                                         \
+      se = cudaFuncSetAttribute(pair_all_kernel<M, P>,                                          \
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);          \
+    if (se == cudaSuccess)                                                                      \
+      pair_all_kernel<M, P><<<pair_all_blocks(a.ns), ALL_WARPS * 32, sm, L.s>>>(                \
+          a, pj, ptab, erd, eru, sx, sy, sz, cq, sg);                                           \
+  } while (0)
+    if (polar) { if (measure) PAIR_ALL(true, true); else PAIR_ALL(false, true); }
+    else { if (measure) PAIR_ALL(true, false); else PAIR_ALL(false, false); }
+#undef PAIR_ALL
+    if (se != cudaSuccess) return se;
+    LAUNCHED(L);
+    return cudaGetLastError();
+  }
+  if (a.group && a.newton) {
     const size_t gsm = sizeof(PairFS) * (size_t)a.nkind * a.nkind;
     cudaError_t ge = cudaSuccess;
+    // with the static part (up to 23 KB) this may pass 48 KB
 #define PAIR_HALF(M, P)                                                                         \
   do {                                                                                          \
-    if (gsm > 48 * 1024)                                                                        \
+    if (gsm > 24 * 1024)                                                                        \
       ge = cudaFuncSetAttribute(pair_half_mixed_kernel<M, P, GROUP_WARPS>,                     \
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm);         \
     if (ge == cudaSuccess)                                                                      \
-      pair_half_mixed_kernel<M, P, GROUP_WARPS><<<a.ngrid, GROUP_WARPS * 32, gsm, L.s>>>(      \
-          a, pj, ptab, erd, eru, sx, sy, sz, cq, sg);                                           \
+      pair_half_mixed_kernel<M, P, GROUP_WARPS>                                                 \
+          <<<a.ngrid * a.split, GROUP_WARPS * 32, gsm, L.s>>>(a, pj, ptab, erd, eru, sx, sy, sz, \
+                                                              cq, sg);                          \
   } while (0)
-#define PAIR_HALF_T(M)                                                                          \
-  do {                                                                                          \
-    if (gsm > 48 * 1024)                                                                        \
-      ge = cudaFuncSetAttribute(pair_half_t_mixed_kernel<M, GROUP_WARPS>,                      \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm);         \
-    if (ge == cudaSuccess)                                                                      \
-      pair_half_t_mixed_kernel<M, GROUP_WARPS><<<a.ngrid, GROUP_WARPS * 32, gsm, L.s>>>(       \
-          a, pj, ptab, erd, eru, sx, sy, sz, cq, sg);                                           \
-  } while (0)
-    // lanes on the neighbours (newton 2) without shells; with shells the
-    // lane-per-home kernel
     if (polar) { if (measure) PAIR_HALF(true, true); else PAIR_HALF(false, true); }
-    else if (a.newton == 2) { if (measure) PAIR_HALF_T(true); else PAIR_HALF_T(false); }
     else { if (measure) PAIR_HALF(true, false); else PAIR_HALF(false, false); }
-#undef PAIR_HALF_T
 #undef PAIR_HALF
     if (ge != cudaSuccess) return ge;
     LAUNCHED(L);
@@ -1418,7 +1554,7 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
     LAUNCHED(L);
     return cudaGetLastError();
   }
-  if (a.group && rel) {
+  if (a.group) {
     const size_t gsm = sizeof(PairFS) * (size_t)a.nkind * a.nkind;
     cudaError_t ge = cudaSuccess;
 #define PAIR_GROUP(M, P)                                                                        \
@@ -1446,35 +1582,30 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
   const size_t dsm = sizeof(PairFS) * (size_t)a.nkind * a.nkind +
                      (stab ? sizeof(float4) * (size_t)a.ntab : 0);
   cudaError_t e = cudaSuccess;
-#define PAIR_MIXED(M, P, R, W, S)                                                               \
+#define PAIR_MIXED(M, P, W, S)                                                                  \
   do {                                                                                          \
     if (dsm > 48 * 1024)                                                                        \
-      e = cudaFuncSetAttribute(pair_mixed_kernel<M, P, R, W, S>,                                \
+      e = cudaFuncSetAttribute(pair_mixed_kernel<M, P, W, S>,                                   \
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);          \
     if (e == cudaSuccess)                                                                       \
-      pair_mixed_kernel<M, P, R, W, S><<<ncell, W * 32, dsm, L.s>>>(a, pj, ptab, erd, eru, sx,  \
-                                                                     sy, sz, cq, sg, al);       \
+      pair_mixed_kernel<M, P, W, S><<<ncell, W * 32, dsm, L.s>>>(a, pj, ptab, erd, eru, sx, sy, \
+                                                                 sz, cq, sg, al);               \
   } while (0)
-#define PAIR_MIXED_W(M, P, R)                              \
-  do {                                                     \
-    if (nw == 16) {                                        \
-      if (stab) PAIR_MIXED(M, P, R, 16, true);             \
-      else PAIR_MIXED(M, P, R, 16, false);                 \
-    } else if (nw == 8) {                                  \
-      if (stab) PAIR_MIXED(M, P, R, 8, true);              \
-      else PAIR_MIXED(M, P, R, 8, false);                  \
-    } else {                                               \
-      if (stab) PAIR_MIXED(M, P, R, 4, true);              \
-      else PAIR_MIXED(M, P, R, 4, false);                  \
-    }                                                      \
+#define PAIR_MIXED_W(M, P)                              \
+  do {                                                  \
+    if (nw == 16) {                                     \
+      if (stab) PAIR_MIXED(M, P, 16, true);             \
+      else PAIR_MIXED(M, P, 16, false);                 \
+    } else if (nw == 8) {                               \
+      if (stab) PAIR_MIXED(M, P, 8, true);              \
+      else PAIR_MIXED(M, P, 8, false);                  \
+    } else {                                            \
+      if (stab) PAIR_MIXED(M, P, 4, true);              \
+      else PAIR_MIXED(M, P, 4, false);                  \
+    }                                                   \
   } while (0)
-  if (polar) {
-    if (measure) { if (rel) PAIR_MIXED_W(true, true, true); else PAIR_MIXED_W(true, true, false); }
-    else { if (rel) PAIR_MIXED_W(false, true, true); else PAIR_MIXED_W(false, true, false); }
-  } else {
-    if (measure) { if (rel) PAIR_MIXED_W(true, false, true); else PAIR_MIXED_W(true, false, false); }
-    else { if (rel) PAIR_MIXED_W(false, false, true); else PAIR_MIXED_W(false, false, false); }
-  }
+  if (polar) { if (measure) PAIR_MIXED_W(true, true); else PAIR_MIXED_W(false, true); }
+  else { if (measure) PAIR_MIXED_W(true, false); else PAIR_MIXED_W(false, false); }
 #undef PAIR_MIXED_W
 #undef PAIR_MIXED
   if (e != cudaSuccess) return e;
@@ -1495,9 +1626,13 @@ __global__ void __launch_bounds__(PAIR_THREADS)
   const int nk = a.nkind, ntab = a.ntab;
   for (int t = threadIdx.x; t < nk * nk; t += PAIR_THREADS) ptab[t] = ptab_g[t];
   __syncthreads();
-  const int c = blockIdx.x;
+  // one cell (all pairs): the CTA takes 32 sites, its warps batches of all
+  // sites in turn; else the sites of its cell, the warps the stencil
+  const bool one = a.allpairs != 0;
+  const int c = one ? 0 : blockIdx.x;
   const int cz = c % a.ncz, cy = (c / a.ncz) % a.ncy, cx = c / (a.ncy * a.ncz);
-  const int i0 = a.cell_start[c], ni = a.cell_start[c + 1] - i0;
+  const int i0 = one ? 32 * (int)blockIdx.x : a.cell_start[c],
+            ni = (one ? min(a.ns, i0 + 32) : a.cell_start[c + 1]) - i0;
   const double cq = a.cutoff_sq, sgrid = a.sgrid, alpha = a.alpha;
   double en[NEN];
 #pragma unroll
@@ -1510,7 +1645,7 @@ __global__ void __launch_bounds__(PAIR_THREADS)
     const long long wi = __double_as_longlong(me.w);
     const int kind_i = (int)(wi & 255), mol_i = (int)(wi >> 8);
     double fx = 0, fy = 0, fz = 0, gx = 0, gy = 0, gz = 0;
-    for (int s = warp; s < a.nstencil; s += NWARP) {
+    for (int s = one ? 0 : warp; s < a.nstencil; s += NWARP) {
       const int4 o = a.stencil[s];
       int x2 = cx + o.x, y2 = cy + o.y, z2 = cz + o.z;
       double shx = 0, shy = 0, shz = 0;
@@ -1520,7 +1655,7 @@ __global__ void __launch_bounds__(PAIR_THREADS)
       const double xs = me.x - shx, ys = me.y - shy, zs = me.z - shz;
       const int c2 = (x2 * a.ncy + y2) * a.ncz + z2;
       const int j0 = a.cell_start[c2], nj = a.cell_start[c2 + 1] - j0;
-      for (int jb = 0; jb < nj; jb += 32) {
+      for (int jb = one ? 32 * warp : 0; jb < nj; jb += one ? 32 * NWARP : 32) {
         if (jb + lane < nj) {
           sj[warp][lane] = pd[j0 + jb + lane];
           if (POLAR) sjd[warp][lane] = a.pdd[j0 + jb + lane];
@@ -1744,7 +1879,8 @@ cudaError_t k_excl_mixed(const Launch& L, const ExclArgs& a, bool measure, bool 
 
 cudaError_t k_pair_fp64(const Launch& L, const PairArgs& a, const double4* pd, const PairD* ptab,
                         const double* ertab, bool measure, bool polar) {
-  int ncell = a.ncx * a.ncy * a.ncz;
+  // one cell: a CTA per 32 sites
+  const int ncell = a.allpairs ? cdiv(a.ns, 32) : a.ncx * a.ncy * a.ncz;
   if (polar) {
     if (measure)
       pair_fp64_kernel<true, true><<<ncell, PAIR_THREADS, 0, L.s>>>(a, pd, ptab, ertab);
@@ -2636,6 +2772,7 @@ namespace mg {
 
 int cell_site_blocks(int ns) { return cdiv(ns, 256); }
 int cell_order_blocks(int ncell) { return cdiv(ncell, ORDER_THREADS / 32); }
+int pair_all_blocks(int ns) { return cdiv(ns, ALL_SITES); }
 
 __global__ void batch_cell_count_kernel(const BoxStep* __restrict__ B) {
   const BoxStep& e = B[blockIdx.y];
@@ -2663,12 +2800,25 @@ __global__ void __launch_bounds__(ORDER_THREADS) batch_cell_order_kernel(const B
 }
 
 template <bool MEASURE>
-__global__ void __launch_bounds__(4 * 32) batch_pair_kernel(const BoxStep* __restrict__ B) {
+__global__ void __launch_bounds__(GROUP_WARPS * 32, MEASURE ? 4 : 6)
+    batch_pair_half_kernel(const BoxStep* __restrict__ B) {
   const BoxStep& e = B[blockIdx.y];
-  if ((int)blockIdx.x >= e.g_pair) return;
-  pair_mixed_kernel_body<MEASURE, false, true, 4, false>(e.pa, e.pj, e.ptab, e.erd, e.eru, e.sx,
-                                                         e.sy, e.sz, e.cq, e.sg, e.al,
-                                                         blockIdx.x, 0);
+  if ((int)blockIdx.x >= e.g_half) return;
+  pair_half_kernel_body<MEASURE, false, GROUP_WARPS>(e.pa, e.pj, e.ptab, e.erd, e.eru, e.sx, e.sy,
+                                                     e.sz, e.cq, e.sg, blockIdx.x);
+}
+
+__global__ void batch_finish_kernel(const BoxStep* __restrict__ B) {
+  const BoxStep& e = B[blockIdx.y];
+  if (e.g_half > 0) finish_forces(e.ns, 1, e.pa.order, e.pa.facc, e.pa.f);
+}
+
+template <bool MEASURE>
+__global__ void __launch_bounds__(ALL_WARPS * 32, 2) batch_pair_all_kernel(const BoxStep* __restrict__ B) {
+  const BoxStep& e = B[blockIdx.y];
+  if ((int)blockIdx.x >= e.g_all) return;
+  pair_all_kernel_body<MEASURE, false>(e.pa, e.pj, e.ptab, e.erd, e.eru, e.sx, e.sy, e.sz, e.cq,
+                                       e.sg, blockIdx.x);
 }
 
 template <bool MEASURE>
@@ -2735,23 +2885,29 @@ cudaError_t k_batch_cells(const Launch& L, const BoxStep* d, int nbox, const Bat
 cudaError_t k_batch_pairs(const Launch& L, const BoxStep* d, int nbox, const BatchGrid& g,
                           bool measure) {
   cudaError_t e = cudaSuccess;
-  if (measure) {
-    if (g.pair_smem > 48 * 1024)
-      e = cudaFuncSetAttribute(batch_pair_kernel<true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pair_smem);
-    if (e == cudaSuccess)
-      batch_pair_kernel<true><<<dim3(g.pair, nbox), 128, g.pair_smem, L.s>>>(d);
-    if (g.excl > 0) batch_excl_kernel<true><<<dim3(g.excl, nbox), EXCL_THREADS, 0, L.s>>>(d);
-  } else {
-    if (g.pair_smem > 48 * 1024)
-      e = cudaFuncSetAttribute(batch_pair_kernel<false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pair_smem);
-    if (e == cudaSuccess)
-      batch_pair_kernel<false><<<dim3(g.pair, nbox), 128, g.pair_smem, L.s>>>(d);
-    if (g.excl > 0) batch_excl_kernel<false><<<dim3(g.excl, nbox), EXCL_THREADS, 0, L.s>>>(d);
-  }
-  if (e != cudaSuccess) return e;
-  *L.counter += 1 + (g.excl > 0 ? 1 : 0);
+  // the boxes of the half-shell kernel, those of the all-pairs kernel, the
+  // exclusions
+#define BATCH_PAIRS(M)                                                                          \
+  do {                                                                                          \
+    if (g.half > 0 && g.pair_smem > 24 * 1024)                                                  \
+      e = cudaFuncSetAttribute(batch_pair_half_kernel<M>,                                       \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pair_smem);  \
+    if (e == cudaSuccess && g.all > 0 && g.pair_smem > 24 * 1024)                               \
+      e = cudaFuncSetAttribute(batch_pair_all_kernel<M>,                                        \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pair_smem);  \
+    if (e != cudaSuccess) return e;                                                             \
+    if (g.half > 0) {                                                                           \
+      batch_pair_half_kernel<M><<<dim3(g.half, nbox), GROUP_WARPS * 32, g.pair_smem, L.s>>>(d); \
+      batch_finish_kernel<<<dim3(g.site, nbox), 256, 0, L.s>>>(d);                              \
+    }                                                                                           \
+    if (g.all > 0)                                                                              \
+      batch_pair_all_kernel<M><<<dim3(g.all, nbox), ALL_WARPS * 32, g.pair_smem, L.s>>>(d);     \
+    if (g.excl > 0) batch_excl_kernel<M><<<dim3(g.excl, nbox), EXCL_THREADS, 0, L.s>>>(d);      \
+  } while (0)
+  if (measure) BATCH_PAIRS(true);
+  else BATCH_PAIRS(false);
+#undef BATCH_PAIRS
+  *L.counter += (g.half > 0 ? 2 : 0) + (g.all > 0 ? 1 : 0) + (g.excl > 0 ? 1 : 0);
   // the FP32-core phase rows (none when every box is on the tensor cores)
   if (g.charge > 0) {
     batch_charge_fixed_kernel<<<dim3(g.charge, nbox), 256, 0, L.s>>>(d);

@@ -117,6 +117,12 @@ struct mg_ctx {
   int* d_mol_cfirst = nullptr;
   int2* d_cons = nullptr;
   double *d_bondq = nullptr, *d_imass = nullptr, *d_mass = nullptr;
+  // three-site tables of SHAKE (ShakeArgs) and of the exclusions (ExclArgs)
+  unsigned char* d_kind3 = nullptr;
+  double* d_ctab = nullptr;
+  float4* d_ftab = nullptr;
+  int* d_xbase3 = nullptr;
+  cudaEvent_t ev_draw0 = nullptr, ev_draw = nullptr;   // Bussi draws beside the step
   double* d_kinpart = nullptr;
   double* d_meas = nullptr;  // [nblocks * 13] constraint virial and kinetic tensor sums
   int* d_status = nullptr;
@@ -464,6 +470,8 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   CK(cudaStreamCreateWithFlags(&ctx->kstream, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ctx->ev_draw0, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ctx->ev_draw, cudaEventDisableTiming));
   const int ns = t->ns;
 
   // ---- site kinds: distinct (LJ type, charge, Drude charge) combinations
@@ -942,6 +950,17 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
         }
       xfirst[n + 1] = (int)xpair.size();
     }
+    std::vector<int> base3(t->nmol, -1);
+    for (int n = 0; n < t->nmol; n++) {
+      const int p = xfirst[n];
+      if (xfirst[n + 1] - p != 3) continue;
+      const int b = xpair[p].x;
+      if (xpair[p].y == b + 1 && xpair[p + 1].x == b && xpair[p + 1].y == b + 2 &&
+          xpair[p + 2].x == b + 1 && xpair[p + 2].y == b + 2 && xq[p].x != 0 && xq[p + 1].x != 0 &&
+          xq[p + 2].x != 0)
+        base3[n] = b;
+    }
+    CK(upload(&ctx->d_xbase3, base3.data(), base3.size()));
     CK(upload(&ctx->d_xfirst, xfirst.data(), xfirst.size()));
     CK(upload(&ctx->d_xpair, xpair.data(), xpair.size()));
     CK(upload(&ctx->d_xq, xq.data(), xq.size()));
@@ -949,10 +968,51 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   CK(upload(&ctx->d_mol_cfirst, mcf.data(), mcf.size()));
   CK(upload(&ctx->d_cons, cons.data(), cons.size()));
   CK(upload(&ctx->d_bondq, bondq.data(), bondq.size()));
+  {
+    // per constraint factors of the three-site sweeps, and which molecules
+    // run them
+    std::vector<double> ct(6 * (size_t)std::max(ctx->nc, 0));
+    std::vector<float> ft(8 * (size_t)std::max(ctx->nc, 0), 0.f);
+    for (int c = 0; c < ctx->nc; c++) {
+      const double bq = bondq[c], mi = imass[cons[c].x], mj = imass[cons[c].y];
+      const double wq = ctx->omega / (mi + mj) * (1.0 / bq);
+      double* q = &ct[6 * (size_t)c];
+      q[0] = bq;
+      q[1] = ctx->epsc * bq;
+      q[2] = mi * wq;
+      q[3] = -(mj * wq);
+      q[4] = ctx->omega / (mi + mj);
+      q[5] = q[4] / bq;
+      float* f = &ft[8 * (size_t)c];
+      f[0] = (float)bq;
+      f[1] = (float)(bq - (double)f[0]);
+      f[2] = (float)q[1];
+      f[3] = (float)q[2];
+      f[4] = (float)q[3];
+    }
+    std::vector<unsigned char> k3(t->nmol, 0);
+    for (int n = 0; n < t->nmol; n++) {
+      const int i0 = t->mol_first[n], i1 = t->mol_first[n + 1], c0 = mcf[n];
+      if (i1 - i0 < 3 || mcf[n + 1] - c0 != 3) continue;
+      bool first3 = true, order = true, tail = true;
+      const int ci[3] = {0, 0, 1}, cj[3] = {1, 2, 2};
+      for (int q = 0; q < 3; q++) {
+        const int x = cons[c0 + q].x - i0, y = cons[c0 + q].y - i0;
+        first3 = first3 && x >= 0 && x < 3 && y >= 0 && y < 3;
+        order = order && x == ci[q] && y == cj[q];
+      }
+      for (int i = i0 + 3; i < i1; i++) tail = tail && mass[i] == 0;
+      if (first3 && order && tail) k3[n] = 1;
+      else if (first3 && i1 - i0 == 3) k3[n] = 2;
+    }
+    CK(upload(&ctx->d_ctab, ct.data(), ct.size()));
+    CK(upload((float**)&ctx->d_ftab, ft.data(), ft.size()));
+    CK(upload(&ctx->d_kind3, k3.data(), k3.size()));
+  }
   CK(upload(&ctx->d_imass, imass.data(), ns));
   CK(upload(&ctx->d_mass, mass.data(), ns));
-  CK(dalloc(&ctx->d_kinpart, (size_t)(t->nmol + 127) / 128 + 1));
-  CK(dalloc(&ctx->d_meas, 13 * ((size_t)(t->nmol + 127) / 128 + 1)));
+  CK(dalloc(&ctx->d_kinpart, (size_t)shake_blocks(t->nmol) + 1));
+  CK(dalloc(&ctx->d_meas, 13 * ((size_t)shake_blocks(t->nmol) + 1)));
   // dependants: parents and dependants of one molecule, consecutive per
   // molecule, no dependant a parent, weights summing to 1 (cook fixes
   // other sums with a warning, cook/simdef.c:390)
@@ -1006,7 +1066,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   // momentum (sim/siminit.c:518-530)
   ctx->thermo_f = p->thermo_f > 0 ? p->thermo_f : 3.0 * (ns - t->ndep) - t->nc - 3;
   ctx->nchi = 2 * PARTITION_SMS;
-  CK(dalloc(&ctx->d_chi, (size_t)ctx->nchi));
+  CK(dalloc(&ctx->d_chi, (size_t)ctx->nchi + 1));
   CK(dalloc(&ctx->d_zth, 1));
   CK(dalloc(&ctx->d_step, 1));
   CK(cudaMemset(ctx->d_step, 0, sizeof(long long)));
@@ -1181,6 +1241,7 @@ ExclArgs excl_args(mg_ctx* ctx, const double* r_dev, double* f) {
   ExclArgs a;
   a.nmol = ctx->nmol;
   a.ns = ctx->ns;
+  a.base3 = ctx->d_xbase3;
   a.xfirst = ctx->d_xfirst;
   a.xpair = ctx->d_xpair;
   a.xq = ctx->d_xq;
@@ -1419,10 +1480,12 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
                                   f_dev));
   ctx->have_cells = true;
   if (measure) {
-    PROF("reduce", k_reduce_sum(L, ctx->d_epart, nerows, 10, ctx->d_sums));
     if (ctx->nq > 0)
-      PROF("reduce", k_reduce_sum(L, ctx->d_ekpart, ctx->nf ? NF_CS * (ctx->Kx + 1) : ctx->nkblocks, 7,
+      PROF("reduce", k_reduce_two(L, ctx->d_epart, nerows, 10, ctx->d_sums, ctx->d_ekpart,
+                                  ctx->nf ? NF_CS * (ctx->Kx + 1) : ctx->nkblocks, 7,
                                   ctx->d_sums + 10));
+    else
+      PROF("reduce", k_reduce_sum(L, ctx->d_epart, nerows, 10, ctx->d_sums));
   }
   return MG_OK;
 }
@@ -1526,6 +1589,9 @@ ShakeArgs shake_args(mg_ctx* ctx, bool measure) {
   ShakeArgs sa;
   sa.meas_part = measure ? ctx->d_meas : nullptr;
   sa.nmol = ctx->nmol;
+  sa.kind3 = ctx->d_kind3;
+  sa.ctab = ctx->d_ctab;
+  sa.ftab = ctx->d_ftab;
   sa.mol_first = ctx->d_mol_first;
   sa.mol_cfirst = ctx->d_mol_cfirst;
   sa.cons = ctx->d_cons;
@@ -1591,7 +1657,7 @@ ThermoArgs thermo_args(mg_ctx* ctx) {
   ThermoArgs t;
   t.kind = ctx->thermostat;
   t.ns = ctx->ns;
-  t.nkin = (ctx->nmol + 127) / 128;
+  t.nkin = shake_blocks(ctx->nmol);
   t.nchi = ctx->nchi;
   t.nf = ctx->thermo_f;
   t.T = ctx->T;
@@ -1605,21 +1671,47 @@ ThermoArgs thermo_args(mg_ctx* ctx) {
   return t;
 }
 
+// the Bussi thermostat's draws of the step on the k-space stream, beside SHAKE
+// (they need nothing of the step: 9 us on 12544 sites that the step does not
+// wait for); thermostat_join waits for them
+int thermostat_fork(mg_ctx* ctx) {
+  if (ctx->thermostat != 2) return MG_OK;
+  cudaStream_t ks = ctx->overlap ? ctx->kstream : ctx->stream;
+  if (ctx->overlap) {
+    CK(cudaEventRecord(ctx->ev_draw0, ctx->stream));
+    CK(cudaStreamWaitEvent(ks, ctx->ev_draw0, 0));
+  }
+  Launch LK{ks, &ctx->launches};
+  PROFS("thermostat", ks, k_bussi_draw(LK, thermo_args(ctx), ctx->d_chi));
+  if (ctx->overlap) CK(cudaEventRecord(ctx->ev_draw, ks));
+  return MG_OK;
+}
+int thermostat_join(mg_ctx* ctx) {
+  Launch L = launch(ctx);
+  if (ctx->thermostat == 2 && ctx->overlap) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_draw, 0));
+  PROF("thermostat", k_thermostat(L, thermo_args(ctx), ctx->d_kinpart, ctx->d_chi, ctx->d_r1));
+  return MG_OK;
+}
+
 // one leap-frog + SHAKE step of a non-polar box with cells re-binned at the
 // force evaluation: kernels only, no host synchronisation (graph capture)
 int md_step_enqueue(mg_ctx* ctx, bool measure) {
   Launch L = launch(ctx);
   int rc = forces_async(ctx, ctx->d_r, ctx->d_f, measure);
   if (rc) return rc;
+  rc = thermostat_fork(ctx);
+  if (rc) return rc;
   CK(depend_f_enqueue(ctx, L, measure));
   CK(k_shake(L, shake_args(ctx, measure)));
   CK(k_depend_r(L, depend_args(ctx), ctx->d_r));
   if (measure) {
-    CK(k_reduce_sum(L, ctx->d_kinpart, (ctx->nmol + 127) / 128, 1, ctx->d_sums + 17));
-    CK(k_reduce_sum(L, ctx->d_meas, (ctx->nmol + 127) / 128, 13, ctx->d_sums + 32));
+    CK(k_reduce_two(L, ctx->d_kinpart, shake_blocks(ctx->nmol), 1, ctx->d_sums + 17, ctx->d_meas,
+                    shake_blocks(ctx->nmol), 13, ctx->d_sums + 32));
   }
-  if (ctx->thermostat)
-    CK(k_thermostat(L, thermo_args(ctx), ctx->d_kinpart, ctx->d_chi, ctx->d_r1));
+  if (ctx->thermostat) {
+    rc = thermostat_join(ctx);
+    if (rc) return rc;
+  }
   if (ctx->drmax > 0) CK(k_bounddr(L, ctx->ns, ctx->drmax, ctx->d_r1, ctx->d_bdrep));
   if (ctx->drift_step)
     CK(k_remove_drift(L, ctx->ns, ctx->d_mass, ctx->total_mass, ctx->d_r1, ctx->d_driftpart,
@@ -1661,7 +1753,7 @@ int check_status(mg_ctx* ctx) {
 // the steps kernel by kernel (Drude boxes, neighbour lists, profiling)
 int md_steps_launched(mg_ctx* ctx, int nsteps, mg_energy* en) {
   Launch L = launch(ctx);
-  const int nkin = (ctx->nmol + 127) / 128;
+  const int nkin = shake_blocks(ctx->nmol);
   for (int s = 0; s < nsteps; s++) {
     const bool last = s == nsteps - 1;
     const bool measure = last && en != nullptr;
@@ -1705,6 +1797,10 @@ int md_steps_launched(mg_ctx* ctx, int nsteps, mg_energy* en) {
       int rc = forces_async(ctx, ctx->d_r, ctx->d_f, measure);
       if (rc) return rc;
     }
+    {
+      int rc = thermostat_fork(ctx);
+      if (rc) return rc;
+    }
     // forces on dependants to their parents (sim/constrd.c:747), the step,
     // and dependant positions for the next force evaluation: the same
     // positions cook's depend_r makes at the start of its next step
@@ -1722,11 +1818,13 @@ int md_steps_launched(mg_ctx* ctx, int nsteps, mg_energy* en) {
       ctx->dmax_pending = true;
     }
     if (measure) {
-      PROF("reduce", k_reduce_sum(L, ctx->d_kinpart, nkin, 1, ctx->d_sums + 17));
-      PROF("reduce", k_reduce_sum(L, ctx->d_meas, nkin, 13, ctx->d_sums + 32));
+      PROF("reduce", k_reduce_two(L, ctx->d_kinpart, nkin, 1, ctx->d_sums + 17, ctx->d_meas, nkin,
+                                  13, ctx->d_sums + 32));
     }
-    if (ctx->thermostat)
-      PROF("thermostat", k_thermostat(L, thermo_args(ctx), ctx->d_kinpart, ctx->d_chi, ctx->d_r1));
+    if (ctx->thermostat) {
+      int rc = thermostat_join(ctx);
+      if (rc) return rc;
+    }
     // cook calls bounddr after Shake (and its thermostat) and normalize
     // (sim/main.c:1607-1623)
     if (ctx->drmax > 0)
@@ -1807,6 +1905,7 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_mol,    ctx->d_key,     ctx->d_pfix,   ctx->d_idx,   ctx->d_key_s,  ctx->d_order,
                   ctx->d_cell_start, ctx->d_ccount, ctx->d_ccursor, ctx->d_spans, ctx->d_gstart,
                   ctx->d_hspans, ctx->d_facc, ctx->d_tcb, ctx->d_nf, ctx->d_nfmem, ctx->d_far,
+                  ctx->d_kind3, ctx->d_ctab, ctx->d_ftab, ctx->d_xbase3,
                   ctx->d_gcell, ctx->d_pj, ctx->d_pd,  ctx->d_stencil,
                   ctx->d_ptabf,  ctx->d_ptabd,   ctx->d_erd,   ctx->d_eru,    ctx->d_ert,
                   ctx->d_epart,  ctx->d_qsite,   ctx->d_qval,  ctx->d_task,   ctx->d_col,
@@ -1836,6 +1935,8 @@ int mg_destroy(mg_ctx* ctx) {
   if (ctx->kstream) cudaStreamDestroy(ctx->kstream);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  if (ctx->ev_draw0) cudaEventDestroy(ctx->ev_draw0);
+  if (ctx->ev_draw) cudaEventDestroy(ctx->ev_draw);
   delete ctx;
   return MG_OK;
 }
@@ -2880,7 +2981,7 @@ int build_fused(mg_batch* b) {
     e.qf = c->d_qfix;
     e.part = (float2*)c->d_part;
     e.sa = shake_args(c, true);
-    const int nkin = (c->nmol + 127) / 128;
+    const int nkin = shake_blocks(c->nmol);
     e.rpart[0] = c->d_epart;
     e.rrows[0] = c->nprows + c->nxblocks;
     e.rwidth[0] = 10;
@@ -2908,7 +3009,7 @@ int build_fused(mg_batch* b) {
     e.g_p1y = c->nchunk;
     e.g_skr = (c->nk + 255) / 256;
     e.g_kf = kf_mixed_blocks(c->nq);
-    e.g_shake = (c->nmol + 127) / 128;
+    e.g_shake = shake_blocks(c->nmol);
     TcBox& t = tc[i];
     if (c->nf) {
       // non-uniform transforms, with the arguments of the box's single

@@ -221,6 +221,8 @@ cudaError_t k_sk_gemm_fp64(const Launch& L, const KArgs& a, const double2* tab, 
 cudaError_t k_kf_gemm_mixed(const Launch& L, const KArgs& a, const float2* tab);
 cudaError_t k_kf_gemm_fp64(const Launch& L, const KArgs& a, const double2* tab);
 cudaError_t k_reduce_sum(const Launch& L, const double* part, int nrows, int width, double* out);
+cudaError_t k_reduce_two(const Launch& L, const double* pa, int ra, int wa, double* oa,
+                         const double* pb, int rb, int wb, double* ob);
 // the dipole term of Ewald(2): M = sum q r into M[0..2] (part: [dipole_blocks(nq) * 3]
 // scratch), then forces q (-c_d M_d) added to f (none when c is zero)
 int dipole_blocks(int nq);
@@ -304,8 +306,19 @@ cudaError_t k_batch_sk_tc(const Launch& L, const TcBox* d, int nbox, int grid, s
 cudaError_t k_batch_kf_tc(const Launch& L, const TcBox* d, int nbox, int gvb, int gkf,
                           size_t smem);
 
+constexpr int SHAKE_THREADS = 32;
+int shake_blocks(int nmol);
 struct ShakeArgs {
   int nmol;
+  // per molecule: 1 three constraints (0,1), (0,2), (1,2) over its first three
+  // sites, further sites massless and unconstrained; 2 other three over those
+  // (exactly three sites); 0 anything else
+  const unsigned char* kind3;
+  // per constraint: {b^2, eps b^2, m_i^-1 w, -m_j^-1 w, omega/(m_i^-1 +
+  // m_j^-1), that / b^2} with w the last; and as floats {b^2 hi, lo, eps b^2,
+  // m_i^-1 w, -m_j^-1 w, 0, 0, 0}
+  const double* ctab;
+  const float4* ftab;
   const int* mol_first;
   const int* mol_cfirst;
   const int2* cons;
@@ -351,6 +364,8 @@ constexpr int MG_NOSE_MAXPRED = 8;
 // molecule (mixed cell path: the pair kernel skips these pairs)
 struct ExclArgs {
   int nmol, ns;
+  const int* base3;     // [nmol] first of three consecutive sites that the
+                        // molecule's three pairs (0,1), (0,2), (1,2) join, or -1
   const int* xfirst;    // [nmol+1] pair range of each molecule
   const int2* xpair;    // (i, j), i < j, sites of one molecule
   const double4* xq;    // charge products: centre-centre, Drude(i)-centre(j),
@@ -361,7 +376,7 @@ struct ExclArgs {
   double* f;            // forces, added to
   double* epart;        // [nblocks * 10] energy rows (measure)
 };
-constexpr int EXCL_THREADS = 128;
+constexpr int EXCL_THREADS = 32;
 cudaError_t k_excl_mixed(const Launch& L, const ExclArgs& a, bool measure, bool polar);
 
 // ---- batches: one launch per kernel over all boxes ----
@@ -528,8 +543,11 @@ cudaError_t k_bounddr(const Launch& L, int ns, double drmax, double* r1, unsigne
 int drift_blocks(int ns);
 cudaError_t k_remove_drift(const Launch& L, int ns, const double* mass, double total_mass,
                            double* r1, double* part, double* P, double* vout);
+// the Bussi thermostat's random numbers of the step into chi_part [nchi + 1];
+// they depend on nothing else of the step
+cudaError_t k_bussi_draw(const Launch& L, const ThermoArgs& a, double* chi_part);
 cudaError_t k_thermostat(const Launch& L, const ThermoArgs& a, const double* kin_part,
-                         double* chi_part, double* r1);
+                         const double* chi_part, double* r1);
 
 // adjoint constants of one pair of site kinds (FP64)
 struct AdjPair {

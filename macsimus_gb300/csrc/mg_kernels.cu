@@ -1802,14 +1802,47 @@ __device__ __forceinline__ double near_img(double d, double L, double iL) {
   return d - L * rint(d * iL);
 }
 
+// A warp per CTA (a molecule's pairs are one chain of loads and FP64 products,
+// so the molecules spread over the SMs); rigid three-site molecules keep their
+// sites in registers.  864 waters 9.0 -> 6.2 us, measured 15 -> 8.5 us.
 template <bool MEASURE, bool POLAR>
 MG_BODY void excl_mixed_kernel_body(const ExclArgs& a,
     const int bx_,
     const int by_) {
-  __shared__ double red[EXCL_THREADS];
+  static_assert(EXCL_THREADS == 32, "one warp per CTA");
   const int n = bx_ * EXCL_THREADS + threadIdx.x;
   double en[7] = {0, 0, 0, 0, 0, 0, 0};
   if (n < a.nmol) {
+    const int b = POLAR ? -1 : a.base3[n];
+    if (b >= 0) {
+      // the three pairs (0,1), (0,2), (1,2) of sites b, b+1, b+2: positions and
+      // forces read once, the same additions in the same order
+      double x[3][3], F[3][3];
+      const double* r = a.r + 3 * (long)b;
+      double* f = a.f + 3 * (long)b;
+#pragma unroll
+      for (int s = 0; s < 3; s++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          x[s][d] = r[3 * s + d];
+          F[s][d] = f[3 * s + d];
+        }
+      const int p0 = a.xfirst[n];
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        const int i = p == 2 ? 1 : 0, j = p == 0 ? 1 : 2;
+        const double q = a.xq[p0 + p].x;
+        const double dx = near_img(x[i][0] - x[j][0], a.Lx, a.iLx),
+                     dy = near_img(x[i][1] - x[j][1], a.Ly, a.iLy),
+                     dz = near_img(x[i][2] - x[j][2], a.Lz, a.iLz);
+        if (excl_r2(dx, dy, dz) < a.cutoff_sq)
+          excl_pair<MEASURE>(dx, dy, dz, q, a.alpha, F[i], F[j], en);
+      }
+#pragma unroll
+      for (int s = 0; s < 3; s++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) f[3 * s + d] = F[s][d];
+    } else {
     const long ns3 = 3 * (long)a.ns;
     for (int p = a.xfirst[n]; p < a.xfirst[n + 1]; p++) {
       const int2 ij = a.xpair[p];
@@ -1838,22 +1871,19 @@ MG_BODY void excl_mixed_kernel_body(const ExclArgs& a,
       }
     }
   }
+  }
   if (MEASURE) {
     // row layout of the pair kernels: el, lj, vir, Pvir[6], spare
-    constexpr int slot[7] = {0, 3, 4, 5, 6, 7, 8};
-    for (int k = 0; k < 10; k++) {
-      double v = 0;
 #pragma unroll
-      for (int m = 0; m < 7; m++)
-        if (slot[m] == k) v = en[m];
-      red[threadIdx.x] = v;
-      __syncthreads();
-      for (int w = EXCL_THREADS / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) a.epart[bx_ * NEN + k] = red[0];
-      __syncthreads();
+    for (int m = 0; m < 7; m++)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) en[m] += __shfl_xor_sync(0xffffffffu, en[m], o);
+    if (threadIdx.x == 0) {
+      double* e = a.epart + (long)bx_ * NEN;
+      e[0] = en[0];
+      e[1] = e[2] = e[9] = 0;
+#pragma unroll
+      for (int m = 1; m < 7; m++) e[m + 2] = en[m];
     }
   }
 }
@@ -2241,34 +2271,64 @@ cudaError_t k_kforce_fp64(const Launch& L, const KArgs& a, const double2* tab) {
   return cudaGetLastError();
 }
 
-// out[k] = sum over rows of part[row*width+k], fixed order (one CTA)
+// out[k] = sum over rows of part[row*width+k], in a fixed order (one CTA): the
+// warps share the columns, several warps a column where there are fewer
+// columns than warps; lanes take rows in turn; the two tables of a phase in one
+// launch.  (One column after the other with a CTA-wide tree each, a launch per
+// table: 13 us a launch on 864 waters; this 6.8 us for both.)
+constexpr int RED_THREADS = 512;
 MG_BODY void reduce_rows_kernel_body(const double* __restrict__ part,
     int nrows,
     int width,
     double* __restrict__ out,
     const int bx_,
     const int by_) {
-  __shared__ double red[256];
-  for (int k = 0; k < width; k++) {
-    double s = 0;
-    for (int r = threadIdx.x; r < nrows; r += 256) s += part[(long)r * width + k];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-      __syncthreads();
+  constexpr int NW = RED_THREADS / 32;
+  __shared__ double red[NW];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k0 = 0; k0 < width; k0 += NW) {
+    const int nc = min(NW, width - k0), ns = NW / nc;   // columns, warps a column
+    const int c = warp % nc, sh = warp / nc;
+    double v = 0;
+    if (sh < ns) {
+      const int step = 32 * ns;
+#pragma unroll 8
+      for (int r = 32 * sh + lane; r < nrows; r += step) v += part[(long)r * width + k0 + c];
     }
-    if (threadIdx.x == 0) out[k] = red[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    if (threadIdx.x < nc) {
+      double t = 0;
+      for (int q = 0; q < ns; q++) t += red[q * nc + threadIdx.x];
+      out[k0 + threadIdx.x] = t;
+    }
     __syncthreads();
   }
 }
 
-__global__ void reduce_rows_kernel(const double* __restrict__ part, int nrows, int width, double* __restrict__ out) {
-  reduce_rows_kernel_body(part, nrows, width, out, blockIdx.x, 0);
+// up to two tables in a launch, one CTA each
+struct RedTab {
+  const double* part;
+  int nrows, width;
+  double* out;
+};
+__global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const __grid_constant__ RedTab a,
+                                                                  const __grid_constant__ RedTab b) {
+  if (blockIdx.x == 0) reduce_rows_kernel_body(a.part, a.nrows, a.width, a.out, 0, 0);
+  else reduce_rows_kernel_body(b.part, b.nrows, b.width, b.out, 0, 0);
 }
 
 cudaError_t k_reduce_sum(const Launch& L, const double* part, int nrows, int width, double* out) {
-  reduce_rows_kernel<<<1, 256, 0, L.s>>>(part, nrows, width, out);
+  const RedTab a{part, nrows, width, out};
+  reduce_rows_kernel<<<1, RED_THREADS, 0, L.s>>>(a, a);
+  LAUNCHED(L);
+  return cudaGetLastError();
+}
+cudaError_t k_reduce_two(const Launch& L, const double* pa, int ra, int wa, double* oa,
+                         const double* pb, int rb, int wb, double* ob) {
+  reduce_rows_kernel<<<2, RED_THREADS, 0, L.s>>>(RedTab{pa, ra, wa, oa}, RedTab{pb, rb, wb, ob});
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -2281,7 +2341,8 @@ cudaError_t k_reduce_sum(const Launch& L, const double* part, int nrows, int wid
 // positions are then wrapped as cook's normalize(-1) does after the step
 // (sim/norm.c:415-444): the molecule's lowest coordinate over its massive
 // sites decides a shift of +L (below r0), -L (at or above r0 + L) or none.
-constexpr int SH_THREADS = 128;
+constexpr int SH_THREADS = SHAKE_THREADS;
+int shake_blocks(int nmol) { return cdiv(nmol, SHAKE_THREADS); }
 
 __device__ __forceinline__ double wrap_shift(double lo, double r0, double L) {
   return lo < r0 ? L : (lo >= r0 + L ? -L : 0.0);
@@ -2417,15 +2478,15 @@ __device__ __forceinline__ void ff_diff(int i, int j, const float (&h)[3], const
 // sweeps; dsum: the deviations summed per constraint (measured steps)
 template <bool MEAS>
 __device__ __forceinline__ bool shake3_ff(double3 (&P)[3], const int (&ci)[3], const int (&cj)[3],
-                                          const double (&bq)[3], const double (&tol)[3],
-                                          const double (&awi)[3], const double (&awj)[3],
+                                          const float4* __restrict__ ftab,
                                           const double (&rx)[3], const double (&ry)[3],
                                           const double (&rz)[3], int maxit,
                                           double (&dsum)[3]) {
   const double3 o = P[0];
   float hx[3], hy[3], hz[3], lx[3], ly[3], lz[3];
+  hx[0] = hy[0] = hz[0] = lx[0] = ly[0] = lz[0] = 0.f;
 #pragma unroll
-  for (int s = 0; s < 3; s++) {
+  for (int s = 1; s < 3; s++) {
     const double ux = P[s].x - o.x, uy = P[s].y - o.y, uz = P[s].z - o.z;
     hx[s] = __double2float_rn(ux);
     hy[s] = __double2float_rn(uy);
@@ -2437,11 +2498,12 @@ __device__ __forceinline__ bool shake3_ff(double3 (&P)[3], const int (&ci)[3], c
   float bqh[3], bql[3], tf[3], wi[3], wj[3], qx[3], qy[3], qz[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    bqh[q] = __double2float_rn(bq[q]);
-    bql[q] = __double2float_rn(bq[q] - (double)bqh[q]);
-    tf[q] = __double2float_rn(tol[q]);
-    wi[q] = __double2float_rn(awi[q]);
-    wj[q] = __double2float_rn(awj[q]);
+    const float4 u = __ldg(ftab + 2 * q), v = __ldg(ftab + 2 * q + 1);
+    bqh[q] = u.x;
+    bql[q] = u.y;
+    tf[q] = u.z;
+    wi[q] = u.w;
+    wj[q] = v.x;
     qx[q] = __double2float_rn(rx[q]);
     qy[q] = __double2float_rn(ry[q]);
     qz[q] = __double2float_rn(rz[q]);
@@ -2489,89 +2551,121 @@ __device__ __forceinline__ bool shake3_ff(double3 (&P)[3], const int (&ci)[3], c
   return over;
 }
 
+// the sweeps on the three sites P at the displacements' directions r_ij of the
+// old positions R, constraint order (ci, cj); true if they did not converge
+template <bool MEAS, bool DF>
+__device__ __forceinline__ bool shake3(const ShakeArgs& a, const bool df, int c0,
+                                       const int (&ci)[3], const int (&cj)[3],
+                                       const double3 (&R)[3], double3 (&P)[3], ShakeMeas& ms) {
+  double rx[3], ry[3], rz[3];
+  double dsum[3] = {0, 0, 0};
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const double3 ri = sh_get(ci[q], R[0], R[1], R[2]), rj = sh_get(cj[q], R[0], R[1], R[2]);
+    rx[q] = ri.x - rj.x;
+    ry[q] = ri.y - rj.y;
+    rz[q] = ri.z - rj.z;
+  }
+  const double* t = a.ctab + 6 * (long)c0;
+  bool over = false;
+  if (DF && df) {
+    over = shake3_ff<MEAS>(P, ci, cj, a.ftab + 2 * (long)c0, rx, ry, rz, a.maxit, dsum);
+  } else {
+    double bq[3], tol[3], awi[3], awj[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      bq[q] = t[6 * q];
+      tol[q] = t[6 * q + 1];
+      awi[q] = t[6 * q + 2];
+      awj[q] = t[6 * q + 3];
+    }
+    int it = 0;
+    do {
+      it++;
+      over = false;
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const double3 pi = sh_get(ci[q], P[0], P[1], P[2]), pj = sh_get(cj[q], P[0], P[1], P[2]);
+        const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
+        const double d = bq[q] - (px * px + py * py + pz * pz);
+        over |= fabs(d) > tol[q];
+        if constexpr (MEAS) dsum[q] += d;
+        sh_add(ci[q], P[0], P[1], P[2], d * awi[q], rx[q], ry[q], rz[q]);
+        sh_add(cj[q], P[0], P[1], P[2], d * awj[q], rx[q], ry[q], rz[q]);
+      }
+    } while (over && it < a.maxit);
+  }
+  if constexpr (MEAS) {
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      meas_cons(ms, dsum[q] * t[6 * q + 4], dsum[q] * t[6 * q + 5], rx[q], ry[q], rz[q]);
+  }
+  return over;
+}
+
+// A warp per CTA: a molecule's set-up and sweeps are one chain, so what counts
+// is how many SMs share the work (and their narrow FP64 pipes).  Molecules with
+// three constraints over their first three sites (rigid water; TIP4P with its
+// massless site behind) keep the sites in registers; where the constraints are
+// (0,1), (0,2), (1,2) the indices are compile-time constants and a sweep needs
+// no selection.  The per-constraint factors come from a table (formed per call
+// they cost six FP64 divisions a molecule).  Measured, float-float sweeps: 864
+// waters 43 -> 13.7 us, 32768 waters 55 -> 21 us.
 template <bool NOSE, bool MEAS, bool DF>
 MG_BODY void shake_kernel_body(const ShakeArgs& a,
     const int bx_,
     const int by_) {
-  __shared__ double red[SH_THREADS];
-  const int n = bx_ * SH_THREADS + threadIdx.x;
+  static_assert(SHAKE_THREADS == 32, "one warp per CTA");
+  const int n = bx_ * SHAKE_THREADS + threadIdx.x;
   double kin = 0;
-  [[maybe_unused]] ShakeMeas ms;
+  ShakeMeas ms;
   if constexpr (MEAS) meas_zero(ms);
   [[maybe_unused]] NoseStep nose;
   if constexpr (NOSE) nose = nose_begin(a);
   if (n < a.nmol) {
     const int i0 = a.mol_first[n], i1 = a.mol_first[n + 1];
     const int c0 = a.mol_cfirst[n], c1 = a.mol_cfirst[n + 1];
-    if (i1 - i0 == 3 && c1 - c0 == 3) {
-      double3 P[3], R[3];
-      double im[3];
+    // 1: the constraints are (0,1), (0,2), (1,2); 2: others over the first
+    // three sites; 0: anything else
+    const int kind = a.kind3[n];
+    if (kind) {
+      double3 P[3], R[3], V[3];
 #pragma unroll
       for (int s = 0; s < 3; s++) {
         const int i = i0 + s;
         R[s] = make_double3(a.r[3 * i], a.r[3 * i + 1], a.r[3 * i + 2]);
-        im[s] = a.imass[i];
+        V[s] = make_double3(a.r1[3 * i], a.r1[3 * i + 1], a.r1[3 * i + 2]);
+        const double hm = a.hh * a.imass[i];
         if constexpr (NOSE) {
-          const double dx = nose_dof(a, nose, 3 * i, a.r1[3 * i]);
-          const double dy = nose_dof(a, nose, 3 * i + 1, a.r1[3 * i + 1]);
-          const double dz = nose_dof(a, nose, 3 * i + 2, a.r1[3 * i + 2]);
-          P[s] = make_double3(a.f[3 * i] * (a.hh * im[s]) + dx + R[s].x + a.r1[3 * i],
-                              a.f[3 * i + 1] * (a.hh * im[s]) + dy + R[s].y + a.r1[3 * i + 1],
-                              a.f[3 * i + 2] * (a.hh * im[s]) + dz + R[s].z + a.r1[3 * i + 2]);
+          const double dx = nose_dof(a, nose, 3 * i, V[s].x);
+          const double dy = nose_dof(a, nose, 3 * i + 1, V[s].y);
+          const double dz = nose_dof(a, nose, 3 * i + 2, V[s].z);
+          P[s] = make_double3(a.f[3 * i] * hm + dx + R[s].x + V[s].x,
+                              a.f[3 * i + 1] * hm + dy + R[s].y + V[s].y,
+                              a.f[3 * i + 2] * hm + dz + R[s].z + V[s].z);
         } else {
-          P[s] = make_double3(a.f[3 * i] * (a.hh * im[s]) + R[s].x + a.r1[3 * i],
-                              a.f[3 * i + 1] * (a.hh * im[s]) + R[s].y + a.r1[3 * i + 1],
-                              a.f[3 * i + 2] * (a.hh * im[s]) + R[s].z + a.r1[3 * i + 2]);
+          P[s] = make_double3(a.f[3 * i] * hm + R[s].x + V[s].x,
+                              a.f[3 * i + 1] * hm + R[s].y + V[s].y,
+                              a.f[3 * i + 2] * hm + R[s].z + V[s].z);
         }
       }
-      // per constraint: the tolerance as a bound on |d| (eps bq, so no
-      // product per sweep) and the factors m_i^-1 wq, m_j^-1 wq that turn d
-      // into the two displacements along r_ij
-      int ci[3], cj[3];
-      double bq[3], tol[3], awi[3], awj[3], rx[3], ry[3], rz[3];
-      [[maybe_unused]] double dsum[3] = {0, 0, 0};
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        const int2 ij = a.cons[c0 + q];
-        ci[q] = ij.x - i0;
-        cj[q] = ij.y - i0;
-        bq[q] = a.bondq[c0 + q];
-        const double mi = a.imass[ij.x], mj = a.imass[ij.y];
-        const double wq = a.omega / (mi + mj) * (1.0 / bq[q]);
-        tol[q] = a.eps * bq[q];
-        awi[q] = mi * wq;
-        awj[q] = -(mj * wq);
-        const double3 ri = sh_get(ci[q], R[0], R[1], R[2]), rj = sh_get(cj[q], R[0], R[1], R[2]);
-        rx[q] = ri.x - rj.x;
-        ry[q] = ri.y - rj.y;
-        rz[q] = ri.z - rj.z;
-      }
-      int it = 0;
-      bool over = false;
-      if constexpr (DF) over = shake3_ff<MEAS>(P, ci, cj, bq, tol, awi, awj, rx, ry, rz, a.maxit, dsum);
-      else do {
-        it++;
-        over = false;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          const double3 pi = sh_get(ci[q], P[0], P[1], P[2]), pj = sh_get(cj[q], P[0], P[1], P[2]);
-          const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
-          const double d = bq[q] - (px * px + py * py + pz * pz);
-          over |= fabs(d) > tol[q];
-          if constexpr (MEAS) dsum[q] += d;
-          sh_add(ci[q], P[0], P[1], P[2], d * awi[q], rx[q], ry[q], rz[q]);
-          sh_add(cj[q], P[0], P[1], P[2], d * awj[q], rx[q], ry[q], rz[q]);
-        }
-      } while (over && it < a.maxit);
-      if (over) atomicOr(a.status, 1);
-      if constexpr (MEAS) {
+      // float-float sweeps for molecules of exactly three sites
+      const bool df = i1 - i0 == 3;
+      bool over;
+      if (kind == 1) {
+        const int ci[3] = {0, 0, 1}, cj[3] = {1, 2, 2};
+        over = shake3<MEAS, DF>(a, df, c0, ci, cj, R, P, ms);
+      } else {
+        int ci[3], cj[3];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
           const int2 ij = a.cons[c0 + q];
-          const double wb = a.omega / (a.imass[ij.x] + a.imass[ij.y]);
-          meas_cons(ms, dsum[q] * wb, dsum[q] * wb / bq[q], rx[q], ry[q], rz[q]);
+          ci[q] = ij.x - i0;
+          cj[q] = ij.y - i0;
         }
+        over = shake3<MEAS, DF>(a, df, c0, ci, cj, R, P, ms);
       }
+      if (over) atomicOr(a.status, 1);
       double sx = 0, sy = 0, sz = 0;
       if (a.normalize) {
         double lx = 9e9, ly = 9e9, lz = 9e9;
@@ -2589,7 +2683,7 @@ MG_BODY void shake_kernel_body(const ShakeArgs& a,
 #pragma unroll
       for (int s = 0; s < 3; s++) {
         const int i = i0 + s;
-        const double v1x = a.r1[3 * i], v1y = a.r1[3 * i + 1], v1z = a.r1[3 * i + 2];
+        const double v1x = V[s].x, v1y = V[s].y, v1z = V[s].z;
         const double v2x = P[s].x - R[s].x, v2y = P[s].y - R[s].y, v2z = P[s].z - R[s].z;
         double v1s = 0, v2s = 0;
         v1s += v1x * v1x;
@@ -2607,6 +2701,16 @@ MG_BODY void shake_kernel_body(const ShakeArgs& a,
         a.r[3 * i + 1] = P[s].y + sy;
         a.r[3 * i + 2] = P[s].z + sz;
       }
+      // massless sites behind the three: moved along, placed by their parents
+      for (int i = i0 + 3; i < i1; i++)
+        for (int k = 0; k < 3; k++) {
+          const double r = a.r[3 * i + k], v = a.r1[3 * i + k];
+          double p = a.f[3 * i + k] * (a.hh * a.imass[i]);
+          if constexpr (NOSE) p = p + nose_dof(a, nose, 3 * i + k, v);
+          p = p + r + v;
+          a.r1[3 * i + k] = p - r;
+          a.r[3 * i + k] = p + (k == 0 ? sx : (k == 1 ? sy : sz));
+        }
     } else {
     double* p = a.p;
     for (int i = i0; i < i1; i++)
@@ -2672,17 +2776,11 @@ MG_BODY void shake_kernel_body(const ShakeArgs& a,
     }
     }
   }
-  red[threadIdx.x] = kin;
-  __syncthreads();
-  for (int w = SH_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) a.kin_part[bx_] = red[0];
+  // the CTA's sums: a shuffle tree, in a fixed order
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) kin += __shfl_down_sync(0xffffffffu, kin, o);
+  if (threadIdx.x == 0) a.kin_part[bx_] = kin;
   if constexpr (MEAS) {
-    // the 13 measured sums of the CTA in a fixed order: a shuffle tree per
-    // warp, then the warps' sums in warp order (red[] is free again)
-    __syncthreads();
     double v[13];
     v[0] = ms.virc;
 #pragma unroll
@@ -2690,19 +2788,11 @@ MG_BODY void shake_kernel_body(const ShakeArgs& a,
       v[1 + k] = ms.pt[k];
       v[7 + k] = ms.pk[k];
     }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < 13; k++) {
-      double x = v[k];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) red[wid * 13 + k] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < 13) {
-      double x = 0;
-      for (int w = 0; w < SH_THREADS / 32; w++) x += red[w * 13 + threadIdx.x];
-      a.meas_part[(long)bx_ * 13 + threadIdx.x] = x;
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      if (threadIdx.x == 0) a.meas_part[(long)bx_ * 13 + k] = v[k];
     }
   }
 }
@@ -2856,7 +2946,7 @@ __global__ void __launch_bounds__(SH_THREADS) batch_shake_kernel(const BoxStep* 
 }
 
 // sums k0..k1-1 of every box (one CTA each)
-__global__ void batch_reduce_kernel(const BoxStep* __restrict__ B, int k0, int k1) {
+__global__ void __launch_bounds__(RED_THREADS) batch_reduce_kernel(const BoxStep* __restrict__ B, int k0, int k1) {
   const BoxStep& e = B[blockIdx.y];
   for (int k = k0; k < k1; k++)
     reduce_rows_kernel_body(e.rpart[k], e.rrows[k], e.rwidth[k], e.rout[k], 0, 0);
@@ -2931,9 +3021,9 @@ cudaError_t k_batch_step(const Launch& L, const BoxStep* d, int nbox, const Batc
                          bool measure) {
   if (measure) {
     // the energies of the force evaluation (rows 0, 1), the step, its sums (2, 3)
-    batch_reduce_kernel<<<dim3(1, nbox), 256, 0, L.s>>>(d, 0, 2);
+    batch_reduce_kernel<<<dim3(1, nbox), RED_THREADS, 0, L.s>>>(d, 0, 2);
     batch_shake_kernel<true><<<dim3(g.shake, nbox), SH_THREADS, 0, L.s>>>(d);
-    batch_reduce_kernel<<<dim3(1, nbox), 256, 0, L.s>>>(d, 2, 4);
+    batch_reduce_kernel<<<dim3(1, nbox), RED_THREADS, 0, L.s>>>(d, 2, 4);
     *L.counter += 3;
   } else {
     batch_shake_kernel<false><<<dim3(g.shake, nbox), SH_THREADS, 0, L.s>>>(d);

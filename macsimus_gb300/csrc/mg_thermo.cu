@@ -44,7 +44,8 @@ __device__ __forceinline__ double th_gauss(unsigned long long seed, long long st
   return sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
 }
 
-// Bussi: sum of squares of Gaussians 1..f-1 of the step, per block
+// Bussi: sum of squares of Gaussians 1..f-1 of the step, per block; Gaussian 0
+// behind them
 __global__ void bussi_chi2_kernel(long long nf, unsigned long long seed,
                                   const long long* __restrict__ stepp, double* __restrict__ part) {
   __shared__ double red[TH_THREADS];
@@ -61,18 +62,39 @@ __global__ void bussi_chi2_kernel(long long nf, unsigned long long seed,
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = red[0];
+    if (blockIdx.x == 0) part[gridDim.x] = th_gauss(seed, step, 0);
+  }
+}
+
+// the sum of v[0..n) in a fixed order, in every thread of the CTA.  (One
+// thread adding the few hundred partial sums one by one: 27 us a step on 12544 sites, this
+// 9.1 us.)
+__device__ __forceinline__ double th_sum(const double* __restrict__ v, int n) {
+  __shared__ double red[TH_THREADS / 32];
+  double s = 0;
+  for (int i = threadIdx.x; i < n; i += TH_THREADS) s += v[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0;
+#pragma unroll
+  for (int w = 0; w < TH_THREADS / 32; w++) s += red[w];
+  return s;
 }
 
 // the factor z (every block computes it from the same sums in the same
 // order) and r1 *= z
-__global__ void thermostat_scale_kernel(ThermoArgs a, const double* __restrict__ kin_part,
-                                        const double* __restrict__ chi_part,
-                                        double* __restrict__ r1) {
+__global__ void __launch_bounds__(TH_THREADS)
+    thermostat_scale_kernel(ThermoArgs a, const double* __restrict__ kin_part,
+                            const double* __restrict__ chi_part, double* __restrict__ r1) {
   __shared__ double zs;
+  const double k = th_sum(kin_part, a.nkin);
+  const double uf = a.kind == 2 ? th_sum(chi_part, a.nchi) : 0;
   if (threadIdx.x == 0) {
-    double k = 0;
-    for (int b = 0; b < a.nkin; b++) k += kin_part[b];
     // cook's doubled kinetic energy sum m (V1^2 + V2^2) / (2 h^2) -> En.T
     const double ET = k / (2 * a.h * a.h) / a.nf;
     double z = 1;
@@ -81,14 +103,17 @@ __global__ void thermostat_scale_kernel(ThermoArgs a, const double* __restrict__
                   : (ET * 7.38905609893065022723 < a.T ? -1 : log(ET / a.T) / 2);
       z = exp(bl * -a.h / a.tau);
     } else if (a.kind == 2) {
-      double uf = 0;
-      for (int b = 0; b < a.nchi; b++) uf += chi_part[b];
-      const double u1 = th_gauss(a.seed, *a.step, 0);
+      const double u1 = chi_part[a.nchi];
       const double e = exp(-a.h / a.tau), c = a.T / (a.nf * ET);
       z = sqrt(e + c * (1 - e) * (u1 * u1 + uf) + 2 * e * sqrt(c * (1 - e)) * u1);
     }
     zs = z;
-    if (blockIdx.x == 0 && a.zout) *a.zout = z;
+    if (blockIdx.x == 0) {
+      if (a.zout) *a.zout = z;
+      // the step counter of the Bussi stream lives on the device (so that a
+      // captured step replays with fresh draws)
+      if (a.kind == 2) ++*a.step;
+    }
   }
   __syncthreads();
   const double z = zs;
@@ -99,10 +124,10 @@ __global__ void thermostat_scale_kernel(ThermoArgs a, const double* __restrict__
 
 // Nose-Hoover: one thread advances the thermostat state (NoseSlot) with the
 // kinetic energy of the step, summed in the order of thermostat_scale_kernel
-__global__ void nose_update_kernel(ThermoArgs a, const double* __restrict__ kin_part) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double k = 0;
-  for (int b = 0; b < a.nkin; b++) k += kin_part[b];
+__global__ void __launch_bounds__(TH_THREADS)
+    nose_update_kernel(ThermoArgs a, const double* __restrict__ kin_part) {
+  const double k = th_sum(kin_part, a.nkin);
+  if (threadIdx.x != 0) return;
   const double ET = k / (2 * a.h * a.h) / a.nf;
   double* s = a.nh;
   const int kk = (int)s[NH_K], knew = min(a.pred, kk + 1);
@@ -118,28 +143,22 @@ __global__ void nose_update_kernel(ThermoArgs a, const double* __restrict__ kin_
   if (a.zout) *a.zout = 1;
 }
 
-// the step counter of the Bussi stream lives on the device (so that a
-// captured step replays with fresh draws)
-__global__ void step_increment_kernel(long long* step) { ++*step; }
+cudaError_t k_bussi_draw(const Launch& L, const ThermoArgs& a, double* chi_part) {
+  bussi_chi2_kernel<<<a.nchi, TH_THREADS, 0, L.s>>>((long long)a.nf, a.seed, a.step, chi_part);
+  ++*L.counter;
+  return cudaGetLastError();
+}
 
 cudaError_t k_thermostat(const Launch& L, const ThermoArgs& a, const double* kin_part,
-                         double* chi_part, double* r1) {
+                         const double* chi_part, double* r1) {
   if (a.kind == 3) {
-    nose_update_kernel<<<1, 32, 0, L.s>>>(a, kin_part);
+    nose_update_kernel<<<1, TH_THREADS, 0, L.s>>>(a, kin_part);
     ++*L.counter;
     return cudaGetLastError();
-  }
-  if (a.kind == 2) {
-    bussi_chi2_kernel<<<a.nchi, TH_THREADS, 0, L.s>>>((long long)a.nf, a.seed, a.step, chi_part);
-    ++*L.counter;
   }
   const int grid = (int)std::min<long long>((3LL * a.ns + TH_THREADS - 1) / TH_THREADS, 4 * PARTITION_SMS);
   thermostat_scale_kernel<<<grid, TH_THREADS, 0, L.s>>>(a, kin_part, chi_part, r1);
   ++*L.counter;
-  if (a.kind == 2) {
-    step_increment_kernel<<<1, 1, 0, L.s>>>(a.step);
-    ++*L.counter;
-  }
   return cudaGetLastError();
 }
 

@@ -19,6 +19,29 @@ using namespace mg;
 // length of the reduction-output block d_sums / h_sums (doubles)
 constexpr int NSUMS = 56;
 
+// workspace of the sorted Widom insertions (at most about 500 MB), kept by
+// its context or batch and freed with it
+struct WidomWork {
+  void* mem = nullptr;
+  size_t cap = 0;
+  bool fit(size_t n) {
+    if (n <= cap) return true;
+    release();
+    if (cudaMalloc(&mem, n) != cudaSuccess) {
+      cudaGetLastError();   // no room: the insertions run unsorted
+      mem = nullptr;
+      return false;
+    }
+    cap = n;
+    return true;
+  }
+  void release() {
+    if (mem) cudaFree(mem);
+    mem = nullptr;
+    cap = 0;
+  }
+};
+
 struct mg_ctx {
   std::string err;
   int precision = MG_MIXED;
@@ -190,6 +213,7 @@ struct mg_ctx {
   PairD* d_wtabd = nullptr;
   double *d_wgeom = nullptr, *d_wpart = nullptr;
   WidomBox* d_wbox = nullptr;
+  WidomWork wwork;
   // adjoint scratch (FP64 contexts)
   AdjPair* d_adjtab = nullptr;
   double *d_ag = nullptr, *d_aq = nullptr, *d_apart = nullptr, *d_adEq = nullptr,
@@ -1925,6 +1949,7 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_xq, ctx->d_za, ctx->d_vb, ctx->d_tcrows, ctx->d_zb, ctx->d_tckrows};
   for (void* b : bufs)
     if (b) cudaFree(b);
+  ctx->wwork.release();
   if (ctx->h_sums) cudaFreeHost(ctx->h_sums);
   if (ctx->h_dmax) cudaFreeHost(ctx->h_dmax);
   if (ctx->ev_dmax) cudaEventDestroy(ctx->ev_dmax);
@@ -2344,10 +2369,17 @@ int mg_widom(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigned lon
     if (d_U) cudaFree(d_U);
     return rc;
   }
-  const int nblk = widom_blocks(ninsert);
+  const bool fp64 = ctx->precision != MG_MIXED;
+  WidomPlan plan = widom_plan(&box, 1, ninsert, fp64);
+  if (plan.sorted && !ctx->wwork.fit(plan.bytes())) {
+    plan = WidomPlan();
+    plan.nblk = widom_blocks(ninsert);
+  }
+  if (plan.sorted) widom_layout(plan, &box, 1, ctx->wwork.mem);
+  const int nblk = plan.nblk;
   CK(cudaMemcpyAsync(ctx->d_wbox, &box, sizeof(WidomBox), cudaMemcpyHostToDevice, ctx->stream));
   Launch L = launch(ctx);
-  cudaError_t e = k_widom(L, ctx->d_wbox, 1, ninsert, ctx->precision != MG_MIXED);
+  cudaError_t e = k_widom(L, ctx->d_wbox, 1, ninsert, fp64, plan, ctx->wwork.mem);
   if (e != cudaSuccess) {
     if (d_U) cudaFree(d_U);
     return fail(ctx, MG_ERR_CUDA, std::string("widom: ") + cudaGetErrorString(e));
@@ -2771,6 +2803,7 @@ struct mg_batch {
   int launches_step = 0, launches = 0;
   WidomBox* d_wbox = nullptr;
   int wcap = 0;
+  WidomWork wwork;
   // one launch per kernel over all boxes, when every box qualifies
   // (fused_ok): the boxes' kernel arguments on the device, the largest
   // grids, one captured graph per kind of step
@@ -2900,6 +2933,7 @@ int mg_batch_destroy(mg_batch* b) {
   if (b->d_stat) cudaFree(b->d_stat);
   if (b->h_stat) cudaFreeHost(b->h_stat);
   if (b->d_wbox) cudaFree(b->d_wbox);
+  b->wwork.release();
   for (cudaEvent_t e : b->ev_join)
     if (e) cudaEventDestroy(e);
   for (cudaStream_t s : b->lanes)
@@ -3277,13 +3311,20 @@ int mg_batch_widom(mg_batch* b, const mg_probe* probes, int probe_per_box, long 
     BCK(cudaMalloc((void**)&b->d_wbox, sizeof(WidomBox) * nbox));
     b->wcap = nbox;
   }
+  const bool fp64 = b->box[0]->precision != MG_MIXED;
+  WidomPlan plan = widom_plan(desc.data(), nbox, ninsert, fp64);
+  if (plan.sorted && !b->wwork.fit(plan.bytes())) {
+    plan = WidomPlan();
+    plan.nblk = widom_blocks(ninsert);
+  }
+  if (plan.sorted) widom_layout(plan, desc.data(), nbox, b->wwork.mem);
   BCK(cudaMemcpyAsync(b->d_wbox, desc.data(), sizeof(WidomBox) * nbox, cudaMemcpyHostToDevice,
                       b->main));
   int cnt = 0;
   Launch L{b->main, &cnt};
-  BCK(k_widom(L, b->d_wbox, nbox, ninsert, b->box[0]->precision != MG_MIXED));
+  BCK(k_widom(L, b->d_wbox, nbox, ninsert, fp64, plan, b->wwork.mem));
   b->launches = cnt;
-  const int nblk = widom_blocks(ninsert);
+  const int nblk = plan.nblk;
   std::vector<double> part((size_t)nblk * nbox);
   for (int i = 0; i < nbox; i++)
     BCK(cudaMemcpyAsync(part.data() + (size_t)i * nblk, b->box[i]->d_wpart, sizeof(double) * nblk,

@@ -571,8 +571,25 @@ struct WidomBox {
   const PairD* tabd;
   const float4* eru;    // erfc energy spline (mixed)
   const double* ert;    // erfc splines (FP64)
+  // sorted insertions (WidomPlan): bins a box edge, ghost sites {x, y, z,
+  // rank in the bin}, their energies, slots -> site, bin counts and starts
+  int nbx, nby, nbz;
+  int4* pos;
+  double* ue;
+  int *slot, *cnt, *start;
 };
 int widom_blocks(long long n);
+// how n insertions into each of nbox boxes are run: sorted by place, cn
+// insertions into `boxes` boxes at a time, in a workspace of bytes(), or a
+// warp each; nblk sums of Boltzmann factors per box
+struct WidomPlan {
+  bool sorted = false;
+  int cn = 0, boxes = 0, nblk = 0;
+  size_t nent = 0, nbin = 0, nslot = 0;   // per box: ghost sites, bins, slots
+  size_t bytes() const;
+};
+WidomPlan widom_plan(const WidomBox* boxes, int nbox, long long n, bool fp64);
+void widom_layout(const WidomPlan& P, WidomBox* boxes, int nbox, void* work);
 // identity change of whole molecules (cook's XWidom): per listed molecule the
 // r-space energy of its sites with the real and with the virtual constants,
 // against the other molecules in the cell list of the last force evaluation
@@ -594,7 +611,8 @@ struct XWidomArgs {
   const double* ert;
 };
 cudaError_t k_xwidom(const Launch& L, const XWidomArgs& a, bool fp64);
-cudaError_t k_widom(const Launch& L, const WidomBox* boxes, int nbox, long long n, bool fp64);
+cudaError_t k_widom(const Launch& L, const WidomBox* boxes, int nbox, long long n, bool fp64,
+                    const WidomPlan& P, void* work);
 
 cudaError_t k_drude_take(const Launch& L, const DrudeArgs& a, const double* r, double* out);
 cudaError_t k_drude_put(const Launch& L, const DrudeArgs& a, const double* in, double* r);

@@ -12,6 +12,11 @@
 // fixed order, so the result does not depend on scheduling.  blockIdx.y
 // selects the box: one launch serves a whole batch of boxes, each with its
 // own cell list, pair table and ghost.
+//
+// Many insertions a cell (mixed precision) are sorted by place instead, 32
+// neighbouring ghost sites to a warp (widom_sorted_kernel below).
+#include <algorithm>
+
 #include "mg_internal.h"
 
 namespace mg {
@@ -141,6 +146,269 @@ __global__ void __launch_bounds__(WD_THREADS) widom_mixed_kernel(const WidomBox*
     }
   }
   wd_block_sum(wacc, a.part);
+}
+
+// ---- mixed path, sorted by place ------------------------------------------
+//
+// A warp per insertion repeats the ghost's FP64 set-up (three divisions, the
+// Boltzmann factor) in all lanes and fills its lanes with the few sites of
+// single cells: 5.9 ns an insertion into ionic boxes of 500 to 4000 sites
+// (28.3 ms for 48 boxes of 100000); this 0.4 ns (1.9 ms, of which the sorted
+// kernel, bound by its instruction issue at 88 %, takes 1.56).
+// Here the set-up is done once, a thread per insertion, and the ghost sites
+// are counting-sorted into bins (the cells, cut so that a bin gets about
+// WS_FILL sites), each bin's segment padded to whole warps.  A warp
+// then takes 32 ghost sites of one bin, one a lane; its lanes test the sites
+// of the stencil's cells against the bin's box, 32 at a time, and every lane
+// takes every survivor from shared memory.  A ghost site's terms are added in
+// cell-list order to an unevaluated sum of two floats (about 48 bits), so that
+// U depends neither on the sort nor on the bins.
+
+constexpr int WS_FILL = 48;     // ghost sites per bin: beyond this the bins are cut finer
+constexpr int WS_SPAN = 1024;   // insertions per CTA of the finishing kernel
+constexpr int WS_BUF = 64;      // survivors buffered per warp
+
+__device__ __forceinline__ unsigned ws_bin(unsigned u, int n) {
+  return (unsigned)(((unsigned long long)u * n) >> 32);
+}
+
+// sites of the insertions n0..n0+cn-1: fixed-point position and rank within
+// their bin.  A one-site ghost is not turned: its offset, three divisions, is
+// formed once per CTA.
+__global__ void __launch_bounds__(WD_THREADS)
+    widom_place_kernel(const WidomBox* __restrict__ boxes, long long n0, int cn) {
+  __shared__ unsigned off[3];
+  const WidomBox& B = boxes[blockIdx.y];
+  const WidomArgs& a = B.a;
+  const int nps = a.nps;
+  if (nps == 1 && threadIdx.x < 3) {
+    const double Lk = threadIdx.x == 0 ? a.Lx : (threadIdx.x == 1 ? a.Ly : a.Lz);
+    off[threadIdx.x] = (unsigned)(int)llrint(a.geom[threadIdx.x] / Lk * 4294967296.0);
+  }
+  __syncthreads();
+  const int t = blockIdx.x * WD_THREADS + threadIdx.x;
+  if (t >= cn) return;
+  const long long k = n0 + t;
+  const int nbx = B.nbx, nby = B.nby, nbz = B.nbz;
+  const unsigned px = (unsigned)(wd_word(a.seed, k, 0) >> 32),
+                 py = (unsigned)(wd_word(a.seed, k, 1) >> 32),
+                 pz = (unsigned)(wd_word(a.seed, k, 2) >> 32);
+  double R[9];
+  if (nps > 1) wd_rotation(a.seed, k, nps, R);
+  for (int s = 0; s < nps; s++) {
+    unsigned ux = px, uy = py, uz = pz;
+    if (nps > 1) {
+      const double g0 = a.geom[3 * s], g1 = a.geom[3 * s + 1], g2 = a.geom[3 * s + 2];
+      ux += (unsigned)(int)llrint((R[0] * g0 + R[1] * g1 + R[2] * g2) / a.Lx * 4294967296.0);
+      uy += (unsigned)(int)llrint((R[3] * g0 + R[4] * g1 + R[5] * g2) / a.Ly * 4294967296.0);
+      uz += (unsigned)(int)llrint((R[6] * g0 + R[7] * g1 + R[8] * g2) / a.Lz * 4294967296.0);
+    } else {
+      ux += off[0];
+      uy += off[1];
+      uz += off[2];
+    }
+    const int bin = (ws_bin(ux, nbx) * nby + ws_bin(uy, nby)) * nbz + ws_bin(uz, nbz);
+    B.pos[t * nps + s] = make_int4((int)ux, (int)uy, (int)uz, atomicAdd(B.cnt + bin, 1));
+  }
+}
+
+// first slot of every bin, segments padded to whole warps (one CTA a box)
+__global__ void __launch_bounds__(1024) widom_scan_kernel(const WidomBox* __restrict__ boxes) {
+  __shared__ int ws[32];
+  const WidomBox& B = boxes[blockIdx.y];
+  const int nbin = B.nbx * B.nby * B.nbz;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry = 0;
+  for (int b0 = 0; b0 < nbin; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    const int c = b < nbin ? (B.cnt[b] + 31) & ~31 : 0;
+    int v = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) ws[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+      int w = ws[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
+      }
+      ws[lane] = w;
+    }
+    __syncthreads();
+    if (b < nbin) B.start[b] = carry + v - c + (warp ? ws[warp - 1] : 0);
+    carry += ws[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) B.start[nbin] = carry;
+}
+
+__global__ void __launch_bounds__(WD_THREADS)
+    widom_slot_kernel(const WidomBox* __restrict__ boxes, int cn) {
+  const WidomBox& B = boxes[blockIdx.y];
+  const int e = blockIdx.x * WD_THREADS + threadIdx.x;
+  if (e >= cn * B.a.nps) return;
+  const int4 p = B.pos[e];
+  const int bin = (ws_bin(p.x, B.nbx) * B.nby + ws_bin(p.y, B.nby)) * B.nbz + ws_bin(p.z, B.nbz);
+  B.slot[B.start[bin] + p.w] = e;
+}
+
+__global__ void __launch_bounds__(WD_THREADS)
+    widom_sorted_kernel(const WidomBox* __restrict__ boxes) {
+  __shared__ PairFS tab[MAX_WPROBE * MAX_KINDS];
+  __shared__ int4 buf[WD_WARPS][WS_BUF];
+  const WidomBox& B = boxes[blockIdx.y];
+  const WidomArgs& a = B.a;
+  const int ncx = a.ncx, ncy = a.ncy, ncz = a.ncz, nbx = B.nbx, nby = B.nby, nbz = B.nbz;
+  const int nslot = B.start[nbx * nby * nbz];
+  if ((int)blockIdx.x * WD_THREADS >= nslot) return;
+  const int nkind = a.nkind, nps = a.nps, nstencil = a.nstencil;
+  for (int t = threadIdx.x; t < nps * nkind; t += WD_THREADS)
+    tab[t] = *reinterpret_cast<const PairFS*>(B.tabf + t);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = blockIdx.x * WD_THREADS + threadIdx.x;
+  if (slot - lane >= nslot) return;   // whole warps: segments are whole warps
+  const int4* __restrict__ pj = B.pj;
+  const float4* __restrict__ eru = B.eru;
+  const int4* __restrict__ stencil = a.stencil;
+  const int* __restrict__ cell_start = a.cell_start;
+  const int e = B.slot[slot];
+  // the first slot of a segment's warp is always taken; lanes past the
+  // segment's end repeat it
+  const int e0 = __shfl_sync(0xffffffffu, e, 0);
+  const int4 p = B.pos[e < 0 ? e0 : e];
+  const int4 p0 = make_int4(__shfl_sync(0xffffffffu, p.x, 0), __shfl_sync(0xffffffffu, p.y, 0),
+                            __shfl_sync(0xffffffffu, p.z, 0), 0);
+  const int bx = ws_bin(p0.x, nbx), by = ws_bin(p0.y, nby), bz = ws_bin(p0.z, nbz);
+  // a cell is a whole number of bins
+  const int cx = bx / (nbx / ncx), cy = by / (nby / ncy), cz = bz / (nbz / ncz);
+  const unsigned mx = (unsigned)((unsigned long long)(2 * bx + 1) * 2147483648ULL / (unsigned)nbx),
+                 my = (unsigned)((unsigned long long)(2 * by + 1) * 2147483648ULL / (unsigned)nby),
+                 mz = (unsigned)((unsigned long long)(2 * bz + 1) * 2147483648ULL / (unsigned)nbz);
+  const float sx = (float)(a.Lx * 2.3283064365386963e-10), sy = (float)(a.Ly * 2.3283064365386963e-10),
+              sz = (float)(a.Lz * 2.3283064365386963e-10);
+  const float hx = 0.5f * (float)a.Lx / nbx, hy = 0.5f * (float)a.Ly / nby,
+              hz = 0.5f * (float)a.Lz / nbz;
+  // the bin test may keep too many, never too few: rounding is far below 1e-4
+  const float cq = (float)a.cutoff_sq, cqb = 1.0001f * cq, sgrid = (float)a.sgrid;
+  const PairFS* T = tab + (e < 0 ? 0 : e % nps) * nkind;
+  const int ntab1 = a.ntab - 1;
+  const unsigned below = (1u << lane) - 1u;
+  float uh = 0, ul = 0;
+
+  auto term = [&](const int4 q) {
+    const float dx = (float)(int)((unsigned)p.x - (unsigned)q.x) * sx;
+    const float dy = (float)(int)((unsigned)p.y - (unsigned)q.y) * sy;
+    const float dz = (float)(int)((unsigned)p.z - (unsigned)q.z) * sz;
+    const float rr = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (rr < cq) {
+      const PairFS& P = T[q.w & 255];
+      float u = 0;
+      if (rr < P.C2q) {
+        if (rr < P.C1q) {
+          const float x = P.Sq / rr, y = x * x * x;
+          u = P.E4 * fmaf(y, y, -y);
+        } else {
+          const float x = rr - P.C2q;
+          u = P.A * x * x;
+        }
+      }
+      if (P.qq != 0.f) {
+        const float4 s = __ldg(eru + min((int)(rr * sgrid), ntab1));
+        u += (__fdividef(s.y, s.z + rr) + s.x) * P.qq;
+      }
+      // uh + ul += u (Knuth's two-sum)
+      const float t = __fadd_rn(uh, u), b = __fsub_rn(t, uh);
+      ul = __fadd_rn(ul, __fadd_rn(__fsub_rn(uh, __fsub_rn(t, b)), __fsub_rn(u, b)));
+      uh = t;
+    }
+  };
+
+  int head = 0, fill = 0;
+  for (int st0 = 0; st0 < nstencil; st0 += 32) {
+    // 32 cells of the stencil: their sites as one list, 32 of it at a time
+    int j0 = 0, cnt = 0;
+    if (st0 + lane < nstencil) {
+      const int4 o = stencil[st0 + lane];
+      const int c2 = (wd_wrap(cx + o.x, ncx) * ncy + wd_wrap(cy + o.y, ncy)) * ncz +
+                     wd_wrap(cz + o.z, ncz);
+      j0 = cell_start[c2];
+      cnt = cell_start[c2 + 1] - j0;
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    j0 -= incl - cnt;   // site t of the list is j0 + t in its cell
+    for (int base = 0; base < total; base += 32) {
+      const int t = base + lane;
+      int c = 0;   // the cell of t: the number of cells that end at or before it
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int u = __shfl_sync(0xffffffffu, incl, c + o - 1);
+        if (u <= t) c += o;
+      }
+      const int jc = __shfl_sync(0xffffffffu, j0, min(c, 31));
+      bool keep = false;
+      int4 q = make_int4(0, 0, 0, 0);
+      if (t < total) {
+        q = pj[jc + t];
+        const float ex = fmaxf(fabsf((float)(int)((unsigned)q.x - mx) * sx) - hx, 0.f),
+                    ey = fmaxf(fabsf((float)(int)((unsigned)q.y - my) * sy) - hy, 0.f),
+                    ez = fmaxf(fabsf((float)(int)((unsigned)q.z - mz) * sz) - hz, 0.f);
+        keep = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < cqb;
+      }
+      const unsigned vote = __ballot_sync(0xffffffffu, keep);
+      if (keep) buf[warp][(head + fill + __popc(vote & below)) & (WS_BUF - 1)] = q;
+      fill += __popc(vote);
+      __syncwarp();
+      if (fill >= 32) {
+#pragma unroll 4
+        for (int i = 0; i < 32; i++) term(buf[warp][head + i]);
+        head = (head + 32) & (WS_BUF - 1);
+        fill -= 32;
+        __syncwarp();
+      }
+    }
+  }
+  for (int i = 0; i < fill; i++) term(buf[warp][(head + i) & (WS_BUF - 1)]);
+  // an overflowed sum stays what it is
+  if (e >= 0) B.ue[e] = isinf(uh) ? (double)uh : (double)uh + (double)ul;
+}
+
+// U and the Boltzmann factor of every insertion, summed per CTA; a further
+// chunk adds to the sums of the ones before
+__global__ void __launch_bounds__(WD_THREADS)
+    widom_finish_kernel(const WidomBox* __restrict__ boxes, long long n0, int cn) {
+  const WidomBox& B = boxes[blockIdx.y];
+  const WidomArgs& a = B.a;
+  const double beta = -1 / a.T;
+  double acc = 0;
+  for (int t = blockIdx.x * WS_SPAN + threadIdx.x; t < min(cn, ((int)blockIdx.x + 1) * WS_SPAN);
+       t += WD_THREADS) {
+    double U = 0;
+    for (int s = 0; s < a.nps; s++) U += B.ue[t * a.nps + s];
+    if (a.U) a.U[n0 + t] = U;
+    const double e = U * beta;
+    if (e > -700) acc += exp(e);
+  }
+  acc = warp_sum(acc);
+  __shared__ double ws[WD_WARPS];
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = n0 ? a.part[blockIdx.x] : 0;
+    for (int w = 0; w < WD_WARPS; w++) s += ws[w];
+    a.part[blockIdx.x] = s;
+  }
 }
 
 // FP64 path: the same in double, nearest image by rint
@@ -348,7 +616,121 @@ int widom_blocks(long long n) {
   return (int)(b < PARTITION_SMS * 8 ? (b > 0 ? b : 1) : PARTITION_SMS * 8);
 }
 
-cudaError_t k_widom(const Launch& L, const WidomBox* boxes, int nbox, long long n, bool fp64) {
+// Sorted from WS_MIN ghost sites a cell on, so that a warp's fixed work (its
+// stencil, the bin tests) is shared by enough lanes, and from WS_SITES ghost
+// sites in all: a warp's walk through its stencil and the five launches take
+// 100 to 200 us at any number, which a warp per insertion (8 ns a site) reaches
+// at about that many.  Measured, one box of 3000 ions: 4000 insertions 100 us
+// unsorted, 214 sorted; 16000 205 and 225; 64000 644 and 179; 256000 2174 and
+// 309.
+constexpr int WS_MIN = 4;
+constexpr long long WS_SITES = 24576;
+// ghost sites sorted at a time over all boxes of a launch (28 bytes each)
+constexpr long long WS_CHUNK = 1LL << 23;
+
+// bins of a box for nent ghost sites: the cells, cut along the longest edge
+// while that leaves WS_FILL sites a bin.  Finer bins keep fewer sites that
+// only the bin's box, not the ghost site, reaches, but pad more slots.
+// Measured, 100000 insertions into each of 48 boxes of 500 to 4000 ions, cut
+// alike along the edges: 2.45 ms at 96 sites, 1.59 ms at 48.
+int3 widom_bins(const WidomArgs& a, double nent) {
+  int m[3] = {1, 1, 1};
+  const int nc[3] = {a.ncx, a.ncy, a.ncz};
+  const double L[3] = {a.Lx, a.Ly, a.Lz};
+  for (;;) {
+    int k = 0;
+    for (int d = 1; d < 3; d++)
+      if (L[d] / (nc[d] * m[d]) > L[k] / (nc[k] * m[k])) k = d;
+    m[k]++;
+    if ((double)nc[0] * m[0] * nc[1] * m[1] * nc[2] * m[2] * WS_FILL > nent) {
+      m[k]--;
+      return make_int3(nc[0] * m[0], nc[1] * m[1], nc[2] * m[2]);
+    }
+  }
+}
+
+WidomPlan widom_plan(const WidomBox* boxes, int nbox, long long n, bool fp64) {
+  WidomPlan P;
+  long long ncell = 0;
+  int nps = 1;
+  for (int i = 0; i < nbox; i++) {
+    const WidomArgs& a = boxes[i].a;
+    ncell = std::max(ncell, (long long)a.ncx * a.ncy * a.ncz);
+    nps = std::max(nps, a.nps);
+  }
+  P.nblk = widom_blocks(n);
+  if (fp64) return P;
+  // insertions a chunk (parts of them are summed by at most as many CTAs as
+  // the part array has room for), boxes a launch
+  P.cn = (int)std::min(n, std::min(WS_CHUNK / nps, (long long)WS_SPAN * PARTITION_SMS * 8));
+  if ((double)P.cn * nps < (double)WS_MIN * ncell || (long long)nbox * P.cn * nps < WS_SITES ||
+      ncell > (1 << 20))
+    return P;
+  const int most = (int)std::max(1LL, std::min((long long)nbox, WS_CHUNK / ((long long)P.cn * nps)));
+  const int groups = (nbox + most - 1) / most;
+  P.boxes = (nbox + groups - 1) / groups;
+  for (int i = 0; i < nbox; i++) {
+    const int3 b = widom_bins(boxes[i].a, (double)P.cn * boxes[i].a.nps);
+    P.nbin = std::max(P.nbin, (size_t)b.x * b.y * b.z);
+  }
+  P.nblk = (P.cn + WS_SPAN - 1) / WS_SPAN;
+  P.nent = (size_t)P.cn * nps;
+  P.nslot = (P.nent + 31 * P.nbin + WD_THREADS - 1) / WD_THREADS * WD_THREADS;
+  P.sorted = true;
+  return P;
+}
+
+size_t WidomPlan::bytes() const {
+  return boxes * (nent * (sizeof(int4) + sizeof(double)) + (nslot + 2 * nbin + 4) * sizeof(int)) + 64;
+}
+
+// the boxes' parts of the workspace
+void widom_layout(const WidomPlan& P, WidomBox* boxes, int nbox, void* work) {
+  const size_t nb = P.boxes;
+  int4* pos = (int4*)work;
+  double* ue = (double*)(pos + nb * P.nent);
+  int* slot = (int*)(ue + nb * P.nent);
+  int* cnt = slot + nb * P.nslot;
+  int* start = cnt + nb * P.nbin;
+  for (int i = 0; i < nbox; i++) {
+    const size_t g = i % nb;
+    const int3 b = widom_bins(boxes[i].a, (double)P.cn * boxes[i].a.nps);
+    boxes[i].nbx = b.x;
+    boxes[i].nby = b.y;
+    boxes[i].nbz = b.z;
+    boxes[i].pos = pos + g * P.nent;
+    boxes[i].ue = ue + g * P.nent;
+    boxes[i].slot = slot + g * P.nslot;
+    boxes[i].cnt = cnt + g * P.nbin;
+    boxes[i].start = start + g * (P.nbin + 1);
+  }
+}
+
+cudaError_t k_widom(const Launch& L, const WidomBox* boxes, int nbox, long long n, bool fp64,
+                    const WidomPlan& P, void* work) {
+  if (P.sorted) {
+    int* slot = (int*)((double*)((int4*)work + P.boxes * P.nent) + P.boxes * P.nent);
+    for (int g = 0; g < nbox; g += P.boxes) {
+      const int ng = std::min(P.boxes, nbox - g);
+      for (long long n0 = 0; n0 < n; n0 += P.cn) {
+        const int cn = (int)std::min((long long)P.cn, n - n0);
+        // slots empty (-1), counts zero
+        cudaError_t e = cudaMemsetAsync(slot, 0xff, P.boxes * P.nslot * sizeof(int), L.s);
+        if (e == cudaSuccess)
+          e = cudaMemsetAsync(slot + P.boxes * P.nslot, 0, P.boxes * P.nbin * sizeof(int), L.s);
+        if (e != cudaSuccess) return e;
+        const unsigned np = (cn + WD_THREADS - 1) / WD_THREADS,
+                       ne = (unsigned)((P.nent + WD_THREADS - 1) / WD_THREADS);
+        widom_place_kernel<<<dim3(np, ng), WD_THREADS, 0, L.s>>>(boxes + g, n0, cn);
+        widom_scan_kernel<<<dim3(1, ng), 1024, 0, L.s>>>(boxes + g);
+        widom_slot_kernel<<<dim3(ne, ng), WD_THREADS, 0, L.s>>>(boxes + g, cn);
+        widom_sorted_kernel<<<dim3((unsigned)(P.nslot / WD_THREADS), ng), WD_THREADS, 0, L.s>>>(boxes + g);
+        widom_finish_kernel<<<dim3(P.nblk, ng), WD_THREADS, 0, L.s>>>(boxes + g, n0, cn);
+        *L.counter += 5;
+      }
+    }
+    return cudaGetLastError();
+  }
   const dim3 grid(widom_blocks(n), nbox);
   if (fp64)
     widom_fp64_kernel<<<grid, WD_THREADS, 0, L.s>>>(boxes);

@@ -82,6 +82,7 @@ struct mg_ctx {
   int *d_ccount = nullptr, *d_ccursor = nullptr;  // cell counts (kept zero), cursors
   int4* d_pj = nullptr;
   double4* d_pd = nullptr;
+  float4* d_pf = nullptr;
   int4* d_stencil = nullptr;
   // group pair kernel: the stencil as z-runs, first group and cell of every
   // group, its grid; nprows = energy rows of the pair kernel (cell or group)
@@ -681,6 +682,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   }
   ctx->nprows = std::max(std::max(ctx->ncell, ctx->ngroup_grid * (ctx->half ? ctx->split : 1)),
                          pair_all_blocks(ns));
+  if (ctx->precision != MG_MIXED) ctx->nprows = pair64_blocks(ns);
 
   // ---- k-vectors (cook's set), sorted into (kx,ky) columns of consecutive kz
   double kappa = p->kappa;
@@ -950,6 +952,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     }
   } else {
     CK(dalloc(&ctx->d_pd, ns));
+    if (!ctx->use_list) CK(dalloc(&ctx->d_pf, ns));
     CK(upload(&ctx->d_ptabd, pd.data(), pd.size()));
     CK(upload(&ctx->d_ert, ert.data(), ert.size()));
     CK(dalloc((double2**)&ctx->d_tab, (size_t)ctx->nq * ctx->row));
@@ -1297,6 +1300,7 @@ PairArgs make_pair_args(mg_ctx* ctx, double* f_dev) {
   pa.small = ctx->small ? 1 : 0;
   pa.nkind = ctx->nkind;
   pa.cell_start = ctx->d_cell_start;
+  pa.key_s = ctx->d_key_s;
   pa.order = ctx->d_order;
   pa.stencil = ctx->d_stencil;
   pa.Lx = ctx->L[0];
@@ -1475,7 +1479,7 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
     }
   } else {
     PROF("gather", k_gather_fp64(L, ns, r_dev, ctx->d_order, ctx->d_kind, ctx->d_mol, ctx->L[0],
-                                 ctx->L[1], ctx->L[2], ctx->d_pd));
+                                 ctx->L[1], ctx->L[2], ctx->d_pd, ctx->d_pf));
     if (ctx->polar) PROF("gather", k_gather_drude(L, ns, r_dev, ctx->d_order, nullptr, ctx->d_pdd));
     if (ctx->use_list) {
       if (rebuild) {
@@ -1488,7 +1492,7 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
                                          ctx->polar));
       nerows = list_blocks(ns, false);
     } else {
-      PROF("pair_fp64", k_pair_fp64(L, pa, ctx->d_pd, ctx->d_ptabd, ctx->d_ert, measure,
+      PROF("pair_fp64", k_pair_fp64(L, pa, ctx->d_pd, ctx->d_pf, ctx->d_ptabd, ctx->d_ert, measure,
                                     ctx->polar));
     }
     if (ctx->nq > 0) {
@@ -1930,7 +1934,7 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_cell_start, ctx->d_ccount, ctx->d_ccursor, ctx->d_spans, ctx->d_gstart,
                   ctx->d_hspans, ctx->d_facc, ctx->d_tcb, ctx->d_nf, ctx->d_nfmem, ctx->d_far,
                   ctx->d_kind3, ctx->d_ctab, ctx->d_ftab, ctx->d_xbase3,
-                  ctx->d_gcell, ctx->d_pj, ctx->d_pd,  ctx->d_stencil,
+                  ctx->d_gcell, ctx->d_pj, ctx->d_pd, ctx->d_pf, ctx->d_stencil,
                   ctx->d_ptabf,  ctx->d_ptabd,   ctx->d_erd,   ctx->d_eru,    ctx->d_ert,
                   ctx->d_epart,  ctx->d_qsite,   ctx->d_qval,  ctx->d_task,   ctx->d_col,
                   ctx->d_kvec,   ctx->d_ekk,     ctx->d_S,     ctx->d_Wf,     ctx->d_Wd,
@@ -2525,6 +2529,7 @@ PairArgs pair_args(mg_ctx* ctx) {
   pa.small = ctx->small ? 1 : 0;
   pa.nkind = ctx->nkind;
   pa.cell_start = ctx->d_cell_start;
+  pa.key_s = ctx->d_key_s;
   pa.order = ctx->d_order;
   pa.stencil = ctx->d_stencil;
   pa.Lx = ctx->L[0];

@@ -122,14 +122,15 @@ cudaError_t k_gather_mixed(const Launch& L, int ns, const double* r, const int* 
                            const int* kind, const int* mol, const double iL[3], int4* pj);
 cudaError_t k_gather_fp64(const Launch& L, int ns, const double* r, const int* order,
                           const int* kind, const int* mol, double Lx, double Ly, double Lz,
-                          double4* pd);
+                          double4* pd, float4* pf);
 // Drude builds: sorted Drude displacements (second half of r)
 cudaError_t k_gather_drude(const Launch& L, int ns, const double* r, const int* order,
                            float4* pdj, double4* pdd);
 
 struct PairArgs {
   int ns, ncx, ncy, ncz, nstencil, nkind;
-  int allpairs;             // one cell: nearest image taken per pair (FP64 path)
+  int allpairs;             // one cell
+  const int* key_s;         // cell of every sorted site (FP64 path)
   int small;                // FP32 path: the all-pairs kernel (pair_all_kernel)
   const int* cell_start;
   const int* order;         // sorted -> site
@@ -168,8 +169,10 @@ struct PairArgs {
 cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj,
                          const PairF* ptab, const float4* erd, const float4* eru,
                          bool measure, bool polar);
-cudaError_t k_pair_fp64(const Launch& L, const PairArgs& a, const double4* pd,
+// pf: the sorted sites {x, y, z, (molecule << 8) | kind} in FP32
+cudaError_t k_pair_fp64(const Launch& L, const PairArgs& a, const double4* pd, const float4* pf,
                         const PairD* ptab, const double* ertab, bool measure, bool polar);
+int pair64_blocks(int ns);   // its energy rows
 
 struct KArgs {
   int nq, nk, ntask, ncol, nchunk;

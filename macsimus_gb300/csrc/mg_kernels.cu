@@ -3,7 +3,7 @@
 //   cell list      k_cell_list: a counting sort of the sites by cell (count,
 //                  scan, scatter, per-cell rank) with the fixed-point site
 //                  records of the FP32 path; k_gather_* for the FP64 path
-//   r-space sum    k_pair_mixed / k_pair_fp64: one CTA per home cell, its warps
+//   r-space sum    k_pair_mixed: one CTA per home cell, its warps
 //                  split the neighbour-cell stencil; neighbour cells are staged
 //                  per warp in shared memory (16-byte loads) and every lane owns
 //                  one home-cell site (full shell: each pair is evaluated from
@@ -309,7 +309,7 @@ cudaError_t k_gather_mixed(const Launch& L, int ns, const double* r, const int* 
 __global__ void gather_fp64_kernel(int ns, const double* __restrict__ r,
                                    const int* __restrict__ order, const int* __restrict__ kind,
                                    const int* __restrict__ mol, double Lx, double Ly, double Lz,
-                                   double4* __restrict__ pd) {
+                                   double4* __restrict__ pd, float4* __restrict__ pf) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ns) return;
   int i = order[t];
@@ -317,13 +317,15 @@ __global__ void gather_fp64_kernel(int ns, const double* __restrict__ r,
   x -= Lx * floor(x / Lx);
   y -= Ly * floor(y / Ly);
   z -= Lz * floor(z / Lz);
-  pd[t] = make_double4(x, y, z, __longlong_as_double((long long)((mol[i] << 8) | kind[i])));
+  const int w = (mol[i] << 8) | kind[i];
+  pd[t] = make_double4(x, y, z, __longlong_as_double((long long)w));
+  if (pf) pf[t] = make_float4((float)x, (float)y, (float)z, __int_as_float(w));
 }
 
 cudaError_t k_gather_fp64(const Launch& L, int ns, const double* r, const int* order,
                           const int* kind, const int* mol, double Lx, double Ly, double Lz,
-                          double4* pd) {
-  gather_fp64_kernel<<<cdiv(ns, 256), 256, 0, L.s>>>(ns, r, order, kind, mol, Lx, Ly, Lz, pd);
+                          double4* pd, float4* pf) {
+  gather_fp64_kernel<<<cdiv(ns, 256), 256, 0, L.s>>>(ns, r, order, kind, mol, Lx, Ly, Lz, pd, pf);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -1613,152 +1615,6 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
   return cudaGetLastError();
 }
 
-template <bool MEASURE, bool POLAR>
-__global__ void __launch_bounds__(PAIR_THREADS)
-    pair_fp64_kernel(PairArgs a, const double4* __restrict__ pd, const PairD* __restrict__ ptab_g,
-                     const double* __restrict__ ert) {
-  __shared__ PairD ptab[MAX_KINDS * MAX_KINDS];
-  __shared__ double4 sj[NWARP][32];
-  __shared__ double4 sjd[POLAR ? NWARP : 1][32];
-  __shared__ double red[NWARP][32][POLAR ? 6 : 3];
-  __shared__ double ered[PAIR_THREADS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nk = a.nkind, ntab = a.ntab;
-  for (int t = threadIdx.x; t < nk * nk; t += PAIR_THREADS) ptab[t] = ptab_g[t];
-  __syncthreads();
-  // one cell (all pairs): the CTA takes 32 sites, its warps batches of all
-  // sites in turn; else the sites of its cell, the warps the stencil
-  const bool one = a.allpairs != 0;
-  const int c = one ? 0 : blockIdx.x;
-  const int cz = c % a.ncz, cy = (c / a.ncz) % a.ncy, cx = c / (a.ncy * a.ncz);
-  const int i0 = one ? 32 * (int)blockIdx.x : a.cell_start[c],
-            ni = (one ? min(a.ns, i0 + 32) : a.cell_start[c + 1]) - i0;
-  const double cq = a.cutoff_sq, sgrid = a.sgrid, alpha = a.alpha;
-  double en[NEN];
-#pragma unroll
-  for (int k = 0; k < NEN; k++) en[k] = 0;
-  for (int ib = 0; ib < ni; ib += 32) {
-    const bool vi = ib + lane < ni;
-    const int ti = i0 + ib + lane;
-    const double4 me = vi ? pd[ti] : make_double4(0, 0, 0, 0);
-    const double4 md = (POLAR && vi) ? a.pdd[ti] : make_double4(0, 0, 0, 0);
-    const long long wi = __double_as_longlong(me.w);
-    const int kind_i = (int)(wi & 255), mol_i = (int)(wi >> 8);
-    double fx = 0, fy = 0, fz = 0, gx = 0, gy = 0, gz = 0;
-    for (int s = one ? 0 : warp; s < a.nstencil; s += NWARP) {
-      const int4 o = a.stencil[s];
-      int x2 = cx + o.x, y2 = cy + o.y, z2 = cz + o.z;
-      double shx = 0, shy = 0, shz = 0;
-      if (x2 < 0) { x2 += a.ncx; shx = -a.Lx; } else if (x2 >= a.ncx) { x2 -= a.ncx; shx = a.Lx; }
-      if (y2 < 0) { y2 += a.ncy; shy = -a.Ly; } else if (y2 >= a.ncy) { y2 -= a.ncy; shy = a.Ly; }
-      if (z2 < 0) { z2 += a.ncz; shz = -a.Lz; } else if (z2 >= a.ncz) { z2 -= a.ncz; shz = a.Lz; }
-      const double xs = me.x - shx, ys = me.y - shy, zs = me.z - shz;
-      const int c2 = (x2 * a.ncy + y2) * a.ncz + z2;
-      const int j0 = a.cell_start[c2], nj = a.cell_start[c2 + 1] - j0;
-      for (int jb = one ? 32 * warp : 0; jb < nj; jb += one ? 32 * NWARP : 32) {
-        if (jb + lane < nj) {
-          sj[warp][lane] = pd[j0 + jb + lane];
-          if (POLAR) sjd[warp][lane] = a.pdd[j0 + jb + lane];
-        }
-        __syncwarp();
-        const int cnt = min(32, nj - jb);
-        for (int jj = 0; jj < cnt; jj++) {
-          const double4 q = sj[warp][jj];
-          double dx = xs - q.x, dy = ys - q.y, dz = zs - q.z;
-          if (a.allpairs) {
-            dx -= a.Lx * rint(dx / a.Lx);
-            dy -= a.Ly * rint(dy / a.Ly);
-            dz -= a.Lz * rint(dz / a.Lz);
-          }
-          const double rr = dx * dx + dy * dy + dz * dz;
-          if (!vi || rr >= cq || j0 + jb + jj == ti) continue;
-          const long long wj = __double_as_longlong(q.w);
-          const PairD& P = ptab[kind_i * nk + (int)(wj & 255)];
-          const bool excl = (int)(wj >> 8) == mol_i;
-          if (!excl && rr < P.C2q) {
-            double f, U;
-            if (rr < P.C1q) {
-              const double x = P.Sq / rr, y = x * x * x, z = y * y;
-              f = P.E24 * (z + z - y) * x;
-              U = P.E4 * (z - y);
-            } else {
-              const double x = rr - P.C2q;
-              f = P.A4 * x;
-              U = x * x * P.A;
-            }
-            fx += f * dx;
-            fy += f * dy;
-            fz += f * dz;
-            if (MEASURE) {
-              en[1] += U;
-              en[2] += rr * f;
-              en[3] += dx * f * dx;
-              en[4] += dy * f * dy;
-              en[5] += dz * f * dz;
-              en[6] += dz * f * dy;
-              en[7] += dx * f * dz;
-              en[8] += dy * f * dx;
-            }
-          }
-          if (P.qq != 0)
-            term64<MEASURE>(dx, dy, dz, P.qq, excl, ert, sgrid, ntab, alpha, fx, fy, fz, en);
-          if (POLAR) {
-            const double4 qd = sjd[warp][jj];
-            if (P.qpc != 0)
-              term64<MEASURE>(dx + md.x, dy + md.y, dz + md.z, P.qpc, excl, ert, sgrid, ntab,
-                              alpha, gx, gy, gz, en);
-            if (P.qcp != 0)
-              term64<MEASURE>(dx - qd.x, dy - qd.y, dz - qd.z, P.qcp, excl, ert, sgrid, ntab,
-                              alpha, fx, fy, fz, en);
-            if (P.qpp != 0)
-              term64<MEASURE>(dx + md.x - qd.x, dy + md.y - qd.y, dz + md.z - qd.z, P.qpp, excl,
-                              ert, sgrid, ntab, alpha, gx, gy, gz, en);
-          }
-        }
-        __syncwarp();
-      }
-    }
-    red[warp][lane][0] = fx;
-    red[warp][lane][1] = fy;
-    red[warp][lane][2] = fz;
-    if (POLAR) {
-      red[warp][lane][POLAR ? 3 : 0] = gx;
-      red[warp][lane][POLAR ? 4 : 0] = gy;
-      red[warp][lane][POLAR ? 5 : 0] = gz;
-    }
-    __syncthreads();
-    if (warp == 0 && vi) {
-      double g[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-      for (int w = 0; w < NWARP; w++)
-#pragma unroll
-        for (int k = 0; k < (POLAR ? 6 : 3); k++) g[k] += red[w][lane][k];
-      const int site = a.order[ti];
-      a.f[3 * site] = g[0];
-      a.f[3 * site + 1] = g[1];
-      a.f[3 * site + 2] = g[2];
-      if (POLAR) {
-        a.f[3 * (long)a.ns + 3 * site] = g[3];
-        a.f[3 * (long)a.ns + 3 * site + 1] = g[4];
-        a.f[3 * (long)a.ns + 3 * site + 2] = g[5];
-      }
-    }
-    __syncthreads();
-  }
-  if (MEASURE) {
-    for (int k = 0; k < 9; k++) {
-      ered[threadIdx.x] = 0.5 * en[k];
-      __syncthreads();
-      for (int w = PAIR_THREADS / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) ered[threadIdx.x] += ered[threadIdx.x + w];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) a.epart[blockIdx.x * NEN + k] = ered[0];
-      __syncthreads();
-    }
-  }
-}
-
 // ------------------------------------------------ Ewald exclusion terms --
 
 // -erf(alpha r)/r of the intramolecular pairs (cook/ljqqnp.c:131-141, its
@@ -1902,25 +1758,6 @@ cudaError_t k_excl_mixed(const Launch& L, const ExclArgs& a, bool measure, bool 
   } else {
     if (polar) excl_mixed_kernel<false, true><<<nb, EXCL_THREADS, 0, L.s>>>(a);
     else excl_mixed_kernel<false, false><<<nb, EXCL_THREADS, 0, L.s>>>(a);
-  }
-  LAUNCHED(L);
-  return cudaGetLastError();
-}
-
-cudaError_t k_pair_fp64(const Launch& L, const PairArgs& a, const double4* pd, const PairD* ptab,
-                        const double* ertab, bool measure, bool polar) {
-  // one cell: a CTA per 32 sites
-  const int ncell = a.allpairs ? cdiv(a.ns, 32) : a.ncx * a.ncy * a.ncz;
-  if (polar) {
-    if (measure)
-      pair_fp64_kernel<true, true><<<ncell, PAIR_THREADS, 0, L.s>>>(a, pd, ptab, ertab);
-    else
-      pair_fp64_kernel<false, true><<<ncell, PAIR_THREADS, 0, L.s>>>(a, pd, ptab, ertab);
-  } else {
-    if (measure)
-      pair_fp64_kernel<true, false><<<ncell, PAIR_THREADS, 0, L.s>>>(a, pd, ptab, ertab);
-    else
-      pair_fp64_kernel<false, false><<<ncell, PAIR_THREADS, 0, L.s>>>(a, pd, ptab, ertab);
   }
   LAUNCHED(L);
   return cudaGetLastError();

@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(BUILD, "libmacgpu.so")
 SOURCES = ["mg_tables.cpp", "mg_kernels.cu", "mg_kspace.cu", "mg_api.cu", "mg_noalloc.cu", "mg_drude.cu", "mg_nlist.cu", "mg_widom.cu", "mg_adjoint.cu", "mg_thermo.cu", "mg_sites.cu", "mg_tc.cu", "mg_kspace_tc.cu", "mg_nufft.cu",
-           "mg_pair64.cu"]
+           "mg_pair64.cu", "mg_kspace64.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

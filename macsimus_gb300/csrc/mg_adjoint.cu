@@ -14,6 +14,7 @@
 //                  dLoss/dq_i = sum_j (g_i - g_j).r_ij e_ij q_j + g_i.F^k_i/q_i
 //                               + sum_k ekk Im(conj(Phi_i(k)) T(k)),
 //                  T(k) = sum_j q_j (g_j.k/L) Phi_j(k)
+// (the k-space parts: mg_kspace64.cu)
 #include "mg_internal.h"
 #include "mg_device.cuh"
 
@@ -154,103 +155,15 @@ __global__ void __launch_bounds__(ADJ_THREADS)
     part[(long)blockIdx.x * nk2 * 6 + t] = 0.5 * acc[t];
 }
 
-// T_d(k) = sum_j g_jd (q_j Phi_j(k)) over a chunk of charges (grid.y)
-__global__ void kadj_T_kernel(KArgs a, const double2* __restrict__ tab, const double* __restrict__ g,
-                              double2* __restrict__ part) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.nk) return;
-  const int4 kv = a.kvec[k];
-  const int ch = blockIdx.y;
-  const int j0 = (int)((long)a.nq * ch / gridDim.y), j1 = (int)((long)a.nq * (ch + 1) / gridDim.y);
-  const int oy = a.Kx + 1 + a.Ky, oz = a.Kx + 2 * a.Ky + 2 + a.Kz;
-  double2 T[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-  for (int j = j0; j < j1; j++) {
-    const double2* R = tab + (long)j * a.row;
-    const double2 X = R[kv.x], Y = R[oy + kv.y], Z = R[oz + kv.z];
-    const double2 A = make_double2(X.x * Y.x - X.y * Y.y, X.x * Y.y + X.y * Y.x);
-    const double2 P = make_double2(A.x * Z.x - A.y * Z.y, A.x * Z.y + A.y * Z.x);
-    const int site = a.qsite[j];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const double w = g[3 * site + d];
-      T[d].x += w * P.x;
-      T[d].y += w * P.y;
-    }
-  }
-#pragma unroll
-  for (int d = 0; d < 3; d++) part[((long)ch * a.nk + k) * 3 + d] = T[d];
-}
-
-// T(k) = sum_d (k_d/L_d) T_d(k), the chunks in a fixed order
-__global__ void kadj_T_reduce_kernel(KArgs a, int nch, const double2* __restrict__ part,
-                                     double2* __restrict__ T) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.nk) return;
-  const int4 kv = a.kvec[k];
-  const double w[3] = {kv.x / a.Lx, kv.y / a.Ly, kv.z / a.Lz};
-  double tx = 0, ty = 0;
-  for (int c = 0; c < nch; c++)
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const double2 v = part[((long)c * a.nk + k) * 3 + d];
-      tx += w[d] * v.x;
-      ty += w[d] * v.y;
-    }
-  T[k] = make_double2(tx, ty);
-}
-
-// per charge: psi (k-space potential), F^k/q, sum_k ekk Im(conj(Phi) T)
-__global__ void kadj_charge_kernel(KArgs a, const double2* __restrict__ tab,
-                                   const double2* __restrict__ T, const double* __restrict__ g,
-                                   double* __restrict__ dEq, double* __restrict__ dLq) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= a.nq) return;
-  const int oy = a.Kx + 1 + a.Ky, oz = a.Kx + 2 * a.Ky + 2 + a.Kz;
-  const double2* R = tab + (long)j * a.row;
-  const double qj = a.qval[j], iq = 1.0 / qj;
-  double psi = 0, fx = 0, fy = 0, fz = 0, kl = 0;
-  for (int k = 0; k < a.nk; k++) {
-    const int4 kv = a.kvec[k];
-    const double2 X = R[kv.x], Y = R[oy + kv.y], Z = R[oz + kv.z];
-    const double2 A = make_double2(X.x * Y.x - X.y * Y.y, X.x * Y.y + X.y * Y.x);
-    const double px = (A.x * Z.x - A.y * Z.y) * iq, py = (A.x * Z.y + A.y * Z.x) * iq;
-    const double sr = a.S[2 * k], si = a.S[2 * k + 1], ek = a.ekk[k];
-    const double2 t = T[k];
-    psi += ek * (sr * px + si * py);
-    const double im = ek * (sr * py - si * px);
-    fx += kv.x * im;
-    fy += kv.y * im;
-    fz += kv.z * im;
-    kl += ek * (px * t.y - py * t.x);
-  }
-  const int site = a.qsite[j];
-  dEq[site] += psi / (2 * 3.14159265358979323846) - 2 * a.alpha / 1.772453850905516 * qj;
-  if (g)
-    dLq[site] += g[3 * site] * fx / a.Lx + g[3 * site + 1] * fy / a.Ly +
-                 g[3 * site + 2] * fz / a.Lz + kl;
-}
-
 static inline int cdiv_a(long a, long b) { return (int)((a + b - 1) / b); }
 
-cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const KArgs& ka, const double4* pd,
-                      const AdjPair* tab, const double* ert, const double2* ptab, const double* g,
-                      const double* q, double4* gs, double* part, double* dEq, double* dLq,
-                      double2* tpart, int ntch, double2* T) {
+cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const double4* pd, const AdjPair* tab,
+                      const double* ert, const double* g, const double* q, double4* gs,
+                      double* part, double* dEq, double* dLq) {
   const int ncell = pa.ncx * pa.ncy * pa.ncz;
   adj_gather_kernel<<<cdiv_a(pa.ns, 256), 256, 0, L.s>>>(pa.ns, pa.order, g, q, gs);
   adj_pair_kernel<<<ncell, ADJ_THREADS, 0, L.s>>>(pa, pd, gs, tab, ert, part, dEq, dLq);
   *L.counter += 2;
-  if (ka.nq > 0 && ka.nk > 0) {
-    if (g) {
-      kadj_T_kernel<<<dim3(cdiv_a(ka.nk, 128), ntch), 128, 0, L.s>>>(ka, ptab, g, tpart);
-      kadj_T_reduce_kernel<<<cdiv_a(ka.nk, 256), 256, 0, L.s>>>(ka, ntch, tpart, T);
-      *L.counter += 2;
-    } else {
-      cudaMemsetAsync(T, 0, sizeof(double2) * ka.nk, L.s);
-    }
-    kadj_charge_kernel<<<cdiv_a(ka.nq, 128), 128, 0, L.s>>>(ka, ptab, T, g, dEq, dLq);
-    *L.counter += 1;
-  }
   return cudaGetLastError();
 }
 

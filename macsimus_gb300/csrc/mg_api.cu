@@ -68,7 +68,7 @@ struct mg_ctx {
   int ncx = 0, ncy = 0, ncz = 0, ncell = 0, nstencil = 0;
   bool allpairs = false;
   int ntab = 0;
-  int Kx = 0, Ky = 0, Kz = 0, row = 0, ntask = 0, ncol = 0, nchunk = 1;
+  int Kx = 0, Ky = 0, Kz = 0, row = 0, nchunk = 1;
   cudaStream_t stream = nullptr;
   // host copies
   std::vector<int> h_kind, h_mol, h_mol_first;
@@ -101,13 +101,11 @@ struct mg_ctx {
   // k-space
   int* d_qsite = nullptr;
   double* d_qval = nullptr;
-  KTask* d_task = nullptr;
-  KCol* d_col = nullptr;
+  K64 k64{};   // FP64 path: the k set and its scratch
   int4* d_kvec = nullptr;
   double* d_ekk = nullptr;
   double* d_S = nullptr;
   float2* d_Wf = nullptr;
-  double2* d_Wd = nullptr;
   void* d_tab = nullptr;   // float2 or double2 rows
   uint4* d_qfix = nullptr; // FP32 path: fixed-point coordinates of the charges
   void* d_part = nullptr;  // float2 or double2 partials
@@ -220,8 +218,7 @@ struct mg_ctx {
   double *d_ag = nullptr, *d_aq = nullptr, *d_apart = nullptr, *d_adEq = nullptr,
          *d_adLq = nullptr;
   double4* d_ags = nullptr;
-  double2 *d_atpart = nullptr, *d_aT = nullptr;
-  int adj_ntch = 0;
+  double* d_apart64 = nullptr;
   std::vector<PairF> h_wtabf;
   std::vector<PairD> h_wtabd;
   std::vector<double> h_wgeom;
@@ -333,6 +330,46 @@ cudaError_t upload(T** p, const T* h, size_t n) {
   cudaError_t e = dalloc(p, n);
   if (e != cudaSuccess || n == 0) return e;
   return cudaMemcpy(*p, h, sizeof(T) * n, cudaMemcpyHostToDevice);
+}
+
+int k64_extent(const KRow& r) { return std::max(std::abs(r.kzlo), std::abs(r.kzhi)); }
+int k64_items(const std::vector<KRow>& krows) {
+  int n = 0;
+  for (const KRow& r : krows) n += k64_extent(r) + 1;
+  return n;
+}
+
+// the k set of the FP64 sums; krows sorted by extent, the largest first
+int setup_k64(mg_ctx* ctx, const std::vector<KRow>& krows) {
+  K64& k = ctx->k64;
+  std::vector<KRow64> rows;
+  std::vector<KTask64> tasks;
+  std::vector<KItem64> items;
+  for (const KRow& r : krows) {
+    const int ext = k64_extent(r), i0 = (int)items.size();
+    for (int z = 0; z <= ext; z++)
+      items.push_back(KItem64{z >= r.kzlo && z <= r.kzhi ? r.kstart + z - r.kzlo : -1,
+                              z > 0 && -z >= r.kzlo && -z <= r.kzhi ? r.kstart - z - r.kzlo : -1, z,
+                              (int)rows.size()});
+    // runs of about equal length
+    const int nrun = (ext + K64_RUN) / K64_RUN;
+    for (int q = 0; q < nrun; q++) {
+      const int z0 = (ext + 1) * q / nrun, z1 = (ext + 1) * (q + 1) / nrun;
+      tasks.push_back(KTask64{r.kx, r.ky, z0, z1 - z0, i0 + z0, {0, 0, 0}});
+    }
+    rows.push_back(KRow64{(double)r.kx, (double)r.ky, r.kx, r.ky, ext, i0});
+  }
+  std::stable_sort(tasks.begin(), tasks.end(),
+                   [](const KTask64& x, const KTask64& y) { return x.n > y.n; });
+  k.nrow = (int)rows.size();
+  k.ntask = (int)tasks.size();
+  k.nitem = (int)items.size();
+  CK(upload((KRow64**)&k.rows, rows.data(), rows.size()));
+  CK(upload((KTask64**)&k.tasks, tasks.data(), tasks.size()));
+  CK(upload((KItem64**)&k.items, items.data(), items.size()));
+  CK(dalloc(&k.part, (size_t)k64_chunks(k.ntask, ctx->nq, false) * k.nitem * 4));
+  CK(dalloc(&k.pm, (size_t)k.nitem));
+  return MG_OK;
 }
 
 // the arguments, tables and grids of the non-uniform transforms
@@ -711,23 +748,16 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     ctx->Ky = std::max(ctx->Ky, std::abs(kvec[i].y));
     ctx->Kz = std::max(ctx->Kz, std::abs(kvec[i].z));
   }
-  std::vector<KCol> cols;
-  std::vector<KTask> tasks;
+  // rows of the tiled k-space kernels: sorted by kz extent, KTR per tile
+  std::vector<KRow> krows;
   for (int i = 0; i < nk;) {
     int j = i + 1;
     while (j < nk && kvec[j].x == kvec[i].x && kvec[j].y == kvec[i].y &&
            kvec[j].z == kvec[j - 1].z + 1)
       j++;
-    cols.push_back(KCol{kvec[i].x, kvec[i].y, kvec[i].z, j - i, i, {0, 0, 0}});
-    for (int s = i; s < j; s += KZT)
-      tasks.push_back(KTask{kvec[s].x, kvec[s].y, kvec[s].z, std::min(KZT, j - s), s, {0, 0, 0}});
+    krows.push_back(KRow{kvec[i].x, kvec[i].y, kvec[i].z, kvec[i].z + (j - i) - 1, i, {0, 0, 0}});
     i = j;
   }
-  ctx->ncol = (int)cols.size();
-  ctx->ntask = (int)tasks.size();
-  // rows of the tiled k-space kernels: sorted by kz extent, KTR per tile
-  std::vector<KRow> krows;
-  for (const KCol& c : cols) krows.push_back(KRow{c.kx, c.ky, c.kz0, c.kz0 + c.n - 1, c.k0, {0, 0, 0}});
   auto extent = [](const KRow& r) { return std::max(std::abs(r.kzlo), std::abs(r.kzhi)); };
   std::stable_sort(krows.begin(), krows.end(),
                    [&](const KRow& x, const KRow& y) { return extent(x) > extent(y); });
@@ -736,12 +766,8 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   for (int r0 = 0; r0 < (int)krows.size(); r0 += KTR) {
     int n = std::min(KTR, (int)krows.size() - r0), R = 0;
     for (int i = r0; i < r0 + n; i++) R = std::max(R, extent(krows[i]));
-    // pass-1 jobs: |kz| chunks of KZC_MIXED over [0, R] (FP32 kernel, both
-    // signs at once) or kz chunks of 16 over [-R, R] (FP64 kernel)
-    if (ctx->precision == MG_MIXED)
-      for (int kz0 = 0; kz0 <= R; kz0 += KZC_MIXED) p1job.push_back(make_int2((int)tiles.size(), kz0));
-    else
-      for (int kz0 = -R; kz0 <= R; kz0 += 16) p1job.push_back(make_int2((int)tiles.size(), kz0));
+    // pass-1 jobs: |kz| chunks of KZC_MIXED over [0, R], both signs at once
+    for (int kz0 = 0; kz0 <= R; kz0 += KZC_MIXED) p1job.push_back(make_int2((int)tiles.size(), kz0));
     tiles.push_back(KTile{r0, n, R, 0});
   }
   ctx->ntile = (int)tiles.size();
@@ -772,18 +798,18 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   ctx->nq = (int)qsite.size();
   ctx->nd = (int)dsite.size();
   ctx->ndblocks = (ctx->nd + 127) / 128;
-  // charge chunks of pass 1: about 8 (FP64 kernel) or 10 (FP32 kernel) CTAs
-  // per SM of a GB300, at least 512 charges each.  Smaller chunks fill the
+  // charge chunks of the FP32 pass 1: about 10 CTAs per SM of a GB300, at least
+  // 512 charges each.  Smaller chunks fill the
   // GPU with one small box but multiply the partial sums the reduction
   // reads (nk x nchunk): a batch of 256 boxes of 500-4000 ions spent more
   // time reducing 64-charge chunks than in pass 1 itself.  The split is
   // fixed by the box, not by the device, so results do not depend on it.
   const int p1ctas = (p->kspace_ctas_per_sm > 0 ? p->kspace_ctas_per_sm
-                                                : (ctx->precision == MG_MIXED ? 10 : 8)) *
+                                                : 10) *
                      PARTITION_SMS;
   ctx->nchunk = std::max(1, std::min(std::max(1, ctx->nq / 512),
                                      (p1ctas + ctx->np1job - 1) / ctx->np1job));
-  ctx->nkblocks = (nk + 255) / 256;
+  ctx->nkblocks = ctx->precision == MG_MIXED ? (nk + 255) / 256 : k64_red_blocks(k64_items(krows));
   const int nfK[3] = {ctx->Kx, ctx->Ky, ctx->Kz};
   // non-uniform transforms (mg_nufft.cu) need the cells of the present
   // positions (no kept lists) and serve the automatic engine
@@ -880,8 +906,6 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   CK(upload(&ctx->d_qsite, qsite.data(), qsite.size()));
   CK(upload(&ctx->d_qval, qval.data(), qval.size()));
   if (ctx->dipole) CK(dalloc(&ctx->d_dippart, 3 * (size_t)dipole_blocks(std::max(ctx->nq, 1))));
-  CK(upload(&ctx->d_task, tasks.data(), tasks.size()));
-  CK(upload(&ctx->d_col, cols.data(), cols.size()));
   CK(upload(&ctx->d_kvec, kvec.data(), kvec.size()));
   CK(upload(&ctx->d_krows, krows.data(), krows.size()));
   ctx->nkrows = (int)krows.size();
@@ -956,8 +980,8 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     CK(upload(&ctx->d_ptabd, pd.data(), pd.size()));
     CK(upload(&ctx->d_ert, ert.data(), ert.size()));
     CK(dalloc((double2**)&ctx->d_tab, (size_t)ctx->nq * ctx->row));
-    CK(dalloc((double2**)&ctx->d_part, (size_t)ctx->nchunk * nk));
-    CK(dalloc(&ctx->d_Wd, nk));
+    int rc = setup_k64(ctx, krows);
+    if (rc) return rc;
   }
   CK(upload(&ctx->d_mol_first, t->mol_first, t->nmol + 1));
   ctx->h_mol_first.assign(t->mol_first, t->mol_first + t->nmol + 1);
@@ -1336,8 +1360,6 @@ KArgs make_kargs(mg_ctx* ctx, double* f_dev) {
   KArgs ka{};
   ka.nq = ctx->nq;
   ka.nk = ctx->nk;
-  ka.ntask = ctx->ntask;
-  ka.ncol = ctx->ncol;
   ka.nchunk = ctx->nchunk;
   ka.Kx = ctx->Kx;
   ka.Ky = ctx->Ky;
@@ -1347,13 +1369,10 @@ KArgs make_kargs(mg_ctx* ctx, double* f_dev) {
   ka.alpha = ctx->alpha;
   ka.qsite = ctx->d_qsite;
   ka.qval = ctx->d_qval;
-  ka.task = ctx->d_task;
-  ka.col = ctx->d_col;
   ka.kvec = ctx->d_kvec;
   ka.ekk = ctx->d_ekk;
   ka.S = ctx->d_S;
   ka.Wf = ctx->d_Wf;
-  ka.Wd = ctx->d_Wd;
   ka.f = f_dev;
   ka.ek_part = ctx->d_ekpart;
   ka.krows = ctx->d_krows;
@@ -1384,7 +1403,9 @@ int tc_upload_slots(mg_ctx* ctx) {
   return MG_OK;
 }
 
-int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) {
+// kforces false (FP64 path): the k-space forces are left out, S(k) is not
+int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure,
+                 bool kforces = true) {
   Launch L = launch(ctx);
   const int ns = ctx->ns;
   ctx->last_r = r_dev;
@@ -1497,9 +1518,8 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure) 
     }
     if (ctx->nq > 0) {
       PROF("phase_tables", k_phase_tables_fp64(L, ka, r_dev, (double2*)ctx->d_tab));
-      PROF("ewald_sk", k_sk_gemm_fp64(L, ka, (const double2*)ctx->d_tab, (double2*)ctx->d_part));
-      PROF("ewald_sk_reduce", k_sk_reduce_fp64(L, ka, (const double2*)ctx->d_part, measure));
-      PROF("ewald_kforce", k_kf_gemm_fp64(L, ka, (const double2*)ctx->d_tab));
+      PROF("ewald_sk", k_sk64(L, ka, ctx->k64, (const double2*)ctx->d_tab, measure));
+      if (kforces) PROF("ewald_kforce", k_kf64(L, ka, ctx->k64, (const double2*)ctx->d_tab));
     }
   }
   // the dipole term (finite epsinf or Yeh-Berkowitz), after the k-space forces
@@ -1936,8 +1956,8 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_kind3, ctx->d_ctab, ctx->d_ftab, ctx->d_xbase3,
                   ctx->d_gcell, ctx->d_pj, ctx->d_pd, ctx->d_pf, ctx->d_stencil,
                   ctx->d_ptabf,  ctx->d_ptabd,   ctx->d_erd,   ctx->d_eru,    ctx->d_ert,
-                  ctx->d_epart,  ctx->d_qsite,   ctx->d_qval,  ctx->d_task,   ctx->d_col,
-                  ctx->d_kvec,   ctx->d_ekk,     ctx->d_S,     ctx->d_Wf,     ctx->d_Wd,
+                  ctx->d_epart,  ctx->d_qsite,   ctx->d_qval,  
+                  ctx->d_kvec,   ctx->d_ekk,     ctx->d_S,     ctx->d_Wf,
                   ctx->d_tab,    ctx->d_part,    ctx->d_ekpart, ctx->d_mol_first,
                   ctx->d_mol_cfirst, ctx->d_cons, ctx->d_bondq, ctx->d_imass, ctx->d_mass,
                   ctx->d_kinpart, ctx->d_meas, ctx->d_dippart, ctx->d_bdrep, ctx->d_driftpart,
@@ -1947,7 +1967,8 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_nlist, ctx->d_ncount, ctx->d_rbuild, ctx->d_dmax,
                   ctx->d_wtabf, ctx->d_wtabd, ctx->d_wgeom, ctx->d_wpart, ctx->d_wbox,
                   ctx->d_qfix, ctx->d_adjtab, ctx->d_ag, ctx->d_aq, ctx->d_apart, ctx->d_adEq,
-                  ctx->d_adLq, ctx->d_ags, ctx->d_atpart, ctx->d_aT, ctx->d_fk,
+                  ctx->d_adLq, ctx->d_ags, ctx->d_apart64, (void*)ctx->k64.rows, (void*)ctx->k64.tasks,
+                  (void*)ctx->k64.items, ctx->k64.part, ctx->k64.pm, ctx->k64.pt, ctx->d_fk,
                   ctx->d_chi, ctx->d_zth, ctx->d_step, ctx->d_nh, ctx->d_vhist, ctx->d_dep_site, ctx->d_dep_first,
                   ctx->d_dep_parent, ctx->d_dep_w, ctx->d_dep_type, ctx->d_dep_par, ctx->d_deppart, ctx->d_plb, ctx->d_xfirst, ctx->d_xpair,
                   ctx->d_xq, ctx->d_za, ctx->d_vb, ctx->d_tcrows, ctx->d_zb, ctx->d_tckrows};
@@ -2034,8 +2055,6 @@ int mg_ewald(mg_ctx* ctx, const double* r, double* f, double* energy) {
   std::memset(&ka, 0, sizeof(ka));
   ka.nq = ctx->nq;
   ka.nk = ctx->nk;
-  ka.ntask = ctx->ntask;
-  ka.ncol = ctx->ncol;
   ka.nchunk = ctx->nchunk;
   ka.Kx = ctx->Kx;
   ka.Ky = ctx->Ky;
@@ -2045,13 +2064,10 @@ int mg_ewald(mg_ctx* ctx, const double* r, double* f, double* energy) {
   ka.alpha = ctx->alpha;
   ka.qsite = ctx->d_qsite;
   ka.qval = ctx->d_qval;
-  ka.task = ctx->d_task;
-  ka.col = ctx->d_col;
   ka.kvec = ctx->d_kvec;
   ka.ekk = ctx->d_ekk;
   ka.S = ctx->d_S;
   ka.Wf = ctx->d_Wf;
-  ka.Wd = ctx->d_Wd;
   ka.f = ctx->d_fs;
   ka.ek_part = ctx->d_ekpart;
   ka.krows = ctx->d_krows;
@@ -2069,9 +2085,8 @@ int mg_ewald(mg_ctx* ctx, const double* r, double* f, double* energy) {
       CK(kf_mixed(ctx, L, ka));
     } else {
       CK(k_phase_tables_fp64(L, ka, ctx->d_rs, (double2*)ctx->d_tab));
-      CK(k_sk_gemm_fp64(L, ka, (const double2*)ctx->d_tab, (double2*)ctx->d_part));
-      CK(k_sk_reduce_fp64(L, ka, (const double2*)ctx->d_part, true));
-      CK(k_kf_gemm_fp64(L, ka, (const double2*)ctx->d_tab));
+      CK(k_sk64(L, ka, ctx->k64, (const double2*)ctx->d_tab, true));
+      CK(k_kf64(L, ka, ctx->k64, (const double2*)ctx->d_tab));
     }
     CK(k_reduce_sum(L, ctx->d_ekpart, ctx->nkblocks, 7, ctx->d_sums + 10));
     if (ctx->dipole)
@@ -2613,21 +2628,30 @@ int mg_adjoint(mg_ctx* ctx, const double* r, const double* g, mg_adjoint_out* ou
     CK(dalloc(&ctx->d_apart, (size_t)ctx->ncell * nk2 * 6));
     CK(dalloc(&ctx->d_adEq, (size_t)ns));
     CK(dalloc(&ctx->d_adLq, (size_t)ns));
-    ctx->adj_ntch = std::max(1, std::min(64, ctx->nq / 256));
-    CK(dalloc(&ctx->d_atpart, (size_t)ctx->adj_ntch * std::max(1, ctx->nk) * 3));
-    CK(dalloc(&ctx->d_aT, (size_t)std::max(1, ctx->nk)));
+    if (ctx->nq > 0) {
+      // the weighted sums of T(k), twice the width of those of S(k)
+      CK(dalloc(&ctx->d_apart64, (size_t)k64_chunks(ctx->k64.ntask, ctx->nq, true) * ctx->k64.nitem * 8));
+      CK(dalloc(&ctx->k64.pt, (size_t)ctx->k64.nitem));
+    }
   }
   ctx->launches = 0;
   const size_t nb = 3 * (size_t)ns * sizeof(double);
   CK(cudaMemcpyAsync(ctx->d_rs, r, nb, cudaMemcpyHostToDevice, ctx->stream));
   if (g) CK(cudaMemcpyAsync(ctx->d_ag, g, nb, cudaMemcpyHostToDevice, ctx->stream));
-  int rc = forces_async(ctx, ctx->d_rs, ctx->d_fs, true);
+  // energies, S(k) and the cell list; of the forces only F^k enters, which the
+  // charge gradients form themselves
+  int rc = forces_async(ctx, ctx->d_rs, ctx->d_fs, true, false);
   if (rc) return rc;
   ctx->need_build = true;
   Launch L = launch(ctx);
-  CK(k_adjoint(L, pair_args(ctx), kspace_args(ctx), ctx->d_pd, ctx->d_adjtab, ctx->d_ert,
-               (const double2*)ctx->d_tab, g ? ctx->d_ag : nullptr, ctx->d_aq, ctx->d_ags,
-               ctx->d_apart, ctx->d_adEq, ctx->d_adLq, ctx->d_atpart, ctx->adj_ntch, ctx->d_aT));
+  CK(k_adjoint(L, pair_args(ctx), ctx->d_pd, ctx->d_adjtab, ctx->d_ert, g ? ctx->d_ag : nullptr,
+               ctx->d_aq, ctx->d_ags, ctx->d_apart, ctx->d_adEq, ctx->d_adLq));
+  if (ctx->nq > 0) {
+    K64 k = ctx->k64;
+    k.part = ctx->d_apart64;
+    CK(k_adjoint64(L, kspace_args(ctx), k, (const double2*)ctx->d_tab, g ? ctx->d_ag : nullptr,
+                   ctx->d_adEq, ctx->d_adLq));
+  }
   std::vector<double> part((size_t)ctx->ncell * nk2 * 6);
   CK(cudaMemcpyAsync(part.data(), ctx->d_apart, sizeof(double) * part.size(),
                      cudaMemcpyDeviceToHost, ctx->stream));

@@ -47,17 +47,6 @@ struct PairFS {
 };
 static_assert(sizeof(PairF) == 80 && sizeof(PairFS) == 48, "PairFS is the head of PairF");
 
-// one k-space task: a run of <=KZT consecutive kz of one (kx,ky) column
-struct KTask {
-  int kx, ky, kz0, n;   // first kz and count
-  int k0;               // index of (kx,ky,kz0) in the k list
-  int pad[3];
-};
-// a (kx,ky) column of the k list
-struct KCol {
-  int kx, ky, kz0, n, k0, pad[3];
-};
-
 // a (kx,ky) row of the k set: kz in [kzlo,kzhi], k index kstart+(kz-kzlo)
 struct KRow {
   int kx, ky, kzlo, kzhi, kstart, pad[3];
@@ -175,20 +164,17 @@ cudaError_t k_pair_fp64(const Launch& L, const PairArgs& a, const double4* pd, c
 int pair64_blocks(int ns);   // its energy rows
 
 struct KArgs {
-  int nq, nk, ntask, ncol, nchunk;
+  int nq, nk, nchunk;
   int Kx, Ky, Kz, row;      // table extents; row = (Kx+1)+(2Ky+1)+(2Kz+1)
   double Lx, Ly, Lz;
   double iLx, iLy, iLz;     // 1 / box edges (set_box)
   double alpha;
   const int* qsite;         // [nq] site of each charge
   const double* qval;       // [nq]
-  const KTask* task;
-  const KCol* col;
   const int4* kvec;         // [nk] kx,ky,kz
   const double* ekk;        // [nk]
   double* S;                // [2*nk] structure factor (FP64)
   float2* Wf;               // [nk] ekk conj(S) for the mixed back-transform (or NULL)
-  double2* Wd;              // [nk] the same in FP64 (or NULL)
   double* f;                // forces (added)
   double* ek_part;          // [nk-blocks * 7] energy + virial partials
   const KRow* krows;        // rows sorted by kz extent
@@ -213,16 +199,41 @@ cudaError_t k_add_forces(const Launch& L, size_t n, const double* fk, double* f)
 cudaError_t k_phase_tables_mixed(const Launch& L, const KArgs& a, const double* r, float2* tab,
                                  uint4* qf);
 cudaError_t k_phase_tables_fp64(const Launch& L, const KArgs& a, const double* r, double2* tab);
-cudaError_t k_sk_mixed(const Launch& L, const KArgs& a, const float2* tab, float2* part);
-cudaError_t k_sk_fp64(const Launch& L, const KArgs& a, const double2* tab, double2* part);
 cudaError_t k_sk_reduce_mixed(const Launch& L, const KArgs& a, const float2* part, bool measure);
-cudaError_t k_sk_reduce_fp64(const Launch& L, const KArgs& a, const double2* part, bool measure);
-cudaError_t k_kforce_mixed(const Launch& L, const KArgs& a, const float2* tab);
-cudaError_t k_kforce_fp64(const Launch& L, const KArgs& a, const double2* tab);
 cudaError_t k_sk_gemm_mixed(const Launch& L, const KArgs& a, const float2* tab, float2* part);
-cudaError_t k_sk_gemm_fp64(const Launch& L, const KArgs& a, const double2* tab, double2* part);
 cudaError_t k_kf_gemm_mixed(const Launch& L, const KArgs& a, const float2* tab);
-cudaError_t k_kf_gemm_fp64(const Launch& L, const KArgs& a, const double2* tab);
+
+// the FP64 sums (mg_kspace64.cu): rows (kx, ky) sorted by their largest |kz|,
+// items (row, |kz|) numbered row by row, tasks of up to K64_RUN items of one
+// row sorted by length
+constexpr int K64_RUN = 7;
+struct KRow64 {
+  double kx, ky;
+  int ikx, iky, ext, item0;   // items item0 + |kz|, |kz| = 0..ext
+};
+struct KTask64 {
+  int kx, ky, z0, n, item0, pad[3];
+};
+struct KItem64 {
+  int kp, km, z, row;         // k of kz = z and of kz = -z (or -1)
+};
+struct K64 {
+  int nrow, ntask, nitem;
+  const KRow64* rows;
+  const KTask64* tasks;
+  const KItem64* items;
+  double* part;               // [chunks][nitem][4] (adjoint: [8])
+  double4* pm;                // [nitem] sums and differences of ekk conj(S) at kz, -kz
+  double4* pt;                // the same of ekk conj(T) (adjoint)
+};
+int k64_chunks(int ntask, int nq, bool adj);
+int k64_red_blocks(int nitem);   // energy rows
+// S(k), {P, M} and (measure) the energy rows; forces added; charge gradients
+// added to dEq, dLq (g or null)
+cudaError_t k_sk64(const Launch& L, const KArgs& a, const K64& k, const double2* tab, bool measure);
+cudaError_t k_kf64(const Launch& L, const KArgs& a, const K64& k, const double2* tab);
+cudaError_t k_adjoint64(const Launch& L, const KArgs& a, K64 k, const double2* tab, const double* g,
+                        double* dEq, double* dLq);
 cudaError_t k_reduce_sum(const Launch& L, const double* part, int nrows, int width, double* out);
 cudaError_t k_reduce_two(const Launch& L, const double* pa, int ra, int wa, double* oa,
                          const double* pb, int rb, int wb, double* ob);
@@ -558,12 +569,10 @@ struct AdjPair {
   double dA, dA4;   // d/dsigma of the smoothing constants
   double eps, sig;  // epsilon > 0 (1 when the pair has no LJ), sigma
 };
-// per cell CTA: kind-pair sums [ncell][nkind^2][6]; per site dE/dq, dLoss/dq;
-// k-space: tpart [ntch][nk][3], T [nk]
-cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const KArgs& ka, const double4* pd,
-                      const AdjPair* tab, const double* ert, const double2* ptab, const double* g,
-                      const double* q, double4* gs, double* part, double* dEq, double* dLq,
-                      double2* tpart, int ntch, double2* T);
+// per cell CTA: kind-pair sums [ncell][nkind^2][6]; per site dE/dq, dLoss/dq
+cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const double4* pd, const AdjPair* tab,
+                      const double* ert, const double* g, const double* q, double4* gs,
+                      double* part, double* dEq, double* dLq);
 
 // one box of a Widom launch (blockIdx.y): its arguments and data
 struct WidomBox {

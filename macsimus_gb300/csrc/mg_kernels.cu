@@ -1892,93 +1892,6 @@ cudaError_t k_phase_tables_fp64(const Launch& L, const KArgs& a, const double* r
   return cudaGetLastError();
 }
 
-template <typename T2>
-struct CplxOps;
-template <>
-struct CplxOps<float2> {
-  typedef float T;
-  static __device__ __forceinline__ float2 mul(float2 a, float2 b) {
-    return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
-  }
-};
-template <>
-struct CplxOps<double2> {
-  typedef double T;
-  static __device__ __forceinline__ double2 mul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-  }
-};
-
-constexpr int SK_THREADS = 256;
-
-// pass 1: each thread owns one task (<=KZT consecutive kz of a column) and
-// sums q X Y Z over the charges of its chunk; charge rows are staged in
-// shared memory STAGE at a time.
-template <typename T2>
-__global__ void __launch_bounds__(SK_THREADS)
-    sk_kernel(KArgs a, const T2* __restrict__ tab, T2* __restrict__ part, int stage) {
-  extern __shared__ unsigned char smem_raw[];
-  T2* rows = reinterpret_cast<T2*>(smem_raw);
-  const int ch = blockIdx.y;
-  const int j0 = (int)((long)a.nq * ch / a.nchunk), j1 = (int)((long)a.nq * (ch + 1) / a.nchunk);
-  const int tk = blockIdx.x * SK_THREADS + threadIdx.x;
-  const bool valid = tk < a.ntask;
-  KTask tsk = valid ? a.task[tk] : KTask{0, 0, 0, 0, 0, {0, 0, 0}};
-  const int ix = tsk.kx, iy = a.Kx + 1 + a.Ky + tsk.ky,
-            iz = a.Kx + 2 * a.Ky + 2 + a.Kz + tsk.kz0;
-  T2 S[KZT];
-#pragma unroll
-  for (int m = 0; m < KZT; m++) S[m] = T2{0, 0};
-  for (int js = j0; js < j1; js += stage) {
-    const int nst = min(stage, j1 - js);
-    __syncthreads();
-    for (int t = threadIdx.x; t < nst * a.row; t += SK_THREADS)
-      rows[t] = tab[(long)js * a.row + t];
-    __syncthreads();
-    if (valid) {
-      for (int jj = 0; jj < nst; jj++) {
-        const T2* R = rows + jj * a.row;
-        const T2 U = CplxOps<T2>::mul(R[ix], R[iy]);
-#pragma unroll
-        for (int m = 0; m < KZT; m++) {
-          if (m < tsk.n) {
-            const T2 Z = R[iz + m];
-            const T2 p = CplxOps<T2>::mul(U, Z);
-            S[m].x += p.x;
-            S[m].y += p.y;
-          }
-        }
-      }
-    }
-  }
-  if (valid) {
-#pragma unroll
-    for (int m = 0; m < KZT; m++)
-      if (m < tsk.n) part[(long)ch * a.nk + tsk.k0 + m] = S[m];
-  }
-}
-
-template <typename T2>
-static cudaError_t launch_sk(const Launch& L, const KArgs& a, const T2* tab, T2* part) {
-  int stage = (int)(40960 / (a.row * sizeof(T2)));
-  if (stage < 1) stage = 1;
-  if (stage > 64) stage = 64;
-  size_t smem = (size_t)stage * a.row * sizeof(T2);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(sk_kernel<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid(cdiv(a.ntask, SK_THREADS), a.nchunk);
-  sk_kernel<T2><<<grid, SK_THREADS, smem, L.s>>>(a, tab, part, stage);
-  LAUNCHED(L);
-  return cudaGetLastError();
-}
-
-cudaError_t k_sk_mixed(const Launch& L, const KArgs& a, const float2* tab, float2* part) {
-  return launch_sk<float2>(L, a, tab, part);
-}
-cudaError_t k_sk_fp64(const Launch& L, const KArgs& a, const double2* tab, double2* part) {
-  return launch_sk<double2>(L, a, tab, part);
-}
-
 // S(k) = sum over chunks (FP64, fixed order); energy and virial per k
 // (sim/ewpass2m.c: E1 = |S|^2 ekk, ptf = 1/kk + (pi/alpha)^2) reduced per block
 template <typename T2>
@@ -2002,7 +1915,6 @@ MG_BODY void sk_reduce_kernel_body(const KArgs& a,
     a.S[2 * k + 1] = si;
     const double ek = a.ekk[k];
     if (a.Wf) a.Wf[k] = make_float2((float)(ek * sr), (float)(-ek * si));
-    if (a.Wd) a.Wd[k] = make_double2(ek * sr, -ek * si);
     if (measure) {
       const int4 kv = a.kvec[k];
       const double kx = kv.x / a.Lx, ky = kv.y / a.Ly, kz = kv.z / a.Lz;
@@ -2041,73 +1953,6 @@ cudaError_t k_sk_reduce_mixed(const Launch& L, const KArgs& a, const float2* par
   LAUNCHED(L);
   return cudaGetLastError();
 }
-cudaError_t k_sk_reduce_fp64(const Launch& L, const KArgs& a, const double2* part, bool measure) {
-  const double pa = 9.869604401089358 / (a.alpha * a.alpha);
-  sk_reduce_kernel<double2><<<cdiv(a.nk, 256), 256, 0, L.s>>>(a, part, measure, pa);
-  LAUNCHED(L);
-  return cudaGetLastError();
-}
-
-// pass 2 (sim/ewpass2.c + sim/ewaldf.c): F_j += sum_k ekk (k/L) Im(conj(S_k) q_j e^{2 pi i k.r_j/L}).
-// One thread per charge; the k list is walked column by column ((kx,ky) with
-// consecutive kz): the phase at the first kz of a column comes from the
-// per-charge rows (X Y Z products), later ones from the recurrence
-// P <- P e^{2 pi i z/L}.  Column sums are FP32, folded into FP64 every
-// KFOLD columns.
-constexpr int KF_THREADS = 128;
-constexpr int KFOLD = 16;
-
-template <typename T2>
-__global__ void __launch_bounds__(KF_THREADS)
-    kforce_kernel(KArgs a, const T2* __restrict__ tab, const T2* __restrict__ W) {
-  typedef typename CplxOps<T2>::T T;
-  const int j = blockIdx.x * KF_THREADS + threadIdx.x;
-  if (j >= a.nq) return;
-  const T2* R = tab + (long)j * a.row;
-  const int oy = a.Kx + 1 + a.Ky, oz = a.Kx + 2 * a.Ky + 2 + a.Kz;
-  const T2 ez = a.Kz >= 1 ? R[oz + 1] : T2{1, 0};
-  double Fx = 0, Fy = 0, Fz = 0;
-  T gx = 0, gy = 0, gz = 0;
-  int nf = 0;
-  for (int c = 0; c < a.ncol; c++) {
-    const KCol col = a.col[c];
-    T2 P = CplxOps<T2>::mul(CplxOps<T2>::mul(R[col.kx], R[oy + col.ky]), R[oz + col.kz0]);
-    T G = 0, Gz = 0;
-    for (int m = 0; m < col.n; m++) {
-      // W_k = ekk conj(S_k): g = ekk Im(conj(S) P)
-      const T2 Wk = W[col.k0 + m];
-      const T g = Wk.x * P.y + Wk.y * P.x;
-      G += g;
-      Gz += (T)(col.kz0 + m) * g;
-      P = CplxOps<T2>::mul(P, ez);
-    }
-    gx += (T)col.kx * G;
-    gy += (T)col.ky * G;
-    gz += Gz;
-    if (++nf == KFOLD) {
-      nf = 0;
-      Fx += gx; Fy += gy; Fz += gz;
-      gx = gy = gz = 0;
-    }
-  }
-  Fx += gx; Fy += gy; Fz += gz;
-  const int site = a.qsite[j];
-  a.f[3 * site] += Fx / a.Lx;
-  a.f[3 * site + 1] += Fy / a.Ly;
-  a.f[3 * site + 2] += Fz / a.Lz;
-}
-
-cudaError_t k_kforce_mixed(const Launch& L, const KArgs& a, const float2* tab) {
-  kforce_kernel<float2><<<cdiv(a.nq, KF_THREADS), KF_THREADS, 0, L.s>>>(a, tab, a.Wf);
-  LAUNCHED(L);
-  return cudaGetLastError();
-}
-cudaError_t k_kforce_fp64(const Launch& L, const KArgs& a, const double2* tab) {
-  kforce_kernel<double2><<<cdiv(a.nq, KF_THREADS), KF_THREADS, 0, L.s>>>(a, tab, a.Wd);
-  LAUNCHED(L);
-  return cudaGetLastError();
-}
-
 // out[k] = sum over rows of part[row*width+k], in a fixed order (one CTA): the
 // warps share the columns, several warps a column where there are fewer
 // columns than warps; lanes take rows in turn; the two tables of a phase in one

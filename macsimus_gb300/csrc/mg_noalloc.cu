@@ -281,7 +281,6 @@ extern "C" int mg_ewald_kspace_noalloc(const double* r_dev, const double* q_dev,
   ka.ekk = ekk;
   ka.S = S;
   ka.Wf = Wf;
-  ka.Wd = nullptr;
   ka.f = f_dev;
   ka.ek_part = ekpart;
   ka.krows = rows;

@@ -13,7 +13,8 @@
 // ends: meeting it once would halve the arithmetic but scatter the reaction in
 // FP64.  (A lane per home site of a cell left most lanes idle and ran each
 // candidate's FP64 branch for a few of them: 1173 us on 864 waters, with energies
-// and virial 1855; this 173 and 307.  Bound by the FP64 pipe.)
+// and virial 1855; this 153 and 306, with 4 warps per CTA 173 and 307.  Bound by
+// the FP64 pipe.)
 #include "mg_internal.h"
 #include "mg_device.cuh"
 #include "mg_pair64.cuh"

@@ -9,7 +9,7 @@
 
 namespace mg {
 
-constexpr int P64_WARPS = 4;
+constexpr int P64_WARPS = 2;
 constexpr int P64_THREADS = 32 * P64_WARPS;
 // a Lennard-Jones term (and charges), charges alone, one molecule
 constexpr int P64_LJ = 0, P64_Q = 1, P64_EXCL = 2;

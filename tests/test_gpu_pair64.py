@@ -1,5 +1,5 @@
 """The FP64 pair kernel (a warp per site, neighbours queued by class) against
-the oracle: site counts around its 4 sites per CTA, grids of one cell and of
+the oracle: site counts around its sites per CTA, grids of one cell and of
 many, a cutoff just short of half the box, kinds without Lennard-Jones term,
 without charge and with neither, Drude shells; measured and plain forces."""
 import numpy as np

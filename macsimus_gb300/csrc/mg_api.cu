@@ -215,6 +215,8 @@ struct mg_ctx {
   WidomWork wwork;
   // adjoint scratch (FP64 contexts)
   AdjPair* d_adjtab = nullptr;
+  std::vector<double> h_adjeps;
+  double *d_arow = nullptr, *d_asums = nullptr;
   double *d_ag = nullptr, *d_aq = nullptr, *d_apart = nullptr, *d_adEq = nullptr,
          *d_adLq = nullptr;
   double4* d_ags = nullptr;
@@ -1403,9 +1405,10 @@ int tc_upload_slots(mg_ctx* ctx) {
   return MG_OK;
 }
 
-// kforces false (FP64 path): the k-space forces are left out, S(k) is not
+// forces false (FP64 path, for the adjoint): the cell list, the sorted sites and
+// S(k) with its energy alone
 int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure,
-                 bool kforces = true) {
+                 bool forces = true) {
   Launch L = launch(ctx);
   const int ns = ctx->ns;
   ctx->last_r = r_dev;
@@ -1512,14 +1515,14 @@ int forces_async(mg_ctx* ctx, const double* r_dev, double* f_dev, bool measure,
       PROF("pair_fp64", k_pair_list_fp64(L, pa, la, ctx->d_pd, ctx->d_ptabd, ctx->d_ert, measure,
                                          ctx->polar));
       nerows = list_blocks(ns, false);
-    } else {
+    } else if (forces) {
       PROF("pair_fp64", k_pair_fp64(L, pa, ctx->d_pd, ctx->d_pf, ctx->d_ptabd, ctx->d_ert, measure,
                                     ctx->polar));
     }
     if (ctx->nq > 0) {
       PROF("phase_tables", k_phase_tables_fp64(L, ka, r_dev, (double2*)ctx->d_tab));
       PROF("ewald_sk", k_sk64(L, ka, ctx->k64, (const double2*)ctx->d_tab, measure));
-      if (kforces) PROF("ewald_kforce", k_kf64(L, ka, ctx->k64, (const double2*)ctx->d_tab));
+      if (forces) PROF("ewald_kforce", k_kf64(L, ka, ctx->k64, (const double2*)ctx->d_tab));
     }
   }
   // the dipole term (finite epsinf or Yeh-Berkowitz), after the k-space forces
@@ -1967,7 +1970,7 @@ int mg_destroy(mg_ctx* ctx) {
                   ctx->d_nlist, ctx->d_ncount, ctx->d_rbuild, ctx->d_dmax,
                   ctx->d_wtabf, ctx->d_wtabd, ctx->d_wgeom, ctx->d_wpart, ctx->d_wbox,
                   ctx->d_qfix, ctx->d_adjtab, ctx->d_ag, ctx->d_aq, ctx->d_apart, ctx->d_adEq,
-                  ctx->d_adLq, ctx->d_ags, ctx->d_apart64, (void*)ctx->k64.rows, (void*)ctx->k64.tasks,
+                  ctx->d_adLq, ctx->d_ags, ctx->d_apart64, ctx->d_arow, ctx->d_asums, (void*)ctx->k64.rows, (void*)ctx->k64.tasks,
                   (void*)ctx->k64.items, ctx->k64.part, ctx->k64.pm, ctx->k64.pt, ctx->d_fk,
                   ctx->d_chi, ctx->d_zth, ctx->d_step, ctx->d_nh, ctx->d_vhist, ctx->d_dep_site, ctx->d_dep_first,
                   ctx->d_dep_parent, ctx->d_dep_w, ctx->d_dep_type, ctx->d_dep_par, ctx->d_deppart, ctx->d_plb, ctx->d_xfirst, ctx->d_xpair,
@@ -2608,7 +2611,7 @@ int mg_adjoint(mg_ctx* ctx, const double* r, const double* g, mg_adjoint_out* ou
                        ctx->h_tA[tb], ctx->comb_rule, &eps, &sig);
         smooth_lj(eps, sig, ctx->C2, &P);
         AdjPair& A = tab[ka * ctx->nkind + kb];
-        A = AdjPair{P.C1q, P.C2q, P.Sq, P.E4, P.A, P.A4, 0, 0, 1, 1};
+        A = AdjPair{P.C1q, P.C2q, P.Sq, P.E4, P.A, P.A4, 0, 0, 1, 1, 1};
         if (eps != 0) {
           const double h = 1e-5 * sig;
           smooth_lj(eps, sig + h, ctx->C2, &Pp);
@@ -2617,15 +2620,20 @@ int mg_adjoint(mg_ctx* ctx, const double* r, const double* g, mg_adjoint_out* ou
           A.dA4 = (Pp.A4 - Pm.A4) / (2 * h) * c6;
           A.eps = -eps;
           A.sig = sig / c6;
+          A.isig = 1 / A.sig;
         }
       }
     CK(upload(&ctx->d_adjtab, tab.data(), tab.size()));
+    ctx->h_adjeps.resize(nk2);
+    for (int t = 0; t < nk2; t++) ctx->h_adjeps[t] = tab[t].eps;
     std::vector<double> q(ns);
     for (int i = 0; i < ns; i++) q[i] = ctx->kind_q[ctx->h_kind[i]];
     CK(upload(&ctx->d_aq, q.data(), q.size()));
     CK(dalloc(&ctx->d_ag, 3 * (size_t)ns));
     CK(dalloc(&ctx->d_ags, (size_t)ns));
-    CK(dalloc(&ctx->d_apart, (size_t)ctx->ncell * nk2 * 6));
+    CK(dalloc(&ctx->d_arow, (size_t)ns * (6 * ctx->nkind + 1)));
+    CK(dalloc(&ctx->d_apart, (size_t)adj_parts(ns) * (6 * nk2 + 1)));
+    CK(dalloc(&ctx->d_asums, (size_t)6 * nk2 + 1));
     CK(dalloc(&ctx->d_adEq, (size_t)ns));
     CK(dalloc(&ctx->d_adLq, (size_t)ns));
     if (ctx->nq > 0) {
@@ -2638,23 +2646,24 @@ int mg_adjoint(mg_ctx* ctx, const double* r, const double* g, mg_adjoint_out* ou
   const size_t nb = 3 * (size_t)ns * sizeof(double);
   CK(cudaMemcpyAsync(ctx->d_rs, r, nb, cudaMemcpyHostToDevice, ctx->stream));
   if (g) CK(cudaMemcpyAsync(ctx->d_ag, g, nb, cudaMemcpyHostToDevice, ctx->stream));
-  // energies, S(k) and the cell list; of the forces only F^k enters, which the
-  // charge gradients form themselves
+  // the cell list, S(k) and the k-space energy; the r-space energies come out of
+  // the gradient's own sums
   int rc = forces_async(ctx, ctx->d_rs, ctx->d_fs, true, false);
   if (rc) return rc;
   ctx->need_build = true;
   Launch L = launch(ctx);
-  CK(k_adjoint(L, pair_args(ctx), ctx->d_pd, ctx->d_adjtab, ctx->d_ert, g ? ctx->d_ag : nullptr,
-               ctx->d_aq, ctx->d_ags, ctx->d_apart, ctx->d_adEq, ctx->d_adLq));
+  CK(k_adjoint(L, pair_args(ctx), ctx->d_pd, ctx->d_pf, ctx->d_adjtab, ctx->d_ert,
+               g ? ctx->d_ag : nullptr, ctx->d_aq, ctx->d_ags, ctx->d_arow, ctx->d_apart,
+               ctx->d_asums, ctx->d_adEq, ctx->d_adLq));
   if (ctx->nq > 0) {
     K64 k = ctx->k64;
     k.part = ctx->d_apart64;
     CK(k_adjoint64(L, kspace_args(ctx), k, (const double2*)ctx->d_tab, g ? ctx->d_ag : nullptr,
                    ctx->d_adEq, ctx->d_adLq));
   }
-  std::vector<double> part((size_t)ctx->ncell * nk2 * 6);
-  CK(cudaMemcpyAsync(part.data(), ctx->d_apart, sizeof(double) * part.size(),
-                     cudaMemcpyDeviceToHost, ctx->stream));
+  std::vector<double> kp((size_t)nk2 * 6 + 1);
+  CK(cudaMemcpyAsync(kp.data(), ctx->d_asums, sizeof(double) * kp.size(), cudaMemcpyDeviceToHost,
+                     ctx->stream));
   if (out->dE_dq)
     CK(cudaMemcpyAsync(out->dE_dq, ctx->d_adEq, sizeof(double) * ns, cudaMemcpyDeviceToHost,
                        ctx->stream));
@@ -2668,15 +2677,22 @@ int mg_adjoint(mg_ctx* ctx, const double* r, const double* g, mg_adjoint_out* ou
   CK(cudaStreamSynchronize(ctx->stream));
   rc = check_status(ctx);
   if (rc) return rc;
+  // every pair was met from both ends; of u and f, which are linear in
+  // epsilon, the derivatives with respect to it
+  for (int m = 0; m < 3; m++) ctx->h_sums[m] = 0;
+  ctx->h_sums[0] = 0.5 * kp[(size_t)6 * nk2];
+  for (int t = 0; t < nk2; t++) {
+    double* v = kp.data() + 6 * t;
+    for (int m = 0; m < 6; m++) v[m] *= 0.5;
+    ctx->h_sums[1] += v[0];
+    ctx->h_sums[2] += v[2];
+    for (int m = 0; m < 6; m += 2) v[m] /= ctx->h_adjeps[t];
+  }
   mg_energy en;
   fill_energy(ctx, &en);
   out->E = en.el + en.lj;
   out->W = en.vir + en.el;
-  // kind pairs (both orders, halves from the kernel) -> type pairs a <= b,
-  // summed over the cell CTAs in a fixed order
-  std::vector<double> kp((size_t)nk2 * 6, 0.0);
-  for (int c = 0; c < ctx->ncell; c++)
-    for (int t = 0; t < nk2 * 6; t++) kp[t] += part[(size_t)c * nk2 * 6 + t];
+  // kind pairs (both orders) -> type pairs a <= b
   double* dst[3] = {out->dE_pair, out->dW_pair, out->dL_pair};
   for (int m = 0; m < 3; m++)
     if (dst[m]) std::memset(dst[m], 0, sizeof(double) * nt * nt * 2);

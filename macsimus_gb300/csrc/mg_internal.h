@@ -568,11 +568,18 @@ struct AdjPair {
   double C1q, C2q, Sq, E4, A, A4;
   double dA, dA4;   // d/dsigma of the smoothing constants
   double eps, sig;  // epsilon > 0 (1 when the pair has no LJ), sigma
+  double isig;      // 1 / sigma
 };
-// per cell CTA: kind-pair sums [ncell][nkind^2][6]; per site dE/dq, dLoss/dq
-cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const double4* pd, const AdjPair* tab,
-                      const double* ert, const double* g, const double* q, double4* gs,
-                      double* part, double* dEq, double* dLq);
+// sums [6 nkind^2 + 1]: per pair of kinds (home site's first) the sums over
+// sites and neighbours of u, du/dsigma, r^2 f, r^2 df/dsigma, g.r f and g.r
+// df/dsigma, and sum q_i psi_i of the r-space potential; per site dE/dq,
+// dLoss/dq.  Scratch: gs [ns], row [ns][6 nkind + 1], part [adj_parts][6
+// nkind^2 + 1]
+int adj_parts(int ns);
+cudaError_t k_adjoint(const Launch& L, const PairArgs& pa, const double4* pd, const float4* pf,
+                      const AdjPair* tab, const double* ert, const double* g, const double* q,
+                      double4* gs, double* row, double* part, double* sums, double* dEq,
+                      double* dLq);
 
 // one box of a Widom launch (blockIdx.y): its arguments and data
 struct WidomBox {

@@ -21,6 +21,44 @@
 
 namespace mg {
 
+// The force arithmetic rounds explicitly (`_rn`): the measuring instantiation
+// also uses the force for the virial, and a product fused in one instantiation
+// and not in the other would move the sites of a measured step differently.
+__device__ __forceinline__ double p64_r2(double dx, double dy, double dz) {
+  return __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
+}
+// force over separation of a pair of charges; energy to en[0]
+template <bool MEASURE, bool EXCL>
+__device__ __forceinline__ double p64_charge(const PairArgs& a, const double* __restrict__ ert,
+                                             double r2, double qq, double* en) {
+  double f, e;
+  if (EXCL) {
+    e = excl_term<double>(r2, a.alpha, &f);
+  } else {
+    const double* p = ert + 6 * min((int)(r2 * a.sgrid), a.ntab - 1);
+    f = __dadd_rn(__ddiv_rn(p[4], __dadd_rn(p[5], r2)), p[3]);
+    e = p[1] / (p[2] + r2) + p[0];
+  }
+  if (MEASURE) en[0] += e * qq;
+  return __dmul_rn(f, qq);
+}
+template <bool MEASURE>
+__device__ __forceinline__ void p64_add(double f, double dx, double dy, double dz, double& fx,
+                                        double& fy, double& fz, double* en) {
+  fx = __fma_rn(f, dx, fx);
+  fy = __fma_rn(f, dy, fy);
+  fz = __fma_rn(f, dz, fz);
+  if (MEASURE) {
+    const double fdx = f * dx, fdy = f * dy, fdz = f * dz;
+    en[3] += dx * fdx;
+    en[4] += dy * fdy;
+    en[5] += dz * fdz;
+    en[6] += dz * fdy;
+    en[7] += dx * fdz;
+    en[8] += dy * fdx;
+  }
+}
+
 template <bool MEASURE, bool POLAR>
 __global__ void __launch_bounds__(P64_THREADS)
     pair64_kernel(const __grid_constant__ PairArgs a, const double4* __restrict__ pd,
@@ -58,48 +96,45 @@ __global__ void __launch_bounds__(P64_THREADS)
       const double dx = p64_image(me.x - q.x, e.y, a.Lx, tight),
                    dy = p64_image(me.y - q.y, e.y >> 2, a.Ly, tight),
                    dz = p64_image(me.z - q.z, e.y >> 4, a.Lz, tight);
-      const double rr = dx * dx + dy * dy + dz * dz;
+      const double rr = p64_r2(dx, dy, dz);
       if (!(rr < a.cutoff_sq)) return;
       const PairD& P = prow[e.y >> 8];
+      constexpr bool excl = CLS == P64_EXCL;
+      double ft = 0;   // the force of the pair, centres, over its separation
       if (CLS == P64_LJ && rr < P.C2q) {
         double f, U;
         if (rr < P.C1q) {
-          const double x = P.Sq / rr, y = x * x * x, z = y * y;
-          f = P.E24 * (z + z - y) * x;
+          const double x = __ddiv_rn(P.Sq, rr), y = __dmul_rn(__dmul_rn(x, x), x),
+                       z = __dmul_rn(y, y);
+          f = __dmul_rn(__dmul_rn(P.E24, __fma_rn(2, z, -y)), x);
           U = P.E4 * (z - y);
         } else {
-          const double x = rr - P.C2q;
-          f = P.A4 * x;
+          const double x = __dadd_rn(rr, -P.C2q);
+          f = __dmul_rn(P.A4, x);
           U = x * x * P.A;
         }
-        fx += f * dx;
-        fy += f * dy;
-        fz += f * dz;
+        ft = f;
         if (MEASURE) {
           en[1] += U;
           en[2] += rr * f;
-          en[3] += dx * f * dx;
-          en[4] += dy * f * dy;
-          en[5] += dz * f * dz;
-          en[6] += dz * f * dy;
-          en[7] += dx * f * dz;
-          en[8] += dy * f * dx;
         }
       }
-      constexpr bool excl = CLS == P64_EXCL;
-      if (P.qq != 0)
-        term64<MEASURE>(dx, dy, dz, P.qq, excl, ert, a.sgrid, a.ntab, a.alpha, fx, fy, fz, en);
+      if (P.qq != 0) ft = __dadd_rn(ft, p64_charge<MEASURE, excl>(a, ert, rr, P.qq, en));
+      p64_add<MEASURE>(ft, dx, dy, dz, fx, fy, fz, en);
       if (POLAR) {
         const double4 qd = a.pdd[e.x];
+        const double ux = dx + md.x, uy = dy + md.y, uz = dz + md.z;
         if (P.qpc != 0)
-          term64<MEASURE>(dx + md.x, dy + md.y, dz + md.z, P.qpc, excl, ert, a.sgrid, a.ntab,
-                          a.alpha, gx, gy, gz, en);
+          p64_add<MEASURE>(p64_charge<MEASURE, excl>(a, ert, p64_r2(ux, uy, uz), P.qpc, en), ux, uy,
+                           uz, gx, gy, gz, en);
+        const double vx = dx - qd.x, vy = dy - qd.y, vz = dz - qd.z;
         if (P.qcp != 0)
-          term64<MEASURE>(dx - qd.x, dy - qd.y, dz - qd.z, P.qcp, excl, ert, a.sgrid, a.ntab,
-                          a.alpha, fx, fy, fz, en);
+          p64_add<MEASURE>(p64_charge<MEASURE, excl>(a, ert, p64_r2(vx, vy, vz), P.qcp, en), vx, vy,
+                           vz, fx, fy, fz, en);
+        const double wx = ux - qd.x, wy = uy - qd.y, wz = uz - qd.z;
         if (P.qpp != 0)
-          term64<MEASURE>(dx + md.x - qd.x, dy + md.y - qd.y, dz + md.z - qd.z, P.qpp, excl, ert,
-                          a.sgrid, a.ntab, a.alpha, gx, gy, gz, en);
+          p64_add<MEASURE>(p64_charge<MEASURE, excl>(a, ert, p64_r2(wx, wy, wz), P.qpp, en), wx, wy,
+                           wz, gx, gy, gz, en);
       }
     };
     p64_walk(a, pf, ti, flag + kind_i * nk, queue[warp], cqf, work);

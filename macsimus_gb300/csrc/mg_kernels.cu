@@ -83,6 +83,7 @@ __global__ void cell_count_kernel(int ns, const double* __restrict__ r, const __
                                   const int* __restrict__ mol, int4* __restrict__ pfix,
                                   int* __restrict__ key, int* __restrict__ count,
                                   int* __restrict__ status) {
+  after_previous();
   cell_count_kernel_body(ns, r, iL.v, ncx, ncy, ncz, kind, mol, pfix, key, count, status,
                          blockIdx.x);
 }
@@ -168,11 +169,13 @@ MG_BODY void cell_scan_kernel_body(int ncell,
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 cell_scan_kernel(int ncell, int* __restrict__ count, int* __restrict__ start, int* __restrict__ cursor, int* __restrict__ gstart) {
+  after_previous();
   cell_scan_kernel_body(ncell, count, start, cursor, gstart, blockIdx.x, 0);
 }
 
 __global__ void cell_scatter_kernel(int ns, const int* __restrict__ key, int* __restrict__ cursor,
                                     int* __restrict__ slot_site) {
+  after_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ns) return;
   slot_site[atomicAdd(cursor + key[i], 1)] = i;
@@ -234,6 +237,7 @@ MG_BODY void cell_order_kernel_body(int ncell,
 
 __global__ void __launch_bounds__(ORDER_THREADS)
 cell_order_kernel(int ncell, const int* __restrict__ start, const int* __restrict__ slot_site, const int4* __restrict__ pfix, int* __restrict__ order, int* __restrict__ key_s, int4* __restrict__ pj, const int* __restrict__ gstart, int* __restrict__ gcell) {
+  after_previous();
   cell_order_kernel_body(ncell, start, slot_site, pfix, order, key_s, pj, gstart, gcell, blockIdx.x, 0);
 }
 
@@ -245,6 +249,7 @@ __global__ void cell_one_kernel(int ns, const double* __restrict__ r, const __gr
                                 int* __restrict__ key_s, int* __restrict__ start,
                                 int* __restrict__ gstart, int4* __restrict__ pj,
                                 int* __restrict__ gcell) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
     start[0] = gstart[0] = 0;
@@ -277,12 +282,12 @@ cudaError_t k_cell_list(const Launch& L, int ns, const double* r, int* status, c
   cell_count_kernel<<<cdiv(ns, 256), 256, 0, L.s>>>(ns, r, il, ncx, ncy, ncz, kind, mol, pfix, key,
                                                     count, status);
   LAUNCHED(L);
-  cell_scan_kernel<<<1, SCAN_THREADS, 0, L.s>>>(ncell, count, start, cursor, gstart);
+  launch_after(L, cell_scan_kernel, 1, SCAN_THREADS, 0, ncell, count, start, cursor, gstart);
   LAUNCHED(L);
-  cell_scatter_kernel<<<cdiv(ns, 256), 256, 0, L.s>>>(ns, key, cursor, slot_site);
+  launch_after(L, cell_scatter_kernel, cdiv(ns, 256), 256, 0, ns, key, cursor, slot_site);
   LAUNCHED(L);
-  cell_order_kernel<<<cdiv(ncell, ORDER_THREADS / 32), ORDER_THREADS, 0, L.s>>>(
-      ncell, start, slot_site, pfix, order, key_s, pj, gstart, gcell);
+  launch_after(L, cell_order_kernel, cdiv(ncell, ORDER_THREADS / 32), ORDER_THREADS, 0, ncell,
+               start, slot_site, pfix, order, key_s, pj, gstart, gcell);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -1023,6 +1028,7 @@ __global__ void __launch_bounds__(ALL_WARPS * 32, POLAR ? 1 : 2)
                     const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
                     const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
                     float sgrid) {
+  after_previous();
   pair_all_kernel_body<MEASURE, POLAR>(a, pj, ptab_g, erd, eru, sx, sy, sz, cq, sgrid, blockIdx.x);
 }
 
@@ -1478,6 +1484,7 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? (POLAR ? 2 : 3) : (POLAR ? 
                            const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
                            const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
                            float sgrid) {
+  after_previous();
   pair_half_kernel_body<MEASURE, POLAR, NW>(a, pj, ptab_g, erd, eru, sx, sy, sz, cq, sgrid,
                                             blockIdx.x);
 }
@@ -1503,6 +1510,7 @@ __device__ __forceinline__ void finish_forces(int ns, int halves, const int* __r
 
 __global__ void finish_forces_kernel(int ns, int halves, const int* __restrict__ order,
                                      long long* __restrict__ facc, double* __restrict__ f) {
+  after_previous();
   finish_forces(ns, halves, order, facc, f);
 }
 
@@ -1522,8 +1530,8 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
       se = cudaFuncSetAttribute(pair_all_kernel<M, P>,                                          \
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);          \
     if (se == cudaSuccess)                                                                      \
-      pair_all_kernel<M, P><<<pair_all_blocks(a.ns), ALL_WARPS * 32, sm, L.s>>>(                \
-          a, pj, ptab, erd, eru, sx, sy, sz, cq, sg);                                           \
+      launch_after(L, pair_all_kernel<M, P>, pair_all_blocks(a.ns), ALL_WARPS * 32, sm, a, pj,  \
+                   ptab, erd, eru, sx, sy, sz, cq, sg);                                         \
   } while (0)
     if (polar) { if (measure) PAIR_ALL(true, true); else PAIR_ALL(false, true); }
     else { if (measure) PAIR_ALL(true, false); else PAIR_ALL(false, false); }
@@ -1551,8 +1559,8 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
 #undef PAIR_HALF
     if (ge != cudaSuccess) return ge;
     LAUNCHED(L);
-    finish_forces_kernel<<<cdiv(a.ns, 256), 256, 0, L.s>>>(a.ns, polar ? 2 : 1, a.order, a.facc,
-                                                           a.f);
+    launch_after(L, finish_forces_kernel, cdiv(a.ns, 256), 256, 0, a.ns, polar ? 2 : 1, a.order,
+                 a.facc, a.f);
     LAUNCHED(L);
     return cudaGetLastError();
   }
@@ -1746,6 +1754,7 @@ MG_BODY void excl_mixed_kernel_body(const ExclArgs& a,
 
 template <bool MEASURE, bool POLAR>
 __global__ void __launch_bounds__(EXCL_THREADS) excl_mixed_kernel(const __grid_constant__ ExclArgs a) {
+  after_previous();
   excl_mixed_kernel_body<MEASURE, POLAR>(a, blockIdx.x, 0);
 }
 
@@ -1753,11 +1762,11 @@ cudaError_t k_excl_mixed(const Launch& L, const ExclArgs& a, bool measure, bool 
   if (a.nmol <= 0) return cudaSuccess;
   const int nb = cdiv(a.nmol, EXCL_THREADS);
   if (measure) {
-    if (polar) excl_mixed_kernel<true, true><<<nb, EXCL_THREADS, 0, L.s>>>(a);
-    else excl_mixed_kernel<true, false><<<nb, EXCL_THREADS, 0, L.s>>>(a);
+    if (polar) launch_after(L, excl_mixed_kernel<true, true>, nb, EXCL_THREADS, 0, a);
+    else launch_after(L, excl_mixed_kernel<true, false>, nb, EXCL_THREADS, 0, a);
   } else {
-    if (polar) excl_mixed_kernel<false, true><<<nb, EXCL_THREADS, 0, L.s>>>(a);
-    else excl_mixed_kernel<false, false><<<nb, EXCL_THREADS, 0, L.s>>>(a);
+    if (polar) launch_after(L, excl_mixed_kernel<false, true>, nb, EXCL_THREADS, 0, a);
+    else launch_after(L, excl_mixed_kernel<false, false>, nb, EXCL_THREADS, 0, a);
   }
   LAUNCHED(L);
   return cudaGetLastError();
@@ -1998,19 +2007,21 @@ struct RedTab {
 };
 __global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const __grid_constant__ RedTab a,
                                                                   const __grid_constant__ RedTab b) {
+  after_previous();
   if (blockIdx.x == 0) reduce_rows_kernel_body(a.part, a.nrows, a.width, a.out, 0, 0);
   else reduce_rows_kernel_body(b.part, b.nrows, b.width, b.out, 0, 0);
 }
 
 cudaError_t k_reduce_sum(const Launch& L, const double* part, int nrows, int width, double* out) {
   const RedTab a{part, nrows, width, out};
-  reduce_rows_kernel<<<1, RED_THREADS, 0, L.s>>>(a, a);
+  launch_after(L, reduce_rows_kernel, 1, RED_THREADS, 0, a, a);
   LAUNCHED(L);
   return cudaGetLastError();
 }
 cudaError_t k_reduce_two(const Launch& L, const double* pa, int ra, int wa, double* oa,
                          const double* pb, int rb, int wb, double* ob) {
-  reduce_rows_kernel<<<2, RED_THREADS, 0, L.s>>>(RedTab{pa, ra, wa, oa}, RedTab{pb, rb, wb, ob});
+  launch_after(L, reduce_rows_kernel, 2, RED_THREADS, 0, RedTab{pa, ra, wa, oa},
+               RedTab{pb, rb, wb, ob});
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -2481,6 +2492,7 @@ MG_BODY void shake_kernel_body(const ShakeArgs& a,
 
 template <bool NOSE, bool MEAS, bool DF>
 __global__ void __launch_bounds__(SH_THREADS) shake_kernel(const __grid_constant__ ShakeArgs a) {
+  after_previous();
   shake_kernel_body<NOSE, MEAS, DF>(a, blockIdx.x, 0);
 }
 
@@ -2490,14 +2502,14 @@ cudaError_t k_shake(const Launch& L, const ShakeArgs& a) {
   do {                                                                    \
     if (a.vhist) {                                                        \
       if (a.meas_part)                                                    \
-        shake_kernel<true, true, DF><<<nb, SH_THREADS, 0, L.s>>>(a);      \
+        launch_after(L, shake_kernel<true, true, DF>, nb, SH_THREADS, 0, a); \
       else                                                                \
-        shake_kernel<true, false, DF><<<nb, SH_THREADS, 0, L.s>>>(a);     \
+        launch_after(L, shake_kernel<true, false, DF>, nb, SH_THREADS, 0, a); \
     } else {                                                              \
       if (a.meas_part)                                                    \
-        shake_kernel<false, true, DF><<<nb, SH_THREADS, 0, L.s>>>(a);     \
+        launch_after(L, shake_kernel<false, true, DF>, nb, SH_THREADS, 0, a); \
       else                                                                \
-        shake_kernel<false, false, DF><<<nb, SH_THREADS, 0, L.s>>>(a);    \
+        launch_after(L, shake_kernel<false, false, DF>, nb, SH_THREADS, 0, a); \
     }                                                                     \
   } while (0)
   if (a.ffsweep) SHAKE_LAUNCH(true);

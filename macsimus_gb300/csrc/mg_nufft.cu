@@ -222,6 +222,7 @@ constexpr int TILE = NF_TILE, SP_WARPS = 8, TP = TILE * TILE * TILE;
 constexpr int SP_ST = 5 * 32 * TILE;
 
 __global__ void __launch_bounds__(SP_WARPS * 32) nf_spread_kernel(const NfBox* __restrict__ boxes) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int ntz = (b.M[2] + TILE - 1) / TILE, nty = (b.M[1] + TILE - 1) / TILE,
             ntx = (b.M[0] + TILE - 1) / TILE;
@@ -387,6 +388,7 @@ constexpr int DF_COLS = 32, DF_THREADS = 256, PL_THREADS = 128, PL_KC = NF_KC;
 
 // G[x][c] -> A[kx][c], c = (y, z)
 __global__ void __launch_bounds__(DF_THREADS) nf_dft_x_kernel(const NfBox* __restrict__ boxes) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int ncol = b.M[1] * b.M[2], c0 = blockIdx.x * DF_COLS, M = b.M[0], H = M / 2, K = b.K[0];
   if (c0 >= ncol) return;
@@ -442,6 +444,7 @@ __global__ void __launch_bounds__(DF_THREADS) nf_dft_x_kernel(const NfBox* __res
 // with the plane in memory between them: 51 us.)
 __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
     nf_plane_kernel(const NfBox* __restrict__ boxes, const bool measure) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int kx = blockIdx.x / NF_CS;
   if (kx > b.K[0]) return;   // the whole cluster
@@ -685,6 +688,7 @@ __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
 
 // A[kx][c] -> G[x][c]: the real part (the half kx >= 0 carries both signs)
 __global__ void __launch_bounds__(DF_THREADS) nf_idft_x_kernel(const NfBox* __restrict__ boxes) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int ncol = b.M[1] * b.M[2], c0 = blockIdx.x * DF_COLS, M = b.M[0], H = M / 2, K = b.K[0];
   if (c0 >= ncol) return;
@@ -800,6 +804,7 @@ constexpr int IT_LD = 2 * TILE, IT_PL = IT_LD * IT_LD;
 
 __global__ void __launch_bounds__(SP_WARPS * 32)
     nf_interp_tile_kernel(const NfBox* __restrict__ boxes, double* __restrict__ f_or_null) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int ntz = (b.M[2] + TILE - 1) / TILE, nty = (b.M[1] + TILE - 1) / TILE,
             ntx = (b.M[0] + TILE - 1) / TILE, tile = blockIdx.x;
@@ -912,6 +917,7 @@ constexpr int IP_WARPS = 4, IP_SITES = 16;
 
 __global__ void __launch_bounds__(IP_WARPS * 32)
     nf_interp_kernel(const NfBox* __restrict__ boxes, double* __restrict__ f_or_null) {
+  after_previous();
   const NfBox& b = boxes[blockIdx.z];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = (blockIdx.x * IP_WARPS + warp) * IP_SITES;
@@ -1139,7 +1145,7 @@ cudaError_t k_nf_forward(const Launch& L, const NfBox* d, int nbox, const NfGrid
   LAUNCHED(L);
   e = nf_smem((const void*)nf_dft_x_kernel, g.sx);
   if (e != cudaSuccess) return e;
-  nf_dft_x_kernel<<<dim3(g.x, 1, nbox), DF_THREADS, g.sx, L.s>>>(d);
+  launch_after(L, nf_dft_x_kernel, dim3(g.x, 1, nbox), DF_THREADS, g.sx, d);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -1147,7 +1153,7 @@ cudaError_t k_nf_forward(const Launch& L, const NfBox* d, int nbox, const NfGrid
 cudaError_t k_nf_modes(const Launch& L, const NfBox* d, int nbox, const NfGrid& g, bool measure) {
   cudaError_t e = nf_smem((const void*)nf_plane_kernel, g.splane);
   if (e != cudaSuccess) return e;
-  nf_plane_kernel<<<dim3(g.plane, 1, nbox), PL_THREADS, g.splane, L.s>>>(d, measure);
+  launch_after(L, nf_plane_kernel, dim3(g.plane, 1, nbox), PL_THREADS, g.splane, d, measure);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -1155,7 +1161,7 @@ cudaError_t k_nf_modes(const Launch& L, const NfBox* d, int nbox, const NfGrid& 
 cudaError_t k_nf_back(const Launch& L, const NfBox* d, int nbox, const NfGrid& g) {
   cudaError_t e = nf_smem((const void*)nf_idft_x_kernel, g.six);
   if (e != cudaSuccess) return e;
-  nf_idft_x_kernel<<<dim3(g.x, 1, nbox), DF_THREADS, g.six, L.s>>>(d);
+  launch_after(L, nf_idft_x_kernel, dim3(g.x, 1, nbox), DF_THREADS, g.six, d);
   LAUNCHED(L);
   return cudaGetLastError();
 }

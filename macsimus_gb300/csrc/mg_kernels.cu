@@ -849,9 +849,8 @@ __device__ __forceinline__ float drude_force_rn(const float4* __restrict__ erd,
   const int ix = min(__float_as_int(__fmaf_rn(r2, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
   const float4 d = __ldg(erd + ix);
   if (MEASURE) {
-    float ee = 0.f;
-    spline_any<true, true>(erd, eru, r2, sgrid, ntab, q, ee);
-    e += ee;
+    const float4 u = __ldg(eru + ix);
+    e += fmaf(u.y, rcp_approx(u.z + r2), u.x) * q;
   }
   return __fmul_rn(__fmaf_rn(d.y, rcp_approx(__fadd_rn(d.z, r2)), d.x), q);
 }
@@ -1068,6 +1067,11 @@ __global__ void __launch_bounds__(ALL_WARPS * 32, POLAR ? 1 : 2)
 // the plain instantiation move the sites identically; the integer sums make
 // the forces bit-reproducible.
 //
+// The virial of a measured evaluation needs no term per pair: the sum of
+// (r_i - r_j) x f_ij over pairs is that of r_i x F_i over the ends, positions
+// from the cell centre, so each candidate and each home site adds six products
+// to compensated sums.
+//
 // Bound by issue (63 %) and the gathers of the erfc table through L1.  Measured:
 // 0.250 ms on 32768 waters (lane per home site 0.363, without the quads and
 // the side-by-side runs 0.267), 42 us on 12544 sites (61), 23 us on 864 waters
@@ -1211,8 +1215,6 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
       float px = 0.f, py = 0.f, pz = 0.f;            // on the candidate
       float ux = 0.f, uy = 0.f, uz = 0.f;            // on its shell
       float e_el = 0.f, e_lj = 0.f, e_vir = 0.f;
-      PvF pv;
-      pv.zero();
       auto pair = [&](const int i, auto full) {
         constexpr bool HEAVY = decltype(full)::value;
         const float4 h = sh[warp][i];
@@ -1255,7 +1257,6 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
           ux = __fmaf_rn(fc, cx2, ux);
           uy = __fmaf_rn(fc, cy2, uy);
           uz = __fmaf_rn(fc, cz2, uz);
-          if (MEASURE) pv.add(cx2, cy2, cz2, fc);
           if (HEAVY) {
             // shell(i) - centre(j), shell(i) - shell(j)
             const float4 md = shd[POLAR ? warp : 0][i];
@@ -1276,25 +1277,20 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
             ux = __fmaf_rn(fd, sx2, ux);
             uy = __fmaf_rn(fd, sy2, uy);
             uz = __fmaf_rn(fd, sz2, uz);
-            if (MEASURE) {
-              pv.add(ex, ey, ez, fp);
-              pv.add(sx2, sy2, sz2, fd);
-            }
           }
         }
         if (MEASURE) {
-          // energies and virial: no effect on the forces; masked, not
-          // branched around, as the forces are
+          // energies: no effect on the forces; masked, not branched around, as
+          // the forces are
           if (HEAVY) {
             const float xt = rr - P.C2q;
             const float u = rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
             e_lj += ok ? u : 0.f;
             e_vir += ok ? rr * flj : 0.f;
           }
-          float e_el_p = 0.f;
-          spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
-          e_el += ok ? e_el_p + e_p : 0.f;
-          pv.add(dx, dy, dz, f);
+          const float4 eu = __ldg(eru + min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) -
+                                                0x4B400000, ntab - 1));
+          e_el += ok ? fmaf(fmaf(eu.y, rcp_approx(eu.z + rr), eu.x), P.qq, e_p) : 0.f;
         }
       };
       // the two quads in one block, their eight chains interleaved
@@ -1321,8 +1317,19 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
       }
       if (MEASURE) {
         es[0].add(e_el); es[1].add(e_lj); es[2].add(e_vir);
-        es[3].add(pv.p0); es[4].add(pv.p1); es[5].add(pv.p2);
-        es[6].add(pv.p3); es[7].add(pv.p4); es[8].add(pv.p5);
+        // the candidate's end of the virial sum of r x F
+        float w[6] = {q.x * px, q.y * py, q.z * pz, q.z * py, q.x * pz, q.y * px};
+        if (POLAR) {
+          const float tx = q.x + qd.x, ty = q.y + qd.y, tz = q.z + qd.z;
+          w[0] = fmaf(tx, ux, w[0]);
+          w[1] = fmaf(ty, uy, w[1]);
+          w[2] = fmaf(tz, uz, w[2]);
+          w[3] = fmaf(tz, uy, w[3]);
+          w[4] = fmaf(tx, uz, w[4]);
+          w[5] = fmaf(ty, ux, w[5]);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) es[3 + k].add(-w[k]);
       }
       __syncwarp();   // the slots read here may be refilled next
     };
@@ -1413,6 +1420,28 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
       }
     }
     if (qn > 0) run(qh, qn);
+
+    if (MEASURE) {
+      // the home sites' end of the virial sum
+#pragma unroll
+      for (int i = 0; i < GS; i++) {
+        const float4 h = sh[warp][i];
+        float w[6] = {h.x * hx[i], h.y * hy[i], h.z * hz[i], h.z * hy[i], h.x * hz[i], h.y * hx[i]};
+        if (POLAR) {
+          const int ip = POLAR ? i : 0;
+          const float4 d = shd[POLAR ? warp : 0][i];
+          const float tx = h.x + d.x, ty = h.y + d.y, tz = h.z + d.z;
+          w[0] = fmaf(tx, gx[ip], w[0]);
+          w[1] = fmaf(ty, gy[ip], w[1]);
+          w[2] = fmaf(tz, gz[ip], w[2]);
+          w[3] = fmaf(tz, gy[ip], w[3]);
+          w[4] = fmaf(tx, gz[ip], w[4]);
+          w[5] = fmaf(ty, gx[ip], w[5]);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) es[3 + k].add(w[k]);
+      }
+    }
 
     // the home sites' sums: lane 3 i + d ends with component d of slot i
     unsigned long long* facc = reinterpret_cast<unsigned long long*>(a.facc);

@@ -71,10 +71,13 @@ class Energy(C.Structure):
     _tensors = ("Pvir", "Pkin", "Ptens")
 
     def asdict(self):
-        d = {k: getattr(self, k) for k, _ in self._fields_ if k not in self._tensors}
+        d = {k: getattr(self, k) for k in self._numbers}
         for k in self._tensors:
-            d[k] = list(getattr(self, k))
+            d[k] = getattr(self, k)[:]
         return d
+
+
+Energy._numbers = tuple(k for k, _ in Energy._fields_ if k not in Energy._tensors)
 
 
 class AdjointOut(C.Structure):
@@ -192,6 +195,15 @@ def fp32_peak_tflops():
 
 def _arr(a, dt):
     return np.ascontiguousarray(a, dtype=dt)
+
+
+def _ptr(a, ct=C.c_double):
+    """a pointer argument to a contiguous array (ndarray.ctypes.data_as takes
+    4 us, a good part of a small call; this a fifth of it)"""
+    try:
+        return C.byref(ct.from_buffer(a))
+    except (TypeError, ValueError, BufferError):   # read-only or empty
+        return a.ctypes.data_as(C.POINTER(ct))
 
 
 def describe(system, L, cutoff, alpha, kappa, precision="mixed", LJcutoff=None, grid=256,
@@ -369,7 +381,7 @@ class ForcePath:
         r = _arr(r, np.float64).reshape(-1)
         f = np.empty_like(r)
         en = Energy()
-        self._check(library().mg_forces(self._ctx, r.ctypes.data_as(_dp), f.ctypes.data_as(_dp),
+        self._check(library().mg_forces(self._ctx, _ptr(r), _ptr(f),
                                         int(measure), C.byref(en)))
         return f.reshape(-1, 3), (en.asdict() if measure else None)
 
@@ -385,7 +397,7 @@ class ForcePath:
         r = _arr(r, np.float64).reshape(-1)
         f = np.zeros_like(r)
         e = C.c_double()
-        self._check(library().mg_ewald(self._ctx, r.ctypes.data_as(_dp), f.ctypes.data_as(_dp),
+        self._check(library().mg_ewald(self._ctx, _ptr(r), _ptr(f),
                                        C.byref(e)))
         return f.reshape(-1, 3), e.value
 
@@ -402,16 +414,14 @@ class ForcePath:
                         getattr(e, k)[m] = v[m]
                 else:
                     setattr(e, k, v)
-        self._check(library().mg_selffield(self._ctx, r.ctypes.data_as(_dp),
-                                           f.ctypes.data_as(_dp), omega, int(en is not None),
+        self._check(library().mg_selffield(self._ctx, _ptr(r), _ptr(f), omega, int(en is not None),
                                            C.byref(e)))
         return r.reshape(-1, 3), f.reshape(-1, 3), (e.asdict() if en is not None else None)
 
     def md_set_state(self, r, r1):
         r = _arr(r, np.float64).reshape(-1)
         r1 = _arr(r1, np.float64).reshape(-1)
-        self._check(library().mg_md_set_state(self._ctx, r.ctypes.data_as(_dp),
-                                              r1.ctypes.data_as(_dp)))
+        self._check(library().mg_md_set_state(self._ctx, _ptr(r), _ptr(r1)))
 
     def md_get_state(self, out=None):
         """(r, r1) of the device MD state; out = (r, r1): contiguous float64
@@ -424,8 +434,7 @@ class ForcePath:
             for a in (r, r1):
                 if a.dtype != np.float64 or a.size != nv or not a.flags.c_contiguous:
                     raise ValueError("out arrays must be contiguous float64 of %d values" % nv)
-        self._check(library().mg_md_get_state(self._ctx, r.ctypes.data_as(_dp),
-                                              r1.ctypes.data_as(_dp)))
+        self._check(library().mg_md_get_state(self._ctx, _ptr(r), _ptr(r1)))
         return r.reshape(-1, 3), r1.reshape(-1, 3)
 
     def md_load_cfg(self, path):
@@ -474,7 +483,7 @@ class ForcePath:
         w = {"plb": 0, "vlb": 1, "dlb": 2}[what]
         fr = np.empty(3 * (self.ns + 1), np.float32)
         self._check(library().mg_playback_frame(self._ctx, w, int(flags),
-                                                fr.ctypes.data_as(C.POINTER(C.c_float))))
+                                                _ptr(fr, C.c_float)))
         fr = fr.reshape(-1, 3)
         return fr[0].copy(), fr[1:]
 
@@ -551,8 +560,7 @@ class ForcePath:
         dEq, dLq = np.zeros(self.ns), np.zeros(self.ns)
         out = AdjointOut(0.0, 0.0, dEp.ctypes.data_as(_dp), dWp.ctypes.data_as(_dp),
                          dLp.ctypes.data_as(_dp), dEq.ctypes.data_as(_dp), dLq.ctypes.data_as(_dp))
-        self._check(library().mg_adjoint(self._ctx, r.ctypes.data_as(_dp),
-                                         gg.ctypes.data_as(_dp) if gg is not None else None,
+        self._check(library().mg_adjoint(self._ctx, _ptr(r), _ptr(gg) if gg is not None else None,
                                          C.byref(out)))
         sh = (nt, nt, 2)
         return dict(E=out.E, W=out.W, dEp=dEp.reshape(sh), dWp=dWp.reshape(sh),

@@ -2261,8 +2261,8 @@ int mg_md_steps(mg_ctx* ctx, int nsteps, mg_energy* en) {
 namespace {
 
 // Widom set-up of one box: checks, the ghost-site x site-kind pair table and
-// the ghost geometry uploaded (on the context's stream), the cutoff
-// correction, and the launch descriptor
+// the ghost geometry (in the context, on the host), the cutoff correction, and
+// the launch descriptor but for the places of these and of the sums
 int widom_prepare(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigned long long seed,
                   double T, double* d_U, WidomBox* box, double* corr_out) {
   if (!ctx || !probe) return fail(ctx, MG_ERR_ARG, "null argument");
@@ -2286,8 +2286,8 @@ int widom_prepare(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigne
   // the cutoff correction over all (ghost site, box site) pairs
   std::vector<PairF>& tf = ctx->h_wtabf;
   std::vector<PairD>& td = ctx->h_wtabd;
-  tf.assign(MAX_WPROBE * MAX_KINDS, PairF{});
-  td.assign(MAX_WPROBE * MAX_KINDS, PairD{});
+  tf.assign((size_t)nps * ctx->nkind, PairF{});
+  td.assign((size_t)nps * ctx->nkind, PairD{});
   double corr = 0;
   for (int s = 0; s < nps; s++) {
     const int ta = probe->site_type[s];
@@ -2316,22 +2316,7 @@ int widom_prepare(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigne
                                      0.f, 0.f, 0.f, 0.f, qq, 0, 0, 0};
     }
   }
-  if (!ctx->d_wgeom) {
-    CK(dalloc(&ctx->d_wgeom, 3 * MAX_WPROBE));
-    CK(dalloc(&ctx->d_wpart, PARTITION_SMS * 8));
-    CK(dalloc(&ctx->d_wtabf, MAX_WPROBE * MAX_KINDS));
-    CK(dalloc(&ctx->d_wtabd, MAX_WPROBE * MAX_KINDS));
-    CK(dalloc(&ctx->d_wbox, 1));
-  }
   ctx->h_wgeom.assign(probe->geometry, probe->geometry + 3 * nps);
-  CK(cudaMemcpyAsync(ctx->d_wgeom, ctx->h_wgeom.data(), sizeof(double) * 3 * nps,
-                     cudaMemcpyHostToDevice, ctx->stream));
-  if (ctx->precision == MG_MIXED)
-    CK(cudaMemcpyAsync(ctx->d_wtabf, tf.data(), sizeof(PairF) * tf.size(), cudaMemcpyHostToDevice,
-                       ctx->stream));
-  else
-    CK(cudaMemcpyAsync(ctx->d_wtabd, td.data(), sizeof(PairD) * td.size(), cudaMemcpyHostToDevice,
-                       ctx->stream));
   WidomArgs& w = box->a;
   w.n = ninsert;
   w.seed = seed;
@@ -2351,16 +2336,36 @@ int widom_prepare(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigne
   w.Lz = ctx->L[2];
   w.cutoff_sq = ctx->cutoff * ctx->cutoff;
   w.sgrid = ctx->sgrid;
-  w.geom = ctx->d_wgeom;
   w.U = d_U;
-  w.part = ctx->d_wpart;
   box->pj = ctx->d_pj;
   box->pd = ctx->d_pd;
-  box->tabf = ctx->d_wtabf;
-  box->tabd = ctx->d_wtabd;
   box->eru = ctx->d_eru;
   box->ert = ctx->d_ert;
   *corr_out = corr;
+  return MG_OK;
+}
+
+// the tables of widom_prepare uploaded on the context's stream
+int widom_upload(mg_ctx* ctx, WidomBox* box) {
+  if (!ctx->d_wgeom) {
+    CK(dalloc(&ctx->d_wgeom, 3 * MAX_WPROBE));
+    CK(dalloc(&ctx->d_wpart, PARTITION_SMS * 8));
+    CK(dalloc(&ctx->d_wtabf, MAX_WPROBE * MAX_KINDS));
+    CK(dalloc(&ctx->d_wtabd, MAX_WPROBE * MAX_KINDS));
+    CK(dalloc(&ctx->d_wbox, 1));
+  }
+  CK(cudaMemcpyAsync(ctx->d_wgeom, ctx->h_wgeom.data(), sizeof(double) * ctx->h_wgeom.size(),
+                     cudaMemcpyHostToDevice, ctx->stream));
+  if (ctx->precision == MG_MIXED)
+    CK(cudaMemcpyAsync(ctx->d_wtabf, ctx->h_wtabf.data(), sizeof(PairF) * ctx->h_wtabf.size(),
+                       cudaMemcpyHostToDevice, ctx->stream));
+  else
+    CK(cudaMemcpyAsync(ctx->d_wtabd, ctx->h_wtabd.data(), sizeof(PairD) * ctx->h_wtabd.size(),
+                       cudaMemcpyHostToDevice, ctx->stream));
+  box->a.geom = ctx->d_wgeom;
+  box->a.part = ctx->d_wpart;
+  box->tabf = ctx->d_wtabf;
+  box->tabd = ctx->d_wtabd;
   return MG_OK;
 }
 
@@ -2387,6 +2392,7 @@ int mg_widom(mg_ctx* ctx, const mg_probe* probe, long long ninsert, unsigned lon
   WidomBox box;
   double corr = 0;
   int rc = widom_prepare(ctx, probe, ninsert, seed, T, d_U, &box, &corr);
+  if (!rc) rc = widom_upload(ctx, &box);
   if (rc) {
     if (d_U) cudaFree(d_U);
     return rc;
@@ -2846,8 +2852,8 @@ struct mg_batch {
   cudaEvent_t ev_fork = nullptr;
   cudaGraphExec_t g_step = nullptr, g_meas = nullptr;
   int launches_step = 0, launches = 0;
-  WidomBox* d_wbox = nullptr;
-  int wcap = 0;
+  char* d_wmem = nullptr;   // Widom descriptors, sums and tables of all boxes
+  size_t wcap = 0;
   WidomWork wwork;
   // one launch per kernel over all boxes, when every box qualifies
   // (fused_ok): the boxes' kernel arguments on the device, the largest
@@ -2977,7 +2983,7 @@ int mg_batch_destroy(mg_batch* b) {
   if (b->d_statp) cudaFree(b->d_statp);
   if (b->d_stat) cudaFree(b->d_stat);
   if (b->h_stat) cudaFreeHost(b->h_stat);
-  if (b->d_wbox) cudaFree(b->d_wbox);
+  if (b->d_wmem) cudaFree(b->d_wmem);
   b->wwork.release();
   for (cudaEvent_t e : b->ev_join)
     if (e) cudaEventDestroy(e);
@@ -3350,12 +3356,6 @@ int mg_batch_widom(mg_batch* b, const mg_probe* probes, int probe_per_box, long 
       return bfail(b, MG_ERR_ARG, "all boxes of a batch need the same precision");
   }
   for (cudaStream_t s : b->lanes) BCK(cudaStreamSynchronize(s));
-  if (b->wcap < nbox) {
-    if (b->d_wbox) cudaFree(b->d_wbox);
-    b->d_wbox = nullptr;
-    BCK(cudaMalloc((void**)&b->d_wbox, sizeof(WidomBox) * nbox));
-    b->wcap = nbox;
-  }
   const bool fp64 = b->box[0]->precision != MG_MIXED;
   WidomPlan plan = widom_plan(desc.data(), nbox, ninsert, fp64);
   if (plan.sorted && !b->wwork.fit(plan.bytes())) {
@@ -3363,17 +3363,47 @@ int mg_batch_widom(mg_batch* b, const mg_probe* probes, int probe_per_box, long 
     plan.nblk = widom_blocks(ninsert);
   }
   if (plan.sorted) widom_layout(plan, desc.data(), nbox, b->wwork.mem);
-  BCK(cudaMemcpyAsync(b->d_wbox, desc.data(), sizeof(WidomBox) * nbox, cudaMemcpyHostToDevice,
-                      b->main));
+  const int nblk = plan.nblk;
+  // one block of device memory: the descriptors, the sums, and every box's
+  // geometry and pair table; one copy in and one back (three small copies a box
+  // took 0.8 ms for 48 boxes)
+  const size_t tab = fp64 ? sizeof(PairD) : sizeof(PairF);
+  size_t at = (sizeof(WidomBox) * nbox + 255) / 256 * 256;
+  const size_t at_part = at;
+  at += (sizeof(double) * nblk * nbox + 255) / 256 * 256;
+  std::vector<size_t> place(nbox);
+  for (int i = 0; i < nbox; i++) {
+    place[i] = at;
+    at += (sizeof(double) * 3 * MAX_WPROBE + tab * desc[i].a.nps * desc[i].a.nkind + 255) / 256 * 256;
+  }
+  if (b->wcap < at) {
+    if (b->d_wmem) cudaFree(b->d_wmem);
+    b->d_wmem = nullptr;
+    b->wcap = 0;
+    BCK(cudaMalloc((void**)&b->d_wmem, at));
+    b->wcap = at;
+  }
+  std::vector<char> host(at);
+  for (int i = 0; i < nbox; i++) {
+    const mg_ctx* c = b->box[i];
+    const size_t pt = place[i] + sizeof(double) * 3 * MAX_WPROBE;
+    std::memcpy(&host[place[i]], c->h_wgeom.data(), sizeof(double) * c->h_wgeom.size());
+    if (fp64) std::memcpy(&host[pt], c->h_wtabd.data(), tab * c->h_wtabd.size());
+    else std::memcpy(&host[pt], c->h_wtabf.data(), tab * c->h_wtabf.size());
+    desc[i].a.geom = (const double*)(b->d_wmem + place[i]);
+    desc[i].a.part = (double*)(b->d_wmem + at_part) + (size_t)i * nblk;
+    desc[i].tabf = (const PairF*)(b->d_wmem + pt);
+    desc[i].tabd = (const PairD*)(b->d_wmem + pt);
+  }
+  std::memcpy(host.data(), desc.data(), sizeof(WidomBox) * nbox);
+  BCK(cudaMemcpyAsync(b->d_wmem, host.data(), at, cudaMemcpyHostToDevice, b->main));
   int cnt = 0;
   Launch L{b->main, &cnt};
-  BCK(k_widom(L, b->d_wbox, nbox, ninsert, fp64, plan, b->wwork.mem));
+  BCK(k_widom(L, (const WidomBox*)b->d_wmem, nbox, ninsert, fp64, plan, b->wwork.mem));
   b->launches = cnt;
-  const int nblk = plan.nblk;
   std::vector<double> part((size_t)nblk * nbox);
-  for (int i = 0; i < nbox; i++)
-    BCK(cudaMemcpyAsync(part.data() + (size_t)i * nblk, b->box[i]->d_wpart, sizeof(double) * nblk,
-                        cudaMemcpyDeviceToHost, b->main));
+  BCK(cudaMemcpyAsync(part.data(), b->d_wmem + at_part, sizeof(double) * part.size(),
+                      cudaMemcpyDeviceToHost, b->main));
   BCK(cudaStreamSynchronize(b->main));
   for (int i = 0; i < nbox; i++)
     widom_result(b->box[i], part.data() + (size_t)i * nblk, nblk, ninsert, T, corr[i], &out[i]);

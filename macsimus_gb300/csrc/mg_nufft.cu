@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32) nf_spread_kernel(const NfBox* _
 // round trip per few steps, 20 us on 32768 waters), a warp per chunk of
 // outputs.
 constexpr int DF_COLS = 32, DF_THREADS = 256, PL_THREADS = 128, PL_KC = NF_KC;
+constexpr int NF_CSB = 2, NF_TB = 256;   // CTAs a plane and their threads in a batch
 
 // G[x][c] -> A[kx][c], c = (y, z)
 __global__ void __launch_bounds__(DF_THREADS) nf_dft_x_kernel(const NfBox* __restrict__ boxes) {
@@ -442,53 +443,59 @@ __global__ void __launch_bounds__(DF_THREADS) nf_dft_x_kernel(const NfBox* __res
 // shared memory.  Measured, the energy and virial sums of the plane.
 // (One CTA per plane: 26 us on 32768 waters, 21 SMs at work; three launches
 // with the plane in memory between them: 51 us.)
-__global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
+// CS CTAs of T threads a plane: four of 128 for one box, whose planes are too few
+// for the GPU; two of 256 for the plain steps of a batch that fills it, which
+// copy the tables half as often and sum more items each (256 ionic boxes 625 ->
+// 533 us; one of 512 535 us; tables through L1 instead 714).  Every sum of the
+// modes and of the grid is a thread's own, so the split does not change them; it
+// would change the order of the energy sums, and a measured step keeps four.
+template <int CS, int T>
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(T)
     nf_plane_kernel(const NfBox* __restrict__ boxes, const bool measure) {
   after_previous();
   const NfBox& b = boxes[blockIdx.z];
-  const int kx = blockIdx.x / NF_CS;
+  const int kx = blockIdx.x / CS;
   if (kx > b.K[0]) return;   // the whole cluster
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = cluster.block_rank();
   const int My = b.M[1], Mz = b.M[2], Hy = My / 2, Hz = Mz / 2, Ky = b.K[1], Kz = b.K[2],
             NY = 2 * Ky + 1, ld = Mz + 1;   // odd row length: no bank conflicts along ky
-  const int nzq = Mz / NF_CS, zq = rank * nzq;          // this CTA's columns z
-  const int nrow = (NY + NF_CS - 1) / NF_CS, r0 = rank * nrow,
+  const int nzq = Mz / CS, zq = rank * nzq;          // this CTA's columns z
+  const int nrow = (NY + CS - 1) / CS, r0 = rank * nrow,
             nr = max(0, min(nrow, NY - r0));            // and rows ky
   extern __shared__ float4 zs[];
   // the four tables: y forwards, z forwards, z backwards, y backwards
   const int nky = Ky / PL_KC + 1, nkz = Kz / 2 + 1, nz = Hz / 2 + 1, ny = Hy / PL_KC + 1;
   const int n0 = nky * (Hy + 1) * (PL_KC / 2), n1 = nkz * (Hz + 1), n2 = nz * (Kz + 1),
             n3 = ny * (Ky + 1) * (PL_KC / 2);
-  float4* tab0 = zs;
-  float4* tab1 = tab0 + n0;
-  float4* tab2 = tab1 + n1;
-  float4* tab3 = tab2 + n2;
-  float4* pm = tab3 + n3;                                    // [Kz + 1][nrow]
+  const float4 *tab0 = zs, *tab1 = tab0 + n0, *tab2 = tab1 + n1, *tab3 = tab2 + n2;
+  float4* pm = zs + n0 + n1 + n2 + n3;                       // [Kz + 1][nrow]
   float2* rows = reinterpret_cast<float2*>(pm + (Kz + 1) * nrow);  // [nrow][ld]
   float2* cols = rows + nrow * ld + (nrow * ld & 1);         // [max(My, NY)][nzq]
-  __shared__ double red[7][PL_THREADS / 32];
+  __shared__ double red[7][T / 32];
   float2* A = b.A + (long)kx * My * Mz;
   {
-    const float4* src[4] = {
-        reinterpret_cast<const float4*>(b.fwd[1]), reinterpret_cast<const float4*>(b.fwd[2]),
-        reinterpret_cast<const float4*>(b.inv[2]), reinterpret_cast<const float4*>(b.inv[1])};
-    float4* dst[4] = {tab0, tab1, tab2, tab3};
-    const int n[4] = {n0, n1, n2, n3};
     // this CTA's columns (nzq may be odd: 8-byte copies), then the tables
-    for (int i = threadIdx.x; i < My * nzq; i += PL_THREADS) {
+    for (int i = threadIdx.x; i < My * nzq; i += T) {
       const int y = i / nzq;
       nf_copy8(cols + i, A + y * Mz + zq + i - y * nzq);
     }
+    const float4* src[4] = {
+        reinterpret_cast<const float4*>(b.fwd[1]), reinterpret_cast<const float4*>(b.fwd[2]),
+        reinterpret_cast<const float4*>(b.inv[2]), reinterpret_cast<const float4*>(b.inv[1])};
+    const int n[4] = {n0, n1, n2, n3};
+    float4* dst = zs;
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      for (int i = threadIdx.x; i < n[k]; i += PL_THREADS) nf_copy16(dst[k] + i, src[k] + i);
+    for (int k = 0; k < 4; k++) {
+      for (int i = threadIdx.x; i < n[k]; i += T) nf_copy16(dst + i, src[k] + i);
+      dst += n[k];
+    }
     nf_copy_wait();
   }
   cluster.sync();   // every CTA runs and has its data
   // y -> ky: item = (chunk of PL_KC ky, z); row ky to the CTA that holds it
-  for (int it = threadIdx.x; it < nky * nzq; it += PL_THREADS) {
+  for (int it = threadIdx.x; it < nky * nzq; it += T) {
     const int ch = it / nzq, z = it - ch * nzq, k0 = ch * PL_KC;
     const float2* a = cols + z;
     const float4* t = tab0 + ch * (Hy + 1) * (PL_KC / 2);
@@ -536,7 +543,7 @@ __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
   // z -> kz and the potential modes: item = (pair of kz, ky)
   double e[7] = {0, 0, 0, 0, 0, 0, 0};
   const int P = (b.K[0] + 1) * NY;
-  for (int it = threadIdx.x; it < nkz * nr; it += PL_THREADS) {
+  for (int it = threadIdx.x; it < nkz * nr; it += T) {
     const int kp = it / nr, r = it - kp * nr, k0 = 2 * kp;
     const float4* t = tab1 + kp * (Hz + 1);
     const float2* in = rows + r * ld;
@@ -596,7 +603,7 @@ __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
   }
   __syncthreads();
   // kz -> z: item = (pair of z, ky); column z to the CTA that holds it
-  for (int it = threadIdx.x; it < nz * nr; it += PL_THREADS) {
+  for (int it = threadIdx.x; it < nz * nr; it += T) {
     const int zp = it / nr, r = it - zp * nr, z0 = 2 * zp;
     const float4* t = tab2 + zp * (Kz + 1);
     const float4 v0 = pm[r];
@@ -628,7 +635,7 @@ __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
   }
   cluster.sync();
   // ky -> y: item = (chunk of PL_KC y, z)
-  for (int it = threadIdx.x; it < ny * nzq; it += PL_THREADS) {
+  for (int it = threadIdx.x; it < ny * nzq; it += T) {
     const int ch = it / nzq, z = it - ch * nzq, y0 = ch * PL_KC;
     const float4* t = tab3 + ch * (Ky + 1) * (PL_KC / 2);
     const float2* in = cols + Ky * nzq + z;
@@ -680,13 +687,15 @@ __global__ void __cluster_dims__(NF_CS, 1, 1) __launch_bounds__(PL_THREADS)
     __syncthreads();
     if (threadIdx.x < 7) {
       double s = 0;
-      for (int i = 0; i < PL_THREADS / 32; i++) s += red[threadIdx.x][i];
+      for (int i = 0; i < T / 32; i++) s += red[threadIdx.x][i];
       b.ek_part[blockIdx.x * 7 + threadIdx.x] = s;
     }
   }
 }
 
 // A[kx][c] -> G[x][c]: the real part (the half kx >= 0 carries both signs)
+// (half the threads where a batch fills the GPU: 256 ionic boxes 225 -> 189 us,
+// 864 waters 3.2 -> 3.5)
 __global__ void __launch_bounds__(DF_THREADS) nf_idft_x_kernel(const NfBox* __restrict__ boxes) {
   after_previous();
   const NfBox& b = boxes[blockIdx.z];
@@ -696,17 +705,17 @@ __global__ void __launch_bounds__(DF_THREADS) nf_idft_x_kernel(const NfBox* __re
   float2* in = reinterpret_cast<float2*>(zs);    // [K + 1][32]
   float4* tw = zs + (K + 1) * (DF_COLS / 2);     // [chunk][K + 1][NF_KC / 2]
   const int nch = H / NF_KC + 1, ntw = nch * (K + 1) * (NF_KC / 2);
-  for (int i = threadIdx.x; i < (K + 1) * (DF_COLS / 2); i += DF_THREADS) {
+  for (int i = threadIdx.x; i < (K + 1) * (DF_COLS / 2); i += (int)blockDim.x) {
     const int c = c0 + i % (DF_COLS / 2) * 2;
     if (c < ncol) nf_copy16(in + 2 * i, b.A + (long)(i / (DF_COLS / 2)) * ncol + c);
   }
-  for (int i = threadIdx.x; i < ntw; i += DF_THREADS)
+  for (int i = threadIdx.x; i < ntw; i += (int)blockDim.x)
     nf_copy16(tw + i, reinterpret_cast<const float4*>(b.inv[0]) + i);
   nf_copy_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, c = c0 + lane;
   if (c >= ncol) return;
-  for (int ch = threadIdx.x >> 5; ch < nch; ch += DF_THREADS / 32) {
+  for (int ch = threadIdx.x >> 5; ch < nch; ch += (int)blockDim.x / 32) {
     const float2* a = in + lane;
     const float4* t = tw + ch * (K + 1) * (NF_KC / 2);
     float e[NF_KC], o[NF_KC];
@@ -912,10 +921,12 @@ __global__ void __launch_bounds__(SP_WARPS * 32)
 }
 
 // Sparse boxes (a few charges a tile): a warp per 16 sorted sites, the rows
-// from memory.
+// from memory.  The warps wait for these loads, so eight CTAs an SM, at 64
+// registers and a few spills: 256 ionic boxes 330 -> 216 us (at 80 registers
+// five; ten CTAs spill more, 387).
 constexpr int IP_WARPS = 4, IP_SITES = 16;
 
-__global__ void __launch_bounds__(IP_WARPS * 32)
+__global__ void __launch_bounds__(IP_WARPS * 32, 8)
     nf_interp_kernel(const NfBox* __restrict__ boxes, double* __restrict__ f_or_null) {
   after_previous();
   const NfBox& b = boxes[blockIdx.z];
@@ -1071,14 +1082,14 @@ void nf_tables(const int K[3], const int M[3], const std::vector<int4>& kvec,
 }
 
 // shared memory of the plane kernel: potential modes, tables, the plane
-static size_t nf_plane_smem(const int K[3], const int M[3]) {
+static size_t nf_plane_smem(const int K[3], const int M[3], int cs) {
   const int NY = 2 * K[1] + 1, Hy = M[1] / 2, Hz = M[2] / 2;
   const size_t tab = (size_t)(K[1] / PL_KC + 1) * (Hy + 1) * (PL_KC / 2) +
                      (size_t)(K[2] / 2 + 1) * (Hz + 1) + (size_t)(Hz / 2 + 1) * (K[2] + 1) +
                      (size_t)(Hy / PL_KC + 1) * (K[1] + 1) * (PL_KC / 2);
-  const int nrow = (NY + NF_CS - 1) / NF_CS;
+  const int nrow = (NY + cs - 1) / cs;
   return 16 * ((size_t)(K[2] + 1) * nrow + tab) + 8 * ((size_t)(M[2] + 1) * nrow + 1) +
-         8 * (size_t)(M[1] > NY ? M[1] : NY) * (M[2] / NF_CS);
+         8 * (size_t)(M[1] > NY ? M[1] : NY) * (M[2] / cs);
 }
 static size_t nf_x_smem(int K, int M) {
   return 4 * (size_t)DF_COLS * M + 16 * (size_t)(K / NF_KC + 1) * (M / 2 + 1) * (NF_KC / 2);
@@ -1092,7 +1103,7 @@ constexpr int NF_MAX_SMEM = 225 * 1024;
 
 bool nf_fits(const int K[3]) {
   const int M[3] = {nf_grid(K[0]), nf_grid(K[1]), nf_grid(K[2])};
-  return nf_plane_smem(K, M) <= NF_MAX_SMEM && nf_x_smem(K[0], M[0]) <= NF_MAX_SMEM &&
+  return nf_plane_smem(K, M, NF_CS) <= NF_MAX_SMEM && nf_x_smem(K[0], M[0]) <= NF_MAX_SMEM &&
          nf_ix_smem(K[0], M[0]) <= NF_MAX_SMEM;
 }
 
@@ -1116,7 +1127,8 @@ void nf_launch(const NfBox& b, NfGrid* g) {
   else up(g->interp, cdiv(b.ns, IP_WARPS * IP_SITES));
   up(g->sx, (int)nf_x_smem(b.K[0], b.M[0]));
   up(g->six, (int)nf_ix_smem(b.K[0], b.M[0]));
-  up(g->splane, (int)nf_plane_smem(b.K, b.M));
+  up(g->splane, (int)nf_plane_smem(b.K, b.M, NF_CS));
+  up(g->splane_few, (int)nf_plane_smem(b.K, b.M, NF_CSB));
 }
 
 // the same limit whatever the box: a captured launch of a larger box must not
@@ -1150,10 +1162,21 @@ cudaError_t k_nf_forward(const Launch& L, const NfBox* d, int nbox, const NfGrid
   return cudaGetLastError();
 }
 
+// more CTAs than two waves of eight an SM: throughput counts, not the latency of
+// one
+static bool nf_many(long ctas) { return ctas > 16L * PARTITION_SMS; }
+
 cudaError_t k_nf_modes(const Launch& L, const NfBox* d, int nbox, const NfGrid& g, bool measure) {
-  cudaError_t e = nf_smem((const void*)nf_plane_kernel, g.splane);
+  const bool many = !measure && nf_many((long)g.plane * nbox) && g.splane_few <= NF_MAX_SMEM;
+  cudaError_t e = many ? nf_smem((const void*)nf_plane_kernel<NF_CSB, NF_TB>, g.splane_few)
+                       : nf_smem((const void*)nf_plane_kernel<NF_CS, PL_THREADS>, g.splane);
   if (e != cudaSuccess) return e;
-  launch_after(L, nf_plane_kernel, dim3(g.plane, 1, nbox), PL_THREADS, g.splane, d, measure);
+  if (many)
+    launch_after(L, nf_plane_kernel<NF_CSB, NF_TB>, dim3(g.plane / NF_CS * NF_CSB, 1, nbox), NF_TB,
+                 g.splane_few, d, measure);
+  else
+    launch_after(L, nf_plane_kernel<NF_CS, PL_THREADS>, dim3(g.plane, 1, nbox), PL_THREADS, g.splane,
+                 d, measure);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -1161,7 +1184,8 @@ cudaError_t k_nf_modes(const Launch& L, const NfBox* d, int nbox, const NfGrid& 
 cudaError_t k_nf_back(const Launch& L, const NfBox* d, int nbox, const NfGrid& g) {
   cudaError_t e = nf_smem((const void*)nf_idft_x_kernel, g.six);
   if (e != cudaSuccess) return e;
-  launch_after(L, nf_idft_x_kernel, dim3(g.x, 1, nbox), DF_THREADS, g.six, d);
+  launch_after(L, nf_idft_x_kernel, dim3(g.x, 1, nbox),
+               nf_many((long)g.x * nbox) ? DF_THREADS / 2 : DF_THREADS, g.six, d);
   LAUNCHED(L);
   return cudaGetLastError();
 }

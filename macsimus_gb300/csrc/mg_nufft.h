@@ -44,7 +44,7 @@ struct NfBox {
 // the largest grids and shared memory over the boxes of a launch
 struct NfGrid {
   int spread, x, plane, interp, interp_tile;
-  int sx, six, splane;
+  int sx, six, splane, splane_few;
 };
 
 int nf_grid(int K);

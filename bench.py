@@ -186,7 +186,7 @@ def run_ours(args, rank, world, local):
     fd, ed = f64.forces(w["r"], measure=True)
     force_err = float(np.sqrt(((fm - fd) ** 2).sum() / (fd ** 2).sum()))
     # the energies beside the forces: the k-space energy relative to itself
-    # (the tensor-core passes accumulate in FP32 rounded toward zero), the
+    # (the tensor-core engines accumulate in FP32 rounded toward zero), the
     # total potential energy relative to the Ewald energy scale |E_self|
     energy_err = {"ek_rel": (em["ek"] - ed["ek"]) / abs(ed["ek"]),
                   "epot_rel_eself": (em["el"] + em["lj"] - ed["el"] - ed["lj"]) / abs(ed["eself"]),
@@ -288,8 +288,9 @@ def run_ours(args, rank, world, local):
     nq = int((system.q != 0).sum()) + (int((system.qpol != 0).sum()) if system.polar else 0)
     V = w["L"] ** 3
     npairs = ns * (ns - 1) / 2 * (4.0 / 3.0 * math.pi * w["cutoff"] ** 3) / V
-    algo = {"ewald_sk": FLOP_PER_KQ * fp.nkvec * nq, "ewald_kforce": FLOP_PER_KQ * fp.nkvec * nq,
-            "pair_mixed": FLOP_PER_PAIR * npairs}
+    algo = {"pair_mixed": FLOP_PER_PAIR * npairs}
+    if args.kspace_engine:   # the direct sums; the transforms do far less
+        algo["ewald_sk"] = algo["ewald_kforce"] = FLOP_PER_KQ * fp.nkvec * nq
     # the kernel with the largest share among those with algorithmic work
     # (the small cell-list kernels of a small box are mostly launch gaps)
     work = {k: v for k, v in prof.items() if k in algo}
@@ -297,13 +298,11 @@ def run_ours(args, rank, world, local):
     name, (kms, kcnt) = top
     kavg = kms / max(kcnt, 1)
     achieved = algo.get(name, 0) / (kavg * 1e-3) / 1e12 if kavg > 0 else 0.0
-    # the pair step's kernel: the group kernel (pair_variant 8), its half-shell
-    # forms (9: lanes on the home sites, 10: lanes on the neighbours; with
-    # Drude shells 10 runs 9) or the cell kernel
+    # the pair step's kernel: the group kernel (pair_variant 8), the half-shell
+    # kernel (9 and 10) or the cell kernel
     if name == "pair_mixed" and tuned.get("pair_variant", 0) in (8, 9, 10):
         pv = tuned["pair_variant"]
-        name = {8: "pair_group", 9: "pair_half", 10: "pair_half" if system.polar
-                else "pair_half_t"}[pv]
+        name = "pair_group" if pv == 8 else "pair_half"
         algo[name] = algo["pair_mixed"]
         achieved = algo[name] / (kavg * 1e-3) / 1e12 if kavg > 0 else 0.0
     traffic = None
@@ -352,7 +351,7 @@ def run_ours(args, rank, world, local):
                        "autotuned": tuned or "off",
                        "pair_search": ("Verlet lists, skin %.2f A" % args.skin) if args.skin > 0
                        else "cells re-binned every step",
-                       "ewald_kspace": {0: "both passes tensor cores (tcgen05 TF32x3)",
+                       "ewald_kspace": {0: "non-uniform Fourier transforms (FP32)",
                                         1: "both passes FP32 cores",
                                         2: "pass 1 FP32 cores, pass 2 tensor cores (tcgen05 TF32x3)",
                                         3: "both passes tensor cores (tcgen05 TF32x3)"}[
@@ -512,9 +511,10 @@ def run_batch(args, rank, world, local):
     nbytes = sum(a.nbytes + b.nbytes for a, b in host)
     # per stage of the fused step (CUDA events between the launches), and
     # the roofline of the stage with the largest share: its algorithmic
-    # work over its time (Ewald passes: 8 flops per (k-vector, charge), on
-    # the tensor cores as TF32 products, three MMAs per product, at half
-    # the bf16 rate; the pair terms: 45 flops per in-cutoff pair, FP32)
+    # work over its time (the direct Ewald passes of engines 1 to 3: 8 flops per
+    # (k-vector, charge), on the tensor cores as TF32 products, three MMAs per
+    # product, at half the bf16 rate; the pair terms: 45 flops per in-cutoff
+    # pair, FP32; the transforms of the default engine are not a product)
     for i in range(len(boxes)):
         bm.box[i].md_set_state(*states[i])
     stages = bm.profile(5) if bm.fused else {}
@@ -525,7 +525,9 @@ def run_batch(args, rank, world, local):
                 for b in boxes)
     roof = None
     if stages:
-        top = max(stages, key=stages.get)
+        direct = ("ewald_sk", "ewald_kforce") if args.kspace_engine else ()
+        rated = [k for k in stages if k in direct + ("pair",)]
+        top = max(rated or stages, key=stages.get)
         t_top = stages[top] * 1e-3
         if top in ("ewald_sk", "ewald_kforce"):
             peaks = json.load(open(os.path.join(REPO, "MEASURED_PEAKS.json"))) \
@@ -557,7 +559,7 @@ def run_batch(args, rank, world, local):
                                    "all), per-box Ewald, leap-frog dt 2 fs; Widom 1e5 "
                                    "insertions per box" % (nbox, sum(b["system"].ns for b in allb)),
                        "boxes_on_rank0": len(boxes),
-                       "ewald_kspace": {0: "tensor cores where the tiles fit", 1: "FP32 cores",
+                       "ewald_kspace": {0: "non-uniform Fourier transforms (FP32)", 1: "FP32 cores",
                                         2: "pass 2 on tensor cores", 3: "tensor cores"}[engine],
                        "l2": "inputs larger than L2 (per-step working set > 129 MB)"},
             "atom_steps_per_s": round(world * nsite * args.steps / (ms * 1e-3), 1),
@@ -628,17 +630,16 @@ def main():
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-autotune", action="store_true")
     ap.add_argument("--kspace-engine", type=int, default=None,
-                    help="Ewald engine of the FP32 path: 0 tensor cores where they fit, 1 FP32 "
-                         "cores, 2 tensor-core pass 2 only, 3 tensor cores for both passes "
-                         "(default 0: one launch per pass over all boxes of a batch, the "
-                         "boxes whose tiles do not fit on the FP32 cores)")
+                    help="Ewald engine of the FP32 path: 0 non-uniform Fourier transforms "
+                         "(default), 1 direct sums on the FP32 cores, 2 tensor-core pass 2 "
+                         "only, 3 tensor cores for both passes")
     ap.add_argument("--skin", type=float, default=0.0,
                     help="> 0: Verlet lists of cutoff+skin instead of cells re-binned every step")
     ap.add_argument("--equilibrate", type=int, default=400,
                     help="relax the lattice start (rigid molecules, velocity rescaling)")
     ap.add_argument("--pair-variant", type=int, default=None,
                     help="FP32 pair kernel (mg_params.pair_variant; 8 = the group kernel, "
-                         "9 and 10 its half-shell forms), "
+                         "9 and 10 the half-shell kernel), "
                          "instead of the autotuner's choice")
     ap.add_argument("--cells", type=int, default=None,
                     help="cells per cutoff instead of the autotuner's choice")

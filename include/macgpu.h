@@ -128,7 +128,7 @@ typedef struct {
   double skin;       /* A */
   int nl_every;      /* most MD steps between list builds; <=0 selects 50 */
   /* Ewald pass 1 work split: charge chunks sized for this many CTAs per SM;
-     <=0 selects 10 (FP32) / 8 (FP64).  mg_autotune picks it. */
+     <=0 selects 10 (direct FP32 sums).  mg_autotune picks it. */
   int kspace_ctas_per_sm;
   /* FP32 pair kernel: 0 = automatic, the half-shell kernel (every pair once,
      warps with a group of 8 home sites each against neighbours pruned by the
@@ -404,8 +404,8 @@ int mg_xwidom(mg_ctx *ctx, int nlist, const int *mols, const int *vtype, const d
    split (kspace_ctas_per_sm 6, 10, 16) and writes the fastest pair into
    *par, then the fastest of the 8 cell-kernel pair_variant values at that
    choice, of the group kernel (pair_variant 8) at every subdivision and,
-   on the FP32 path, of its half-shell forms (pair_variant 9 and 10) at
-   every subdivision, each timed (FP32 path) with
+   on the FP32 path, of the half-shell kernel (pair_variant 9 and 10, one
+   kernel) at every subdivision, each timed (FP32 path) with
    kspace_serial 0 and 1, the pair chosen together.  Builds and frees its
    own trial contexts; ms[28] (optional) gets the time per evaluation of
    each trial (the best of three blocks of nrep evaluations; cdiv-major,

@@ -95,7 +95,7 @@ struct Launch {
 // graph, where such edges are as fast as the others at best (864 waters 66
 // against 68 us a step, 500 waters 76 against 62, 32768 416 against 393), and not
 // for the pair kernels: set up early, beside a kernel that holds much shared
-// memory, they keep its small L1 (32768 waters, 250 -> 295 us).
+// memory, they keep its small L1 (32768 waters: 24 us a step more).
 template <class... KA, class... A>
 inline void launch_after(const Launch& L, void (*kernel)(KA...), dim3 grid, dim3 block,
                          size_t smem, A&&... args) {

@@ -3,15 +3,14 @@
 //   cell list      k_cell_list: a counting sort of the sites by cell (count,
 //                  scan, scatter, per-cell rank) with the fixed-point site
 //                  records of the FP32 path; k_gather_* for the FP64 path
-//   r-space sum    k_pair_mixed: one CTA per home cell, its warps
-//                  split the neighbour-cell stencil; neighbour cells are staged
-//                  per warp in shared memory (16-byte loads) and every lane owns
-//                  one home-cell site (full shell: each pair is evaluated from
-//                  both ends, so no atomics and a fixed summation order).
-//   k-space        k_phase_tables_* (per-charge e^{2 pi i n x/L} rows),
-//                  k_sk_* (structure factor, FP32 partial sums per charge chunk),
-//                  k_sk_reduce_* (FP64 sum of the partials, energy, virial),
-//                  k_kforce_* (force back-transform, one thread per charge)
+//   r-space sum    k_pair_mixed: the half-shell kernel (every pair once, a warp
+//                  on 8 home sites, lanes on the neighbours), the all-pairs
+//                  kernel of small boxes, the cell and the group kernel;
+//                  k_excl_mixed: the Ewald terms of pairs within a molecule.
+//                  The FP64 path: mg_pair64.cu
+//   k-space        the phase rows and S(k) sums of the direct FP32 engines
+//                  (passes: mg_kspace.cu, mg_kspace_tc.cu; transforms:
+//                  mg_nufft.cu; FP64: mg_kspace64.cu)
 //   integrator     k_shake: leap-frog + SHAKE sweeps, one thread per molecule
 //
 // Mixed precision: positions enter the pair kernel as 32-bit fixed-point

@@ -133,9 +133,11 @@ typedef struct {
   /* FP32 pair kernel: 0 = automatic, the half-shell kernel (every pair once,
      warps with a group of 8 home sites each against neighbours pruned by the
      group's bounding box; forces, of the shells too, summed in 64-bit fixed
-     point, 2^-32 K/A, by integer atomics, so reproducible bit for bit), or all
-     pairs in a small box whose cutoff leaves cells of few sites; 9, 10 = the
-     half-shell kernel; 8 = the group kernel (the same pruning, every pair
+     point, 2^-32 K/A, by integer atomics, so reproducible bit for bit; the
+     force on a site with a term beyond the range of these sums, some 1e6 K/A,
+     or not finite, is formed pair by pair instead), or all pairs in a small
+     box whose cutoff leaves cells of few sites; 9, 10 = the half-shell kernel;
+     8 = the group kernel (the same pruning, every pair
      from both ends, no atomics); 1..7 = the cell kernel with bit 0 = 8 warps
      per home cell (else 4), bit 2 = 16 warps per home cell (over bit 0), bit 1
      = the erfc force spline in shared memory (else read through L1).  A box

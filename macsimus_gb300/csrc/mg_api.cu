@@ -92,6 +92,7 @@ struct mg_ctx {
   int4* d_hspans = nullptr;
   int nhspans = 0;
   long long* d_facc = nullptr;
+  int* d_bad = nullptr;   // its marks of sites whose sums would not hold
   int *d_gstart = nullptr, *d_gcell = nullptr;
   PairF* d_ptabf = nullptr;
   PairD* d_ptabd = nullptr;
@@ -187,6 +188,8 @@ struct mg_ctx {
   bool small = false, half = false;
   int split = 1;
   unsigned heavy = 0, shells = 0;
+  float flim = 0;
+  int maxgroups = 0;
   // thermostat
   int normalize = 1;
   double box_r0 = 0.15;
@@ -719,6 +722,20 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
            cand >= 2 * ctx->split * 128)
       ctx->split *= 2;
   }
+  // its 64-bit sums hold 2^31 K/A.  A site's sum has a term from every group
+  // whose half shell holds it and one from each warp of its own group, so with
+  // at most maxgroups groups a cell terms below flim cannot leave it.  Room for
+  // 1024 terms (flim 2e6 K/A, twenty times the closest contacts of water) or, in
+  // a smaller box, all its groups; for more where cells are large: four times
+  // their mean, and 0.25 sites to the cubic A (water has 0.1)
+  {
+    const int nh = (ctx->nstencil + 1) / 2;
+    const double vol = p->L[0] * p->L[1] * p->L[2] / ctx->ncell;
+    ctx->maxgroups = std::max({1024 / nh, 4 * (ns / ctx->ncell / GROUP_SITES + 1),
+                               (int)std::min(0.25 * vol / GROUP_SITES, 1e6) + 1});
+    const double terms = std::min((double)nh * ctx->maxgroups, ns / (double)GROUP_SITES + ctx->ncell);
+    ctx->flim = (float)(0.999 * 2147483648.0 / (terms + ctx->split));
+  }
   ctx->nprows = std::max(std::max(ctx->ncell, ctx->ngroup_grid * (ctx->half ? ctx->split : 1)),
                          pair_all_blocks(ns));
   if (ctx->precision != MG_MIXED) ctx->nprows = pair64_blocks(ns);
@@ -879,8 +896,10 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
     const size_t nfix = 3 * (size_t)ns * (t->chargepol ? 2 : 1);
     CK(dalloc(&ctx->d_facc, nfix));
     CK(cudaMemset(ctx->d_facc, 0, nfix * sizeof(long long)));
+    CK(dalloc(&ctx->d_bad, ns));
+    CK(cudaMemset(ctx->d_bad, 0, ns * sizeof(int)));
   }
-  CK(dalloc(&ctx->d_gstart, (size_t)ctx->ncell + 1));
+  CK(dalloc(&ctx->d_gstart, (size_t)ctx->ncell + 2));
   CK(dalloc(&ctx->d_gcell, (size_t)ns / GROUP_SITES + ctx->ncell + 1));
   ctx->nxblocks = (t->nmol + EXCL_THREADS - 1) / EXCL_THREADS;
   ctx->nepart = std::max(ctx->nprows + ctx->nxblocks,
@@ -1350,6 +1369,10 @@ PairArgs make_pair_args(mg_ctx* ctx, double* f_dev) {
   pa.hspans = ctx->d_hspans;
   pa.nhspans = ctx->nhspans;
   pa.facc = ctx->d_facc;
+  pa.bad = ctx->d_bad;
+  pa.over = ctx->d_gstart + ctx->ncell + 1;
+  pa.flim = ctx->flim;
+  pa.maxgroups = ctx->maxgroups;
   pa.gstart = ctx->d_gstart;
   pa.gcell = ctx->d_gcell;
   pa.spans = ctx->d_spans;
@@ -1955,7 +1978,7 @@ int mg_destroy(mg_ctx* ctx) {
   void* bufs[] = {ctx->d_rs, ctx->d_fs, ctx->d_r,      ctx->d_f,       ctx->d_r1,    ctx->d_p,      ctx->d_kind,
                   ctx->d_mol,    ctx->d_key,     ctx->d_pfix,   ctx->d_idx,   ctx->d_key_s,  ctx->d_order,
                   ctx->d_cell_start, ctx->d_ccount, ctx->d_ccursor, ctx->d_spans, ctx->d_gstart,
-                  ctx->d_hspans, ctx->d_facc, ctx->d_tcb, ctx->d_nf, ctx->d_nfmem, ctx->d_far,
+                  ctx->d_hspans, ctx->d_facc, ctx->d_bad, ctx->d_tcb, ctx->d_nf, ctx->d_nfmem, ctx->d_far,
                   ctx->d_kind3, ctx->d_ctab, ctx->d_ftab, ctx->d_xbase3,
                   ctx->d_gcell, ctx->d_pj, ctx->d_pd, ctx->d_pf, ctx->d_stencil,
                   ctx->d_ptabf,  ctx->d_ptabd,   ctx->d_erd,   ctx->d_eru,    ctx->d_ert,

@@ -155,7 +155,7 @@ cudaError_t k_gather_drude(const Launch& L, int ns, const double* r, const int* 
 struct PairArgs {
   int ns, ncx, ncy, ncz, nstencil, nkind;
   int allpairs;             // one cell
-  const int* key_s;         // cell of every sorted site (FP64 path)
+  const int* key_s;         // cell of every sorted site
   int small;                // FP32 path: the all-pairs kernel (pair_all_kernel)
   const int* cell_start;
   const int* order;         // sorted -> site
@@ -183,13 +183,19 @@ struct PairArgs {
   // the half-shell kernel (every pair once): the half-shell z-runs, and the
   // 64-bit fixed-point force sums (2^-32 K/A units, sorted order, kept zero
   // between evaluations); split: warps per group; bit masks of the kinds with
-  // a Lennard-Jones term or a shell, and of those with a shell
+  // a Lennard-Jones term or a shell, and of those with a shell; bad: marks of
+  // the sorted sites with a term of flim or more, over: set when a cell holds
+  // more than maxgroups groups; without either no sum can leave its 64 bits
+  // (bad kept zero between evaluations, over cleared by the cell list)
   int newton;
   int split;
   unsigned heavy, shells;
   const int4* hspans;
   int nhspans;
   long long* facc;
+  int *bad, *over;
+  float flim;
+  int maxgroups;
 };
 cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj,
                          const PairF* ptab, const float4* erd, const float4* eru,

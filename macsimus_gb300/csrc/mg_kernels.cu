@@ -91,7 +91,8 @@ __global__ void cell_count_kernel(int ns, const double* __restrict__ r, const __
 // tiles of 4 x 1024 counts (int4 loads; count is padded with zeros to a
 // multiple of 4 entries); the counts are cleared for the next list.  With
 // gstart the same scan of the group counts ceil(count / GROUP_SITES) (the
-// work items of the group pair kernel) goes to gstart[0..ncell].
+// work items of the group pair kernel) goes to gstart[0..ncell]; gstart[ncell + 1],
+// the half-shell kernel's mark (PairArgs::over), is cleared.
 constexpr int SCAN_THREADS = 1024;
 __device__ __forceinline__ int2 add2(int2 a, int2 b) { return make_int2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ int2 shfl_up2(int2 v, int o) {
@@ -162,7 +163,10 @@ MG_BODY void cell_scan_kernel_body(int ncell,
   }
   if (t == 0) {
     start[ncell] = carry_s.x;
-    if (gstart) gstart[ncell] = carry_s.y;
+    if (gstart) {
+      gstart[ncell] = carry_s.y;
+      gstart[ncell + 1] = 0;
+    }
   }
 }
 
@@ -804,6 +808,12 @@ __global__ void __launch_bounds__(NW * 32)
 // does not depend on the order, so the forces come out the same bit for bit
 // on every run.  finish_forces_kernel turns the sums into the FP64 forces
 // (site order) and clears them for the next evaluation.
+//
+// A sum holds 2^31 K/A, less than two oxygens 1 A apart repel each other by, and
+// a conversion makes a number of a NaN.  Every term is therefore compared with
+// PairArgs::flim before its conversion (written so that a NaN fails); where one
+// fails, its site is marked and finish_forces_kernel forms that site's force pair
+// by pair instead (direct_forces).
 constexpr double FIX_SCALE = 4294967296.0;  // 2^32: steps of 2.3e-10 K/A, |F| < 2^31 K/A
 
 
@@ -818,6 +828,12 @@ template <bool B>
 struct BoolC {
   static constexpr bool value = B;
 };
+
+// a store that the compiler need not take for a change of the kernel's other
+// integers (a batch's arguments, in memory, would be read again after it)
+__device__ __forceinline__ void mark(int* flag) {
+  asm volatile("st.global.u32 [%0], 1;" ::"l"(flag));
+}
 
 // the half-shell kernel's pair force factor f (force on i = f (r_i - r_j))
 // with every rounding explicit; flj: the LJ part, y: (Sq / r^2)^3 for its
@@ -1146,6 +1162,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
     const int hs = a.cell_start[c], he = a.cell_start[c + 1];
     const int i0 = hs + GS * (item - a.gstart[c]);
     const int ni = min(GS, he - i0);
+    if (ngroups(he - hs) > a.maxgroups) mark(a.over);
     const unsigned refx = (unsigned)((((unsigned long long)(2 * cx + 1)) << 31) / a.ncx),
                    refy = (unsigned)((((unsigned long long)(2 * cy + 1)) << 31) / a.ncy),
                    refz = (unsigned)((((unsigned long long)(2 * cz + 1)) << 31) / a.ncz);
@@ -1303,6 +1320,10 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
       else if (ni > 4) { quad(0, BoolC<false>()); quad(4, BoolC<false>()); }
       else quad(0, BoolC<false>());
       if (vt) {
+        // a term beyond the sums' range, or not a number
+        float big = fabsf(px) + fabsf(py) + fabsf(pz);
+        if (POLAR) big += fabsf(ux) + fabsf(uy) + fabsf(uz);
+        if (!(big < a.flim)) mark(a.bad + tj);
         unsigned long long* fj = reinterpret_cast<unsigned long long*>(a.facc) + 3 * (long)tj;
         atomicAdd(fj, (unsigned long long)__float2ll_rn(__fmul_rn(px, -(float)FIX_SCALE)));
         atomicAdd(fj + 1, (unsigned long long)__float2ll_rn(__fmul_rn(py, -(float)FIX_SCALE)));
@@ -1456,6 +1477,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
       v[3 * i + 2] = hz[i];
     }
     reduce_scatter(v, lane);
+    if (!(fabsf(v[0]) < a.flim)) mark(a.bad + at / 3);   // lanes from 3 ni on: zero
     if (lane < 3 * ni)
       atomicAdd(facc + at, (unsigned long long)__float2ll_rn(__fmul_rn(v[0], (float)FIX_SCALE)));
     if (POLAR && nh > 0) {
@@ -1469,6 +1491,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
         v[3 * i + 2] = gz[ip];
       }
       reduce_scatter(v, lane);
+      if (!(fabsf(v[0]) < a.flim)) mark(a.bad + at / 3);
       if (lane < 3 * nh)
         atomicAdd(facc + 3 * (long)a.ns + at,
                   (unsigned long long)__float2ll_rn(__fmul_rn(v[0], (float)FIX_SCALE)));
@@ -1517,29 +1540,108 @@ __global__ void __launch_bounds__(NW * 32, MEASURE ? (POLAR ? 2 : 3) : (POLAR ? 
                                             blockIdx.x);
 }
 
-// the fixed-point sums (sorted order) into the FP64 forces (site order),
-// with shells the second half of each; the sums are cleared for the next
-// evaluation
-__device__ __forceinline__ void finish_forces(int ns, int halves, const int* __restrict__ order,
-                                              long long* __restrict__ facc,
-                                              double* __restrict__ f) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ns) return;
-  const int site = order[t];
-  for (int h = 0; h < halves; h++) {
-    const long o = 3 * (long)ns * h;
+// The force on sorted site t from all its pairs by a warp, FP32 pair terms (those
+// of the half-shell kernel) added in FP64: marked sites, overlapping ones of a
+// random start or a hot fluid.  Some 5 us a site.
+template <bool POLAR>
+__device__ __noinline__ void direct_forces(const PairArgs& a, int t, const int4* __restrict__ pj,
+                                           const PairF* __restrict__ ptab,
+                                           const float4* __restrict__ erd, float sx, float sy,
+                                           float sz, float cq, float sgrid) {
+  constexpr int NC = POLAR ? 6 : 3;
+  const int ntab = a.ntab, c = a.key_s[t], lane = threadIdx.x & 31;
+  const int cz = c % a.ncz, cy = (c / a.ncz) % a.ncy, cx = c / (a.ncy * a.ncz);
+  const int4 me = pj[t];
+  const float4 md = POLAR ? a.pdj[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  double F[NC];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      f[o + 3 * (long)site + d] = (double)facc[o + 3 * (long)t + d] * (1.0 / FIX_SCALE);
-      facc[o + 3 * (long)t + d] = 0;
+  for (int k = 0; k < NC; k++) F[k] = 0;
+  auto add = [&](int k, float f, float x, float y, float z) {
+    F[k] += (double)f * x;
+    F[k + 1] += (double)f * y;
+    F[k + 2] += (double)f * z;
+  };
+  for (int s = 0; s < a.nstencil; s++) {
+    const int4 o = a.stencil[s];
+    int x = cx + o.x, y = cy + o.y, z = cz + o.z;
+    x += x < 0 ? a.ncx : (x >= a.ncx ? -a.ncx : 0);
+    y += y < 0 ? a.ncy : (y >= a.ncy ? -a.ncy : 0);
+    z += z < 0 ? a.ncz : (z >= a.ncz ? -a.ncz : 0);
+    const int c2 = (x * a.ncy + y) * a.ncz + z;
+    for (int j = a.cell_start[c2] + lane; j < a.cell_start[c2 + 1]; j += 32) {
+      const int4 q = pj[j];
+      const float dx = __fmul_rn((float)(int)((unsigned)me.x - (unsigned)q.x), sx),
+                  dy = __fmul_rn((float)(int)((unsigned)me.y - (unsigned)q.y), sy),
+                  dz = __fmul_rn((float)(int)((unsigned)me.z - (unsigned)q.z), sz);
+      const float rr = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+      if (!(rr < cq) || ((q.w ^ me.w) >> 8) == 0) continue;
+      const PairFS& P =
+          *reinterpret_cast<const PairFS*>(ptab + (me.w & 255) * a.nkind + (q.w & 255));
+      float flj, lj6;
+      add(0, pair_force_rn(P, rr, erd, sgrid, ntab, flj, lj6), dx, dy, dz);
+      if constexpr (POLAR) {
+        const float4 qd = a.pdj[j];
+        float e = 0.f;
+        const float ex = __fadd_rn(dx, md.x), ey = __fadd_rn(dy, md.y), ez = __fadd_rn(dz, md.z);
+        add(3, drude_force_rn<false>(erd, nullptr, ex, ey, ez, sgrid, ntab, P.qpc, e), ex, ey, ez);
+        const float vx = __fadd_rn(dx, -qd.x), vy = __fadd_rn(dy, -qd.y), vz = __fadd_rn(dz, -qd.z);
+        add(0, drude_force_rn<false>(erd, nullptr, vx, vy, vz, sgrid, ntab, P.qcp, e), vx, vy, vz);
+        const float ux = __fadd_rn(ex, -qd.x), uy = __fadd_rn(ey, -qd.y), uz = __fadd_rn(ez, -qd.z);
+        add(3, drude_force_rn<false>(erd, nullptr, ux, uy, uz, sgrid, ntab, P.qpp, e), ux, uy, uz);
+      }
     }
+  }
+#pragma unroll
+  for (int k = 0; k < NC; k++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) F[k] += __shfl_xor_sync(0xffffffffu, F[k], o);
+    if (lane == 0) a.f[(k < 3 ? 0 : 3 * (long)a.ns) + 3 * (long)a.order[t] + k % 3] = F[k];
   }
 }
 
-__global__ void finish_forces_kernel(int ns, int halves, const int* __restrict__ order,
-                                     long long* __restrict__ facc, double* __restrict__ f) {
+// the fixed-point sums (sorted order) into the FP64 forces (site order),
+// with shells the second half of each; the sums are cleared for the next
+// evaluation, and the marks.  Whole warps.
+template <bool POLAR>
+__device__ __forceinline__ void finish_forces(const PairArgs& a, const int4* __restrict__ pj,
+                                              const PairF* __restrict__ ptab,
+                                              const float4* __restrict__ erd, float sx, float sy,
+                                              float sz, float cq, float sgrid) {
+  constexpr int NH = POLAR ? 2 : 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  bool redo = false;
+  if (t < a.ns) {
+    // every load before the first store
+    const int site = a.order[t], bad = a.bad[t], over = *a.over;
+    long long v[NH][3];
+#pragma unroll
+    for (int h = 0; h < NH; h++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) v[h][k] = a.facc[3 * ((long)a.ns * h + t) + k];
+#pragma unroll
+    for (int h = 0; h < NH; h++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        a.f[3 * ((long)a.ns * h + site) + k] = (double)v[h][k] * (1.0 / FIX_SCALE);
+        a.facc[3 * ((long)a.ns * h + t) + k] = 0;
+      }
+    redo = (bad | over) != 0;
+    if (bad) a.bad[t] = 0;
+  }
+  unsigned m = __ballot_sync(0xffffffffu, redo);
+  __syncwarp();
+  for (; m; m &= m - 1)
+    direct_forces<POLAR>(a, t - (int)(threadIdx.x & 31) + __ffs(m) - 1, pj, ptab, erd, sx, sy, sz,
+                         cq, sgrid);
+}
+
+template <bool POLAR>
+__global__ void __launch_bounds__(256)
+    finish_forces_kernel(const __grid_constant__ PairArgs a, const int4* __restrict__ pj,
+                         const PairF* __restrict__ ptab, const float4* __restrict__ erd, float sx,
+                         float sy, float sz, float cq, float sgrid) {
   after_previous();
-  finish_forces(ns, halves, order, facc, f);
+  finish_forces<POLAR>(a, pj, ptab, erd, sx, sy, sz, cq, sgrid);
 }
 
 cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, const PairF* ptab,
@@ -1587,8 +1689,16 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
 #undef PAIR_HALF
     if (ge != cudaSuccess) return ge;
     LAUNCHED(L);
-    launch_after(L, finish_forces_kernel, cdiv(a.ns, 256), 256, 0, a.ns, polar ? 2 : 1, a.order,
-                 a.facc, a.f);
+    // with shells plainly: set up beside the last pair CTAs, 59 registers a thread,
+    // it cost 32768 Drude waters 19 us a step; without shells set up early (864
+    // waters 138 -> 132 us an evaluation)
+    if (polar) {
+      finish_forces_kernel<true>
+          <<<cdiv(a.ns, 256), 256, 0, L.s>>>(a, pj, ptab, erd, sx, sy, sz, cq, sg);
+    } else {
+      launch_after(L, finish_forces_kernel<false>, cdiv(a.ns, 256), 256, 0, a, pj, ptab, erd, sx,
+                   sy, sz, cq, sg);
+    }
     LAUNCHED(L);
     return cudaGetLastError();
   }
@@ -2622,7 +2732,8 @@ __global__ void __launch_bounds__(GROUP_WARPS * 32, MEASURE ? 4 : 6)
 
 __global__ void batch_finish_kernel(const BoxStep* __restrict__ B) {
   const BoxStep& e = B[blockIdx.y];
-  if (e.g_half > 0) finish_forces(e.ns, 1, e.pa.order, e.pa.facc, e.pa.f);
+  if (e.g_half > 0)
+    finish_forces<false>(e.pa, e.pj, e.ptab, e.erd, e.sx, e.sy, e.sz, e.cq, e.sg);
 }
 
 template <bool MEASURE>

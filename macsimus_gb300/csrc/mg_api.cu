@@ -3346,8 +3346,9 @@ int mg_batch_md_steps(mg_batch* b, int nsteps, mg_energy* en) {
   BCK(cudaStreamSynchronize(b->main));
   for (size_t i = 0; i < b->box.size(); i++) {
     mg_ctx* c = b->box[i];
-    int rc = fetch_status(c);
-    if (!rc && en) rc = fetch_sums(c);
+    // the sums first: the status word goes into the same block
+    int rc = fetch_sums(c);
+    if (!rc) rc = fetch_status(c);
     if (!rc) {
       cudaError_t e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) rc = fail(c, MG_ERR_CUDA, cudaGetErrorString(e));

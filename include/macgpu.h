@@ -232,6 +232,10 @@ const char *mg_last_error(const mg_ctx *ctx);
 double mg_kappa(const mg_ctx *ctx);
 /* number of k-vectors Q->N */
 int mg_nkvec(const mg_ctx *ctx);
+/* the pair kernel that a force evaluation of this context runs: "all-pairs",
+   "half-shell", "group", "cell" (the FP32 path), "fp64", or "list" with kept
+   neighbour lists */
+const char *mg_pair_kernel(const mg_ctx *ctx);
 
 /* cook's forces(B,A): r = A->rp (host, ns or 2*ns vectors), f = B->rp
    (host, overwritten).  measure != 0 fills *en (may be NULL otherwise). */

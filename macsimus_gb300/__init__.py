@@ -115,6 +115,8 @@ def library():
         L.mg_kappa.argtypes = [vp]
         L.mg_kappa.restype = C.c_double
         L.mg_nkvec.argtypes = [vp]
+        L.mg_pair_kernel.argtypes = [vp]
+        L.mg_pair_kernel.restype = C.c_char_p
         L.mg_last_launches.argtypes = [vp]
         L.mg_forces.argtypes = [vp, _dp, _dp, C.c_int, C.POINTER(Energy)]
         L.mg_forces_device.argtypes = [vp, vp, vp, C.c_int, C.POINTER(Energy)]
@@ -375,6 +377,11 @@ class ForcePath:
     @property
     def launches(self):
         return library().mg_last_launches(self._ctx)
+
+    @property
+    def pair_kernel(self):
+        """the pair kernel a force evaluation runs (mg_pair_kernel)"""
+        return library().mg_pair_kernel(self._ctx).decode()
 
     def forces(self, r, measure=False):
         """cook forces(B,A): returns (f [ns,3], energy dict or None)."""

@@ -2020,6 +2020,12 @@ int mg_destroy(mg_ctx* ctx) {
 const char* mg_last_error(const mg_ctx* ctx) { return ctx ? ctx->err.c_str() : "no context"; }
 double mg_kappa(const mg_ctx* ctx) { return ctx ? ctx->kappa : 0; }
 int mg_nkvec(const mg_ctx* ctx) { return ctx ? ctx->nk : 0; }
+const char* mg_pair_kernel(const mg_ctx* ctx) {
+  if (!ctx) return "";
+  if (ctx->use_list) return "list";
+  if (ctx->precision != MG_MIXED) return "fp64";
+  return ctx->small ? "all-pairs" : (ctx->half ? "half-shell" : (ctx->pair_variant == 8 ? "group" : "cell"));
+}
 int mg_last_launches(const mg_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 int mg_forces_device(mg_ctx* ctx, const double* r_dev, double* f_dev, int measure,

@@ -661,7 +661,12 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   // the FP32 pair kernel.  One cell: all pairs; so with cells of fewer than
   // four sites (a cutoff just short of half the box, cut in many to fit) in a
   // box of up to 8192.  Otherwise variants 9, 10 and the default 0 run the
-  // half-shell kernel
+  // half-shell kernel.  Force evaluations of water, all-pairs against half-shell,
+  // us (measured evaluations behind the stroke): 0.9 sites a cell, 1200 sites
+  // 67/93 and 84/93; 0.6, 3000 sites 106/155 and 170/229; 1.6, 8100 sites
+  // 241/386 and 354/474; 3.0 to 3.7 a cell about even (4200 sites 109/187 and
+  // 123/191, 6600 174/292 and 182/266, 8100 213/368 and 211/311); beyond 8192
+  // sites the pairs outside the cutoff, which grow with the square, would win
   ctx->small = allpairs || (ctx->precision == MG_MIXED && !ctx->use_list &&
                             ctx->pair_variant == 0 && ns <= 8192 &&
                             ns < 4L * nc3[0] * nc3[1] * nc3[2]);

@@ -882,8 +882,8 @@ __device__ __forceinline__ float drude_force_rn(const float4* __restrict__ erd,
 // skipped when no lane needs them.  Measured at 1500 sites: 11 us, the cell
 // kernel 85 and the half-shell kernel 17; at 648 sites held in one cell, where
 // one warp of the cell kernel did all the work, a measured evaluation went
-// from 3.2 ms to about 20 us.  From some 2000 sites on the half-shell kernel is
-// the faster one wherever there is a grid for it.  Forces: FP32 per batch, folded into
+// from 3.2 ms to about 20 us.  Where a cell holds more than three or four sites
+// the half-shell kernel is the faster one.  Forces: FP32 per batch, folded into
 // compensated sums, the warps' sums added in order in FP64; every rounding of
 // the force arithmetic is explicit (measured and plain forces are the same).
 constexpr int ALL_WARPS = 16, ALL_SITES = 8;

@@ -385,9 +385,9 @@ int setup_nf(mg_ctx* ctx, const int K[3], const std::vector<int4>& kvec,
   b.ns = ctx->ns;
   b.nsub = ctx->polar ? 2 : 1;
   const int nc[3] = {ctx->ncx, ctx->ncy, ctx->ncz};
+  nf_grids(K, b.M);
   for (int d = 0; d < 3; d++) {
     b.K[d] = K[d];
-    b.M[d] = nf_grid(K[d]);
     b.nc[d] = nc[d];
     b.marg[d] = ctx->polar ? (int)std::ceil(NF_MARGIN * b.M[d] / ctx->L[d]) : 0;
     const double beta = nf_beta(b.M[d], K[d]);
@@ -835,10 +835,11 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
                                      (p1ctas + ctx->np1job - 1) / ctx->np1job));
   ctx->nkblocks = ctx->precision == MG_MIXED ? (nk + 255) / 256 : k64_red_blocks(k64_items(krows));
   const int nfK[3] = {ctx->Kx, ctx->Ky, ctx->Kz};
+  int nfM[3];
   // non-uniform transforms (mg_nufft.cu) need the cells of the present
   // positions (no kept lists) and serve the automatic engine
   ctx->nf = ctx->precision == MG_MIXED && p->kspace_engine == 0 && !ctx->use_list && ctx->nq > 0 &&
-            nf_fits(nfK);
+            nf_grids(nfK, nfM);
 
   // ---- constraints
   ctx->nc = t->nc;

@@ -9,13 +9,15 @@
 //   phi(t) = exp(beta (sqrt(1 - (2t/w)^2) - 1)), |t| < w/2, w = 8 grid steps
 // of Barnett, Magland and af Klinteberg (SIAM J. Sci. Comput. 41, C479
 // (2019)), whose transform is divided out exactly at every k (host
-// quadrature).  The grid has about 1.75 points per resolved mode.
+// quadrature).  The grid has at least 1.86 points per resolved mode.
 //
 // Measured on 32768 waters: 0.11 ms (spread 54 us, x 5, planes 13, x 5, interp
 // 35) against 0.52 ms for the direct tensor-core passes; the MD step
 // 0.87 -> 0.45 ms; 256 ionic boxes 3.3 -> 2.3 ms.  Error against 64 bits,
-// k-space force relative RMS: window 2e-7..5e-7 at these sizes, FP32 arithmetic
-// 7e-7; the direct passes measure 2.3e-6.  Every sum runs in a fixed order (a grid point gathers its charges
+// k-space force relative RMS, mean over 46 boxes of 650 to 98000 sites: 7.2e-7 (the
+// direct tensor-core passes 11.5e-7; 9.8e-7 with 1.75 points a mode, the weights
+// not cut off and the potential taken whole in the interpolation).
+// Every sum runs in a fixed order (a grid point gathers its charges
 // in the sorted order of the cell list; no floating-point atomics), so the
 // results are reproducible bit for bit, alone or in a batch.
 //
@@ -66,14 +68,15 @@ __device__ __forceinline__ float nf_ex2(float x) {
 
 // the window at z = 2 t / w; nb = -beta log2(e).  The exponent is taken as
 // -beta z^2 / (1 + s), s = sqrt(1 - z^2): beta (s - 1) would carry the
-// rounding of s times beta (1e-6 of the weight near its centre).  Beyond the
-// window (|z| > 1, reached by points of a tile that a charge does not touch)
-// the same arithmetic with |1 - z^2| stays below e^-beta = 2e-9, under the
-// rounding of the sums, and needs no test.
+// rounding of s times beta (1e-6 of the weight near its centre).  Zero beyond the
+// window (reached by points of a tile that a charge does not touch): the same
+// arithmetic with |1 - z^2| would leave up to 1e-7 there, which of two boxes of
+// some 75000 sites made 2.3e-6 of the k-space force, 1.3e-6 and 1.5e-6 without.
 __device__ __forceinline__ float nf_window(float z, float nb, float& s) {
   const float z2 = __fmul_rn(z, z);
   s = nf_sqrt(fabsf(__fmaf_rn(-z, z, 1.f)));
-  return nf_ex2(__fmul_rn(__fmul_rn(nb, z2), nf_rcp(__fadd_rn(1.f, s))));
+  const float w = nf_ex2(__fmul_rn(__fmul_rn(nb, z2), nf_rcp(__fadd_rn(1.f, s))));
+  return z2 < 1.f ? w : 0.f;
 }
 
 // pairs of floats: acc += a * w, a * w
@@ -754,6 +757,12 @@ __global__ void __launch_bounds__(DF_THREADS) nf_idft_x_kernel(const NfBox* __re
 // four charges; the sums over y run per x with the 1-D weights and
 // derivatives (each lane computes one of the 8 and passes it on by
 // shuffles): two FMAs per load.
+//
+// The potential of the charge's own grid cell is subtracted from every value.  A
+// constant has no gradient, but the window's derivatives add up to zero only to
+// their rounding and the window's error, both of which it would multiply: the
+// potential is mostly long waves, hundreds of times its change over the window.
+// Of a brine's k-space force (12544 sites) the error fell from 1.2e-6 to 0.9e-6.
 struct NfWeights {
   float w[3], g[3];   // window and derivative of this lane's step, x y z
 
@@ -808,10 +817,11 @@ struct NfForce {
 // offset from the charge's first.  Bound by the shared-memory wavefronts (64
 // loads of four unaligned 32-byte rows each per four charges): 35 us on 32768
 // waters, 8.8 us on 864, where reading the rows from memory (below) takes 36
-// and 12 us.
+// and 12 us.  Two CTAs an SM: left to itself the compiler takes 80 registers and
+// spills, 1 us more on 12544 sites.
 constexpr int IT_LD = 2 * TILE, IT_PL = IT_LD * IT_LD;
 
-__global__ void __launch_bounds__(SP_WARPS * 32)
+__global__ void __launch_bounds__(SP_WARPS * 32, 2)
     nf_interp_tile_kernel(const NfBox* __restrict__ boxes, double* __restrict__ f_or_null) {
   after_previous();
   const NfBox& b = boxes[blockIdx.z];
@@ -851,6 +861,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32)
       NfWeights k;
       k.set(b, l8, fx, fy, fz);
       const float* row = ph + jx * IT_PL + jy * IT_LD + jz + 1 + l8;
+      const float home = ph[(jx + W / 2 - 1) * IT_PL + (jy + W / 2 - 1) * IT_LD + jz + W / 2];
       float wy[W], gy[W];
 #pragma unroll
       for (int c = 0; c < W; c++) {
@@ -865,7 +876,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32)
         float u = 0.f, v = 0.f;
 #pragma unroll
         for (int c = 0; c < W; c++) {
-          const float g = row[a * IT_PL + c * IT_LD];
+          const float g = __fadd_rn(row[a * IT_PL + c * IT_LD], -home);
           u = __fmaf_rn(wy[c], g, u);
           v = __fmaf_rn(gy[c], g, v);
         }
@@ -968,6 +979,7 @@ __global__ void __launch_bounds__(IP_WARPS * 32, 8)
       ax += ax < 0 ? Mx : (ax >= Mx ? -Mx : 0);
       ay += ay < 0 ? My : (ay >= My ? -My : 0);
       az += az < 0 ? Mz : (az >= Mz ? -Mz : 0);
+      const float home = __ldg(G + ((long)jx * My + jy) * Mz + jz);
       ax *= My * Mz;
       ay *= Mz;
       float wy[W], gy[W];
@@ -987,7 +999,7 @@ __global__ void __launch_bounds__(IP_WARPS * 32, 8)
         float u = 0.f, v = 0.f;
 #pragma unroll
         for (int c = 0; c < W; c++) {
-          const float g = __ldg(row + yo[c]);
+          const float g = __fadd_rn(__ldg(row + yo[c]), -home);
           u = __fmaf_rn(wy[c], g, u);
           v = __fmaf_rn(gy[c], g, v);
         }
@@ -1012,12 +1024,10 @@ __global__ void nf_far_kernel(int ns, const float4* __restrict__ pdj, float lim,
 
 // -------------------------------------------------------------- host side --
 
-// the grid of K modes on an edge: the next multiple of 4 of 1.75 (2 K + 1),
-// at least a tile and a window (16).  The window error at the highest modes
-// falls with the number of points (2e-6 of the k-space force at 1.53 points
-// per mode, 5e-7 at 1.75, 2e-7 at 2.1) and the transforms grow with its cube
-int nf_grid(int K) {
-  const int m = ((int)std::ceil(1.75 * (2 * K + 1)) + 3) / 4 * 4;
+// the grid of K modes on an edge: the next multiple of 4 of `points` per mode,
+// (2 K + 1) modes, at least a tile and a window (16)
+static int nf_points(int K, double points) {
+  const int m = ((int)std::ceil(points * (2 * K + 1)) + 3) / 4 * 4;
   return m < 16 ? 16 : m;
 }
 
@@ -1101,10 +1111,21 @@ static size_t nf_ix_smem(int K, int M) {
 // a CTA's 227 KB less the kernels' static part
 constexpr int NF_MAX_SMEM = 225 * 1024;
 
-bool nf_fits(const int K[3]) {
-  const int M[3] = {nf_grid(K[0]), nf_grid(K[1]), nf_grid(K[2])};
-  return nf_plane_smem(K, M, NF_CS) <= NF_MAX_SMEM && nf_x_smem(K[0], M[0]) <= NF_MAX_SMEM &&
-         nf_ix_smem(K[0], M[0]) <= NF_MAX_SMEM;
+// The grids M of the modes K; false where the transforms do not fit a CTA.  The
+// window's error at the highest modes falls with the points per mode and the
+// transforms grow with their cube.  At 1.86 the k-space force is closer to the
+// 64-bit sums than the direct tensor-core passes take it, in every one of 46 boxes
+// of 650 to 98000 sites (water, brine, Drude water, TIP4P; |n| 6 to 20); at 1.75 it
+// was 1.4 and 2.6 times as far for brines with |n| <= 12 and 20.  1.75 only for the
+// largest sets, which fit no more points (|n| 44 and 45).
+bool nf_grids(const int K[3], int M[3]) {
+  for (double points : {1.86, 1.75}) {
+    for (int d = 0; d < 3; d++) M[d] = nf_points(K[d], points);
+    if (nf_plane_smem(K, M, NF_CS) <= NF_MAX_SMEM && nf_x_smem(K[0], M[0]) <= NF_MAX_SMEM &&
+        nf_ix_smem(K[0], M[0]) <= NF_MAX_SMEM)
+      return true;
+  }
+  return false;
 }
 
 static int nf_tiles(const NfBox& b) {

@@ -47,8 +47,7 @@ struct NfGrid {
   int sx, six, splane, splane_few;
 };
 
-int nf_grid(int K);
-bool nf_fits(const int K[3]);
+bool nf_grids(const int K[3], int M[3]);
 double nf_beta(int M, int K);
 int nf_dense(int nq, const int M[3]);
 void nf_tables(const int K[3], const int M[3], const std::vector<int4>& kvec,

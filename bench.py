@@ -29,6 +29,10 @@ METRIC = "ns/day & atom-steps/s, mixed vs plain FP64 GPU path at force RMS err â
 WORKLOAD = "spce32768"
 FLOP_PER_PAIR = 45          # FP32 flops per in-cutoff (half) pair
 FLOP_PER_KQ = 8             # flops per (k-vector, charge) per Ewald pass
+# the roofline's name, and its entry in profiles/traffic_*.json, of each pair
+# kernel a context may run (mg_pair_kernel)
+PAIR_LABEL = {"half-shell": "pair_half", "all-pairs": "pair_all", "group": "pair_group",
+              "cell": "pair_mixed", "list": "pair_list", "fp64": "pair_fp64"}
 
 
 def env_rank():
@@ -298,13 +302,8 @@ def run_ours(args, rank, world, local):
     name, (kms, kcnt) = top
     kavg = kms / max(kcnt, 1)
     achieved = algo.get(name, 0) / (kavg * 1e-3) / 1e12 if kavg > 0 else 0.0
-    # the pair step's kernel: the group kernel (pair_variant 8), the half-shell
-    # kernel (9 and 10) or the cell kernel
-    if name == "pair_mixed" and tuned.get("pair_variant", 0) in (8, 9, 10):
-        pv = tuned["pair_variant"]
-        name = "pair_group" if pv == 8 else "pair_half"
-        algo[name] = algo["pair_mixed"]
-        achieved = algo[name] / (kavg * 1e-3) / 1e12 if kavg > 0 else 0.0
+    if name == "pair_mixed":
+        name = PAIR_LABEL[fp.pair_kernel]
     traffic = None
     tpath = os.path.join(REPO, "profiles", "traffic_%s.json" % args.workload)
     if os.path.exists(tpath):

@@ -408,15 +408,16 @@ int mg_xwidom(mg_ctx *ctx, int nlist, const int *mols, const int *vtype, const d
    No reference counterpart.  Times the force evaluation of the configuration
    r for every cell subdivision (cells_per_cutoff 1..3) and Ewald pass-1
    split (kspace_ctas_per_sm 6, 10, 16) and writes the fastest pair into
-   *par, then the fastest of the 8 cell-kernel pair_variant values at that
-   choice, of the group kernel (pair_variant 8) at every subdivision and,
-   on the FP32 path, of the half-shell kernel (pair_variant 9 and 10, one
-   kernel) at every subdivision, each timed (FP32 path) with
-   kspace_serial 0 and 1, the pair chosen together.  Builds and frees its
-   own trial contexts; ms[28] (optional) gets the time per evaluation of
-   each trial (the best of three blocks of nrep evaluations; cdiv-major,
-   then the 8 cell-kernel variants, the group
-   kernel at cdiv 1..3 and the half-shell group kernel (9) at cdiv 1..3, the
+   *par, then the fastest of the pair_variant values 0..7 at that choice, of
+   the group kernel (pair_variant 8) at every subdivision and, on the FP32
+   path, of the half-shell kernel (pair_variant 9 and 10, one kernel) at
+   every subdivision, each timed (FP32 path) with kspace_serial 0 and 1, the
+   pair chosen together.  Choices that come to the same evaluation share one
+   timing: the splits where no kernel reads the split (*par then keeps its own,
+   or gets 10), the numbers of one pair kernel.  Builds and frees its own trial
+   contexts; ms[28] (optional) gets the time per evaluation of each trial (the
+   best of three blocks of nrep evaluations; cdiv-major, then pair_variant
+   0..7, the group kernel at cdiv 1..3 and pair_variant 9 at cdiv 1..3, the
    faster of the two kspace_serial settings each, then the chosen variant
    with kspace_serial 0 and 1, then pair_variant 10 at cdiv 1..3; -1 if that
    grid is not possible or the trial did not run). */

@@ -3469,10 +3469,28 @@ int mg_autotune(const mg_topology* top, mg_params* par, const double* r, int nre
   // best of three blocks of nrep evaluations (choices within a few per cent
   // of each other, such as the Ewald chain beside or after the r-space
   // chain, flipped between runs on single blocks)
+  // Choices that come to the same evaluation (a split that no kernel reads, two
+  // variants of one kernel) are timed once: of several timings of one thing the
+  // luckiest would be picked.
+  std::map<std::string, double> timed;
+  bool split_counts = false;
   auto trial = [&](const mg_params& p2) -> double {
     int st = 0;
     mg_ctx* c = mg_create(top, &p2, &st);
     if (!c) return -1;
+    // what of the parameters under trial the evaluation depends on; the split
+    // only the direct FP32-core pass 1 reads
+    const bool split = c->precision == MG_MIXED && c->nq > 0 && !c->nf && !c->sk_tc;
+    split_counts = split_counts || split;
+    std::string key = mg_pair_kernel(c);
+    if (key == "cell") key += std::to_string(c->pair_variant & 7);
+    for (int v : {c->ncx, c->ncy, c->ncz, c->overlap ? 1 : 0, split ? p2.kspace_ctas_per_sm : 0})
+      key += " " + std::to_string(v);
+    const auto seen = timed.find(key);
+    if (seen != timed.end()) {
+      mg_destroy(c);
+      return seen->second;
+    }
     double t = -1;
     int e = mg_forces_device(c, r_dev, f_dev, 0, nullptr);  // warm-up
     for (int blk = 0; blk < 3 && !e; blk++) {
@@ -3488,6 +3506,7 @@ int mg_autotune(const mg_topology* top, mg_params* par, const double* r, int nre
       rc = e;
       t = -1;
     }
+    timed[key] = t;
     mg_destroy(c);
     return t;
   };
@@ -3498,6 +3517,11 @@ int mg_autotune(const mg_topology* top, mg_params* par, const double* r, int nre
       mg_params p2 = *par;
       p2.cells_per_cutoff = cd[a];
       p2.kspace_ctas_per_sm = kc[b];
+      // the split does not count: its first timing stands for all three
+      if (b > 0 && !split_counts) {
+        if (ms) ms[3 * a + b] = ms[3 * a];
+        continue;
+      }
       const double t = trial(p2);
       if (ms) ms[3 * a + b] = t;
       if (t > 0 && t < best) {
@@ -3506,6 +3530,8 @@ int mg_autotune(const mg_topology* top, mg_params* par, const double* r, int nre
         bk = kc[b];
       }
     }
+  // where the split does not count it stays the caller's, or the default
+  if (!split_counts) bk = par->kspace_ctas_per_sm > 0 ? par->kspace_ctas_per_sm : 10;
   // the pair-kernel variants at the best split, each with the Ewald chain
   // beside the r-space chain and after it (FP32 path): which is faster
   // depends on how the kernels share the SMs, so the two are chosen together
@@ -3540,8 +3566,7 @@ int mg_autotune(const mg_topology* top, mg_params* par, const double* r, int nre
     // the group pair kernel (variant 8) at every cell subdivision: its
     // pruning favours other cells than the cell kernel does
     for (int a = 0; a < 3 && rc == MG_OK; a++) consider(8, cd[a], ms ? ms + 17 + a : nullptr);
-    // and its half-shell forms (Newton's third law; FP32 path): lanes on the
-    // home sites, and lanes on the neighbours
+    // and the half-shell kernel, which both of its numbers name
     if (par->precision == MG_MIXED) {
       for (int a = 0; a < 3 && rc == MG_OK; a++) consider(9, cd[a], ms ? ms + 20 + a : nullptr);
       for (int a = 0; a < 3 && rc == MG_OK; a++) consider(10, cd[a], ms ? ms + 25 + a : nullptr);

@@ -1330,7 +1330,7 @@ ExclArgs excl_args(mg_ctx* ctx, const double* r_dev, double* f) {
   a.iLy = 1 / ctx->L[1];
   a.iLz = 1 / ctx->L[2];
   a.cutoff_sq = ctx->cutoff * ctx->cutoff;
-  a.alpha = (float)ctx->alpha;
+  a.alpha = ctx->alpha;
   a.r = r_dev;
   a.f = f;
   // energy rows after the pair kernel's

@@ -49,6 +49,42 @@ __device__ __forceinline__ T excl_term(T rr, T alpha, T* erd, bool minus_const =
   return minus_const ? y - A : y;
 }
 
+// The same of the FP32 path, for the sites of a molecule.  With t = (alpha r)^2 the
+// Taylor series of
+//   erf(x)/x = 2/sqrt(pi) (1 - t R(t)),  R = sum (-t)^(n-1) / ((2n+1) n!),
+//   D(t) = (1 - t R - exp(-t)) / t = sum (-t)^(n-1) 2n / ((2n+1) n!),  n >= 1,
+// the first terms left out below 1e-9 up to t = 1/2, the first step and the factors
+// in FP64.  As a difference in FP32 D lost a factor 3/(2t) of its digits, 18 for the OH
+// of water at alpha 0.29 / A: the exclusion forces were good to 3e-6, alike for all
+// molecules, and so most of the error of the virial.
+__device__ __forceinline__ double excl_mixed(double r2, double alpha, double* erd) {
+  const double aq = __dmul_rn(alpha, alpha), t = __dmul_rn(r2, aq),
+               A = __dmul_rn(alpha, -1.1283791670955126);
+  if (t < 0.5) {
+    const float x = -(float)t;
+    float R = 1.f / 685440, D = 1.f / 383040;
+    R = __fmaf_rn(x, R, 1.f / 75600);
+    R = __fmaf_rn(x, R, 1.f / 9360);
+    R = __fmaf_rn(x, R, 1.f / 1320);
+    R = __fmaf_rn(x, R, 1.f / 216);
+    R = __fmaf_rn(x, R, 1.f / 42);
+    R = __fmaf_rn(x, R, 1.f / 10);
+    D = __fmaf_rn(x, D, 1.f / 42840);
+    D = __fmaf_rn(x, D, 1.f / 5400);
+    D = __fmaf_rn(x, D, 1.f / 780);
+    D = __fmaf_rn(x, D, 1.f / 132);
+    D = __fmaf_rn(x, D, 1.f / 27);
+    D = __fmaf_rn(x, D, 1.f / 7);
+    D = __fmaf_rn(x, D, 2.f / 5);
+    *erd = __dmul_rn(__dmul_rn(A, aq), __fma_rn(-t, (double)D, 2.0 / 3));
+    return __dmul_rn(A, __fma_rn(-t, __fma_rn(-t, (double)R, 1.0 / 3), 1.0));
+  }
+  float f;
+  const float e = excl_term<float>((float)r2, (float)alpha, &f);
+  *erd = f;
+  return e;
+}
+
 // f/r of a spline term (erd), energy (eru) added to e when MEASURE
 template <bool MEASURE>
 __device__ __forceinline__ float spline_term(const float4* __restrict__ erd,
@@ -81,19 +117,19 @@ __device__ __forceinline__ float spline_any(const float4* erd, const float4* __r
 }
 
 // excluded intramolecular term: its Ewald correction is large and cancels
-// the self term; evaluated in FP32 (an FP64 erf on a divergent lane would
-// stall the warp on the slow FP64 pipe) and summed into FP64
+// the self term; evaluated in FP32 but for the last steps (an FP64 erf on a
+// divergent lane would stall the warp on the slow FP64 pipe) and summed into FP64
 template <bool MEASURE>
-__device__ __forceinline__ void excl_acc(float dx, float dy, float dz, double qq, float alpha,
+__device__ __forceinline__ void excl_acc(float dx, float dy, float dz, double qq, double alpha,
                                          double& fx, double& fy, double& fz, double* en) {
-  float fe;
-  const float e = excl_term<float>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), alpha, &fe);
-  const double fq = (double)fe * qq;
+  double fe;
+  const double e = excl_mixed(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), alpha, &fe);
+  const double fq = fe * qq;
   fx += fq * dx;
   fy += fq * dy;
   fz += fq * dz;
   if (MEASURE) {
-    en[0] += (double)e * qq;
+    en[0] += e * qq;
     en[3] += fq * dx * dx;
     en[4] += fq * dy * dy;
     en[5] += fq * dz * dz;

@@ -427,7 +427,7 @@ struct ExclArgs {
   const double4* xq;    // charge products: centre-centre, Drude(i)-centre(j),
                         // centre(i)-Drude(j), Drude-Drude
   double Lx, Ly, Lz, iLx, iLy, iLz, cutoff_sq;
-  float alpha;
+  double alpha;
   const double* r;      // positions (+ Drude offsets in the second half)
   double* f;            // forces, added to
   double* epart;        // [nblocks * 10] energy rows (measure)

@@ -1765,8 +1765,8 @@ cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj, con
 
 // -erf(alpha r)/r of the intramolecular pairs (cook/ljqqnp.c:131-141, its
 // Drude forms cook/ljqqpol.c) for the mixed cell path: each pair once, from
-// the FP64 positions (nearest image), the term in FP32 as in the pair
-// kernels, forces and energy summed in FP64.  Pairs beyond the cutoff are
+// the FP64 positions (nearest image), the term in FP32 but for its last steps
+// (excl_mixed), forces and energy summed in FP64.  Pairs beyond the cutoff are
 // skipped, as the cell traversal never meets them.
 // The force arithmetic rounds explicitly (`_rn`): the measuring
 // instantiation also uses the products for the virial, and a product the
@@ -1777,11 +1777,11 @@ __device__ __forceinline__ double excl_r2(double dx, double dy, double dz) {
 }
 
 template <bool MEASURE>
-__device__ __forceinline__ void excl_pair(double dx, double dy, double dz, double qq, float alpha,
+__device__ __forceinline__ void excl_pair(double dx, double dy, double dz, double qq, double alpha,
                                           double* fi, double* fj, double* en) {
-  float fe;
-  const float e = excl_term<float>((float)excl_r2(dx, dy, dz), alpha, &fe);
-  const double fq = __dmul_rn((double)fe, qq);
+  double fe;
+  const double e = excl_mixed(excl_r2(dx, dy, dz), alpha, &fe);
+  const double fq = __dmul_rn(fe, qq);
   const double Fx = __dmul_rn(fq, dx), Fy = __dmul_rn(fq, dy), Fz = __dmul_rn(fq, dz);
   fi[0] = __dadd_rn(fi[0], Fx);
   fi[1] = __dadd_rn(fi[1], Fy);
@@ -1790,7 +1790,7 @@ __device__ __forceinline__ void excl_pair(double dx, double dy, double dz, doubl
   fj[1] = __dadd_rn(fj[1], -Fy);
   fj[2] = __dadd_rn(fj[2], -Fz);
   if (MEASURE) {
-    en[0] += (double)e * qq;
+    en[0] += e * qq;
     en[1] += Fx * dx;
     en[2] += Fy * dy;
     en[3] += Fz * dz;

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NL_THREADS)
     pair_list_mixed_kernel(PairArgs a, ListArgs l, const int4* __restrict__ pj,
                            const PairF* __restrict__ ptab_g, const float4* __restrict__ erd,
                            const float4* __restrict__ eru, float sx, float sy, float sz, float cq,
-                           float sgrid, float alpha) {
+                           float sgrid, double alpha) {
   __shared__ PairF ptab[MAX_KINDS * MAX_KINDS];
   __shared__ double ered[NL_THREADS];
   const int nk = a.nkind, ntab = a.ntab;
@@ -364,7 +364,8 @@ cudaError_t k_pair_list_mixed(const Launch& L, const PairArgs& a, const ListArgs
   const int grid = list_blocks(a.ns, true);
   const float sx = (float)(a.Lx / 4294967296.0), sy = (float)(a.Ly / 4294967296.0),
               sz = (float)(a.Lz / 4294967296.0);
-  const float cq = (float)a.cutoff_sq, sg = (float)a.sgrid, al = (float)a.alpha;
+  const float cq = (float)a.cutoff_sq, sg = (float)a.sgrid;
+  const double al = a.alpha;
 #define LAUNCH_PL(M, P) \
   pair_list_mixed_kernel<M, P><<<grid, NL_THREADS, 0, L.s>>>(a, l, pj, ptab, erd, eru, sx, sy, sz, cq, sg, al)
   if (polar) {

@@ -90,10 +90,12 @@ template <bool MEASURE>
 __device__ __forceinline__ float spline_term(const float4* __restrict__ erd,
                                              const float4* __restrict__ eru, float r2, float sgrid,
                                              int ntab, float qq, float& e) {
-  // floor(r2 sgrid) without a float-to-int conversion: r2 sgrid - 1/2 rounded
-  // to an integer in the mantissa of 1.5 * 2^23 (0 <= r2 sgrid < 2^22; at an
-  // exact knot either neighbouring interval gives the same value)
-  const int ix = min(__float_as_int(fmaf(r2, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+  // floor(r2 sgrid) without a float-to-int conversion: the sum rounded towards
+  // zero to an integer in the mantissa of 1.5 * 2^23 (0 <= r2 sgrid < 2^22).
+  // (Rounded to nearest from 1.5 * 2^23 - 1/2, which no float is, it was the next
+  // interval in the upper half of each: charge terms off by 9e-5 at 0.65 A, 8e-6 at
+  // 1 A, 1e-6 at 1.4 A and 2e-7 at 2 A)
+  const int ix = min(__float_as_int(__fmaf_rz(r2, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
   const float4 d = __ldg(erd + ix);
   if (MEASURE) {
     const float4 u = __ldg(eru + ix);
@@ -107,7 +109,7 @@ __device__ __forceinline__ float spline_term(const float4* __restrict__ erd,
 template <bool MEASURE, bool LDG>
 __device__ __forceinline__ float spline_any(const float4* erd, const float4* __restrict__ eru,
                                             float r2, float sgrid, int ntab, float qq, float& e) {
-  const int ix = min(__float_as_int(fmaf(r2, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+  const int ix = min(__float_as_int(__fmaf_rz(r2, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
   const float4 d = LDG ? __ldg(erd + ix) : erd[ix];
   if (MEASURE) {
     const float4 u = __ldg(eru + ix);

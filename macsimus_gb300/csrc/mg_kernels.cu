@@ -847,7 +847,7 @@ __device__ __forceinline__ float pair_force_rn(const PairFS& P, float rr,
   y = __fmul_rn(__fmul_rn(x, x), x);
   flj = rr < P.C1q ? __fmul_rn(__fmul_rn(P.E24, __fmaf_rn(__fmul_rn(2.f, y), y, -y)), x)
                    : (rr < P.C2q ? __fmul_rn(P.A4, __fadd_rn(rr, -P.C2q)) : 0.f);
-  const int ix = min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+  const int ix = min(__float_as_int(__fmaf_rz(rr, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
   const float4 d = __ldg(erd + ix);
   return __fmaf_rn(__fmaf_rn(d.y, rcp_approx(__fadd_rn(d.z, rr)), d.x), P.qq, flj);
 }
@@ -861,7 +861,7 @@ __device__ __forceinline__ float drude_force_rn(const float4* __restrict__ erd,
                                                 float ey, float ez, float sgrid, int ntab,
                                                 float q, float& e) {
   const float r2 = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
-  const int ix = min(__float_as_int(__fmaf_rn(r2, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+  const int ix = min(__float_as_int(__fmaf_rz(r2, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
   const float4 d = __ldg(erd + ix);
   if (MEASURE) {
     const float4 u = __ldg(eru + ix);
@@ -1249,7 +1249,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
           P.qq = pp->qq;
           // no LJ at this home site
           const int ix =
-              min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) - 0x4B400000, ntab - 1);
+              min(__float_as_int(__fmaf_rz(rr, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
           const float4 d = __ldg(erd + ix);
           f = __fmul_rn(__fmaf_rn(d.y, rcp_approx(__fadd_rn(d.z, rr)), d.x), P.qq);
         }
@@ -1304,7 +1304,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
             e_lj += ok ? u : 0.f;
             e_vir += ok ? rr * flj : 0.f;
           }
-          const float4 eu = __ldg(eru + min(__float_as_int(__fmaf_rn(rr, sgrid, 12582911.5f)) -
+          const float4 eu = __ldg(eru + min(__float_as_int(__fmaf_rz(rr, sgrid, 12582912.f)) -
                                                 0x4B400000, ntab - 1));
           e_el += ok ? fmaf(fmaf(eu.y, rcp_approx(eu.z + rr), eu.x), P.qq, e_p) : 0.f;
         }

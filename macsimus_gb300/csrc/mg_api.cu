@@ -980,13 +980,18 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
   if (ctx->precision == MG_MIXED) {
     CK(dalloc(&ctx->d_pj, ns));
     CK(upload(&ctx->d_ptabf, pf.data(), pf.size()));
-    std::vector<float4> erd(ntab), eru(ntab);
-    for (int i = 0; i < ntab; i++) {
-      erd[i] = make_float4((float)ert[6 * i + 3], (float)ert[6 * i + 4], (float)ert[6 * i + 5], 0);
-      eru[i] = make_float4((float)ert[6 * i], (float)ert[6 * i + 1], (float)ert[6 * i + 2], 0);
+    {
+      double* t = nullptr;
+      CK(dalloc(&ctx->d_erd, ntab));
+      CK(dalloc(&ctx->d_eru, ntab));
+      CK(upload(&t, ert.data(), ert.size()));
+      int cnt = 0;
+      cudaError_t er = k_round_spline(Launch{ctx->stream, &cnt}, ntab, t, ctx->sgrid, ctx->d_erd,
+                                      ctx->d_eru);
+      if (er == cudaSuccess) er = cudaStreamSynchronize(ctx->stream);
+      cudaFree(t);
+      CK(er);
     }
-    CK(upload(&ctx->d_erd, erd.data(), ntab));
-    CK(upload(&ctx->d_eru, eru.data(), ntab));
     {
       // phase rows zero-padded to whole groups of 32 charges (tensor-core pass 1)
       const size_t ntab = (size_t)((ctx->nq + 31) / 32 * 32) * ctx->row;

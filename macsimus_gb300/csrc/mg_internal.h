@@ -197,6 +197,9 @@ struct PairArgs {
   float flim;
   int maxgroups;
 };
+// the erfc splines of the FP32 path from those in FP64, ert [n][6]
+cudaError_t k_round_spline(const Launch& L, int n, const double* ert, double sgrid, float4* erd,
+                           float4* eru);
 cudaError_t k_pair_mixed(const Launch& L, const PairArgs& a, const int4* pj,
                          const PairF* ptab, const float4* erd, const float4* eru,
                          bool measure, bool polar);

@@ -337,6 +337,42 @@ cudaError_t upload(T** p, const T* h, size_t n) {
   return cudaMemcpy(*p, h, sizeof(T) * n, cudaMemcpyHostToDevice);
 }
 
+// The Lennard-Jones constants of the FP32 kernels for separations in units of
+// `s` A, with what their rounding leaves over put where it does not count: a
+// relative error of sigma^2 or of the unit comes out up to 50 times as large in
+// the virial of a liquid (both terms grow with the 6th and the 12th power and
+// nearly cancel), the same for every pair.  With q near sigma^2, k = (sigma^2 / q)^3
+// and y = (q / r^2)^3:  u = E4 k^2 y (y - 1/k), f = 24 eps k^2 y (2 y - 1/k) / r^2.
+// Of the floats next to sigma^2 that q is taken which leaves 1/k and the two
+// factors the smallest rounding.
+PairF pair_f(const PairLJ& P, double s) {
+  PairF F{};
+  const double s2 = s * s;
+  F.C1q = (float)(P.C1q * s2);
+  F.C2q = (float)(P.C2q * s2);
+  F.A = (float)(P.A / (s2 * s2));
+  F.A4 = (float)(P.A4 / (s2 * s));
+  F.lam = 1;
+  if (P.Sq == 0) return F;
+  const double Sq = P.Sq * s2;
+  float q = (float)Sq;
+  for (int n = 0; n < 32; n++) q = std::nextafterf(q, 0.f);
+  double best = 1;
+  for (int n = 0; n < 65; n++, q = std::nextafterf(q, 2 * q)) {
+    const double c = Sq / q, k = c * c * c,
+                 v[3] = {1 / k, P.E4 * k * k, P.E24 * P.Sq * s * k * k / q};
+    double off = 0;
+    for (double x : v) off += x != 0 ? std::fabs((float)x / x - 1) : 0;
+    if (off >= best) continue;
+    best = off;
+    F.Sq = q;
+    F.lam = (float)v[0];
+    F.E4 = (float)v[1];
+    F.E24 = (float)v[2];
+  }
+  return F;
+}
+
 int k64_extent(const KRow& r) { return std::max(std::abs(r.kzlo), std::abs(r.kzhi)); }
 int k64_items(const std::vector<KRow>& krows) {
   int n = 0;
@@ -598,6 +634,13 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
         return fail(ctx, MG_ERR_SETUP, "smooth LJ cutoff cannot be determined");
     }
   int nk2 = ctx->nkind * ctx->nkind;
+  // the FP32 path's separations come out in this unit (A): a fixed-point step in
+  // A is rounded to FP32 for each edge
+  double unit = 1;
+  for (int d = 0; d < 3; d++) {
+    const double step = p->L[d] / 4294967296.0;
+    unit *= std::cbrt((double)(float)step / step);
+  }
   std::vector<PairF> pf(nk2);
   std::vector<PairD> pd(nk2);
   for (int a = 0; a < ctx->nkind; a++)
@@ -607,10 +650,16 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
                    qcp = kind_q[a] * kind_qp[b], qpp = kind_qp[a] * kind_qp[b];
       pd[a * ctx->nkind + b] =
           PairD{P.C1q, P.C2q, P.A4, P.E24, P.Sq, qq, P.A, P.E4, qpc, qcp, qpp, 0.0};
-      pf[a * ctx->nkind + b] = PairF{(float)P.C1q, (float)P.C2q, (float)P.A4, (float)P.E24,
-                                     (float)P.Sq,  (float)qq,    (float)P.A,  (float)P.E4,
-                                     (float)qpc,   (float)qcp,   (float)qpp,  0.f,
-                                     qq,           qpc,          qcp,         qpp};
+      PairF& F = pf[a * ctx->nkind + b];
+      F = pair_f(P, unit);
+      F.qq = (float)qq;
+      F.qpc = (float)qpc;
+      F.qcp = (float)qcp;
+      F.qpp = (float)qpp;
+      F.qqd = qq;
+      F.qpcd = qpc;
+      F.qcpd = qcp;
+      F.qppd = qpp;
     }
 
   for (int k = 0; k < ctx->nkind; k++) {

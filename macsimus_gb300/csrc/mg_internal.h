@@ -33,7 +33,7 @@ void aspc_coefficients(int k, double* B, double* omega);
 struct PairF {
   float C1q, C2q, A4, E24;        // LJ force
   float Sq, qq, A, E4;            // LJ energy, centre-centre charge product
-  float qpc, qcp, qpp, pad;
+  float qpc, qcp, qpp, lam;       // lam: 1 but for the rounding of Sq (pair_f)
   double qqd, qpcd, qcpd, qppd;   // the charge products in FP64 (exclusions)
 };
 struct PairD {
@@ -44,7 +44,7 @@ struct PairD {
 struct PairFS {
   float C1q, C2q, A4, E24;
   float Sq, qq, A, E4;
-  float qpc, qcp, qpp, pad;
+  float qpc, qcp, qpp, lam;
 };
 static_assert(sizeof(PairF) == 80 && sizeof(PairFS) == 48, "PairFS is the head of PairF");
 

@@ -461,8 +461,8 @@ MG_BODY void pair_mixed_kernel_body(const PairArgs& a,
             float U;
             if (rr < P.C1q) {
               const float x = __fdividef(P.Sq, rr), y = x * x * x;
-              f = P.E24 * fmaf(2.f * y, y, -y) * x;
-              U = P.E4 * fmaf(y, y, -y);
+              f = P.E24 * (fmaf(2.f, y, -P.lam) * y) * x;
+              U = P.E4 * ((y - P.lam) * y);
             } else {
               const float x = rr - P.C2q;
               f = P.A4 * x;
@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(NW * 32)
             const PairFS P = ptab[kind_i * nk + (qw & 255)];
             const float x = __fdividef(P.Sq, rr), y = x * x * x, xt = rr - P.C2q;
             const bool core = rr < P.C1q, tail = rr < P.C2q;
-            const float flj = core ? P.E24 * fmaf(2.f * y, y, -y) * x : (tail ? P.A4 * xt : 0.f);
+            const float flj = core ? P.E24 * (fmaf(2.f, y, -P.lam) * y) * x : (tail ? P.A4 * xt : 0.f);
             float e_el_p = 0.f;
             float f = flj + spline_any<MEASURE, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
             f = ok ? f : 0.f;
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(NW * 32)
             ay = fmaf(f, dy, ay);
             az = fmaf(f, dz, az);
             if (MEASURE && ok) {
-              e_lj += core ? P.E4 * fmaf(y, y, -y) : (tail ? P.A * xt * xt : 0.f);
+              e_lj += core ? P.E4 * ((y - P.lam) * y) : (tail ? P.A * xt * xt : 0.f);
               e_vir += rr * flj;
               e_el += e_el_p;
               pv.add(dx, dy, dz, f);
@@ -872,7 +872,7 @@ __device__ __forceinline__ float pair_force_rn(const PairFS& P, float rr,
                                                int ntab, float& flj, float& y) {
   const float x = __fmul_rn(P.Sq, rcp_approx(rr));
   y = __fmul_rn(__fmul_rn(x, x), x);
-  flj = rr < P.C1q ? __fmul_rn(__fmul_rn(P.E24, __fmaf_rn(__fmul_rn(2.f, y), y, -y)), x)
+  flj = rr < P.C1q ? __fmul_rn(__fmul_rn(P.E24, __fmul_rn(__fmaf_rn(2.f, y, -P.lam), y)), x)
                    : (rr < P.C2q ? __fmul_rn(P.A4, __fadd_rn(rr, -P.C2q)) : 0.f);
   const int ix = min(__float_as_int(__fmaf_rz(rr, sgrid, 12582912.f)) - 0x4B400000, ntab - 1);
   const float4 d = __ldg(erd + ix);
@@ -1001,7 +1001,7 @@ MG_BODY void pair_all_kernel_body(const PairArgs& a, const int4* __restrict__ pj
       if (MEASURE && ok) {
         // energies and virial: no effect on the forces
         const float xt = rr - P.C2q;
-        e_lj += rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
+        e_lj += rr < P.C1q ? P.E4 * ((y - P.lam) * y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
         e_vir += rr * flj;
         float e_el_p = 0.f;
         spline_any<true, true>(erd, eru, rr, sgrid, ntab, P.qq, e_el_p);
@@ -1327,7 +1327,7 @@ __device__ __forceinline__ void pair_half_kernel_body(const PairArgs& a, const i
           // the forces are
           if (HEAVY) {
             const float xt = rr - P.C2q;
-            const float u = rr < P.C1q ? P.E4 * fmaf(y, y, -y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
+            const float u = rr < P.C1q ? P.E4 * ((y - P.lam) * y) : (rr < P.C2q ? P.A * xt * xt : 0.f);
             e_lj += ok ? u : 0.f;
             e_vir += ok ? rr * flj : 0.f;
           }

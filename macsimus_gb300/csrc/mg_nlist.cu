@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(NL_THREADS)
         float U;
         if (rr < P.C1q) {
           const float x = __fdividef(P.Sq, rr), y = x * x * x;
-          f = P.E24 * fmaf(2.f * y, y, -y) * x;
-          U = P.E4 * fmaf(y, y, -y);
+          f = P.E24 * (fmaf(2.f, y, -P.lam) * y) * x;
+          U = P.E4 * ((y - P.lam) * y);
         } else {
           const float x = rr - P.C2q;
           f = P.A4 * x;

@@ -245,7 +245,9 @@ int mg_forces(mg_ctx *ctx, const double *r, double *f, int measure, mg_energy *e
 int mg_forces_device(mg_ctx *ctx, const double *r_dev, double *f_dev, int measure,
                      mg_energy *en);
 /* Ewald(1,...)+Ewald(2,...): k-space forces only (added to f), returns the
-   k-space + self + dipole energy in *energy when energy != NULL */
+   k-space + self + dipole energy in *energy when energy != NULL.  Runs the
+   direct passes on the FP32 path; a context whose force evaluations run the
+   transforms (kspace_engine 0) allocates their buffers at its first call */
 int mg_ewald(mg_ctx *ctx, const double *r, double *f, double *energy);
 
 /* One SCF iteration of the Drude displacements, cook's

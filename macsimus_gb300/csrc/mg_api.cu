@@ -244,6 +244,7 @@ struct mg_ctx {
   cudaStream_t kstream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   double* d_fk = nullptr;
+  bool direct = false;   // direct_buffers
   // the tensor-core passes' arguments (TcBox) for the position and force
   // buffers of the context's own calls: slot 3 ri + fi for r = (d_r, d_rs)[ri],
   // f = (d_f, d_fs, d_fk)[fi]; slot 6 for a caller's buffers
@@ -1000,8 +1001,6 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
       return fail(ctx, MG_ERR_SIZE, "the k set is too large for the tensor-core tiles");
     ctx->kspace_tc = fits && ctx->nq > 0;
     if (ctx->kspace_tc) {
-      CK(dalloc(&ctx->d_za, kf_tc_za_floats(kd)));
-      CK(dalloc(&ctx->d_vb, kf_tc_vb_floats(kd, ctx->nkrows)));
       std::vector<TcRow> tr;
       std::vector<KRow> tck = krows;
       std::sort(tck.begin(), tck.end(), [](const KRow& x, const KRow& y) {
@@ -1013,12 +1012,7 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
       if (p->kspace_engine == 3 && !sk_tc_fits(kd))
         return fail(ctx, MG_ERR_SIZE, "the k set is too large for the tensor-core pass 1");
       ctx->sk_tc = p->kspace_engine == 3 || (p->kspace_engine == 0 && sk_tc_fits(kd));
-      if (ctx->sk_tc) {
-        const size_t nzb = sk_tc_zb_floats(kd);
-        CK(dalloc(&ctx->d_zb, nzb));
-        CK(cudaMemset(ctx->d_zb, 0, nzb * sizeof(float)));
-        sk_tc_split(kd, ctx->nkrows, &ctx->sk_nch, &ctx->sk_gpc);
-      }
+      if (ctx->sk_tc) sk_tc_split(kd, ctx->nkrows, &ctx->sk_nch, &ctx->sk_gpc);
     }
   }
   CK(upload(&ctx->d_tiles, tiles.data(), tiles.size()));
@@ -1041,16 +1035,6 @@ int setup(mg_ctx* ctx, const mg_topology* t, const mg_params* p) {
       cudaFree(t);
       CK(er);
     }
-    {
-      // phase rows zero-padded to whole groups of 32 charges (tensor-core pass 1)
-      const size_t ntab = (size_t)((ctx->nq + 31) / 32 * 32) * ctx->row;
-      CK(dalloc((float2**)&ctx->d_tab, ntab));
-      CK(cudaMemset(ctx->d_tab, 0, ntab * sizeof(float2)));
-    }
-    CK(dalloc(&ctx->d_qfix, std::max(1, ctx->nq)));
-    CK(dalloc(&ctx->d_fk, 3 * (size_t)ns * (ctx->polar ? 2 : 1)));
-    CK(dalloc((float2**)&ctx->d_part, (size_t)std::max(ctx->nchunk, ctx->sk_nch) * nk));
-    CK(dalloc(&ctx->d_Wf, nk));
     if (ctx->nf) {
       int rc = setup_nf(ctx, nfK, kvec, ekk, kind_q, kind_qp);
       if (rc) return rc;
@@ -1486,6 +1470,54 @@ int tc_upload_slots(mg_ctx* ctx) {
   CK(dalloc(&ctx->d_tcb, 7));
   CK(cudaMemcpy(ctx->d_tcb, ctx->h_tcb, 7 * sizeof(TcBox), cudaMemcpyHostToDevice));
   return MG_OK;
+}
+
+// the buffers of the direct FP32 passes (phase rows, operand planes, partial sums:
+// 200 MB on 98304 sites), for a context that runs them: with the transforms only
+// mg_ewald does, which calls this
+int direct_buffers(mg_ctx* ctx) {
+  if (ctx->precision != MG_MIXED || ctx->direct) return MG_OK;
+  KArgs kd;
+  kd.Kx = ctx->Kx;
+  kd.Ky = ctx->Ky;
+  kd.Kz = ctx->Kz;
+  kd.nq = ctx->nq;
+  kd.row = ctx->row;
+  // phase rows zero-padded to whole groups of 32 charges (tensor-core pass 1)
+  const size_t ntab = (size_t)((ctx->nq + 31) / 32 * 32) * ctx->row,
+               nzb = ctx->sk_tc ? sk_tc_zb_floats(kd) : 0;
+  struct {
+    void** p;
+    size_t bytes;
+    bool clear;
+  } want[] = {{&ctx->d_tab, ntab * sizeof(float2), true},
+              {(void**)&ctx->d_qfix, std::max(1, ctx->nq) * sizeof(uint4), false},
+              {(void**)&ctx->d_fk, 3 * (size_t)ctx->ns * (ctx->polar ? 2 : 1) * sizeof(double), false},
+              {&ctx->d_part, (size_t)std::max(ctx->nchunk, ctx->sk_nch) * ctx->nk * sizeof(float2), false},
+              {(void**)&ctx->d_Wf, ctx->nk * sizeof(float2), false},
+              {(void**)&ctx->d_za, ctx->kspace_tc ? kf_tc_za_floats(kd) * sizeof(float) : 0, false},
+              {(void**)&ctx->d_vb, ctx->kspace_tc ? kf_tc_vb_floats(kd, ctx->nkrows) * sizeof(float) : 0, false},
+              {(void**)&ctx->d_zb, nzb * sizeof(float), true}};
+  cudaError_t e = cudaSuccess;
+  for (auto& w : want) {
+    if (!w.bytes || *w.p) continue;
+    e = cudaMalloc(w.p, w.bytes);
+    if (e == cudaSuccess && w.clear) e = cudaMemsetAsync(*w.p, 0, w.bytes, ctx->stream);
+    if (e != cudaSuccess) break;
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) {
+    // nothing half-made stays behind: a later call may find room
+    for (auto& w : want) {
+      if (*w.p) cudaFree(*w.p);
+      *w.p = nullptr;
+    }
+    cudaGetLastError();
+    return fail(ctx, MG_ERR_CUDA, std::string("direct Ewald passes: ") + cudaGetErrorString(e));
+  }
+  const int rc = tc_upload_slots(ctx);
+  ctx->direct = rc == MG_OK;
+  return rc;
 }
 
 // forces false (FP64 path, for the adjoint): the cell list, the sorted sites and
@@ -2022,7 +2054,7 @@ extern "C" {
 mg_ctx* mg_create(const mg_topology* top, const mg_params* par, int* status) {
   mg_ctx* ctx = new mg_ctx();
   int rc = setup(ctx, top, par);
-  if (rc == MG_OK) rc = tc_upload_slots(ctx);
+  if (rc == MG_OK && !ctx->nf) rc = direct_buffers(ctx);
   if (rc != MG_OK) {
     fprintf(stderr, "mg_create: %s\n", ctx->err.c_str());
     mg_destroy(ctx);
@@ -2139,6 +2171,8 @@ int mg_ewald(mg_ctx* ctx, const double* r, double* f, double* energy) {
   // full forces minus the r-space part is not separable cheaply here: run
   // the k-space kernels alone on a zeroed force buffer
   ctx->launches = 0;
+  int rc = direct_buffers(ctx);
+  if (rc) return rc;
   const size_t nb = 3 * (size_t)ctx->ns * (ctx->polar ? 2 : 1) * sizeof(double);
   Launch L = launch(ctx);
   CK(cudaMemcpyAsync(ctx->d_rs, r, nb, cudaMemcpyHostToDevice, ctx->stream));
@@ -2186,7 +2220,7 @@ int mg_ewald(mg_ctx* ctx, const double* r, double* f, double* energy) {
   }
   std::vector<double> fk(nb / sizeof(double));
   CK(cudaMemcpyAsync(fk.data(), ctx->d_fs, nb, cudaMemcpyDeviceToHost, ctx->stream));
-  int rc = fetch_sums(ctx);
+  rc = fetch_sums(ctx);
   if (rc) return rc;
   rc = fetch_status(ctx);
   if (rc) return rc;

@@ -1115,10 +1115,10 @@ __global__ void __launch_bounds__(ALL_WARPS * 32, POLAR ? 1 : 2)
 // to compensated sums.
 //
 // Bound by issue (63 %) and the gathers of the erfc table through L1.  Measured:
-// 0.250 ms on 32768 waters (lane per home site 0.363, without the quads and
-// the side-by-side runs 0.267), 42 us on 12544 sites (61), 23 us on 864 waters
+// 0.255 ms on 32768 waters (lane per home site 0.363, without the quads and
+// the side-by-side runs 0.267), 45 us on 12544 sites (61), 25 us on 864 waters
 // (61; cell kernel 110), 0.59 ms with 32768 shells (lane per home site 0.67),
-// 0.61 ms on a batch of 256 ionic boxes (cell kernel 0.94).
+// 0.65 ms on a batch of 256 ionic boxes (cell kernel 0.94).
 
 // the z-ranges of half-shell span sp around cell (cx, cy, cz): column index
 // col; run [ra0, ra1] and, where the run wraps through the box, [rb0, rb1]
@@ -1833,7 +1833,8 @@ __device__ __forceinline__ double near_img(double d, double L, double iL) {
 
 // A warp per CTA (a molecule's pairs are one chain of loads and FP64 products,
 // so the molecules spread over the SMs); rigid three-site molecules keep their
-// sites in registers.  864 waters 9.0 -> 6.2 us, measured 15 -> 8.5 us.
+// sites in registers.  864 waters 9.0 -> 7.4 us, measured 15 -> 10.5 us (6.2 and 8.5
+// with the terms as FP32 differences, good to 3e-6 where the series are to 1e-7).
 template <bool MEASURE, bool POLAR>
 MG_BODY void excl_mixed_kernel_body(const ExclArgs& a,
     const int bx_,

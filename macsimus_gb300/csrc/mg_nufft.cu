@@ -11,9 +11,9 @@
 // (2019)), whose transform is divided out exactly at every k (host
 // quadrature).  The grid has at least 1.86 points per resolved mode.
 //
-// Measured on 32768 waters: 0.11 ms (spread 54 us, x 5, planes 13, x 5, interp
-// 35) against 0.52 ms for the direct tensor-core passes; the MD step
-// 0.87 -> 0.45 ms; 256 ionic boxes 3.3 -> 2.3 ms.  Error against 64 bits,
+// Measured on 32768 waters: 0.13 ms (spread 57 us, x 6, planes 16, x 6, interp
+// 45) against 0.52 ms for the direct tensor-core passes; the MD step
+// 0.87 -> 0.43 ms; 256 ionic boxes 3.3 -> 2.7 ms.  Error against 64 bits,
 // k-space force relative RMS, mean over 46 boxes of 650 to 98000 sites: 7.2e-7 (the
 // direct tensor-core passes 11.5e-7; 9.8e-7 with 1.75 points a mode, the weights
 // not cut off and the potential taken whole in the interpolation).
@@ -449,7 +449,8 @@ __global__ void __launch_bounds__(DF_THREADS) nf_dft_x_kernel(const NfBox* __res
 // CS CTAs of T threads a plane: four of 128 for one box, whose planes are too few
 // for the GPU; two of 256 for the plain steps of a batch that fills it, which
 // copy the tables half as often and sum more items each (256 ionic boxes 625 ->
-// 533 us; one of 512 535 us; tables through L1 instead 714).  Every sum of the
+// 533 us; one of 512 535 us; tables through L1 instead 714; 564 with 1.86 points a
+// mode).  Every sum of the
 // modes and of the grid is a thread's own, so the split does not change them; it
 // would change the order of the energy sums, and a measured step keeps four.
 template <int CS, int T>
@@ -698,7 +699,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(T)
 
 // A[kx][c] -> G[x][c]: the real part (the half kx >= 0 carries both signs)
 // (half the threads where a batch fills the GPU: 256 ionic boxes 225 -> 189 us,
-// 864 waters 3.2 -> 3.5)
+// 864 waters 3.2 -> 3.5, on grids of 1.75 points a mode; 223 and 4.5 at 1.86)
 __global__ void __launch_bounds__(DF_THREADS) nf_idft_x_kernel(const NfBox* __restrict__ boxes) {
   after_previous();
   const NfBox& b = boxes[blockIdx.z];
@@ -815,10 +816,11 @@ struct NfForce {
 // charges whose grid cell lies in the tile come from the cell list as in the
 // spreading, and every row of a window is a shared-memory load at a fixed
 // offset from the charge's first.  Bound by the shared-memory wavefronts (64
-// loads of four unaligned 32-byte rows each per four charges): 35 us on 32768
-// waters, 8.8 us on 864, where reading the rows from memory (below) takes 36
-// and 12 us.  Two CTAs an SM: left to itself the compiler takes 80 registers and
-// spills, 1 us more on 12544 sites.
+// loads of four unaligned 32-byte rows each per four charges): 45 us on 32768
+// waters, 10 us on 864, with the charge's own potential taken out; before that 35
+// and 8.8, where reading the rows from memory (below) took 36 and 12.  Two CTAs an
+// SM: left to itself the compiler takes 80 registers and spills, 1 us more on 12544
+// sites.
 constexpr int IT_LD = 2 * TILE, IT_PL = IT_LD * IT_LD;
 
 __global__ void __launch_bounds__(SP_WARPS * 32, 2)

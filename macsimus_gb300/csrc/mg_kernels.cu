@@ -2069,9 +2069,8 @@ cudaError_t k_phase_tables_fp64(const Launch& L, const KArgs& a, const double* r
 
 // S(k) = sum over chunks (FP64, fixed order); energy and virial per k
 // (sim/ewpass2m.c: E1 = |S|^2 ekk, ptf = 1/kk + (pi/alpha)^2) reduced per block
-template <typename T2>
 MG_BODY void sk_reduce_kernel_body(const KArgs& a,
-    const T2* __restrict__ part,
+    const float2* __restrict__ part,
     bool measure,
     double pi2_over_a2,
     const int bx_,
@@ -2082,7 +2081,7 @@ MG_BODY void sk_reduce_kernel_body(const KArgs& a,
   if (k < a.nk) {
     double sr = 0, si = 0;
     for (int c = 0; c < a.nchunk; c++) {
-      T2 v = part[(long)c * a.nk + k];
+      const float2 v = part[(long)c * a.nk + k];
       sr += v.x;
       si += v.y;
     }
@@ -2117,14 +2116,13 @@ MG_BODY void sk_reduce_kernel_body(const KArgs& a,
     for (int m = 0; m < 7; m++) a.ek_part[bx_ * 7 + m] = red[0][m];
 }
 
-template <typename T2>
-__global__ void sk_reduce_kernel(const __grid_constant__ KArgs a, const T2* __restrict__ part, bool measure, double pi2_over_a2) {
-  sk_reduce_kernel_body<T2>(a, part, measure, pi2_over_a2, blockIdx.x, 0);
+__global__ void sk_reduce_kernel(const __grid_constant__ KArgs a, const float2* __restrict__ part, bool measure, double pi2_over_a2) {
+  sk_reduce_kernel_body(a, part, measure, pi2_over_a2, blockIdx.x, 0);
 }
 
 cudaError_t k_sk_reduce_mixed(const Launch& L, const KArgs& a, const float2* part, bool measure) {
   const double pa = 9.869604401089358 / (a.alpha * a.alpha);
-  sk_reduce_kernel<float2><<<cdiv(a.nk, 256), 256, 0, L.s>>>(a, part, measure, pa);
+  sk_reduce_kernel<<<cdiv(a.nk, 256), 256, 0, L.s>>>(a, part, measure, pa);
   LAUNCHED(L);
   return cudaGetLastError();
 }
@@ -2795,7 +2793,7 @@ __global__ void batch_sk_reduce_kernel(const BoxStep* __restrict__ B, bool measu
   const BoxStep& e = B[blockIdx.y];
   if ((int)blockIdx.x >= e.g_skr) return;
   const double pa = 9.869604401089358 / (e.ka.alpha * e.ka.alpha);
-  sk_reduce_kernel_body<float2>(e.ka, e.part, measure, pa, blockIdx.x, 0);
+  sk_reduce_kernel_body(e.ka, e.part, measure, pa, blockIdx.x, 0);
 }
 
 template <bool MEAS>
